@@ -3,7 +3,7 @@
 // Layout in HBM (V = B*C views, T = tiles per view):
 //   ViewCam   cams[V]             camera set-up, one per view
 //   TriFrame  tri_frame[B*F]      per-frame triangle constants (scaled vertices, plane normal)
-//   TriView   tri_view[V*F]       per-view triangle constants (ray-plane numerator, pixel bbox)
+//   TriView   tri_view[V*F]       per-view triangle constants (footprint, ray-plane numerator, pixel bbox)
 //   int2      tile_state[V*T]     (binned count, spill slot + 1)
 //   int       bins[V*T*CAP]       triangle ids per tile
 //   int4      spill[S]            (view, tile, triangle) pairs beyond CAP
@@ -57,14 +57,13 @@ struct TriFrame {    // 48 bytes: s0.xyz n.x | s1.xyz n.y | s2.xyz n.z
     float4 a, b, c;
 };
 
-struct TriView {     // 64 bytes per (view, triangle), written by the binning pass
+struct __align__(16) TriView {  // 48 bytes per (view, triangle), written by the binning pass
+    float4 e01;      // 2-D footprint edges 0 and 1: (a0, b0, a1, b1)
+    float4 e2c;      // edge 2 and two offsets: (a2, b2, c0, c1)
+    float c2;        // the third offset
     float num;       // dot(s0, n) - dot(ro_s, n)
     int x01;         // bbox x0 | x1 << 16
     int y01;         // bbox y0 | y1 << 16
-    int dqmin;       // lower bound of the quantised depth; bit 31 set = back-facing
-    float4 e01;      // 2-D footprint edges 0 and 1: (a0, b0, a1, b1)
-    float4 e2c;      // edge 2 and two offsets: (a2, b2, c0, c1)
-    float4 e2o;      // (c2, 0, 0, 0)
 };
 
 struct TriS;
@@ -106,18 +105,46 @@ __device__ __forceinline__ TriS tri_from(const TriFrame& f) {
     return t;
 }
 
-// Conservative lower bound of int(t * 1e4) over the triangle.  For a unit
-// ray direction t is the distance from the camera centre to the hit point,
-// which is at least (a) the distance to the triangle's plane, |num| / |n|,
-// and (b) the distance to the nearest vertex minus the longest edge (every
-// point of a triangle lies within its longest edge of some vertex).  The
-// larger of the two is lowered by 1e-4 relative and 2 quanta so float
-// rounding of either side cannot break it.
-__device__ __forceinline__ int depth_lower_bound(float num, float3 n, const TriS& T, float3 o) {
-    const float pd = fabsf(num) / sqrtf(dot(n, n));
-    // the minimum / maximum taken on the squared lengths and rooted once: the
-    // correctly rounded square root is monotone, so the values are those of
-    // the per-vertex and per-edge lengths
+// The unnormalised camera rays of a tile's pixel centres: u(x, y) = c + x ux +
+// y uy for |x|, |y| <= h pixels from the tile's centre (pixel_ray's affine
+// form before its normalisation).  min_len bounds |u| from below; slack
+// bounds the float error of u . n over |n|.
+struct TileRays {
+    float3 c, ux, uy;  // ux, uy scaled by h
+    float min_len, slack;
+};
+
+__device__ __forceinline__ TileRays tile_rays(const ViewCam& cam, float x, float y, float h) {
+    const float* m = cam.invP;
+    TileRays r;
+    const float3 o = make_float3(cam.ro[0], cam.ro[1], cam.ro[2]);
+    r.c = make_float3(1000.f * (m[0] * x + m[1] * y + m[2]) + m[3] - o.x,
+                      1000.f * (m[4] * x + m[5] * y + m[6]) + m[7] - o.y,
+                      1000.f * (m[8] * x + m[9] * y + m[10]) + m[11] - o.z);
+    const float k = 1000.f * h;
+    r.ux = make_float3(k * m[0], k * m[4], k * m[8]);
+    r.uy = make_float3(k * m[1], k * m[5], k * m[9]);
+    const float len = sqrtf(dot(r.c, r.c)), far = fabsf(o.x) + fabsf(o.y) + fabsf(o.z);
+    r.slack = 2e-6f * (len + far);
+    r.min_len = fmaxf(len - sqrtf(dot(r.ux, r.ux)) - sqrtf(dot(r.uy, r.uy)) - r.slack, 0.f);
+    return r;
+}
+
+// Conservative lower bound of int(t * 1e4) of a triangle's hits in a tile.
+// For the unit ray direction u / |u|, t is the distance from the camera
+// centre to the hit point.  It is (a) on the triangle's plane, t = num |u| /
+// (u . n), so at least |num| min |u| / max |u . n|, the maximum of the affine
+// u . n over the tile being |c . n| + |ux . n| + |uy . n|; and (b) at least the
+// distance to the nearest vertex minus the longest edge (every point of a
+// triangle lies within its longest edge of some vertex).  The larger of the
+// two is lowered by 1e-4 relative and 2 quanta so float rounding of either
+// side cannot break it.  (a) is nearly the triangle's depth in the tile: the
+// bound of the whole triangle that it replaced left long thin triangles, whose
+// nearest point lies far outside the tile, at the head of many tiles.
+__device__ __forceinline__ int depth_lower_bound(float num, const TriS& T, float3 o, const TileRays& r) {
+    const float most = fabsf(dot(r.c, T.n)) + fabsf(dot(r.ux, T.n)) + fabsf(dot(r.uy, T.n)) +
+                       r.slack * (fabsf(T.n.x) + fabsf(T.n.y) + fabsf(T.n.z));
+    const float pd = most > 0.f ? fabsf(num) * r.min_len / most : 0.f;
     const float3 a0 = T.s0 - o, a1 = T.s1 - o, a2 = T.s2 - o;
     const float dmin = sqrtf(fminf(dot(a0, a0), fminf(dot(a1, a1), dot(a2, a2))));
     const float3 e0 = T.s1 - T.s0, e1 = T.s2 - T.s1, e2 = T.s0 - T.s2;

@@ -253,13 +253,11 @@ __global__ void __launch_bounds__(256, 6) k_bin(int V, int C, int F, int N, int 
         const int cx0 = min(x0, W), cy0 = min(y0, H);
         tv.x01 = (cx0 & 0xffff) | (cx1 << 16);
         tv.y01 = (cy0 & 0xffff) | (cy1 << 16);
-        // front-facing: the plane normal points towards the camera (num < 0)
-        tv.dqmin = depth_lower_bound(tv.num, T.n, T, ro_s) | (tv.num < 0.f ? 0 : (int)0x80000000);
         fp = footprint(p0, p1, p2);
-        // the tile resolve stages this record as it is (no vertex gathers there)
+        // the tile resolve copies this record as it is (no vertex gathers there)
         tv.e01 = make_float4(fp.a[0], fp.b[0], fp.a[1], fp.b[1]);
         tv.e2c = make_float4(fp.a[2], fp.b[2], fp.c[0], fp.c[1]);
-        tv.e2o = make_float4(fp.c[2], 0.f, 0.f, 0.f);
+        tv.c2 = fp.c[2];
         tri_view[i] = tv;
     }
     const bool nonempty = live && x1 >= x0 && y1 >= y0;
@@ -526,37 +524,33 @@ __device__ __forceinline__ float3 shade_pixel(const ShadeArgs& A, const ViewCam&
     return color;
 }
 
-struct TileTri {
-    int4 hdr;        // column mask, row mask (tile-relative bbox), depth lower bound, face id
-    float4 ea;       // footprint edges 0, 1: (a0, b0, a1, b1)
-    float4 nm;       // ray-plane numerator, footprint offsets c0, c1, c2
-    float4 eb;       // footprint edge 2: (a2, b2, -, -)
-    float4 a, b, c;  // TriFrame
-};
-
 // Hit test with an early depth rejection: the quantised depth int(t * 1e4) is
 // known as soon as t is, so a triangle that cannot reach the pixel's current
-// best depth skips the edge tests.  Accepted hits and their depth / barycentrics
-// are those of raster_hit.
+// best depth skips the edge tests; so does a pixel known to lie inside.
+// Accepted hits and their depth are those of raster_hit.  The barycentric
+// window (a, b <= 1.001 |N|^2 after the sign tests) is decided without the two
+// divisions unless a value is near its end or |N|^2 is near underflow.
 __device__ __forceinline__ bool raster_hit_below(float3 ro_s, float3 dir, const TriS& T, float num,
-                                                 unsigned best_d, int& depth_q, float& a, float& b) {
+                                                 unsigned best_d, bool inside, int& depth_q) {
     const float ndr = dot(dir, T.n);
     if (fabsf(ndr) < 0.0000001f) return false;
     const float t = num / ndr;
     if (t < 0.f) return false;
     depth_q = (int)(t * 10000.f);
     if ((unsigned)depth_q > best_d) return false;
+    if (inside) return true;
     const float3 P = ro_s + t * dir;
     float3 C = cross(T.s1 - T.s0, P - T.s0);
     if (dot(T.n, C) < 0.f) return false;
     C = cross(T.s2 - T.s1, P - T.s1);
-    if ((a = dot(T.n, C)) < 0.f) return false;
+    const float a = dot(T.n, C);
+    if (a < 0.f) return false;
     C = cross(T.s0 - T.s2, P - T.s2);
-    if ((b = dot(T.n, C)) < 0.f) return false;
+    const float b = dot(T.n, C);
+    if (b < 0.f) return false;
     const float denom = dot(T.n, T.n);
-    a /= denom;
-    b /= denom;
-    return (a >= -0.001f) && (b >= -0.001f) && (a <= 1.001f) && (b <= 1.001f);
+    if (denom > 1e-30f && fmaxf(a, b) <= 1.0005f * denom) return true;
+    return (a / denom >= -0.001f) && (b / denom >= -0.001f) && (a / denom <= 1.001f) && (b / denom <= 1.001f);
 }
 
 // bits lo..hi of a 32-bit mask (empty when hi < lo)
@@ -564,9 +558,91 @@ __device__ __forceinline__ unsigned bit_range(int lo, int hi) {
     return hi < lo ? 0u : ((2u << hi) - 1u) & ~((1u << lo) - 1u);
 }
 
+// Rows of a 32 x 32 bit matrix (one per lane) to columns: lane i ends with
+// bit j = lane j's bit i.  Five rounds of block swaps.
+__device__ __forceinline__ unsigned transpose_bits(unsigned x, int lane) {
+    unsigned m = 0x0000ffffu;
+#pragma unroll
+    for (int j = 16; j > 0; j >>= 1) {
+        const unsigned y = __shfl_xor_sync(0xffffffffu, x, j);
+        x = (lane & j) ? ((x & ~m) | ((y >> j) & m)) : ((x & m) | ((y << j) & ~m));
+        m ^= m << (j >> 1);
+    }
+    return x;
+}
+
+// The pixels of a warp (RW rows of TS pixels; the first pixel is (X0, Y0))
+// that a triangle can hit: its bounding box exactly, and its footprint from
+// the x interval that each edge leaves of a row, widened by kMaskSlack px in
+// the edge's value (the float error of that value is below 0.03 px in the
+// admitted coordinate range, and the reciprocal's far below that).
+// Bit r * TS + x is pixel (X0 + x, Y0 + r).
+constexpr float kMaskSlack = 0.0625f;
+
+template <int TS, int RW>
+__device__ __forceinline__ unsigned pixel_mask(const float4* rec, int X0, int Y0) {
+    const float4 e01 = rec[0], e2c = rec[1], q = rec[2];
+    const int x01 = __float_as_int(q.z), y01 = __float_as_int(q.w);
+    const int bx0 = max((x01 & 0xffff) - X0, 0), bx1 = min((x01 >> 16) - X0, TS - 1);
+    const int by0 = (y01 & 0xffff) - Y0, by1 = (y01 >> 16) - Y0;
+    if (bx1 < bx0 || by1 < 0 || by0 >= RW) return 0u;
+    const float fx = X0 + 0.5f, fy = Y0 + 0.5f;
+    const float ea[3] = {e01.x, e01.z, e2c.x}, eb[3] = {e01.y, e01.w, e2c.y}, ec[3] = {e2c.z, e2c.w, q.x};
+    float s[3], inv[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        s[k] = ea[k] * fx + eb[k] * fy + ec[k] + kMaskSlack;
+        inv[k] = fabsf(ea[k]) > 1e-6f ? __fdividef(-1.f, ea[k]) : 0.f;  // 0: the edge leaves every x
+    }
+    unsigned mask = 0u;
+#pragma unroll
+    for (int r = 0; r < RW; ++r) {
+        float lo = (float)bx0, hi = (float)bx1;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float x = (s[k] + eb[k] * r) * inv[k];  // where the edge's value is -kMaskSlack
+            lo = fmaxf(lo, inv[k] < 0.f ? x : lo);
+            hi = fminf(hi, inv[k] > 0.f ? x : hi);
+        }
+        const int xl = (int)ceilf(lo), xh = (int)floorf(hi);
+        if (r >= by0 && r <= by1) mask |= bit_range(xl, xh) << (r * TS);
+    }
+    return mask;
+}
+
 // TIES: the call asked for the per-pixel count of hits at the winning depth
 // (diagnostics); without it the count is compiled out, which frees a register
 // of the scan and shortens its updates
+//
+// Resident CTAs claim the tiles of the call (the frame's cameras
+// concatenated) from a counter, `claim_n` consecutive tiles per atomic: no
+// launch cost per tile, and tiles of very different cost still balance.
+//
+// A chunk of the tile's bin is copied to shared memory, six consecutive
+// threads per 96-byte record, so a warp's copy touches as few lines as the
+// records have and passes through no registers (a lane per record takes 32
+// lines for each 16-byte piece).  It is then ordered by (back-facing, lower
+// bound of the depth within the tile): 32-bit keys (facing | bound | slot) are
+// distinct; each warp sorts its 32 keys with a shuffle bitonic network, and a
+// key's rank in the chunk is its lane plus its lower bound in every other
+// warp's sorted keys (5-step binary searches).
+//
+// Each warp turns 32 ordered records at a time into per-pixel lists: a lane
+// forms the 32-bit mask of the warp's pixels that its triangle can hit
+// (pixel_mask), and a bit-matrix transpose hands every pixel the mask of the
+// records that can hit it.  A pixel visits only those, nearest bound first,
+// front faces before back faces, and leaves a run at the first triangle whose
+// bound exceeds its best depth: that one can neither win nor tie, nor can any
+// after it in the run.  (Walking all records in lockstep, a pixel visited 19
+// and tested 4, and the warp paid every test that one of its pixels needed.)
+// The result is the minimum (depth, id) over the triangles whose box holds the
+// pixel, as in one unordered pass.
+//
+// Bound by instruction issue (DRAM at 3-8 % of its rate).  Lists instead of
+// the lockstep walk, the bound within the tile instead of the triangle's, and
+// claims sized to the call: 16 x 8 views of 1024^2, 8-px tiles 7.50 -> 6.73 ms;
+// 2 x 4 mixed-size views of a mesh of long thin triangles 751 -> 496 us;
+// 4 x 2048^2 at 16 px 1265 -> 968 us; one 512^2 view 84 -> 20 us.
 template <int TS, bool TIES>
 __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_resolve(ShadeArgs A, FastDiv fd_frame,
                                                    const int* __restrict__ tile_cam, int cap,
@@ -576,29 +652,34 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
                                                    const int2* __restrict__ tile_state,
                                                    const int* __restrict__ bins,
                                                    const unsigned long long* __restrict__ spill_keys,
-                                                   int spill_tile_cap, long long n_tiles,
+                                                   int spill_tile_cap, long long n_tiles, int claim_n,
                                                    unsigned long long* __restrict__ claim) {
     constexpr int NT = TS * TS;
+    constexpr int RW = 32 / TS;                 // pixel rows of a warp
     constexpr int CHUNK = NT > 256 ? 256 : NT;  // triangles staged per round
     constexpr int SB = CHUNK == 64 ? 6 : 8;     // slot bits of a sort key
     constexpr unsigned kNoKey = 0xffffffffu;
-    __shared__ TileTri s_tri[CHUNK];             // staged triangles in key order
-    __shared__ unsigned s_key[CHUNK];            // per warp: its keys, sorted
-    __shared__ unsigned char s_rank[CHUNK];       // position of each slot in key order
-    // Resident CTAs claim the tiles of the call from a counter (the frame's
-    // cameras concatenated), kClaim consecutive tiles per atomic: no launch
-    // cost per tile, tiles of very different cost still balance, and the one
-    // counter sees a quarter of the atomics.  Thread 0 claims into the slot of
-    // this claim's parity; the slot is rewritten two claims later, after every
-    // thread has passed the next claim's barrier.
-    constexpr int kClaim = 4;
+    constexpr int kRec = (sizeof(TriView) + sizeof(TriFrame)) / 16;  // 16-byte pieces of a record
+    constexpr int kViewRec = sizeof(TriView) / 16;
+    __shared__ float4 s_rec[CHUNK * kRec];  // staged records (TriView, TriFrame), by slot
+    __shared__ unsigned s_key[CHUNK];       // per warp: its keys, sorted
+    __shared__ unsigned s_ord[CHUNK];       // the chunk's keys in order
+    __shared__ int s_face[CHUNK];           // triangle of each slot
+    // thread 0 claims into the slot of this claim's parity; the slot is
+    // rewritten two claims later, after every thread has passed the next
+    // claim's barrier
     __shared__ long long s_g[2];
-    for (int it = 0;; ++it) {
-    if (it % kClaim == 0) {
-        if (threadIdx.x == 0) s_g[(it / kClaim) & 1] = (long long)atomicAdd(claim, (unsigned long long)kClaim);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int left = 0, par = 1;  // tiles left of the current claim; its slot
+    long long g = 0;
+    for (;; --left, ++g) {
+    if (left == 0) {
+        par ^= 1;
+        if (threadIdx.x == 0) s_g[par] = (long long)atomicAdd(claim, (unsigned long long)claim_n);
         __syncthreads();
+        g = s_g[par];
+        left = claim_n;
     }
-    const long long g = s_g[(it / kClaim) & 1] + it % kClaim;
     if (g >= n_tiles) break;
     // tile -> (frame, camera, tile of the camera): the call has < 2^31 tiles
     const int b = (int)fd_frame.div((unsigned)g);
@@ -607,9 +688,7 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
     const int tile = (int)(g - cam.tile_base);
     const int W = cam.W, H = cam.H;
     const int ty = (int)cam.fd_tiles_x.div((unsigned)tile), tx = (int)cam.fd_tiles_x.mod((unsigned)tile, ty);
-    const int lx = threadIdx.x % TS, ly = threadIdx.x / TS;
-    const int px = tx * TS + lx, py = ty * TS + ly;
-    const unsigned col_bit = 1u << lx, row_bit = 1u << ly;
+    const int px = tx * TS + threadIdx.x % TS, py = ty * TS + threadIdx.x / TS;
     const float cx = px + 0.5f, cy = py + 0.5f;
     const bool valid = px < W && py < H;
     const float3 ro_s = make_float3(cam.ro_s[0], cam.ro_s[1], cam.ro_s[2]);
@@ -621,126 +700,111 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
     int best_f = 0x7fffffff;
     int ties = 0;
     int best_e = -1;  // bin entry (base + slot) of the winner, -1 when it came from the spill
-    // Each staged chunk is sorted by (back-facing, depth lower bound) and
-    // staged once: its front faces are tested first, nearest bound first, then
-    // its back faces.  A triangle whose bound exceeds the pixel's current best
-    // depth can neither win nor tie, and
-    // neither can any triangle after it in the same run (their bounds are at
-    // least as large), so a pixel stops scanning a run there.  The result is
-    // the same minimum (depth, id) as one unordered pass.  Per pixel a
-    // triangle is only tested when the pixel lies in its bounding box (a
-    // column and a row bit mask relative to the tile) and in its conservative
-    // footprint.
-    //
-    // Sort: 32-bit keys (facing | bound | slot) are distinct; each
-    // warp sorts its 32 keys with a shuffle bitonic network, and a key's rank
-    // in the chunk is its lane plus its lower bound in every other warp's
-    // sorted keys (5-step binary searches).
-    int n_front = 0;
-    const int lane = threadIdx.x & 31;
     for (int base = 0; base < n; base += CHUNK) {
-        for (int pass = 0; pass < 2; ++pass) {
-            const int m = min(CHUNK, n - base);
-            if (pass == 0) {
-                __syncthreads();  // the previous chunk's readers are done
-                bool front = false;
-                unsigned key = kNoKey;
-                TileTri t;
-                if ((int)threadIdx.x < m) {
-                    const int f = tb[base + threadIdx.x];
-                    const TriView tv = tri_view[(long long)view * A.F + f];
-                    front = tv.dqmin >= 0;
-                    const TriFrame tf = tri_frame[(long long)b * A.F + f];
-                    const int x0 = tv.x01 & 0xffff, x1 = tv.x01 >> 16;
-                    const int y0 = tv.y01 & 0xffff, y1 = tv.y01 >> 16;
-                    // the bound, clamped to the key's 31 - SB bits (exact below ~2^25 quanta, a
-                    // lower bound above) and kept below the all-ones key of an empty slot
-                    const unsigned coarse = min((unsigned)(tv.dqmin & 0x7fffffff), (1u << (31 - SB)) - 2u);
-                    t.hdr = make_int4((int)bit_range(max(x0 - tx * TS, 0), min(x1 - tx * TS, TS - 1)),
-                                      (int)bit_range(max(y0 - ty * TS, 0), min(y1 - ty * TS, TS - 1)),
-                                      (int)coarse, f);
-                    t.ea = tv.e01;
-                    t.nm = make_float4(tv.num, tv.e2c.z, tv.e2c.w, tv.e2o.x);
-                    t.eb = make_float4(tv.e2c.x, tv.e2c.y, 0.f, 0.f);
-                    t.a = tf.a;
-                    t.b = tf.b;
-                    t.c = tf.c;
-                    key = (front ? 0u : 0x80000000u) | (coarse << SB) | threadIdx.x;
-                }
-                if (threadIdx.x < CHUNK && (int)(threadIdx.x & ~31u) < m) {  // whole warps that hold keys
+        const int m = min(CHUNK, n - base);
+        __syncthreads();  // the previous chunk's readers are done
+        for (int i = threadIdx.x; i < m * kRec; i += NT) {
+            const int r = i / kRec, c = i - r * kRec;
+            const int f = tb[base + r];
+            if (c == 0) s_face[r] = f;
+            const float4* src = c < kViewRec
+                                    ? reinterpret_cast<const float4*>(tri_view + (long long)view * A.F + f) + c
+                                    : reinterpret_cast<const float4*>(tri_frame + (long long)b * A.F + f) + (c - kViewRec);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(
+                             (unsigned)__cvta_generic_to_shared(&s_rec[i])),
+                         "l"(src));
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncthreads();
+        bool front = false;
+        unsigned key = kNoKey;
+        if ((int)threadIdx.x < m) {
+            const float4* rec = s_rec + threadIdx.x * kRec;
+            TriFrame tf;
+            tf.a = rec[kViewRec];
+            tf.b = rec[kViewRec + 1];
+            tf.c = rec[kViewRec + 2];
+            const float num = rec[2].y;
+            const TileRays rays = tile_rays(cam, tx * TS + 0.5f * TS, ty * TS + 0.5f * TS, 0.5f * (TS - 1));
+            front = num < 0.f;  // the plane normal points towards the camera
+            // the bound, clamped to the key's 31 - SB bits (exact below ~2^25 quanta, a
+            // lower bound above) and kept below the all-ones key of an empty slot
+            const unsigned coarse = min((unsigned)depth_lower_bound(num, tri_from(tf), ro_s, rays),
+                                        (1u << (31 - SB)) - 2u);
+            key = (front ? 0u : 0x80000000u) | (coarse << SB) | threadIdx.x;
+        }
+        if (threadIdx.x < CHUNK && (int)(threadIdx.x & ~31u) < m) {  // whole warps that hold keys
 #pragma unroll
-                    for (int size = 2; size <= 32; size <<= 1) {
+            for (int size = 2; size <= 32; size <<= 1) {
 #pragma unroll
-                        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                            const unsigned o = __shfl_xor_sync(0xffffffffu, key, stride);
-                            const bool keep_min = ((lane & stride) == 0) == ((lane & size) == 0);
-                            key = keep_min ? min(key, o) : max(key, o);
-                        }
-                    }
-                    s_key[threadIdx.x] = key;
+                for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                    const unsigned o = __shfl_xor_sync(0xffffffffu, key, stride);
+                    const bool keep_min = ((lane & stride) == 0) == ((lane & size) == 0);
+                    key = keep_min ? min(key, o) : max(key, o);
                 }
-                n_front = __syncthreads_count(front);
-                if (threadIdx.x < CHUNK && key != kNoKey) {
-                    int r = lane;
-                    const int me = threadIdx.x >> 5, nw = (m + 31) >> 5;
-                    for (int w = 0; w < nw; ++w) {
-                        if (w == me) continue;
-                        const unsigned* L = s_key + 32 * w;
-                        int lo = 0;
-#pragma unroll
-                        for (int step = 16; step > 0; step >>= 1) lo += L[lo + step] < key ? step : 0;
-                        r += lo + (L[lo] < key ? 1 : 0);
-                    }
-                    s_rank[key & (CHUNK - 1)] = (unsigned char)r;
-                }
-                __syncthreads();
-                if ((int)threadIdx.x < m) s_tri[s_rank[threadIdx.x]] = t;
-                __syncthreads();
             }
-            const int j0 = pass == 0 ? 0 : n_front;
-            const int j1 = pass == 0 ? n_front : m;
-            if (valid) {
-                for (int slot = j0; slot < j1; ++slot) {
-                    // one 16-byte header load decides whether the ray test runs
-                    const int4 h = s_tri[slot].hdr;
-                    if ((unsigned)h.z > best_d) break;  // neither this nor a later one can reach the best depth
-                    if (!((unsigned)h.x & col_bit) || !((unsigned)h.y & row_bit)) continue;
-                    const float4 ea = s_tri[slot].ea, nm = s_tri[slot].nm, eb = s_tri[slot].eb;
-                    const float e0 = ea.x * cx + ea.y * cy + nm.y, e1 = ea.z * cx + ea.w * cy + nm.z,
-                                e2 = eb.x * cx + eb.y * cy + nm.w;
-                    if (e0 < 0.f || e1 < 0.f || e2 < 0.f) continue;  // clearly outside the projected triangle
-                    int dq;
-                    if (e0 >= kEdgeInterior && e1 >= kEdgeInterior && e2 >= kEdgeInterior) {
-                        // clearly inside: the edge tests would pass, only the depth is needed
-                        // (the same operations as ray_tri up to t)
-                        const float3 n = make_float3(s_tri[slot].a.w, s_tri[slot].b.w, s_tri[slot].c.w);
-                        const float ndr = dot(dir, n);
-                        if (fabsf(ndr) < 0.0000001f) continue;
-                        const float t = nm.x / ndr;
-                        if (t < 0.f) continue;
-                        dq = (int)(t * 10000.f);
-                        if ((unsigned)dq > best_d) continue;
-                    } else {
-                        TriFrame tf;
-                        tf.a = s_tri[slot].a;
-                        tf.b = s_tri[slot].b;
-                        tf.c = s_tri[slot].c;
-                        float a, bb;
-                        if (!raster_hit_below(ro_s, dir, tri_from(tf), nm.x, best_d, dq, a, bb)) continue;
-                    }
-                    const int f = h.w;
-                    if ((unsigned)dq < best_d) {
-                        best_d = (unsigned)dq;
+            s_key[threadIdx.x] = key;
+        }
+        const int n_front = __syncthreads_count(front);
+        if (threadIdx.x < CHUNK && key != kNoKey) {
+            int r = lane;
+            const int nw = (m + 31) >> 5;
+            for (int w = 0; w < nw; ++w) {
+                if (w == warp) continue;
+                const unsigned* L = s_key + 32 * w;
+                int lo = 0;
+#pragma unroll
+                for (int step = 16; step > 0; step >>= 1) lo += L[lo + step] < key ? step : 0;
+                r += lo + (L[lo] < key ? 1 : 0);
+            }
+            s_ord[r] = key;
+        }
+        __syncthreads();
+        for (int s0 = 0; s0 < m; s0 += 32) {  // warp-uniform
+            const int cnt = min(32, m - s0), nf = min(max(n_front - s0, 0), cnt);  // records, front faces of the group
+            // no pixel of the warp can be reached by the group's nearest front or back face
+            const unsigned bf = nf > 0 ? s_ord[s0] >> SB : kNoKey;
+            const unsigned bb = nf < cnt ? (s_ord[s0 + nf] & 0x7fffffffu) >> SB : kNoKey;
+            if (!__any_sync(0xffffffffu, valid && min(bf, bb) <= best_d)) continue;
+            unsigned w = 0u;
+            if (lane < cnt) w = pixel_mask<TS, RW>(s_rec + (s_ord[s0 + lane] & (CHUNK - 1)) * kRec, tx * TS,
+                                                     ty * TS + warp * RW);
+            w = transpose_bits(w, lane);
+            if (!valid) w = 0u;
+            const unsigned fm = nf == 32 ? 0xffffffffu : (1u << nf) - 1u;  // the front faces' bits
+            while (w) {
+                const unsigned k = s_ord[s0 + __ffs(w) - 1];
+                w &= w - 1u;
+                if ((k & 0x7fffffffu) >> SB > best_d) {  // neither this nor a later one of its run can reach the best depth
+                    w &= (k >> 31) ? 0u : ~fm;
+                    continue;
+                }
+                const int slot = (int)(k & (CHUNK - 1));
+                const float4* rec = s_rec + slot * kRec;
+                const float4 ea = rec[0], eb = rec[1], q = rec[2];
+                const float e0 = ea.x * cx + ea.y * cy + eb.z, e1 = ea.z * cx + ea.w * cy + eb.w,
+                            e2 = eb.x * cx + eb.y * cy + q.x;
+                if (e0 < 0.f || e1 < 0.f || e2 < 0.f) continue;  // clearly outside the projected triangle
+                TriFrame tf;
+                tf.a = rec[kViewRec];
+                tf.b = rec[kViewRec + 1];
+                tf.c = rec[kViewRec + 2];
+                // clearly inside: the edge tests would pass, only the depth is needed
+                const bool inside = e0 >= kEdgeInterior && e1 >= kEdgeInterior && e2 >= kEdgeInterior;
+                int dq;
+                if (!raster_hit_below(ro_s, dir, tri_from(tf), q.y, best_d, inside, dq)) continue;
+                const int f = s_face[slot];
+                if ((unsigned)dq < best_d) {
+                    best_d = (unsigned)dq;
+                    best_f = f;
+                    best_e = base + slot;
+                    ties = 1;
+                } else {  // equal depth (deeper hits were rejected)
+                    if (f < best_f) {
                         best_f = f;
                         best_e = base + slot;
-                        ties = 1;
-                    } else {  // equal depth (deeper hits were rejected)
-                        if (f < best_f) {
-                            best_f = f;
-                            best_e = base + slot;
-                        }
-                        ++ties;
                     }
+                    ++ties;
                 }
             }
         }
@@ -781,19 +845,19 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
             const float3 tg = l1m ? ld3(A.l1_target + 3 * pix) : make_float3(0.f, 0.f, 0.f);
             // recompute the winner's barycentrics (same arithmetic as the hit test)
             // the winner's triangle and plane offset: from the staged chunk when
-            // the winner is in the last one staged (s_tri is rewritten only
+            // the winner is in the last one staged (s_rec is rewritten only
             // after the next tile's first barrier), else from global memory
             const int last_base = n > 0 ? ((n - 1) / CHUNK) * CHUNK : 0;
             TriS Tw;
             float wnum;
             if (best_e >= last_base) {
-                const TileTri& w = s_tri[best_e - last_base];
+                const float4* rec = s_rec + (best_e - last_base) * kRec;
                 TriFrame tf;
-                tf.a = w.a;
-                tf.b = w.b;
-                tf.c = w.c;
+                tf.a = rec[kViewRec];
+                tf.b = rec[kViewRec + 1];
+                tf.c = rec[kViewRec + 2];
                 Tw = tri_from(tf);
-                wnum = w.nm.x;
+                wnum = rec[2].y;
             } else {
                 Tw = tri_from(tri_frame[(long long)b * A.F + best_f]);
                 wnum = tri_view[(long long)view * A.F + best_f].num;
@@ -824,8 +888,8 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
             l1c += __shfl_xor_sync(0xffffffffu, l1c, o);
         }
         if (lane == 0) {
-            A.l1_sum[g * (NT / 32) + (threadIdx.x >> 5)] = l1s;
-            A.l1_cnt[g * (NT / 32) + (threadIdx.x >> 5)] = l1c;
+            A.l1_sum[g * (NT / 32) + warp] = l1s;
+            A.l1_cnt[g * (NT / 32) + warp] = l1c;
         }
     }
     }
@@ -870,6 +934,14 @@ static unsigned resident_grid(K kernel, int threads, long long items) {
         per_sm = 1;
     return (unsigned)std::max<long long>(1, std::min((long long)sms * per_sm, items));
 }
+// Tiles a CTA of the tile resolve claims per atomic: four, so that the one
+// counter sees a quarter of the atomics, but no more than leave every CTA at
+// least four claims (a 512 x 512 view has 1024 tiles of 16 px for 740 CTAs:
+// claims of four would leave two thirds of them idle)
+static int claim_size(long long tiles, unsigned grid) {
+    return (int)std::max<long long>(1, std::min<long long>(4, tiles / (4ll * grid)));
+}
+
 // Per-camera layout of a frame for the current tile size: each camera's
 // resolution, tile grids and offsets, and the camera of every tile (the tile
 // resolve and the adjoint launch one CTA per tile of the whole call).
@@ -1031,16 +1103,14 @@ hc_status raster_forward(const Topology& topo, RasterWorkspace& ws, cudaStream_t
     const unsigned long long* kspill = ws.spill_keys.as<unsigned long long>();
     ws.clock.begin(kKResolve, s);
 #define HC_RESOLVE_CASE(TSV)                                                                                   \
-    case TSV:                                                                                                  \
-        if (A.tie_count)                                                                                       \
-            k_resolve<TSV, true><<<resident_grid(k_resolve<TSV, true>, TSV * TSV, tiles), TSV * TSV, 0, s>>>(  \
-                A, FastDiv((unsigned)ws.T_frame), tcam, ws.bin_cap, cams, tf, tv, tstate, kbins, kspill,       \
-                ws.spill_tile_cap, tiles, claim);                                                              \
-        else                                                                                                   \
-            k_resolve<TSV, false><<<resident_grid(k_resolve<TSV, false>, TSV * TSV, tiles), TSV * TSV, 0, s>>>( \
-                A, FastDiv((unsigned)ws.T_frame), tcam, ws.bin_cap, cams, tf, tv, tstate, kbins, kspill,       \
-                ws.spill_tile_cap, tiles, claim);                                                              \
-        break;
+    case TSV: {                                                                                                \
+        auto kernel = A.tie_count ? k_resolve<TSV, true> : k_resolve<TSV, false>;                              \
+        const unsigned grid = resident_grid(kernel, TSV * TSV, tiles);                                         \
+        kernel<<<grid, TSV * TSV, 0, s>>>(A, FastDiv((unsigned)ws.T_frame), tcam, ws.bin_cap, cams, tf, tv, tstate, \
+                                          kbins, kspill, ws.spill_tile_cap, tiles,                             \
+                                          claim_size(tiles, grid), claim);                                     \
+        break;                                                                                                 \
+    }
     switch (TS) {
         HC_RESOLVE_CASE(8)
         HC_RESOLVE_CASE(16)
