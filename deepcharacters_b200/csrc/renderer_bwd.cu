@@ -11,7 +11,7 @@
 //    reference's 3x9 product (which is kept as the parity mode);
 //  * per-vertex contributions (position, colour, pixel-normal gradients) are
 //    merged inside each warp (lanes matched by face id, a leader sums up to
-//    8 members) before one global reduction per vertex and leader;
+//    8 members) before 16-byte global reductions per vertex and leader;
 //  * SH gradients are reduced over the CTA (warp shuffles) before one atomic
 //    per coefficient;
 //  * the shaded-mode normal chain is split in two: pixels accumulate the
@@ -56,11 +56,9 @@ struct BwdArgs {
     const float* vnormal;   // [V,N,3]
     const float* bary;      // [V,H,W,2]
     const int* face;        // [V,H,W]
-    float* vpos_grad;       // [B,N,3]
-    float* vcol_grad;       // [B,N,3]
+    float* vacc;            // [B,N,VertexSums::kStride] per-vertex sums (cleared before the launch)
     float* tex_grad;        // [B,TH,TW,3]
     float* sh_grad;         // [V,27]
-    float* nrm_grad;        // [B,N,3] workspace: d loss / d (unnormalised vertex normal)
     // fused image L1: the image gradient is formed from the render and the
     // target instead of read from grad (NULL state: not fused)
     const L1State* l1_state;
@@ -233,12 +231,38 @@ __device__ __forceinline__ void taps_fs(const float4* s_tgt, int s0, float3 G, f
 // whose albedo has no parameters (normal, lighting, mask, position, depth, uv).
 enum { kAlbVcol = 0, kAlbTex = 1, kAlbNone = 2, kAlbTexBilinear = 3 };
 
+// The values the adjoint sums per (frame, vertex): position, colour (vertex
+// colours only) and unnormalised-normal gradient (shaded only), in that order.
+// They are summed in a workspace of kStride floats per vertex, a multiple of
+// 16 bytes, so that a leader issues one 16-byte reduction per four values
+// instead of one per float (6 instead of 18 reductions per leader with vertex
+// colours); k_vertex_grad writes the op's outputs from it.
+template <bool SHADED, int ALB>
+struct VertexSums {
+    static constexpr int kVals = 3 + (ALB == kAlbVcol ? 3 : 0) + (SHADED ? 3 : 0);
+    static constexpr int kStride = (kVals + 3) / 4 * 4;
+    static constexpr int kNormal = ALB == kAlbVcol ? 6 : 3;  // first normal value
+};
+
+// sum kVals values into a vertex's slot (16-byte aligned)
+template <int VALS>
+__device__ __forceinline__ void add_vertex(float* slot, const float* a) {
+#pragma unroll
+    for (int k = 0; k + 4 <= VALS; k += 4)
+        atomicAdd(reinterpret_cast<float4*>(slot + k), make_float4(a[k], a[k + 1], a[k + 2], a[k + 3]));
+    constexpr int rest = VALS % 4, at = VALS - rest;
+    if constexpr (rest == 3) atomicAdd(reinterpret_cast<float4*>(slot + at), make_float4(a[at], a[at + 1], a[at + 2], 0.f));
+    if constexpr (rest == 2) atomicAdd(reinterpret_cast<float2*>(slot + at), make_float2(a[at], a[at + 1]));
+    if constexpr (rest == 1) atomicAdd(slot + at, a[at]);
+}
+
 template <bool SHADED, int ALB, bool PARITY, bool DYN>
 __global__ void __launch_bounds__(BNT, SHADED ? 2 : 4) k_render_grad(BwdArgs A, const ViewCam* __restrict__ cams, long long n_tiles,
                                                                      const __grid_constant__ CUtensorMap tmap,
                                                                      int use_tma) {
-    constexpr int NVV = SHADED ? 9 : 6;               // values per vertex
-    constexpr int NROW = (3 * NVV + 3) / 4 * 4;       // per-lane row, padded for float4 loads
+    using Sums = VertexSums<SHADED, ALB>;
+    constexpr int NVV = Sums::kVals;                  // values per vertex
+    constexpr int NROW = (3 * NVV + 3) / 4 * 4;       // per-lane row, a multiple of 16 bytes
     __shared__ __align__(16) float s_red[BNT / 32][32][NROW];
     __shared__ float s_sh[SHADED ? BNT / 32 : 1][27];
     __shared__ __align__(128) float4 s_tgt2[2][TILE_S * TILE_S];  // target tile + halo, double-buffered
@@ -400,8 +424,10 @@ __global__ void __launch_bounds__(BNT, SHADED ? 2 : 4) k_render_grad(BwdArgs A, 
     const int W = cam.W, H = cam.H;
     const int tyi = (int)cam.fd_tiles_x_b.div((unsigned)tile);
     const int tx0 = (int)cam.fd_tiles_x_b.mod((unsigned)tile, tyi) * BT, ty0 = tyi * BT;
-    const int px = tx0 + threadIdx.x % BT;
-    const int py = ty0 + threadIdx.x / BT;
+    // a warp takes 8 x 4 pixels: fewer faces meet in it than in 16 x 2, so
+    // fewer leaders reduce below
+    const int px = tx0 + (warp & 1) * 8 + (lane & 7);
+    const int py = ty0 + (warp >> 1) * 4 + (lane >> 3);
     const float* tgt = A.target + cam.pix_base * 3;
     float shg[SHADED ? 27 : 1];
 #pragma unroll
@@ -647,22 +673,29 @@ __global__ void __launch_bounds__(BNT, SHADED ? 2 : 4) k_render_grad(BwdArgs A, 
     // shared memory and issues one reduction per value and vertex.  The cap
     // bounds the loop (unrolled, its loads issue together) at the cost of a
     // second set of reductions for the rare group of more than 8 lanes.
-    {
-        float* row = s_red[warp][lane];
+    if (__any_sync(0xffffffffu, f >= 0)) {
+        float val[NROW];
+#pragma unroll
+        for (int k = 3 * NVV; k < NROW; ++k) val[k] = 0.f;
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            row[NVV * i + 0] = gp[3 * i];
-            row[NVV * i + 1] = gp[3 * i + 1];
-            row[NVV * i + 2] = gp[3 * i + 2];
-            row[NVV * i + 3] = gA.x * bw[i];
-            row[NVV * i + 4] = gA.y * bw[i];
-            row[NVV * i + 5] = gA.z * bw[i];
+            val[NVV * i + 0] = gp[3 * i];
+            val[NVV * i + 1] = gp[3 * i + 1];
+            val[NVV * i + 2] = gp[3 * i + 2];
+            if constexpr (vcol) {
+                val[NVV * i + 3] = gA.x * bw[i];
+                val[NVV * i + 4] = gA.y * bw[i];
+                val[NVV * i + 5] = gA.z * bw[i];
+            }
             if constexpr (SHADED) {
-                row[NVV * i + 6] = gnu.x * bw[i];
-                row[NVV * i + 7] = gnu.y * bw[i];
-                row[NVV * i + 8] = gnu.z * bw[i];
+                val[NVV * i + Sums::kNormal + 0] = gnu.x * bw[i];
+                val[NVV * i + Sums::kNormal + 1] = gnu.y * bw[i];
+                val[NVV * i + Sums::kNormal + 2] = gnu.z * bw[i];
             }
         }
+        float4* row = reinterpret_cast<float4*>(s_red[warp][lane]);  // rows of 12, 20 or 28 words: no bank conflicts
+#pragma unroll
+        for (int k = 0; k < NROW / 4; ++k) row[k] = make_float4(val[4 * k], val[4 * k + 1], val[4 * k + 2], val[4 * k + 3]);
         __syncwarp();
         const unsigned grp = __match_any_sync(0xffffffffu, f);
         const int rank = __popc(grp & ((1u << lane) - 1u));
@@ -684,22 +717,8 @@ __global__ void __launch_bounds__(BNT, SHADED ? 2 : 4) k_render_grad(BwdArgs A, 
             }
             const float* a = reinterpret_cast<const float*>(acc);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                const long long o3 = ((long long)b * A.N + vid[i]) * 3;
-                atomicAdd(A.vpos_grad + o3 + 0, a[NVV * i + 0]);
-                atomicAdd(A.vpos_grad + o3 + 1, a[NVV * i + 1]);
-                atomicAdd(A.vpos_grad + o3 + 2, a[NVV * i + 2]);
-                if constexpr (vcol) {
-                    atomicAdd(A.vcol_grad + o3 + 0, a[NVV * i + 3]);
-                    atomicAdd(A.vcol_grad + o3 + 1, a[NVV * i + 4]);
-                    atomicAdd(A.vcol_grad + o3 + 2, a[NVV * i + 5]);
-                }
-                if constexpr (SHADED) {
-                    atomicAdd(A.nrm_grad + o3 + 0, a[NVV * i + 6]);
-                    atomicAdd(A.nrm_grad + o3 + 1, a[NVV * i + 7]);
-                    atomicAdd(A.nrm_grad + o3 + 2, a[NVV * i + 8]);
-                }
-            }
+            for (int i = 0; i < 3; ++i)
+                add_vertex<NVV>(A.vacc + ((long long)b * A.N + vid[i]) * Sums::kStride, a + NVV * i);
         }
     }
     // SH: reduce over the CTA, one atomic per coefficient
@@ -725,32 +744,46 @@ __global__ void __launch_bounds__(BNT, SHADED ? 2 : 4) k_render_grad(BwdArgs A, 
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
-// Normal chain, per (frame, vertex): for every incident face g = (x, y, z)
-// with unnormalised normal N_g = (y - x) x (z - x), the gradient reaching N_g
-// is the sum of the three vertex-normal gradients; d N_g / d vertex gives
+// The op's per-vertex outputs from the adjoint's sums, a thread per (frame,
+// vertex): the colour gradient (zeros where the albedo has none) and the
+// position gradient, to which shading adds the normal chain: for every
+// incident face g = (x, y, z) with unnormalised normal N_g = (y - x) x (z - x),
+// the gradient reaching N_g is the sum of the three vertex-normal gradients;
+// d N_g / d vertex gives
 //   x: g x (z - y),  y: (z - x) x g,  z: g x (y - x).
-__global__ void k_normal_chain(int B, int N, const int3* __restrict__ faces, const int* __restrict__ vf,
-                               const int2* __restrict__ vf_id, const float* __restrict__ verts,
-                               const float* __restrict__ nrm_grad, float* __restrict__ vpos_grad) {
+// Bound by its gathers; the sums are at most 48 bytes per vertex.
+template <bool SHADED, int ALB>
+__global__ void k_vertex_grad(int B, int N, const int3* __restrict__ faces, const int* __restrict__ vf,
+                              const int2* __restrict__ vf_id, const float* __restrict__ verts,
+                              const float* __restrict__ vacc, float* __restrict__ vpos_grad,
+                              float* __restrict__ vcol_grad) {
+    using Sums = VertexSums<SHADED, ALB>;
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= (long long)B * N) return;
-    const int b = (int)(i / N), v = (int)(i % N);
-    const float* P = verts + (long long)b * N * 3;
-    const float* Gn = nrm_grad + (long long)b * N * 3;
-    const int2 r = vf_id[v];
-    float3 acc = make_float3(0.f, 0.f, 0.f);
-    for (int k = r.x; k < r.x + r.y; ++k) {
-        const int3 f = faces[vf[k]];
-        const float3 g = ld3(Gn + 3 * f.x) + ld3(Gn + 3 * f.y) + ld3(Gn + 3 * f.z);
-        const float3 x = ld3(P + 3 * f.x), y = ld3(P + 3 * f.y), z = ld3(P + 3 * f.z);
-        if (v == f.x) acc += cross(g, z - y);
-        else if (v == f.y) acc += cross(z - x, g);
-        else acc += cross(g, y - x);
+    const float* S = vacc + i * Sums::kStride;
+    if (vcol_grad) st3(vcol_grad + 3 * i, ALB == kAlbVcol ? ld3(S + 3) : make_float3(0.f, 0.f, 0.f));
+    if (!vpos_grad) return;
+    float3 g0 = ld3(S);
+    if constexpr (SHADED) {
+        const int b = (int)(i / N), v = (int)(i % N);
+        const float* P = verts + (long long)b * N * 3;
+        const float* Gn = vacc + (long long)b * N * Sums::kStride + Sums::kNormal;
+        const int2 r = vf_id[v];
+        float3 acc = make_float3(0.f, 0.f, 0.f);
+        for (int k = r.x; k < r.x + r.y; ++k) {
+            const int3 f = faces[vf[k]];
+            const float3 g = ld3(Gn + (long long)Sums::kStride * f.x) + ld3(Gn + (long long)Sums::kStride * f.y) +
+                             ld3(Gn + (long long)Sums::kStride * f.z);
+            const float3 x = ld3(P + 3 * f.x), y = ld3(P + 3 * f.y), z = ld3(P + 3 * f.z);
+            if (v == f.x) acc += cross(g, z - y);
+            else if (v == f.y) acc += cross(z - x, g);
+            else acc += cross(g, y - x);
+        }
+        g0.x += acc.x;
+        g0.y += acc.y;
+        g0.z += acc.z;
     }
-    float* o = vpos_grad + i * 3;
-    o[0] += acc.x;
-    o[1] += acc.y;
-    o[2] += acc.z;
+    st3(vpos_grad + 3 * i, g0);
 }
 
 }  // namespace
@@ -809,7 +842,7 @@ static bool target_tensor_map(const RasterWorkspace& ws, const float* target, in
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& nrm_ws, cudaStream_t s, int B, int C,
+hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vacc, cudaStream_t s, int B, int C,
                           int albedo, int shading, int ifs, int tfs, const float* grad,
                           const float* verts, const float* colors, const float* texture, int tex_h, int tex_w,
                           const float* sh, const float* target, const float* vnormal, const float* bary,
@@ -819,13 +852,16 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& nrm
     HC_TRY(raster_layout(ws));
     HC_TRY(ws.cams.ensure(sizeof(ViewCam) * (size_t)std::max(V, ws.cap_views)));
     const bool shaded = shading == kShaded;
-    if (shaded) HC_TRY(nrm_ws.ensure(sizeof(float) * 3 * (size_t)B * N));
-    if (vpos_grad) HC_CUDA(cudaMemsetAsync(vpos_grad, 0, sizeof(float) * 3 * (size_t)B * N, s));
-    if (vcol_grad) HC_CUDA(cudaMemsetAsync(vcol_grad, 0, sizeof(float) * 3 * (size_t)B * N, s));
+    const int alb = albedo == kVertexColor ? kAlbVcol
+                    : albedo == kTextured ? kAlbTex
+                    : albedo == kTexturedBilinear ? kAlbTexBilinear : kAlbNone;
+    const int stride = (3 + (alb == kAlbVcol ? 3 : 0) + (shaded ? 3 : 0) + 3) / 4 * 4;  // VertexSums::kStride
+    const size_t vacc_bytes = sizeof(float) * (size_t)stride * (size_t)B * N;
+    HC_TRY(vacc.ensure(vacc_bytes));
+    HC_CUDA(cudaMemsetAsync(vacc.ptr, 0, vacc_bytes, s));
     if (tex_grad && tex_h > 0 && tex_w > 0)
         HC_CUDA(cudaMemsetAsync(tex_grad, 0, sizeof(float) * 3 * (size_t)B * tex_h * tex_w, s));
     if (sh_grad) HC_CUDA(cudaMemsetAsync(sh_grad, 0, sizeof(float) * 27 * (size_t)V, s));
-    if (shaded) HC_CUDA(cudaMemsetAsync(nrm_ws.ptr, 0, sizeof(float) * 3 * (size_t)B * N, s));
     ViewCam* cams = ws.cams.as<ViewCam>();
     k_view_setup<<<div_up(V, 64), 64, 0, s>>>(V, C, extr, intr, ws.layout.as<CamLayout>(), ws.P_frame, ws.T_frame,
                                               ws.Tb_frame, cams);
@@ -856,11 +892,9 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& nrm
     A.vnormal = vnormal;
     A.bary = bary;
     A.face = face;
-    A.vpos_grad = vpos_grad;
-    A.vcol_grad = vcol_grad;
+    A.vacc = vacc.as<float>();
     A.tex_grad = tex_grad;
     A.sh_grad = sh_grad;
-    A.nrm_grad = shaded ? nrm_ws.as<float>() : nullptr;
     HC_TRY(ws.stats.ensure(sizeof(RasterStats)));
     A.err = &ws.stats.as<RasterStats>()->overflow;
     A.l1_state = l1 ? l1->state : nullptr;
@@ -877,9 +911,6 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& nrm
     memset(&tmap, 0, sizeof(tmap));
     const int use_tma = target_tensor_map(ws, target, V, ifs, &tmap) ? 1 : 0;
     ws.clock.begin(kKRenderGrad, s);
-    const int alb = albedo == kVertexColor ? kAlbVcol
-                    : albedo == kTextured ? kAlbTex
-                    : albedo == kTexturedBilinear ? kAlbTexBilinear : kAlbNone;
     const int sel = (shaded ? 8 : 0) + alb * 2 + (parity ? 1 : 0);
     switch (sel) {
 #define HC_GRAD_CASE(SH, AL, PA)                                                                              \
@@ -911,14 +942,26 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& nrm
     }
     HC_CHECK_LAUNCH();
     ws.clock.end(kKRenderGrad, s);
-    if (shaded) {
-        ws.clock.begin(kKNormalChain, s);
-        k_normal_chain<<<div_up((long long)B * N, 256), 256, 0, s>>>(B, N, topo.faces.as<int3>(), topo.vf.as<int>(),
-                                                                     topo.vf_id.as<int2>(), verts, nrm_ws.as<float>(),
-                                                                     vpos_grad);
-        HC_CHECK_LAUNCH();
-        ws.clock.end(kKNormalChain, s);
+    ws.clock.begin(kKNormalChain, s);
+    switch ((shaded ? 4 : 0) + alb) {
+#define HC_VERTEX_CASE(SH, AL)                                                                                \
+    case (SH ? 4 : 0) + AL:                                                                                   \
+        k_vertex_grad<SH, AL><<<div_up((long long)B * N, 256), 256, 0, s>>>(                                  \
+            B, N, topo.faces.as<int3>(), topo.vf.as<int>(), topo.vf_id.as<int2>(), verts, vacc.as<float>(),   \
+            vpos_grad, vcol_grad);                                                                            \
+        break;
+        HC_VERTEX_CASE(false, kAlbVcol)
+        HC_VERTEX_CASE(false, kAlbTex)
+        HC_VERTEX_CASE(false, kAlbNone)
+        HC_VERTEX_CASE(false, kAlbTexBilinear)
+        HC_VERTEX_CASE(true, kAlbVcol)
+        HC_VERTEX_CASE(true, kAlbTex)
+        HC_VERTEX_CASE(true, kAlbNone)
+        HC_VERTEX_CASE(true, kAlbTexBilinear)
+#undef HC_VERTEX_CASE
     }
+    HC_CHECK_LAUNCH();
+    ws.clock.end(kKNormalChain, s);
     return HC_OK;
 }
 
