@@ -3,6 +3,10 @@
 
 #include "hc_common.cuh"
 
+#include <map>
+#include <mutex>
+#include <utility>
+
 namespace hc {
 
 static thread_local std::string g_last_error;
@@ -20,6 +24,22 @@ void clear_error() { g_last_error.clear(); }
 
 static std::atomic<long long> g_launches{0};
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
+
+int resident_ctas(const void* kernel, int threads) {
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, int> known;  // a few kernels per device
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = known.find({kernel, dev});
+    if (it != known.end()) return it->second;
+    int sms = 0, per_sm = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess || per_sm <= 0)
+        per_sm = 1;
+    known[{kernel, dev}] = sms * per_sm;
+    return sms * per_sm;
+}
 
 }  // namespace hc
 

@@ -82,6 +82,19 @@ hc_status upload(DevBuf& b, const T* host, size_t count) {
     return HC_OK;
 }
 
+// CTAs of a kernel that are resident on the current device at once (SMs x CTAs
+// per SM without dynamic shared memory); looked up once per kernel and device
+int resident_ctas(const void* kernel, int threads);
+
+// grid of a persistent kernel: as many CTAs as are resident at once (a second
+// partial wave would run its work after everything else), never more than the
+// work items
+template <typename K>
+unsigned resident_grid(K kernel, int threads, long long items) {
+    const long long g = resident_ctas(reinterpret_cast<const void*>(kernel), threads);
+    return (unsigned)(items < 1 ? 1 : items < g ? items : g);
+}
+
 inline int div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace hc

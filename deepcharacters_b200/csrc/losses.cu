@@ -230,12 +230,7 @@ extern "C" hc_status hc_sum_squares_loss(void* stream, int64_t n, const float* x
     HC_CUDA(cudaMemsetAsync(acc, 0, sizeof(double), s));
     // grid-stride: as many CTAs as are resident at once, so that no partial
     // second wave runs after the rest
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sumsq_fused, 256, 0) != cudaSuccess || per_sm <= 0)
-        per_sm = 1;
-    const int blocks = (int)std::max<long long>(1, std::min<long long>((long long)sms * per_sm, n / 1024 + 1));
+    const unsigned blocks = resident_grid(k_sumsq_fused, 256, n / 1024 + 1);
     const int vec = n % 4 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)grad & 15) == 0;
     k_sumsq_fused<<<blocks, 256, 0, s>>>(n, x, weight, acc, grad, vec);
     HC_CHECK_LAUNCH();

@@ -788,24 +788,6 @@ __global__ void k_vertex_grad(int B, int N, const int3* __restrict__ faces, cons
 
 }  // namespace
 
-// CTAs of a persistent launch: as many as fit on the GPU at once (each walks
-// tiles blockIdx.x, + gridDim.x, ...), never more than the tiles
-template <class K>
-static unsigned persistent_grid(K kernel, long long tiles) {
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 148;
-    }
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, BNT, 0) != cudaSuccess || per_sm <= 0)
-        per_sm = 1;
-    const long long g = (long long)sms * per_sm;
-    return (unsigned)std::max<long long>(1, std::min(g, tiles));
-}
-
 hc_status raster_layout(RasterWorkspace& ws);
 
 // The target image [V][H][W][3] as a 3-D tensor map {3W, H, V} (floats) with a
@@ -916,10 +898,10 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vac
 #define HC_GRAD_CASE(SH, AL, PA)                                                                              \
     case (SH ? 8 : 0) + AL * 2 + PA:                                                                          \
         if (dyn)                                                                                              \
-            k_render_grad<SH, AL, PA, true><<<persistent_grid(k_render_grad<SH, AL, PA, true>, tiles), BNT, 0, s>>>( \
+            k_render_grad<SH, AL, PA, true><<<resident_grid(k_render_grad<SH, AL, PA, true>, BNT, tiles), BNT, 0, s>>>( \
                 A, cams, tiles, tmap, use_tma);                                                               \
         else                                                                                                  \
-            k_render_grad<SH, AL, PA, false><<<persistent_grid(k_render_grad<SH, AL, PA, false>, tiles), BNT, 0, s>>>( \
+            k_render_grad<SH, AL, PA, false><<<resident_grid(k_render_grad<SH, AL, PA, false>, BNT, tiles), BNT, 0, s>>>( \
                 A, cams, tiles, tmap, use_tma);                                                               \
         break;
         HC_GRAD_CASE(false, kAlbVcol, false)

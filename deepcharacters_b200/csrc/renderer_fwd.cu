@@ -923,17 +923,6 @@ __global__ void k_l1_loss(const L1State* __restrict__ state, float* __restrict__
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-// grid of a persistent kernel: as many CTAs as are resident at once (SMs x
-// CTAs per SM), never more than the work items
-template <typename K>
-static unsigned resident_grid(K kernel, int threads, long long items) {
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess || per_sm <= 0)
-        per_sm = 1;
-    return (unsigned)std::max<long long>(1, std::min((long long)sms * per_sm, items));
-}
 // Tiles a CTA of the tile resolve claims per atomic: four, so that the one
 // counter sees a quarter of the atomics, but no more than leave every CTA at
 // least four claims (a 512 x 512 view has 1024 tiles of 16 px for 740 CTAs:

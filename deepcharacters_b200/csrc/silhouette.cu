@@ -1166,19 +1166,6 @@ long long max_view_pixels(const ImgLayout& L) {
 }
 
 // every view's pixel count a multiple of 4 (so every view starts 4-aligned)
-// grid of a persistent kernel: as many CTAs as are resident at once (a
-// second partial wave would run its strided work after everything else),
-// never more than `items`
-template <typename K>
-unsigned resident_blocks(K kernel, int threads, long long items) {
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess || per_sm <= 0)
-        per_sm = 1;
-    return (unsigned)std::max<long long>(1, std::min<long long>(items, (long long)sms * per_sm));
-}
-
 bool pixels_by_four(const ImgLayout& L) {
     for (int c = 0; c < L.n_cam; ++c)
         if (((long long)L.cam[c].W * L.cam[c].H) % 4 != 0) return false;
@@ -1313,13 +1300,13 @@ static hc_status mesh_boundary_run(hc_mesh_boundary h, void* stream, int32_t bat
         HC_CUDA(cudaMemsetAsync(cb.n_items, 0, sizeof(int), s));
         k_cov_cull<<<dim3(div_up(h->F, 256), (unsigned)views), 256, 0, s>>>(h->N, h->F, h->faces.as<int>(), p2, cb, L);
         HC_CHECK_LAUNCH();
-        k_cov_bin_list<<<resident_blocks(k_cov_bin_list, 256, views * h->F / 256 + 1), 256, 0, s>>>(
+        k_cov_bin_list<<<resident_grid(k_cov_bin_list, 256, views * h->F / 256 + 1), 256, 0, s>>>(
             h->N, h->F, h->faces.as<int>(), p2, cb, L);
     } else {
         k_cov_bin<<<dim3(div_up(h->F, 256), (unsigned)views), 256, 0, s>>>(h->N, h->F, h->faces.as<int>(), p2, cb, L);
     }
     HC_CHECK_LAUNCH();
-    k_cov_tile<<<resident_blocks(k_cov_tile, kCovTile * kCovTile, n_keys), kCovTile * kCovTile, 0, s>>>(h->F, n_keys,
+    k_cov_tile<<<resident_grid(k_cov_tile, kCovTile * kCovTile, n_keys), kCovTile * kCovTile, 0, s>>>(h->F, n_keys,
                                                                                                       cb, L);
     HC_CHECK_LAUNCH();
     k_boundary_cover<<<div_up(nv, 256), 256, 0, s>>>(batch, n_cameras, h->N, L, p2d, h->cover.as<unsigned char>(),

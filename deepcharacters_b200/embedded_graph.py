@@ -127,6 +127,7 @@ class _EGFn(torch.autograd.Function):
         ctx.eng = eng
         ctx.save_for_backward(da, sa, dT, disp)
         ctx.mark_non_differentiable(da, sa)
+        ctx.set_materialize_grads(False)  # only the vertices' and markers' gradients are read
         return v, n, m, g, da, sa
 
     @staticmethod

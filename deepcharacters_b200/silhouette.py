@@ -52,8 +52,9 @@ class _ProjFn(torch.autograd.Function):
         points, vectors, extrinsics, intrinsics = ctx.saved_tensors
         gp = camera_projection_backward(g, points, extrinsics, intrinsics, ctx.is_point)
         # normals / cameras get zero gradients (CameraProjectionGPU.py:60-71)
-        return (gp, None if vectors is None else torch.zeros_like(vectors), torch.zeros_like(extrinsics),
-                torch.zeros_like(intrinsics), None)
+        rest = [torch.zeros_like(t) if need else None
+                for t, need in zip((vectors, extrinsics, intrinsics), ctx.needs_input_grad[1:4])]
+        return (gp, *rest, None)
 
 
 class CameraProjectionGpu:
@@ -274,6 +275,7 @@ class _SilFn(torch.autograd.Function):
         res, res1, dtg, cid = eng.forward(points, normals, is_boundary, dt, crops)
         ctx.save_for_backward(dtg, cid, crops)
         ctx.mark_non_differentiable(dtg, cid)
+        ctx.set_materialize_grads(False)
         return res, res1, dtg, cid
 
     @staticmethod

@@ -148,8 +148,10 @@ class SkinningEngine:
             torch.as_tensor(node_vertex, dtype=torch.int32, device=dofs.device)
         if weights.shape != (self.N, self.K):
             raise ValueError(f"skin weights must be [{self.N},{self.K}], got {tuple(weights.shape)}")
-        if nv.numel() and (int(nv.min()) < 0 or int(nv.max()) >= self.N):
-            raise ValueError("node_vertex index out of range")
+        if nv.numel():
+            host = nv.cpu().numpy()  # one copy instead of two reductions and two reads
+            if int(host.min()) < 0 or int(host.max()) >= self.N:
+                raise ValueError("node_vertex index out of range")
         B, M = dofs.shape[0], nv.numel()
         t = torch.empty((B, M, 3), device=dofs.device)
         a = torch.empty((B, M, 3), device=dofs.device)
@@ -201,6 +203,7 @@ class _DQFn(torch.autograd.Function):
         ctx.eng = eng
         ctx.save_for_backward(v, gp, ga, dq, w)
         ctx.mark_non_differentiable(gp, ga, dq, w)
+        ctx.set_materialize_grads(False)  # only the positions' gradient is read
         return v, n, gp, ga, dq, w
 
     @staticmethod
@@ -219,6 +222,7 @@ class _LBSFn(torch.autograd.Function):
         ctx.eng = eng
         ctx.save_for_backward(v, gp, ga, xf, w, disp)
         ctx.mark_non_differentiable(gp, ga, xf, w)
+        ctx.set_materialize_grads(False)  # only the positions' gradient is read
         return v, n, gp, ga, xf, w
 
     @staticmethod
