@@ -52,15 +52,29 @@ __host__ __device__ inline void axis_angle(const float* a, float th, float* R) {
 }
 
 __host__ __device__ inline void xf_mul(const Xf& A, const Xf& B, Xf& O) {
+#pragma unroll
     for (int i = 0; i < 3; ++i) {
+#pragma unroll
         for (int j = 0; j < 3; ++j)
             O.r[3 * i + j] = A.r[3 * i] * B.r[j] + A.r[3 * i + 1] * B.r[3 + j] + A.r[3 * i + 2] * B.r[6 + j];
         O.t[i] = A.r[3 * i] * B.t[0] + A.r[3 * i + 1] * B.t[1] + A.r[3 * i + 2] * B.t[2] + A.t[i];
     }
 }
 
+// the branch of mat_to_quat for the largest diagonal entry I
+template <int I>
+__device__ __forceinline__ void quat_from_largest(const float* R, float* q) {
+    constexpr int j = (I + 1) % 3, k = (j + 1) % 3;
+    float s = sqrtf(R[3 * I + I] - R[3 * j + j] - R[3 * k + k] + 1.f);
+    q[I] = 0.5f * s;
+    s = 0.5f / s;
+    q[3] = (R[3 * k + j] - R[3 * j + k]) * s;
+    q[j] = (R[3 * j + I] + R[3 * I + j]) * s;
+    q[k] = (R[3 * k + I] + R[3 * I + k]) * s;
+}
+
 // quaternion (x, y, z, w) of a rotation matrix (Shepperd's method), normalised
-__host__ __device__ inline void mat_to_quat(const float* R, float* q) {
+__device__ __forceinline__ void mat_to_quat(const float* R, float* q) {
     const float tr = R[0] + R[4] + R[8];
     if (tr > 0.f) {
         float s = sqrtf(tr + 1.f);
@@ -69,17 +83,12 @@ __host__ __device__ inline void mat_to_quat(const float* R, float* q) {
         q[0] = (R[7] - R[5]) * s;
         q[1] = (R[2] - R[6]) * s;
         q[2] = (R[3] - R[1]) * s;
+    } else if (R[4] > R[0]) {
+        if (R[8] > R[4]) quat_from_largest<2>(R, q);
+        else quat_from_largest<1>(R, q);
     } else {
-        int i = 0;
-        if (R[4] > R[0]) i = 1;
-        if (R[8] > R[3 * i + i]) i = 2;
-        const int j = (i + 1) % 3, k = (j + 1) % 3;
-        float s = sqrtf(R[3 * i + i] - R[3 * j + j] - R[3 * k + k] + 1.f);
-        q[i] = 0.5f * s;
-        s = 0.5f / s;
-        q[3] = (R[3 * k + j] - R[3 * j + k]) * s;
-        q[j] = (R[3 * j + i] + R[3 * i + j]) * s;
-        q[k] = (R[3 * k + i] + R[3 * i + k]) * s;
+        if (R[8] > R[0]) quat_from_largest<2>(R, q);
+        else quat_from_largest<0>(R, q);
     }
     const float n = sqrtf(q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
     for (int c = 0; c < 4; ++c) q[c] /= n;
@@ -99,6 +108,17 @@ struct Skel {
     const float* skin_scale;  // [S]
     const float* t0inv;    // [S,12] inverse rest transform (R 9 + t 3)
     const unsigned char* in_chain;  // [S,J]
+    // the joints' dof entries in dof order, and the joints by depth in the tree
+    int levels;
+    const int* joint_off;    // [J+1]
+    const int* joint_dof;    // [E]
+    const float* joint_w;    // [E]
+    const int* level_off;    // [levels+1]
+    const int* level_joint;  // [J]: joint << 16 | parent + 1
+    // the adjoint's vertex blocks: each block's (vertex, slot) pairs by skinning joint
+    int grad_block;          // vertices per block
+    const int* bone_off;     // [blocks, S+1]
+    const int2* bone_slot;   // [N,K]: (vertex * K + slot, vertex) within the block
     const int* skin_idx;   // [N,K] skinning joint per vertex slot
     const float* base_v;   // [N,3]
     const float* base_n;   // [N,3]
@@ -106,114 +126,116 @@ struct Skel {
     const float4* base_n4;  // [N]
 };
 
-// Forward kinematics, one CTA per frame: the joint parameters and every
-// joint's local transform are formed in parallel in shared memory, one thread
-// composes the chain (parents precede children), and the outputs -- joint
-// transforms [B,J], global joint positions / axes [B,J,3], skinning
-// transforms [B,S] -- are written in parallel.
-__global__ void k_fk(Skel sk, int B, const float* __restrict__ dofs, Xf* __restrict__ joints, float* __restrict__ gpos,
-                     float* __restrict__ gaxis, Xf* __restrict__ skin_xf, float* __restrict__ params) {
+// Forward kinematics, one CTA per frame.  Every joint sums its dof entries (in
+// dof order, the reference's) and forms its local transform in parallel; the
+// chain is composed level by level of the tree, twelve threads per joint, and
+// the outputs -- global joint positions / axes [B,J,3] and the skinning
+// transforms [B,S], as dual quaternions (8 floats; DualQuaternion.h:58-69) or
+// as rotation + translation (12 floats) -- are written in parallel.
+// Bound by latency: a few dependent loads and one short step per level (21
+// levels for 24 joints of three revolute axes).  One thread composing all 72
+// joints in turn, with the transforms' conversion in a kernel of its own, took
+// 27 us; this takes 7.7 us.
+constexpr int kFkBlock = 128;
+
+__global__ void __launch_bounds__(kFkBlock) k_fk(Skel sk, const float* __restrict__ dofs, float* __restrict__ gpos,
+                                                 float* __restrict__ gaxis, float* __restrict__ dq_out,
+                                                 float* __restrict__ xf_out) {
     extern __shared__ float fk_sm[];
     const int b = blockIdx.x;
-    const int J4 = (sk.J + 3) & ~3, E = sk.dof_off[sk.D], E4 = (E + 3) & ~3;
-    float* P = fk_sm;                                        // [J]
-    Xf* Lx = reinterpret_cast<Xf*>(fk_sm + J4);              // [J] local transforms
-    Xf* T = Lx + sk.J;                                       // [J] global transforms
-    int* par = reinterpret_cast<int*>(T + sk.J);             // [J] parents
-    float* prod = reinterpret_cast<float*>(par + J4);        // [E] dof weight * dof value
-    int* ent_joint = reinterpret_cast<int*>(prod + E4);      // [E] joint of each dof entry
-    // DOF -> joint parameters (dof.cpp:9-17): the products in parallel, then
-    // every joint sums its entries in dof order, the reference's order
-    for (int d = threadIdx.x; d < sk.D; d += blockDim.x) {
-        const float v = dofs[(long long)b * sk.D + d];
-        for (int e = sk.dof_off[d]; e < sk.dof_off[d + 1]; ++e) {
-            prod[e] = sk.dof_w[e] * v;
-            ent_joint[e] = sk.dof_joint[e];
-        }
-    }
-    for (int j = threadIdx.x; j < sk.J; j += blockDim.x) par[j] = sk.parent[j];
-    __syncthreads();
-    for (int j = threadIdx.x; j < sk.J; j += blockDim.x) {
-        float acc = 0.f;
-        for (int e = 0; e < E; ++e)
-            if (ent_joint[e] == j) acc += prod[e];
-        P[j] = acc;
-    }
-    __syncthreads();
-    for (int j = threadIdx.x; j < sk.J; j += blockDim.x) {
+    float* L = fk_sm;                                   // [J][12] local transforms
+    float* T = L + 12 * sk.J;                           // [J][12] global transforms
+    int* ord = reinterpret_cast<int*>(T + 12 * sk.J);   // [J] joints by level
+    for (int j = threadIdx.x; j < sk.J; j += kFkBlock) {
+        // DOF -> joint parameter (dof.cpp:9-17), each product rounded on its own
+        float th = 0.f;
+        const int e1 = sk.joint_off[j + 1];
+        for (int e = sk.joint_off[j]; e < e1; ++e)
+            th = __fadd_rn(th, __fmul_rn(sk.joint_w[e], dofs[(long long)b * sk.D + sk.joint_dof[e]]));
         Xf local;
         const float s = sk.jscale[j];
         const float* ax = sk.axis + 3 * j;
         if (sk.type[j] == kRevolute) {
-            axis_angle(ax, P[j], local.r);
+            axis_angle(ax, th, local.r);
             for (int c = 0; c < 3; ++c) local.t[c] = sk.offset[3 * j + c] * s;
         } else {
             for (int c = 0; c < 9; ++c) local.r[c] = (c % 4 == 0) ? 1.f : 0.f;
-            for (int c = 0; c < 3; ++c) local.t[c] = sk.offset[3 * j + c] * s + ax[c] * P[j];
+            for (int c = 0; c < 3; ++c) local.t[c] = sk.offset[3 * j + c] * s + ax[c] * th;
         }
-        Lx[j] = local;
+#pragma unroll
+        for (int c = 0; c < 9; ++c) L[12 * j + c] = local.r[c];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) L[12 * j + 9 + c] = local.t[c];
+        ord[j] = sk.level_joint[j];
+    }
+    int l0 = 0;  // level_off[0]
+    for (int l = 0; l < sk.levels; ++l) {  // T[j] = T[parent] L[j], the operations of xf_mul
+        const int l1 = sk.level_off[l + 1];
+        __syncthreads();
+        for (int i = threadIdx.x; i < 12 * (l1 - l0); i += kFkBlock) {
+            const int q = i / 12, e = i - 12 * q, jp = ord[l0 + q], j = jp >> 16, p = (jp & 0xffff) - 1;
+            const float* Bm = L + 12 * j;
+            float r = Bm[e];
+            if (p >= 0) {
+                const int row = e < 9 ? e / 3 : e - 9, col = e < 9 ? e - 3 * row : 9, step = e < 9 ? 3 : 1;
+                const float* A = T + 12 * p;
+                r = A[3 * row] * Bm[col] + A[3 * row + 1] * Bm[col + step] + A[3 * row + 2] * Bm[col + 2 * step];
+                if (e >= 9) r += A[9 + row];
+            }
+            T[12 * j + e] = r;
+        }
+        l0 = l1;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int j = 0; j < sk.J; ++j) {
-            const int p = par[j];
-            if (p >= 0) xf_mul(T[p], Lx[j], T[j]);
-            else T[j] = Lx[j];
-        }
-    }
-    __syncthreads();
-    for (int j = threadIdx.x; j < sk.J; j += blockDim.x) {
-        const Xf X = T[j];
-        joints[(long long)b * sk.J + j] = X;
-        params[(long long)b * sk.J + j] = P[j];
+    for (int j = threadIdx.x; j < sk.J; j += kFkBlock) {
+        const float* X = T + 12 * j;
         const float* ax = sk.axis + 3 * j;
         float* gp = gpos + ((long long)b * sk.J + j) * 3;
         float* ga = gaxis + ((long long)b * sk.J + j) * 3;
         for (int c = 0; c < 3; ++c) {
-            gp[c] = X.t[c];
-            ga[c] = X.r[3 * c] * ax[0] + X.r[3 * c + 1] * ax[1] + X.r[3 * c + 2] * ax[2];
+            gp[c] = X[9 + c];
+            ga[c] = X[3 * c] * ax[0] + X[3 * c + 1] * ax[1] + X[3 * c + 2] * ax[2];
         }
     }
     // skinning transforms J * scale * J0^-1 (DQSkinningGPUOp.cpp:274-306); the
     // rotation part has the uniform scale divided out (Eigen rotation())
-    for (int si = threadIdx.x; si < sk.S; si += blockDim.x) {
-        Xf A = T[sk.skin_joint[si]];
+    for (int si = threadIdx.x; si < sk.S; si += kFkBlock) {
+        const float* X = T + 12 * sk.skin_joint[si];
         const float sc = sk.skin_scale[si];
-        Xf I0;
+        Xf A, I0, O;
+#pragma unroll
+        for (int c = 0; c < 9; ++c) A.r[c] = X[c];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) A.t[c] = X[9 + c];
+#pragma unroll
         for (int c = 0; c < 9; ++c) I0.r[c] = sk.t0inv[12 * si + c] * sc;
+#pragma unroll
         for (int c = 0; c < 3; ++c) I0.t[c] = sk.t0inv[12 * si + 9 + c] * sc;
-        Xf O;
         xf_mul(A, I0, O);
+#pragma unroll
         for (int c = 0; c < 9; ++c) O.r[c] /= sc;
-        skin_xf[(long long)b * sk.S + si] = O;
+        if (dq_out) {
+            float q[4];
+            mat_to_quat(O.r, q);
+            const float* t = O.t;
+            float* o = dq_out + 8 * ((long long)b * sk.S + si);
+            o[0] = q[0];
+            o[1] = q[1];
+            o[2] = q[2];
+            o[3] = q[3];
+            o[7] = -0.5f * (t[0] * q[0] + t[1] * q[1] + t[2] * q[2]);
+            o[4] = 0.5f * (t[0] * q[3] + t[1] * q[2] - t[2] * q[1]);
+            o[5] = 0.5f * (-t[0] * q[2] + t[1] * q[3] + t[2] * q[0]);
+            o[6] = 0.5f * (t[0] * q[1] - t[1] * q[0] + t[2] * q[3]);
+        }
+        if (xf_out) {
+            float* o = xf_out + 12 * ((long long)b * sk.S + si);
+#pragma unroll
+            for (int c = 0; c < 9; ++c) o[c] = O.r[c];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) o[9 + c] = O.t[c];
+        }
     }
-}
-
-// dual quaternions of the skinning transforms: rotation (x,y,z,w), translation (x,y,z,w)
-// (DualQuaternion.h:58-69)
-__global__ void k_dq_from_xf(int BS, const Xf* __restrict__ xf, float* __restrict__ dq) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= BS) return;
-    const Xf X = xf[i];
-    float q[4];
-    mat_to_quat(X.r, q);
-    const float* t = X.t;
-    float* o = dq + 8LL * i;
-    o[0] = q[0];
-    o[1] = q[1];
-    o[2] = q[2];
-    o[3] = q[3];
-    o[7] = -0.5f * (t[0] * q[0] + t[1] * q[1] + t[2] * q[2]);
-    o[4] = 0.5f * (t[0] * q[3] + t[1] * q[2] - t[2] * q[1]);
-    o[5] = 0.5f * (-t[0] * q[2] + t[1] * q[3] + t[2] * q[0]);
-    o[6] = 0.5f * (t[0] * q[1] - t[1] * q[0] + t[2] * q[3]);
-}
-
-__global__ void k_xf_to_lbs(int BS, const Xf* __restrict__ xf, float* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= BS) return;
-    for (int c = 0; c < 9; ++c) out[12LL * i + c] = xf[i].r[c];
-    for (int c = 0; c < 3; ++c) out[12LL * i + 9 + c] = xf[i].t[c];
 }
 
 __device__ __forceinline__ float dot4(float4 a, float4 b) { return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
@@ -257,25 +279,6 @@ __device__ __forceinline__ void dq_rotmat(float4 q, float* R) {
     R[6] = txz - twy;
     R[7] = tyz + twx;
     R[8] = 1.f - txx - tyy;
-}
-
-// sign-aligned weighted blend of a vertex's dual quaternions (DQSkinningGPUOp.cu:65-92)
-__device__ __forceinline__ void dq_blend(const Skel& sk, int b, int v, const float* __restrict__ dq,
-                                         const float* __restrict__ w, float4& br, float4& bt) {
-    br = make_float4(0.f, 0.f, 0.f, 0.f);
-    bt = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 first = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int k = 0; k < sk.K; ++k) {
-        const int s = sk.skin_idx[(long long)v * sk.K + k];
-        const float wk = w[((long long)b * sk.N + v) * sk.K + k];
-        const float* q = dq + ((long long)b * sk.S + s) * 8;
-        const float4 r = f4(q), t = f4(q + 4);
-        float sign = 1.0f;
-        if (k == 0) first = r;
-        if (dot4(first, r) < 0.f && k != 0) sign = -1.0f;
-        br = add4(br, mul4(mul4(r, wk), sign));
-        bt = add4(bt, mul4(mul4(t, wk), sign));
-    }
 }
 
 // Shared-memory staging of a skinning block (grid (vertex blocks, frames),
@@ -412,73 +415,46 @@ __global__ void __launch_bounds__(kSkinBlock) k_lbs_skin(Skel sk, int B, const f
 // adjoints
 // ---------------------------------------------------------------------------
 
-// per-bone moments A_s = sum w (v x g), G_s = sum w g over the vertices of a
-// frame; one CTA covers 256 vertices of one frame (grid.y = frame)
-__global__ void k_bone_moments(Skel sk, const float* __restrict__ vpos, const float* __restrict__ gv,
-                               const float* __restrict__ w, float* __restrict__ mom) {
-    extern __shared__ float s_mom[];  // [S][6]
-    const int b = blockIdx.y;
-    for (int i = threadIdx.x; i < sk.S * 6; i += blockDim.x) s_mom[i] = 0.f;
-    __syncthreads();
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < sk.N) {
-        const long long vi = (long long)b * sk.N + v;
-        const float3 p = ld3(vpos + 3 * vi), g = ld3(gv + 3 * vi);
-        const float3 pg = cross(p, g);
-        for (int k = 0; k < sk.K; ++k) {
-            const int s = sk.skin_idx[(long long)v * sk.K + k];
-            const float wk = w[vi * sk.K + k];
-            float* m = s_mom + 6 * s;
-            atomicAdd(m + 0, wk * pg.x);
-            atomicAdd(m + 1, wk * pg.y);
-            atomicAdd(m + 2, wk * pg.z);
-            atomicAdd(m + 3, wk * g.x);
-            atomicAdd(m + 4, wk * g.y);
-            atomicAdd(m + 5, wk * g.z);
-        }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < sk.S * 6; i += blockDim.x)
-        if (s_mom[i] != 0.f) atomicAdd(mom + (long long)b * sk.S * 6 + i, s_mom[i]);
+// dynamic shared memory of an adjoint block: the joint table, the block's
+// weights and joint indices, and six values per vertex
+__host__ __device__ constexpr size_t skin_grad_smem(int S, int table_floats, int K, int threads) {
+    return skin_block_smem(S, table_floats, K, threads) + sizeof(float) * 6 * (size_t)threads;
 }
 
-// dof gradient from the bone moments: a dof collects, for every joint it
-// drives, axis . (A_s - c x G_s) (revolute) or axis . G_s (prismatic) of the
-// bones whose kinematic chain contains that joint
-__global__ void k_dof_grad(Skel sk, int B, const float* __restrict__ mom, const float* __restrict__ gpos,
-                           const float* __restrict__ gaxis, float* __restrict__ gdof) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B * sk.D) return;
-    const int b = i / sk.D, d = i % sk.D;
-    float acc = 0.f;
-    for (int e = sk.dof_off[d]; e < sk.dof_off[d + 1]; ++e) {
-        const int j = sk.dof_joint[e];
-        const float3 ax = ld3(gaxis + ((long long)b * sk.J + j) * 3);
-        const float3 c = ld3(gpos + ((long long)b * sk.J + j) * 3);
-        for (int s = 0; s < sk.S; ++s) {
-            if (!sk.in_chain[s * sk.J + j]) continue;
-            const float* m = mom + ((long long)b * sk.S + s) * 6;
-            const float3 A = make_float3(m[0], m[1], m[2]), G = make_float3(m[3], m[4], m[5]);
-            acc += sk.type[j] == kRevolute ? dot(ax, A - cross(c, G)) : dot(ax, G);
+// Sums of eight values over the warp: value lane & 7 is returned in every lane
+// (three rounds halve the values each lane carries, two more add the rest:
+// 9 shuffles instead of 40).
+__device__ __forceinline__ float warp_sum8(float v[8], int lane) {
+#pragma unroll
+    for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const float keep = (lane & h) ? v[i + h] : v[i], send = (lane & h) ? v[i] : v[i + h];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
         }
-    }
-    gdof[i] = acc;
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 8);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
+    return v[0];
 }
 
-// DQ weight gradient (DQSkinningGPUOpGrad.cu:12-141).  `parity` keeps the
-// reference's Jacobian of the rotated point (DQHelper.h:121-174, which adds
-// vert.z instead of multiplying by it); otherwise the exact Jacobian.
-__global__ void k_dq_weight_grad(Skel sk, int B, const float* __restrict__ dq, const float* __restrict__ w,
-                                 const float* __restrict__ gv, int parity, float* __restrict__ gw) {
-    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (idx >= (long long)B * sk.N * sk.K) return;
-    const int kk = (int)(idx % sk.K);
-    const long long vi = idx / sk.K;
-    const int b = (int)(vi / sk.N), v = (int)(vi % sk.N);
-    float4 br, bt;
-    dq_blend(sk, b, v, dq, w, br, bt);
-    const int s0 = sk.skin_idx[(long long)v * sk.K];
-    const float4 first = f4(dq + ((long long)b * sk.S + s0) * 8);
+// DQ weight gradients of a vertex's slots (DQSkinningGPUOpGrad.cu:12-141).
+// `parity` keeps the reference's Jacobian of the rotated point
+// (DQHelper.h:121-174, which adds vert.z instead of multiplying by it);
+// otherwise the exact Jacobian.  I holds the slots' joints and receives the
+// gradients in their place.
+__device__ __forceinline__ void dq_weight_grads(int K, const float* s_dq, const float* Wt, int* I, float3 vb, float3 g,
+                                                int parity) {
+    // sign-aligned weighted blend (DQSkinningGPUOp.cu:65-92)
+    float4 br = make_float4(0.f, 0.f, 0.f, 0.f), bt = br, first = br;
+    for (int k = 0; k < K; ++k) {
+        const float* q = s_dq + I[k] * 8;
+        const float4 r = f4(q), t = f4(q + 4);
+        float sign = 1.0f;
+        if (k == 0) first = r;
+        if (dot4(first, r) < 0.f && k != 0) sign = -1.0f;
+        br = add4(br, mul4(mul4(r, Wt[k]), sign));
+        bt = add4(bt, mul4(mul4(t, Wt[k]), sign));
+    }
     float scale = sqrtf(dot4(br, br));
     const float4 ir = br, it = bt;
     bool small = false;
@@ -488,91 +464,177 @@ __global__ void k_dq_weight_grad(Skel sk, int B, const float* __restrict__ dq, c
     }
     br = mul4(br, 1.f / scale);
     bt = mul4(bt, 1.f / scale);
-    const int s = sk.skin_idx[(long long)v * sk.K + kk];
-    const float* q = dq + ((long long)b * sk.S + s) * 8;
-    float4 fr = f4(q), ft = f4(q + 4);
-    const float sign = (dot4(first, fr) < 0.f && kk != 0) ? -1.f : 1.f;
-    fr = mul4(fr, sign);
-    ft = mul4(ft, sign);
-    float ds = dot4(mul4(ir, 1.f / scale), fr);
-    if (small) ds = 0.f;
     const float s2 = scale * scale;
-    fr = mul4(add4(mul4(fr, scale), mul4(ir, -ds)), 1.f / s2);
-    ft = mul4(add4(mul4(ft, scale), mul4(it, -ds)), 1.f / s2);
-    // d(point)/d(rotation quaternion) and d(translation)/d(dq) applied to (fr, ft)
-    const float3 vb = ld3(sk.base_v + 3LL * v);
     const float x = br.x, y = br.y, z = br.z, ww = br.w;
-    const float qd[4] = {fr.x, fr.y, fr.z, fr.w};
-    // rows of dR/dq entries (R00..R22 w.r.t. x,y,z,w)
+    // rows of dR/dq entries (R00..R22 w.r.t. x,y,z,w), contracted with the base vertex
     const float dR[9][4] = {{0.f, -4.f * y, -4.f * z, 0.f},      {2.f * y, 2.f * x, -2.f * ww, -2.f * z},
                             {2.f * z, 2.f * ww, 2.f * x, 2.f * y}, {2.f * y, 2.f * x, 2.f * ww, 2.f * z},
                             {-4.f * x, 0.f, -4.f * z, 0.f},      {-2.f * ww, 2.f * z, 2.f * y, -2.f * x},
                             {2.f * z, -2.f * ww, 2.f * x, -2.f * y}, {2.f * ww, 2.f * z, 2.f * y, 2.f * x},
                             {-4.f * x, -4.f * y, 0.f, 0.f}};
-    float3 g = make_float3(0.f, 0.f, 0.f);
-    float gr[3];
-    for (int r = 0; r < 3; ++r) {
-        float acc = 0.f;
+    float jac[3][4];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
         for (int c = 0; c < 4; ++c) {
             const float a0 = dR[3 * r + 0][c], a1 = dR[3 * r + 1][c], a2 = dR[3 * r + 2][c];
-            const float jac = parity ? (a0 * vb.x + a1 * vb.y + a2 + vb.z) : (a0 * vb.x + a1 * vb.y + a2 * vb.z);
-            acc += jac * qd[c];
+            jac[r][c] = parity ? (a0 * vb.x + a1 * vb.y + a2 + vb.z) : (a0 * vb.x + a1 * vb.y + a2 * vb.z);
         }
-        gr[r] = acc;
-    }
-    g = make_float3(gr[0], gr[1], gr[2]);
     // translation: t = 2 (-t.w r.xyz + t.xyz r.w + ...) (DQHelper.h:184-235)
     const float4 tq = bt;
     const float dTr[3][4] = {{-tq.w, tq.z, -tq.y, tq.x}, {-tq.z, -tq.w, tq.x, tq.y}, {tq.y, -tq.x, -tq.w, tq.z}};
     const float dTt[3][4] = {{ww, -z, y, -x}, {z, ww, -x, -y}, {-y, x, ww, -z}};
-    const float ftd[4] = {ft.x, ft.y, ft.z, ft.w};
-    for (int r = 0; r < 3; ++r) {
-        float acc = 0.f;
-        for (int c = 0; c < 4; ++c) acc += 2.f * dTr[r][c] * qd[c] + 2.f * dTt[r][c] * ftd[c];
-        gr[r] = acc;
+    for (int k = 0; k < K; ++k) {
+        const float* q = s_dq + I[k] * 8;
+        float4 fr = f4(q), ft = f4(q + 4);
+        const float sign = (dot4(first, fr) < 0.f && k != 0) ? -1.f : 1.f;
+        fr = mul4(fr, sign);
+        ft = mul4(ft, sign);
+        float ds = dot4(mul4(ir, 1.f / scale), fr);
+        if (small) ds = 0.f;
+        fr = mul4(add4(mul4(fr, scale), mul4(ir, -ds)), 1.f / s2);
+        ft = mul4(add4(mul4(ft, scale), mul4(it, -ds)), 1.f / s2);
+        // d(point)/d(rotation quaternion) and d(translation)/d(dq) applied to (fr, ft)
+        const float qd[4] = {fr.x, fr.y, fr.z, fr.w}, ftd[4] = {ft.x, ft.y, ft.z, ft.w};
+        float gr[3], gt[3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            gr[r] = gt[r] = 0.f;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                gr[r] += jac[r][c] * qd[c];
+                gt[r] += 2.f * dTr[r][c] * qd[c] + 2.f * dTt[r][c] * ftd[c];
+            }
+        }
+        I[k] = __float_as_int(dot(make_float3(gr[0], gr[1], gr[2]) + make_float3(gt[0], gt[1], gt[2]), g));
     }
-    g = g + make_float3(gr[0], gr[1], gr[2]);
-    gw[idx] = dot(g, ld3(gv + 3 * vi));
 }
 
-// LBS weight / displacement gradients (LBSkinningGPUOpGrad.cu:11-88).  In the
-// parity mode the reference's indexing is kept: the weight gradient reads the
-// transform of slot k instead of the vertex's k-th bone and ignores the
-// displacement; the displacement gradient reads the weights without the frame
-// offset, the transform of slot k, and skips weights below 1e-4.
-__global__ void k_lbs_weight_grad(Skel sk, int B, const float* __restrict__ xf12, const float* __restrict__ disp,
-                                  const float* __restrict__ gv, int parity, float* __restrict__ gw) {
-    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (idx >= (long long)B * sk.N * sk.K) return;
-    const int kk = (int)(idx % sk.K);
-    const long long vi = idx / sk.K;
-    const int b = (int)(vi / sk.N), v = (int)(vi % sk.N);
-    const int s = parity ? kk : sk.skin_idx[(long long)v * sk.K + kk];
-    const float* X = xf12 + ((long long)b * sk.S + s) * 12;
-    float3 p = ld3(sk.base_v + 3LL * v);
-    if (!parity) p = p + ld3(disp + 3 * vi);
-    const float3 o = make_float3(X[0] * p.x + X[1] * p.y + X[2] * p.z, X[3] * p.x + X[4] * p.y + X[5] * p.z,
-                                 X[6] * p.x + X[7] * p.y + X[8] * p.z) + make_float3(X[9], X[10], X[11]);
-    gw[idx] = dot(o, ld3(gv + 3 * vi));
-}
-
-__global__ void k_lbs_disp_grad(Skel sk, int B, const float* __restrict__ xf12, const float* __restrict__ w,
-                                const float* __restrict__ gv, int parity, float* __restrict__ gd) {
-    const long long vi = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (vi >= (long long)B * sk.N) return;
-    const int b = (int)(vi / sk.N), v = (int)(vi % sk.N);
+// LBS weight and displacement gradients of a vertex (LBSkinningGPUOpGrad.cu:11-88).
+// In the parity mode the reference's indexing is kept: the weight gradient
+// reads the transform of slot k instead of the vertex's k-th bone and ignores
+// the displacement; the displacement gradient reads the weights without the
+// frame offset, the transform of slot k, and skips weights below 1e-4.
+// I as in dq_weight_grads.
+__device__ __forceinline__ float3 lbs_grads(const Skel& sk, int B, int b, int v, const float* s_xf,
+                                            const float* __restrict__ xf12, const float* __restrict__ w,
+                                            const float* __restrict__ disp, const float* Wt, int* I, float3 g,
+                                            int parity) {
+    const float4 b4 = sk.base_v4[v];
+    float3 p = make_float3(b4.x, b4.y, b4.z);
+    if (!parity) p = p + ld3(disp + 3 * ((long long)b * sk.N + v));
     float M[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // sum w R^T
     for (int k = 0; k < sk.K; ++k) {
-        const float wk = parity ? w[(long long)v * sk.K + k] : w[vi * sk.K + k];
+        const float* X = s_xf + 12 * (parity ? k : I[k]);
+        // slots past the last skinning joint read on into the next frame's, as the reference does
+        if (parity && k >= sk.S) X = (long long)b * sk.S + k < (long long)B * sk.S ? xf12 + 12 * ((long long)b * sk.S + k) : s_xf;
+        const float3 o = make_float3(X[0] * p.x + X[1] * p.y + X[2] * p.z, X[3] * p.x + X[4] * p.y + X[5] * p.z,
+                                     X[6] * p.x + X[7] * p.y + X[8] * p.z) + make_float3(X[9], X[10], X[11]);
+        I[k] = __float_as_int(dot(o, g));
+        const float wk = parity ? w[(long long)v * sk.K + k] : Wt[k];
         if (parity && wk < 1e-4f) continue;
-        const int s = parity ? k : sk.skin_idx[(long long)v * sk.K + k];
-        const float* X = xf12 + ((long long)b * sk.S + s) * 12;
+#pragma unroll
         for (int r = 0; r < 3; ++r)
+#pragma unroll
             for (int c = 0; c < 3; ++c) M[3 * c + r] += X[3 * r + c] * wk;
     }
-    const float3 g = ld3(gv + 3 * vi);
-    st3(gd + 3 * vi, make_float3(M[0] * g.x + M[1] * g.y + M[2] * g.z, M[3] * g.x + M[4] * g.y + M[5] * g.z,
-                                 M[6] * g.x + M[7] * g.y + M[8] * g.z));
+    return make_float3(M[0] * g.x + M[1] * g.y + M[2] * g.z, M[3] * g.x + M[4] * g.y + M[5] * g.z,
+                       M[6] * g.x + M[7] * g.y + M[8] * g.z);
+}
+
+// The skinning adjoint of a block of vertices of one frame (grid (vertex
+// blocks, frames)): a thread per vertex forms the gradients of its weights
+// (and, LBS, its displacement) from the staged joint table, and the block adds
+// its part of the bone moments A_s = sum w (v x g), G_s = sum w g.  The block's
+// (vertex, slot) pairs are listed by bone when the handle is made, so a warp
+// sums a bone's pairs in registers and adds six values per bone.
+// Reads and writes 100 bytes per vertex at K = 4; bound by instruction issue.
+// 16 frames x 40,962 vertices, 24 joints: 41 us, where six shared-memory
+// atomics per pair took 159 us and a thread per (vertex, slot), each blending
+// the vertex again, 55 us.
+template <bool DQ>
+__global__ void __launch_bounds__(256) k_skin_grad(Skel sk, int B, const float* __restrict__ tab,
+                                                   const float* __restrict__ w, const float* __restrict__ vpos,
+                                                   const float* __restrict__ gv, const float* __restrict__ disp,
+                                                   int parity, int vec, float* __restrict__ gw, float* __restrict__ gd,
+                                                   float* __restrict__ mom) {
+    extern __shared__ __align__(16) float s_dyn[];
+    constexpr int TF = DQ ? 8 : 12;
+    const int G = blockDim.x, b = blockIdx.y, K = sk.K;
+    float* s_tab = s_dyn;
+    float* s_w = s_tab + sk.S * TF;
+    int* s_idx = reinterpret_cast<int*>(s_w + G * K);
+    float* s_m = reinterpret_cast<float*>(s_idx + G * K);  // [6][G]: v x g, g
+    const int v0 = stage_skin_block(sk, b, tab, TF, w, vec, s_tab, s_w, s_idx);
+    const int lv = threadIdx.x, v = v0 + lv;
+    if (v < sk.N) {
+        const long long vi = (long long)b * sk.N + v;
+        const float3 p = ld3(vpos + 3 * vi), g = ld3(gv + 3 * vi);
+        const float3 pg = cross(p, g);
+        s_m[lv] = pg.x;
+        s_m[G + lv] = pg.y;
+        s_m[2 * G + lv] = pg.z;
+        s_m[3 * G + lv] = g.x;
+        s_m[4 * G + lv] = g.y;
+        s_m[5 * G + lv] = g.z;
+        if constexpr (DQ) {
+            const float4 b4 = sk.base_v4[v];
+            dq_weight_grads(K, s_tab, s_w + lv * K, s_idx + lv * K, make_float3(b4.x, b4.y, b4.z), g, parity);
+        } else {
+            st3(gd + 3 * vi, lbs_grads(sk, B, b, v, s_tab, tab, w, disp, s_w + lv * K, s_idx + lv * K, g, parity));
+        }
+    }
+    __syncthreads();
+    // the weight gradients, left in the place of the joint indices
+    const int n = min(G, sk.N - v0) * K;
+    float* out = gw + ((long long)b * sk.N + v0) * K;
+    if (vec) {
+        for (int e = threadIdx.x; e < n / 4; e += G)
+            reinterpret_cast<float4*>(out)[e] = reinterpret_cast<const float4*>(s_idx)[e];
+    } else {
+        for (int e = threadIdx.x; e < n; e += G) out[e] = __int_as_float(s_idx[e]);
+    }
+    const int lane = threadIdx.x & 31;
+    const int* off = sk.bone_off + (long long)blockIdx.x * (sk.S + 1);
+    for (int s = threadIdx.x >> 5; s < sk.S; s += G >> 5) {  // warp-uniform
+        const int e0 = off[s], e1 = off[s + 1];
+        if (e0 == e1) continue;
+        float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int e = e0 + lane; e < e1; e += 32) {
+            const int2 q = sk.bone_slot[e];
+            const float wk = s_w[q.x];
+#pragma unroll
+            for (int c = 0; c < 6; ++c) a[c] += wk * s_m[c * G + q.y];
+        }
+        const float t = warp_sum8(a, lane);
+        if (lane < 6 && t != 0.f) atomicAdd(mom + ((long long)b * sk.S + s) * 6 + lane, t);
+    }
+}
+
+// dof gradient from the bone moments, a warp per (frame, dof): a dof collects,
+// for every joint it drives, axis . (A_s - c x G_s) (revolute) or axis . G_s
+// (prismatic) of the bones (a lane each) whose kinematic chain contains that
+// joint
+__global__ void k_dof_grad(Skel sk, int B, const float* __restrict__ mom, const float* __restrict__ gpos,
+                           const float* __restrict__ gaxis, float* __restrict__ gdof) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= B * sk.D) return;  // warp-uniform
+    const int b = i / sk.D, d = i % sk.D;
+    float acc = 0.f;
+    for (int e = sk.dof_off[d]; e < sk.dof_off[d + 1]; ++e) {
+        const int j = sk.dof_joint[e];
+        const float3 ax = ld3(gaxis + ((long long)b * sk.J + j) * 3);
+        const float3 c = ld3(gpos + ((long long)b * sk.J + j) * 3);
+        for (int s = lane; s < sk.S; s += 32) {
+            if (!sk.in_chain[s * sk.J + j]) continue;
+            const float* m = mom + ((long long)b * sk.S + s) * 6;
+            const float3 A = make_float3(m[0], m[1], m[2]), G = make_float3(m[3], m[4], m[5]);
+            acc += sk.type[j] == kRevolute ? dot(ax, A - cross(c, G)) : dot(ax, G);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) gdof[i] = acc;
 }
 
 // Node-level skinning of the embedded graph (Pose2EmbeddedGraphCPUOp.cpp:129-300):
@@ -769,12 +831,12 @@ __global__ void k_pose2eg_grad_nodes(Skel sk, int M, const int* __restrict__ nod
     }
 }
 
-// per (frame, dof): sum over the dof's joints and the skinning joints below them
+// per (frame, dof), a warp: sum over the dof's joints and the skinning joints below them (a lane each)
 __global__ void k_pose2eg_grad_dofs(Skel sk, int B, const float* __restrict__ dq, const float* __restrict__ gdq,
                                     const float* __restrict__ gpos, const float* __restrict__ gaxis,
                                     float* __restrict__ gdof) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B * sk.D) return;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= B * sk.D) return;  // warp-uniform
     const int b = i / sk.D, d = i % sk.D;
     float acc = 0.f;
     for (int e = sk.dof_off[d]; e < sk.dof_off[d + 1]; ++e) {
@@ -782,7 +844,7 @@ __global__ void k_pose2eg_grad_dofs(Skel sk, int B, const float* __restrict__ dq
         const float3 ax = ld3(gaxis + ((long long)b * sk.J + j) * 3);
         const float3 c = ld3(gpos + ((long long)b * sk.J + j) * 3);
         float gj = 0.f;
-        for (int s = 0; s < sk.S; ++s) {
+        for (int s = lane; s < sk.S; s += 32) {
             if (!sk.in_chain[s * sk.J + j]) continue;
             const float* q = dq + ((long long)b * sk.S + s) * 8;
             const float4 r = f4(q), tq = f4(q + 4);
@@ -803,7 +865,9 @@ __global__ void k_pose2eg_grad_dofs(Skel sk, int B, const float* __restrict__ dq
         }
         acc += sk.dof_w[e] * gj;
     }
-    gdof[i] = acc;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) gdof[i] = acc;
 }
 
 }  // namespace
@@ -819,7 +883,9 @@ struct hc_skin_s {
     int parity = 1;
     DevBuf parent, type, offset, axis, jscale, dof_off, dof_joint, dof_w, skin_joint, skin_scale, t0inv, in_chain,
         skin_idx, base_v, base_n, base_v4, base_n4;
-    DevBuf joints, params, skin_xf, mom, lbs_xf, gpos, gaxis, dq_ws, gdq;
+    DevBuf joint_off, joint_dof, joint_w, level_off, level_joint, bone_off, bone_slot;
+    DevBuf mom, gpos, gaxis, dq_ws, gdq;
+    int levels = 0, grad_block = 0;
     Skel skel() const {
         Skel s;
         s.J = J;
@@ -844,20 +910,25 @@ struct hc_skin_s {
         s.base_n = base_n.as<float>();
         s.base_v4 = base_v4.as<float4>();
         s.base_n4 = base_n4.as<float4>();
+        s.levels = levels;
+        s.joint_off = joint_off.as<int>();
+        s.joint_dof = joint_dof.as<int>();
+        s.joint_w = joint_w.as<float>();
+        s.level_off = level_off.as<int>();
+        s.level_joint = level_joint.as<int>();
+        s.grad_block = grad_block;
+        s.bone_off = bone_off.as<int>();
+        s.bone_slot = bone_slot.as<int2>();
         return s;
     }
 };
 
-// Opt a kernel in to more than 48 KB of dynamic shared memory, once per device.
+// Opt a kernel in to more than 48 KB of dynamic shared memory (hc_skin_create
+// bounds what a handle needs).
 template <typename K>
 static hc_status skin_allow_smem(K kernel, size_t bytes) {
-    static unsigned long long done = 0;  // one bit per device
     if (bytes <= (48u << 10)) return HC_OK;
-    int dev = 0;
-    HC_CUDA(cudaGetDevice(&dev));
-    if (dev < 64 && (done >> dev & 1ull)) return HC_OK;
     HC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    if (dev < 64) done |= 1ull << dev;
     return HC_OK;
 }
 
@@ -960,6 +1031,56 @@ extern "C" hc_status hc_skin_create(hc_skin* out, int32_t n_joints, const int32_
         UP(base_v4, bv4.data(), bv4.size());
         UP(base_n4, bn4.data(), bn4.size());
     }
+    {
+        // the dof entries by joint (in dof order), and the joints by depth
+        std::vector<int> joff(n_joints + 1, 0), jdof(std::max(E, 1), 0), depth(n_joints, 0);
+        std::vector<float> jw(std::max(E, 1), 0.f);
+        for (int e = 0; e < E; ++e) joff[dof_joint[e] + 1]++;
+        for (int j = 0; j < n_joints; ++j) joff[j + 1] += joff[j];
+        std::vector<int> at(joff.begin(), joff.end() - 1);
+        for (int d = 0; d < n_dofs; ++d)
+            for (int e = dof_offsets[d]; e < dof_offsets[d + 1]; ++e) {
+                jdof[at[dof_joint[e]]] = d;
+                jw[at[dof_joint[e]]++] = dof_weight[e];
+            }
+        for (int j = 0; j < n_joints; ++j) {
+            depth[j] = parent[j] < 0 ? 0 : depth[parent[j]] + 1;
+            h->levels = std::max(h->levels, depth[j] + 1);
+        }
+        std::vector<int> loff(h->levels + 1, 0), lj;
+        for (int l = 0; l < h->levels; ++l) {
+            for (int j = 0; j < n_joints; ++j)
+                if (depth[j] == l) lj.push_back((int)((unsigned)j << 16 | (unsigned)(parent[j] + 1)));
+            loff[l + 1] = (int)lj.size();
+        }
+        UP(joint_off, joff.data(), joff.size());
+        UP(joint_dof, jdof.data(), jdof.size());
+        UP(joint_w, jw.data(), jw.size());
+        UP(level_off, loff.data(), loff.size());
+        UP(level_joint, lj.data(), lj.size());
+    }
+    {
+        // each adjoint block's (vertex, slot) pairs by skinning joint, vertices ascending
+        const int G = h->grad_block = skin_grad_smem(n_skin, 12, k, 256) <= (96u << 10) ? 256 : 128;
+        const int blocks = div_up(n_vertices, G);
+        std::vector<int> off;
+        std::vector<int2> slot((size_t)n_vertices * k);
+        off.reserve((size_t)blocks * (n_skin + 1));
+        std::vector<int> cnt(n_skin + 1);
+        for (int q = 0; q < blocks; ++q) {
+            const int v0 = q * G, v1 = std::min(v0 + G, n_vertices);
+            std::fill(cnt.begin(), cnt.end(), 0);
+            for (long long i = (long long)v0 * k; i < (long long)v1 * k; ++i) cnt[skin_index[i] + 1]++;
+            cnt[0] = v0 * k;
+            for (int s = 0; s < n_skin; ++s) cnt[s + 1] += cnt[s];
+            off.insert(off.end(), cnt.begin(), cnt.end());
+            for (int v = v0; v < v1; ++v)
+                for (int c = 0; c < k; ++c)
+                    slot[cnt[skin_index[(long long)v * k + c]]++] = make_int2((v - v0) * k + c, v - v0);
+        }
+        UP(bone_off, off.data(), off.size());
+        UP(bone_slot, slot.data(), slot.size());
+    }
 #undef UP
     if (st != HC_OK) {
         delete h;
@@ -974,7 +1095,8 @@ extern "C" hc_status hc_skin_destroy(hc_skin h) {
     if (!h) return HC_OK;
     DevBuf* bufs[] = {&h->parent, &h->type, &h->offset, &h->axis, &h->jscale, &h->dof_off, &h->dof_joint, &h->dof_w,
                       &h->skin_joint, &h->skin_scale, &h->t0inv, &h->in_chain, &h->skin_idx, &h->base_v,
-                      &h->base_n, &h->joints, &h->params, &h->skin_xf, &h->mom, &h->lbs_xf, &h->gpos, &h->gaxis,
+                      &h->base_n, &h->joint_off, &h->joint_dof, &h->joint_w, &h->level_off, &h->level_joint,
+                      &h->bone_off, &h->bone_slot, &h->mom, &h->gpos, &h->gaxis,
                       &h->dq_ws, &h->gdq};
     for (DevBuf* b : bufs) b->release();
     delete h;
@@ -988,15 +1110,13 @@ extern "C" hc_status hc_skin_set_parity(hc_skin h, int32_t parity) {
     return HC_OK;
 }
 
-static hc_status fk(hc_skin h, cudaStream_t s, int B, const float* dofs, float* gpos, float* gaxis) {
-    HC_TRY(h->joints.ensure(sizeof(Xf) * (size_t)B * h->J));
-    HC_TRY(h->params.ensure(sizeof(float) * (size_t)B * h->J));
-    HC_TRY(h->skin_xf.ensure(sizeof(Xf) * (size_t)B * h->S));
-    const size_t smem = sizeof(float) * (2 * (size_t)((h->J + 3) & ~3) + 2 * (size_t)((h->E + 3) & ~3)) +
+static hc_status fk(hc_skin h, cudaStream_t s, int B, const float* dofs, float* gpos, float* gaxis, float* dq,
+                    float* xf) {
+    // two transforms and up to two words per joint, two per dof entry
+    const size_t most = sizeof(float) * (2 * (size_t)((h->J + 3) & ~3) + 2 * (size_t)((h->E + 3) & ~3)) +
                         2 * sizeof(Xf) * (size_t)h->J;
-    HC_REQUIRE(smem <= 48 * 1024, "skeleton too large for the kinematics kernel (%d joints)", h->J);
-    k_fk<<<B, 128, smem, s>>>(h->skel(), B, dofs, h->joints.as<Xf>(), gpos, gaxis, h->skin_xf.as<Xf>(),
-                              h->params.as<float>());
+    HC_REQUIRE(most <= 48 * 1024, "skeleton too large for the kinematics kernel (%d joints)", h->J);
+    k_fk<<<B, kFkBlock, (2 * sizeof(Xf) + sizeof(int)) * (size_t)h->J, s>>>(h->skel(), dofs, gpos, gaxis, dq, xf);
     HC_CHECK_LAUNCH();
     return HC_OK;
 }
@@ -1004,11 +1124,7 @@ static hc_status fk(hc_skin h, cudaStream_t s, int B, const float* dofs, float* 
 extern "C" hc_status hc_skin_reserve(hc_skin h, int32_t batch) {
     clear_error();
     HC_REQUIRE(h && batch > 0, "invalid handle or batch");
-    HC_TRY(h->joints.ensure(sizeof(Xf) * (size_t)batch * h->J));
-    HC_TRY(h->params.ensure(sizeof(float) * (size_t)batch * h->J));
-    HC_TRY(h->skin_xf.ensure(sizeof(Xf) * (size_t)batch * h->S));
     HC_TRY(h->mom.ensure(sizeof(float) * 6 * (size_t)batch * h->S));
-    HC_TRY(h->lbs_xf.ensure(sizeof(float) * 12 * (size_t)batch * h->S));
     HC_TRY(h->gpos.ensure(sizeof(float) * 3 * (size_t)batch * h->J));
     HC_TRY(h->gaxis.ensure(sizeof(float) * 3 * (size_t)batch * h->J));
     return HC_OK;
@@ -1025,10 +1141,7 @@ extern "C" hc_status hc_dq_skinning_forward(hc_skin h, void* stream, int32_t bat
                    global_joint_position && global_joint_axis && dual_quaternions,
                "NULL input/output pointer");
     cudaStream_t s = (cudaStream_t)stream;
-    HC_TRY(fk(h, s, batch, dofs, global_joint_position, global_joint_axis));
-    const int BS = batch * h->S;
-    k_dq_from_xf<<<div_up(BS, 128), 128, 0, s>>>(BS, h->skin_xf.as<Xf>(), dual_quaternions);
-    HC_CHECK_LAUNCH();
+    HC_TRY(fk(h, s, batch, dofs, global_joint_position, global_joint_axis, dual_quaternions, nullptr));
     HC_REQUIRE(batch <= 65535, "too many frames in one call (%d)", batch);
     HC_TRY(skin_allow_smem(k_dq_skin, skin_block_smem(h->S, 8, h->K, kSkinBlock)));
     k_dq_skin<<<dim3(div_up(h->N, kSkinBlock), batch), kSkinBlock, skin_block_smem(h->S, 8, h->K, kSkinBlock), s>>>(
@@ -1038,14 +1151,22 @@ extern "C" hc_status hc_dq_skinning_forward(hc_skin h, void* stream, int32_t bat
     return HC_OK;
 }
 
-static hc_status dof_grad(hc_skin h, cudaStream_t s, int B, const float* vpos, const float* gv, const float* w,
-                          const float* gpos, const float* gaxis, float* gdof) {
+// The skinning adjoint's two launches: per vertex block the weight (and, LBS,
+// displacement) gradients and the bone moments, then the dof gradient.
+template <bool DQ>
+static hc_status skin_grad(hc_skin h, cudaStream_t s, int B, const float* vpos, const float* gv, const float* tab,
+                           const float* w, const float* disp, const float* gpos, const float* gaxis, float* gdof,
+                           float* gw, float* gd) {
+    HC_REQUIRE(B <= 65535, "too many frames in one call (%d)", B);
     HC_TRY(h->mom.ensure(sizeof(float) * 6 * (size_t)B * h->S));
     HC_CUDA(cudaMemsetAsync(h->mom.ptr, 0, sizeof(float) * 6 * (size_t)B * h->S, s));
-    const dim3 grid(div_up(h->N, 256), B);
-    k_bone_moments<<<grid, 256, sizeof(float) * 6 * h->S, s>>>(h->skel(), vpos, gv, w, h->mom.as<float>());
+    const size_t smem = skin_grad_smem(h->S, DQ ? 8 : 12, h->K, h->grad_block);
+    HC_TRY(skin_allow_smem(k_skin_grad<DQ>, smem));
+    const int vec = slots_by_four(h, w) && ((uintptr_t)gw & 15) == 0;
+    k_skin_grad<DQ><<<dim3(div_up(h->N, h->grad_block), B), h->grad_block, smem, s>>>(
+        h->skel(), B, tab, w, vpos, gv, disp, h->parity, vec, gw, gd, h->mom.as<float>());
     HC_CHECK_LAUNCH();
-    k_dof_grad<<<div_up(B * h->D, 128), 128, 0, s>>>(h->skel(), B, h->mom.as<float>(), gpos, gaxis, gdof);
+    k_dof_grad<<<div_up(32ll * B * h->D, 128), 128, 0, s>>>(h->skel(), B, h->mom.as<float>(), gpos, gaxis, gdof);
     HC_CHECK_LAUNCH();
     return HC_OK;
 }
@@ -1062,12 +1183,9 @@ extern "C" hc_status hc_dq_skinning_backward(hc_skin h, void* stream, int32_t ba
                    global_joint_axis && dual_quaternions && skinning_weights && dofs_grad && skinning_weights_grad,
                "NULL input/output pointer");
     cudaStream_t s = (cudaStream_t)stream;
-    HC_TRY(dof_grad(h, s, batch, skinned_vertex_positions, skinned_vertex_positions_grad, skinning_weights,
-                    global_joint_position, global_joint_axis, dofs_grad));
-    const long long n = (long long)batch * h->N * h->K;
-    k_dq_weight_grad<<<div_up(n, 128), 128, 0, s>>>(h->skel(), batch, dual_quaternions, skinning_weights,
-                                                    skinned_vertex_positions_grad, h->parity, skinning_weights_grad);
-    HC_CHECK_LAUNCH();
+    HC_TRY(skin_grad<true>(h, s, batch, skinned_vertex_positions, skinned_vertex_positions_grad, dual_quaternions,
+                           skinning_weights, nullptr, global_joint_position, global_joint_axis, dofs_grad,
+                           skinning_weights_grad, nullptr));
     return HC_OK;
 }
 
@@ -1082,10 +1200,7 @@ extern "C" hc_status hc_lb_skinning_forward(hc_skin h, void* stream, int32_t bat
                    global_joint_position && global_joint_axis && transformation,
                "NULL input/output pointer");
     cudaStream_t s = (cudaStream_t)stream;
-    HC_TRY(fk(h, s, batch, dofs, global_joint_position, global_joint_axis));
-    const int BS = batch * h->S;
-    k_xf_to_lbs<<<div_up(BS, 128), 128, 0, s>>>(BS, h->skin_xf.as<Xf>(), transformation);
-    HC_CHECK_LAUNCH();
+    HC_TRY(fk(h, s, batch, dofs, global_joint_position, global_joint_axis, nullptr, transformation));
     HC_REQUIRE(batch <= 65535, "too many frames in one call (%d)", batch);
     HC_TRY(skin_allow_smem(k_lbs_skin, skin_block_smem(h->S, 12, h->K, kSkinBlock)));
     k_lbs_skin<<<dim3(div_up(h->N, kSkinBlock), batch), kSkinBlock, skin_block_smem(h->S, 12, h->K, kSkinBlock), s>>>(
@@ -1110,16 +1225,9 @@ extern "C" hc_status hc_lb_skinning_backward(hc_skin h, void* stream, int32_t ba
                "NULL input/output pointer");
     HC_REQUIRE(h->parity || displacement, "the exact LBS weight gradient needs the displacement input");
     cudaStream_t s = (cudaStream_t)stream;
-    HC_TRY(dof_grad(h, s, batch, skinned_vertex_positions, skinned_vertex_positions_grad, skinning_weights,
-                    global_joint_position, global_joint_axis, dofs_grad));
-    const long long n = (long long)batch * h->N * h->K;
-    k_lbs_weight_grad<<<div_up(n, 128), 128, 0, s>>>(h->skel(), batch, transformation, displacement,
-                                                     skinned_vertex_positions_grad, h->parity, skinning_weights_grad);
-    HC_CHECK_LAUNCH();
-    k_lbs_disp_grad<<<div_up((long long)batch * h->N, 128), 128, 0, s>>>(
-        h->skel(), batch, transformation, skinning_weights, skinned_vertex_positions_grad, h->parity,
-        displacement_grad);
-    HC_CHECK_LAUNCH();
+    HC_TRY(skin_grad<false>(h, s, batch, skinned_vertex_positions, skinned_vertex_positions_grad, transformation,
+                            skinning_weights, displacement, global_joint_position, global_joint_axis, dofs_grad,
+                            skinning_weights_grad, displacement_grad));
     return HC_OK;
 }
 
@@ -1135,10 +1243,7 @@ extern "C" hc_status hc_pose2eg_forward(hc_skin h, void* stream, int32_t batch, 
     cudaStream_t s = (cudaStream_t)stream;
     HC_TRY(h->gpos.ensure(sizeof(float) * 3 * (size_t)batch * h->J));
     HC_TRY(h->gaxis.ensure(sizeof(float) * 3 * (size_t)batch * h->J));
-    HC_TRY(fk(h, s, batch, dofs, h->gpos.as<float>(), h->gaxis.as<float>()));
-    const int BS = batch * h->S;
-    k_dq_from_xf<<<div_up(BS, 128), 128, 0, s>>>(BS, h->skin_xf.as<Xf>(), dual_quaternions);
-    HC_CHECK_LAUNCH();
+    HC_TRY(fk(h, s, batch, dofs, h->gpos.as<float>(), h->gaxis.as<float>(), dual_quaternions, nullptr));
     k_pose2eg<<<div_up((long long)batch * n_nodes, 128), 128, 0, s>>>(h->skel(), batch, n_nodes, node_vertex,
                                                                        dual_quaternions, vertex_weights,
                                                                        nodes_skinned_translation,
@@ -1162,10 +1267,7 @@ extern "C" hc_status hc_pose2eg_backward(hc_skin h, void* stream, int32_t batch,
     HC_TRY(hc_skin_reserve(h, batch));
     HC_TRY(h->dq_ws.ensure(sizeof(float) * 8 * (size_t)batch * h->S));
     HC_TRY(h->gdq.ensure(sizeof(float) * 8 * (size_t)batch * h->S));
-    HC_TRY(fk(h, s, batch, dofs, h->gpos.as<float>(), h->gaxis.as<float>()));
-    const int BS = batch * h->S;
-    k_dq_from_xf<<<div_up(BS, 128), 128, 0, s>>>(BS, h->skin_xf.as<Xf>(), h->dq_ws.as<float>());
-    HC_CHECK_LAUNCH();
+    HC_TRY(fk(h, s, batch, dofs, h->gpos.as<float>(), h->gaxis.as<float>(), h->dq_ws.as<float>(), nullptr));
     const size_t smem = sizeof(float) * 8 * (size_t)h->S * 4;  // 4 warps
     HC_REQUIRE(smem <= 48 * 1024, "too many skinning joints (%d)", h->S);
     HC_CUDA(cudaMemsetAsync(h->gdq.ptr, 0, sizeof(float) * 8 * (size_t)batch * h->S, s));
@@ -1174,7 +1276,7 @@ extern "C" hc_status hc_pose2eg_backward(hc_skin h, void* stream, int32_t batch,
                                                   vertex_weights, nodes_skinned_translation_grad,
                                                   nodes_skinned_rotation_grad, h->gdq.as<float>());
     HC_CHECK_LAUNCH();
-    k_pose2eg_grad_dofs<<<div_up(batch * h->D, 128), 128, 0, s>>>(h->skel(), batch, h->dq_ws.as<float>(),
+    k_pose2eg_grad_dofs<<<div_up(32ll * batch * h->D, 128), 128, 0, s>>>(h->skel(), batch, h->dq_ws.as<float>(),
                                                                   h->gdq.as<float>(), h->gpos.as<float>(),
                                                                   h->gaxis.as<float>(), dofs_grad);
     HC_CHECK_LAUNCH();
