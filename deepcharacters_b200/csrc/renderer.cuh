@@ -308,6 +308,62 @@ __device__ __forceinline__ bool footprint_overlaps(const Footprint& fp, int x0, 
     return true;
 }
 
+// bits lo..hi of a 32-bit mask (empty when hi < lo)
+__device__ __forceinline__ unsigned bit_range(int lo, int hi) {
+    return hi < lo ? 0u : ((2u << hi) - 1u) & ~((1u << lo) - 1u);
+}
+
+// Rows of a 32 x 32 bit matrix (one per lane) to columns: lane i ends with
+// bit j = lane j's bit i.  Five rounds of block swaps.
+__device__ __forceinline__ unsigned transpose_bits(unsigned x, int lane) {
+    unsigned m = 0x0000ffffu;
+#pragma unroll
+    for (int j = 16; j > 0; j >>= 1) {
+        const unsigned y = __shfl_xor_sync(0xffffffffu, x, j);
+        x = (lane & j) ? ((x & ~m) | ((y >> j) & m)) : ((x & m) | ((y << j) & ~m));
+        m ^= m << (j >> 1);
+    }
+    return x;
+}
+
+// The pixels of a warp (RW rows of TS pixels; the first pixel is (X0, Y0))
+// that a triangle can cover: its bounding box (x01, y01: first | last << 16)
+// exactly, and its footprint edges (a, b, c) from the x interval that each
+// leaves of a row, widened by kMaskSlack px in the edge's value (the float
+// error of that value is below 0.03 px in the admitted coordinate range, and
+// the reciprocal's far below that).  Bit r * TS + x is pixel (X0 + x, Y0 + r).
+constexpr float kMaskSlack = 0.0625f;
+
+template <int TS, int RW>
+__device__ __forceinline__ unsigned pixel_mask(float a0, float b0, float c0, float a1, float b1, float c1, float a2,
+                                               float b2, float c2, int x01, int y01, int X0, int Y0) {
+    const int bx0 = max((x01 & 0xffff) - X0, 0), bx1 = min((x01 >> 16) - X0, TS - 1);
+    const int by0 = (y01 & 0xffff) - Y0, by1 = (y01 >> 16) - Y0;
+    if (bx1 < bx0 || by1 < 0 || by0 >= RW) return 0u;
+    const float fx = X0 + 0.5f, fy = Y0 + 0.5f;
+    const float ea[3] = {a0, a1, a2}, eb[3] = {b0, b1, b2}, ec[3] = {c0, c1, c2};
+    float s[3], inv[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        s[k] = ea[k] * fx + eb[k] * fy + ec[k] + kMaskSlack;
+        inv[k] = fabsf(ea[k]) > 1e-6f ? __fdividef(-1.f, ea[k]) : 0.f;  // 0: the edge leaves every x
+    }
+    unsigned mask = 0u;
+#pragma unroll
+    for (int r = 0; r < RW; ++r) {
+        float lo = (float)bx0, hi = (float)bx1;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float x = (s[k] + eb[k] * r) * inv[k];  // where the edge's value is -kMaskSlack
+            lo = fmaxf(lo, inv[k] < 0.f ? x : lo);
+            hi = fminf(hi, inv[k] > 0.f ? x : hi);
+        }
+        const int xl = __float2int_ru(lo), xh = __float2int_rd(hi);
+        if (r >= by0 && r <= by1) mask |= bit_range(xl, xh) << (r * TS);
+    }
+    return mask;
+}
+
 // Bilinear texture lookup at texel coordinates (x, y), texel centres at
 // integer + 0.5, clamp-to-edge addressing: the four texel offsets (floats,
 // x3 channels) and weights.

@@ -553,63 +553,6 @@ __device__ __forceinline__ bool raster_hit_below(float3 ro_s, float3 dir, const 
     return (a / denom >= -0.001f) && (b / denom >= -0.001f) && (a / denom <= 1.001f) && (b / denom <= 1.001f);
 }
 
-// bits lo..hi of a 32-bit mask (empty when hi < lo)
-__device__ __forceinline__ unsigned bit_range(int lo, int hi) {
-    return hi < lo ? 0u : ((2u << hi) - 1u) & ~((1u << lo) - 1u);
-}
-
-// Rows of a 32 x 32 bit matrix (one per lane) to columns: lane i ends with
-// bit j = lane j's bit i.  Five rounds of block swaps.
-__device__ __forceinline__ unsigned transpose_bits(unsigned x, int lane) {
-    unsigned m = 0x0000ffffu;
-#pragma unroll
-    for (int j = 16; j > 0; j >>= 1) {
-        const unsigned y = __shfl_xor_sync(0xffffffffu, x, j);
-        x = (lane & j) ? ((x & ~m) | ((y >> j) & m)) : ((x & m) | ((y << j) & ~m));
-        m ^= m << (j >> 1);
-    }
-    return x;
-}
-
-// The pixels of a warp (RW rows of TS pixels; the first pixel is (X0, Y0))
-// that a triangle can hit: its bounding box exactly, and its footprint from
-// the x interval that each edge leaves of a row, widened by kMaskSlack px in
-// the edge's value (the float error of that value is below 0.03 px in the
-// admitted coordinate range, and the reciprocal's far below that).
-// Bit r * TS + x is pixel (X0 + x, Y0 + r).
-constexpr float kMaskSlack = 0.0625f;
-
-template <int TS, int RW>
-__device__ __forceinline__ unsigned pixel_mask(const float4* rec, int X0, int Y0) {
-    const float4 e01 = rec[0], e2c = rec[1], q = rec[2];
-    const int x01 = __float_as_int(q.z), y01 = __float_as_int(q.w);
-    const int bx0 = max((x01 & 0xffff) - X0, 0), bx1 = min((x01 >> 16) - X0, TS - 1);
-    const int by0 = (y01 & 0xffff) - Y0, by1 = (y01 >> 16) - Y0;
-    if (bx1 < bx0 || by1 < 0 || by0 >= RW) return 0u;
-    const float fx = X0 + 0.5f, fy = Y0 + 0.5f;
-    const float ea[3] = {e01.x, e01.z, e2c.x}, eb[3] = {e01.y, e01.w, e2c.y}, ec[3] = {e2c.z, e2c.w, q.x};
-    float s[3], inv[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        s[k] = ea[k] * fx + eb[k] * fy + ec[k] + kMaskSlack;
-        inv[k] = fabsf(ea[k]) > 1e-6f ? __fdividef(-1.f, ea[k]) : 0.f;  // 0: the edge leaves every x
-    }
-    unsigned mask = 0u;
-#pragma unroll
-    for (int r = 0; r < RW; ++r) {
-        float lo = (float)bx0, hi = (float)bx1;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float x = (s[k] + eb[k] * r) * inv[k];  // where the edge's value is -kMaskSlack
-            lo = fmaxf(lo, inv[k] < 0.f ? x : lo);
-            hi = fminf(hi, inv[k] > 0.f ? x : hi);
-        }
-        const int xl = (int)ceilf(lo), xh = (int)floorf(hi);
-        if (r >= by0 && r <= by1) mask |= bit_range(xl, xh) << (r * TS);
-    }
-    return mask;
-}
-
 // TIES: the call asked for the per-pixel count of hits at the winning depth
 // (diagnostics); without it the count is compiled out, which frees a register
 // of the scan and shortens its updates
@@ -767,8 +710,12 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
             const unsigned bb = nf < cnt ? (s_ord[s0 + nf] & 0x7fffffffu) >> SB : kNoKey;
             if (!__any_sync(0xffffffffu, valid && min(bf, bb) <= best_d)) continue;
             unsigned w = 0u;
-            if (lane < cnt) w = pixel_mask<TS, RW>(s_rec + (s_ord[s0 + lane] & (CHUNK - 1)) * kRec, tx * TS,
-                                                     ty * TS + warp * RW);
+            if (lane < cnt) {
+                const float4* rec = s_rec + (s_ord[s0 + lane] & (CHUNK - 1)) * kRec;
+                const float4 ea = rec[0], eb = rec[1], q = rec[2];
+                w = pixel_mask<TS, RW>(ea.x, ea.y, eb.z, ea.z, ea.w, eb.w, eb.x, eb.y, q.x, __float_as_int(q.z),
+                                       __float_as_int(q.w), tx * TS, ty * TS + warp * RW);
+            }
             w = transpose_bits(w, lane);
             if (!valid) w = 0u;
             const unsigned fm = nf == 32 ? 0xffffffffu : (1u << nf) - 1u;  // the front faces' bits

@@ -595,13 +595,22 @@ __global__ void __launch_bounds__(256, 4) k_cov_bin_list(int N, int F, const int
 }
 
 // Persistent CTAs over the tiles that received entries (the binning pass
-// lists them), one thread per pixel of the current tile: a pixel stops at the
-// first binned triangle that covers it, the tile at the chunk after which all
-// its pixels are covered.
+// lists them), one thread per pixel of the current tile.  A chunk of 64 records
+// is copied to shared memory, five consecutive threads per 80-byte record.
+// Each warp turns 32 records at a time into per-pixel lists, as the tile
+// resolve does: a lane forms the mask of the warp's uncovered pixels that its
+// triangle can cover, the bit matrix is transposed, and a pixel tests only its
+// own records until one covers it (walked in lockstep, a warp paid every
+// record that one of its open pixels still needed).  A warp stops when all its
+// pixels are covered, the tile at the chunk after which all are.
+// Bound by instruction issue.  16 views of 81,920 triangles at 1024^2: 552 ->
+// 382 us.
 __global__ void __launch_bounds__(kCovTile* kCovTile) k_cov_tile(int F, long long n_keys, CovBins cb,
                                                                   const __grid_constant__ ImgLayout L) {
-    __shared__ CovTileTri s_t[kCovTile * kCovTile];
-    const int listed = *cb.n_tiles;
+    constexpr int NT = kCovTile * kCovTile, RW = 32 / kCovTile, kRec = sizeof(CovTileTri) / 16;
+    static_assert(sizeof(CovTileTri) == 16 * kRec, "records are copied in 16-byte pieces");
+    __shared__ __align__(16) CovTileTri s_t[NT];
+    const int listed = *cb.n_tiles, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int it = blockIdx.x; it < listed; it += gridDim.x) {
         const long long key = cb.tiles[it];
         const int n = min(cb.count[key], kCovCap);
@@ -613,17 +622,40 @@ __global__ void __launch_bounds__(kCovTile* kCovTile) k_cov_tile(int F, long lon
         const bool valid = px < vi.W && py < vi.H;
         unsigned char* pix = cb.cover + vi.pix + (long long)py * vi.W + px;
         bool covered = !valid || *pix;
-        const CovTileTri* R = cb.rec + (long long)view * F;
+        const bool was = covered;
+        const float4* R = reinterpret_cast<const float4*>(cb.rec + (long long)view * F);
+        const int* bin = cb.bins + key * kCovCap;
         // every chunk starts with a barrier (so does the next tile: the staged
         // records of this one are no longer read there)
-        for (int base = 0; base < n; base += kCovTile * kCovTile) {
-            const int m = min(kCovTile * kCovTile, n - base);
+        for (int base = 0; base < n; base += NT) {
+            const int m = min(NT, n - base);
             if (__syncthreads_and(covered)) break;  // every pixel of the tile is covered: stop staging
-            if ((int)threadIdx.x < m) s_t[threadIdx.x] = R[cb.bins[key * kCovCap + base + threadIdx.x]];
+            for (int i = threadIdx.x; i < m * kRec; i += NT) {
+                const int r = i / kRec, c = i - r * kRec;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(
+                                 (unsigned)__cvta_generic_to_shared(reinterpret_cast<float4*>(s_t) + i)),
+                             "l"(R + (long long)bin[base + r] * kRec + c));
+            }
+            asm volatile("cp.async.wait_all;\n" ::: "memory");
             __syncthreads();
-            for (int j = 0; j < m && !covered; ++j) covered = cover_record_test(s_t[j], px, py);
+            for (int s0 = 0; s0 < m; s0 += 32) {  // warp-uniform
+                const unsigned open = __ballot_sync(0xffffffffu, !covered);
+                if (!open) break;
+                unsigned w = 0u;
+                if (s0 + lane < m) {
+                    const CovTileTri& e = s_t[s0 + lane];
+                    w = open & pixel_mask<kCovTile, RW>(e.e0.x, e.e0.y, e.e0.z, e.e0.w, e.e1.x, e.e1.y, e.e1.z, e.e1.w,
+                                                        e.e2.x, e.bb.x, e.bb.y, tx * kCovTile,
+                                                        ty * kCovTile + warp * RW);
+                }
+                w = transpose_bits(w, lane);
+                while (w && !covered) {
+                    covered = cover_record_test(s_t[s0 + __ffs(w) - 1], px, py);
+                    w &= w - 1u;
+                }
+            }
         }
-        if (valid && covered && !*pix) *pix = 1;
+        if (covered && !was) *pix = 1;
     }
 }
 
