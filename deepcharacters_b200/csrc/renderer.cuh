@@ -308,9 +308,11 @@ __device__ __forceinline__ bool footprint_overlaps(const Footprint& fp, int x0, 
     return true;
 }
 
-// bits lo..hi of a 32-bit mask (empty when hi < lo)
-__device__ __forceinline__ unsigned bit_range(int lo, int hi) {
-    return hi < lo ? 0u : ((2u << hi) - 1u) & ~((1u << lo) - 1u);
+// bit n alone; 0 for n = 32 (the hardware shift saturates)
+__device__ __forceinline__ unsigned bit_at(unsigned n) {
+    unsigned r;
+    asm("shl.b32 %0, 1, %1;" : "=r"(r) : "r"(n));
+    return r;
 }
 
 // Rows of a 32 x 32 bit matrix (one per lane) to columns: lane i ends with
@@ -342,11 +344,17 @@ __device__ __forceinline__ unsigned pixel_mask(float a0, float b0, float c0, flo
     if (bx1 < bx0 || by1 < 0 || by0 >= RW) return 0u;
     const float fx = X0 + 0.5f, fy = Y0 + 0.5f;
     const float ea[3] = {a0, a1, a2}, eb[3] = {b0, b1, b2}, ec[3] = {c0, c1, c2};
-    float s[3], inv[3];
+    // where edge k's value is -kMaskSlack in row r: x0 + r dx; the pixels right
+    // of it (a > 0) or left of it remain, all of them where a is nearly 0
+    float x0[3], dx[3];
+    bool right[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        s[k] = ea[k] * fx + eb[k] * fy + ec[k] + kMaskSlack;
-        inv[k] = fabsf(ea[k]) > 1e-6f ? __fdividef(-1.f, ea[k]) : 0.f;  // 0: the edge leaves every x
+        const float s = ea[k] * fx + eb[k] * fy + ec[k] + kMaskSlack, inv = __fdividef(-1.f, ea[k]);
+        const bool bounds = fabsf(ea[k]) > 1e-6f;
+        right[k] = !bounds || ea[k] > 0.f;
+        x0[k] = bounds ? s * inv : -1.f;
+        dx[k] = bounds ? eb[k] * inv : 0.f;
     }
     unsigned mask = 0u;
 #pragma unroll
@@ -354,12 +362,15 @@ __device__ __forceinline__ unsigned pixel_mask(float a0, float b0, float c0, flo
         float lo = (float)bx0, hi = (float)bx1;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const float x = (s[k] + eb[k] * r) * inv[k];  // where the edge's value is -kMaskSlack
-            lo = fmaxf(lo, inv[k] < 0.f ? x : lo);
-            hi = fminf(hi, inv[k] > 0.f ? x : hi);
+            const float x = x0[k] + r * dx[k];
+            if (right[k]) lo = fmaxf(lo, x);
+            else hi = fminf(hi, x);
         }
-        const int xl = __float2int_ru(lo), xh = __float2int_rd(hi);
-        if (r >= by0 && r <= by1) mask |= bit_range(xl, xh) << (r * TS);
+        // ceil(lo) and floor(hi) + 1 by directed rounding at 2^23 (full-rate
+        // additions; conversions run at a quarter of their rate)
+        const unsigned l = __float_as_uint(__fadd_ru(fminf(lo, (float)TS), 8388608.f)) & 63u;
+        const unsigned h = max(__float_as_uint(__fadd_rd(fmaxf(hi, -1.f), 8388609.f)) & 63u, l);
+        if (r >= by0 && r <= by1) mask |= (bit_at(h) - bit_at(l)) << (r * TS);
     }
     return mask;
 }

@@ -188,19 +188,21 @@ struct CamImg {
     int W, H;          // image size (the distance image's U, V)
     int tiles_x;       // 8x8 coverage tiles per row
     int gx, gy;        // boundary-grid cells (edge: the search radius)
+    int words_x;       // needed-tile words (8x8 coverage tiles each) per row
     long long pix;     // first pixel in the frame
     long long tile;    // first coverage tile in the frame
     long long cell;    // first grid cell in the frame
+    long long word;    // first needed-tile word in the frame
 };
 struct ImgLayout {
     int n_cam;
-    long long P, T, G;  // pixels, coverage tiles, grid cells of a frame
+    long long P, T, G, Q;  // pixels, coverage tiles, grid cells, needed-tile words of a frame
     FastDiv fd_T;       // division by T
     CamImg cam[kMaxLayoutCams];
 };
 struct ViewImg {       // one view's image in the call's buffers
-    int W, H, tiles_x, gx, gy;
-    long long pix, tile, cell;
+    int W, H, tiles_x, gx, gy, words_x;
+    long long pix, tile, cell, word;
 };
 
 __device__ __forceinline__ ViewImg view_img(const ImgLayout& L, int view) {
@@ -215,6 +217,8 @@ __device__ __forceinline__ ViewImg view_img(const ImgLayout& L, int view) {
     v.pix = b * L.P + k.pix;
     v.tile = b * L.T + k.tile;
     v.cell = b * L.G + k.cell;
+    v.words_x = k.words_x;
+    v.word = b * L.Q + k.word;
     return v;
 }
 
@@ -228,12 +232,12 @@ __device__ __forceinline__ int view_of_tile(const ImgLayout& L, long long key, i
     return (int)b * L.n_cam + c;
 }
 
-__device__ __forceinline__ void cover_tri(int view, int f, int N, int W, int H, const int* __restrict__ faces,
-                                          const float2* __restrict__ p2d, CoverTri& t) {
+__device__ __forceinline__ void cover_tri(int view, int N, int W, int H, int3 id, const float2* __restrict__ p2d,
+                                          CoverTri& t) {
     const float2* P = p2d + (long long)view * N;
-    t.a = P[faces[3 * f]];
-    t.b = P[faces[3 * f + 1]];
-    t.c = P[faces[3 * f + 2]];
+    t.a = P[id.x];
+    t.b = P[id.y];
+    t.c = P[id.z];
     const float2 a = t.a, b = t.b, c = t.c;
     t.x0 = (int)fmaxf(fminf(a.x, fminf(b.x, c.x)) - 0.5f, 0);
     t.y0 = (int)fmaxf(fminf(a.y, fminf(b.y, c.y)) - 0.5f, 0);
@@ -308,8 +312,7 @@ struct CovBins {
     int* bins;         // [tiles of the call * kCovCap]
     CovTileTri* rec;   // [V*F]
     unsigned char* cover;       // coverage image, the layout's pixels
-    const unsigned char* need;  // [tiles of the call] tiles with a pixel still open (NULL: every tile)
-    const int* need_sum;        // [tiles of the call] per view: inclusive 2-D prefix sums of need (NULL: none)
+    const unsigned long long* need;  // tiles with a pixel still open: a word per 8x8 tiles of a view, bit 8 row + column
     int* tiles;                 // [tiles of the call]: the tiles that received an entry, in no order
     int* n_tiles;               // their number (cleared before the binning pass)
     int* items;                 // [V*F]: hinted binning, the (view * F + triangle) pairs left by the cull
@@ -324,14 +327,20 @@ __device__ __forceinline__ int cov_claim(const CovBins& cb, long long key) {
     return slot;
 }
 
-// needed tiles of a view in the tile box [tx0, tx1] x [ty0, ty1] (inclusive),
-// from the view's 2-D prefix sums S (row-major, tiles_x per row)
-__device__ __forceinline__ int need_in_box(const int* S, int tiles_x, int tx0, int ty0, int tx1, int ty1) {
-    const int a = S[ty1 * tiles_x + tx1];
-    const int b = ty0 > 0 ? S[(ty0 - 1) * tiles_x + tx1] : 0;
-    const int c = tx0 > 0 ? S[ty1 * tiles_x + tx0 - 1] : 0;
-    const int d = ty0 > 0 && tx0 > 0 ? S[(ty0 - 1) * tiles_x + tx0 - 1] : 0;
-    return a - b - c + d;
+// the tiles of word (wx, wy) inside the tile box [tx0, tx1] x [ty0, ty1] (inclusive; the word touches it)
+__device__ __forceinline__ unsigned long long word_box(int wx, int wy, int tx0, int ty0, int tx1, int ty1) {
+    const int x0 = max(tx0 - 8 * wx, 0), x1 = min(tx1 - 8 * wx, 7), y0 = max(ty0 - 8 * wy, 0), y1 = min(ty1 - 8 * wy, 7);
+    const unsigned long long row = (2ull << x1) - (1ull << x0);
+    return row * 0x0101010101010101ull & (~0ull >> (56 - 8 * y1)) & (~0ull << (8 * y0));
+}
+
+// a needed tile of a view lies in the box
+__device__ __forceinline__ bool need_in_box(const unsigned long long* need, const ViewImg& vi, int tx0, int ty0, int tx1,
+                                            int ty1) {
+    for (int wy = ty0 >> 3; wy <= ty1 >> 3; ++wy)
+        for (int wx = tx0 >> 3; wx <= tx1 >> 3; ++wx)
+            if (need[vi.word + (long long)wy * vi.words_x + wx] & word_box(wx, wy, tx0, ty0, tx1, ty1)) return true;
+    return false;
 }
 
 // the pixels of one tile that a triangle covers, written at once (a pair
@@ -360,12 +369,41 @@ __device__ void cov_sweep(const CovBins& cb, const ViewImg& vi, int tile, const 
 // window that holds the pixel.
 constexpr unsigned char kPending = 2;
 
+// the flag of a vertex whose window around (u, v) has the pixels `open` left
+// (bit 3 j + k: row j, column k); pending windows are written and marked
+__device__ __forceinline__ unsigned char window_flag(unsigned open, int u, int v, const ViewImg& vi,
+                                                     unsigned char* __restrict__ cover,
+                                                     unsigned long long* __restrict__ need) {
+    if (!open) return 0;
+    const int tx0 = (u - 1) / kCovTile, ty0 = (v - 1) / kCovTile;
+    unsigned tiles = 0;  // bit 2 j + k: tile (tx0 + k, ty0 + j) holds an open pixel
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int rr = v - 1 + j, c = u - 1 + k;
+            const bool op = (open >> (3 * j + k)) & 1u;
+            cover[vi.pix + (long long)rr * vi.W + c] = op ? 0 : 1;
+            if (op) tiles |= 1u << (2 * (rr / kCovTile - ty0) + (c / kCovTile - tx0));
+        }
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        if (!((tiles >> t) & 1u)) continue;
+        const int tx = tx0 + (t & 1), ty = ty0 + (t >> 1);
+        unsigned long long* w = need + vi.word + (long long)(ty >> 3) * vi.words_x + (tx >> 3);
+        const unsigned long long bit = 1ull << (8 * (ty & 7) + (tx & 7));
+        // most marks repeat an earlier one: read at L2, where the atomics act
+        if (!(__ldcg(w) & bit)) atomicOr(w, bit);
+    }
+    return kPending;
+}
+
 // (6 CTAs of 256 per SM: the kernel waits on dependent gathers, and more
 // resident warps hide them better than the registers they cost)
 __global__ void __launch_bounds__(256, 6) k_bnd_hint(long long n, int N, int F, const __grid_constant__ ImgLayout L,
                            const float2* __restrict__ p2d, const int* __restrict__ faces,
                            const int* __restrict__ hint, unsigned char* __restrict__ cover,
-                           unsigned char* __restrict__ need, unsigned char* __restrict__ out) {
+                           unsigned long long* __restrict__ need, unsigned char* __restrict__ out) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int view = (int)(i / N);
@@ -387,99 +425,49 @@ __global__ void __launch_bounds__(256, 6) k_bnd_hint(long long n, int N, int F, 
                 bool cov = false;
                 if (f >= 0 && f < F) {
                     if (f != last) {  // neighbouring pixels mostly share their hint face
-                        cover_tri(view, f, N, W, H, faces, p2d, t);
+                        cover_tri(view, N, W, H, make_int3(faces[3 * f], faces[3 * f + 1], faces[3 * f + 2]), p2d, t);
                         last = f;
                     }
                     cov = c >= t.x0 && c <= t.x1 && rr >= t.y0 && rr <= t.y1 && cover_test(t, c + 0.5f, rr + 0.5f);
                 }
                 open |= (cov ? 0u : 1u) << (3 * j + k);
             }
-        if (open) {  // only a pending window's pixels are read again
-            r = kPending;
-#pragma unroll
-            for (int j = 0; j < 3; ++j)
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const int rr = v - 1 + j, c = u - 1 + k;
-                    const bool op = (open >> (3 * j + k)) & 1u;
-                    cover[vi.pix + (long long)rr * W + c] = op ? 0 : 1;
-                    if (op) need[vi.tile + (long long)(rr / kCovTile) * vi.tiles_x + c / kCovTile] = 1;
-                }
-        }
+        r = window_flag(open, u, v, vi, cover, need);
     }
     out[i] = r;
 }
 
-// Per view, the inclusive 2-D prefix sums of the needed-tile flags, so that
-// the binning pass drops a triangle whose tile box holds no needed tile with
-// four loads.  One CTA per view: a warp per row (shuffle prefix sums over 32
-// tiles at a time, carried along the row), then a thread per column down the
-// rows.
-constexpr int kNeedSumThreads = 512;
-__global__ void __launch_bounds__(kNeedSumThreads) k_need_sum(const __grid_constant__ ImgLayout L,
-                                                              const unsigned char* __restrict__ need,
-                                                              int* __restrict__ sum) {
-    const ViewImg vi = view_img(L, blockIdx.x);
-    const int tx = vi.tiles_x, ty = (vi.H + kCovTile - 1) / kCovTile;
-    const unsigned char* nd = need + vi.tile;
-    int* S = sum + vi.tile;
-    const int lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
-    for (int y = threadIdx.x >> 5; y < ty; y += nwarp) {
-        int carry = 0;
-        for (int x0 = 0; x0 < tx; x0 += 32) {  // warp-uniform
-            const int x = x0 + lane;
-            int v = x < tx ? nd[y * tx + x] : 0;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, v, o);
-                if (lane >= o) v += u;
-            }
-            if (x < tx) S[y * tx + x] = carry + v;
-            carry += __shfl_sync(0xffffffffu, v, 31);
-        }
-    }
-    __syncthreads();
-    for (int x = threadIdx.x; x < tx; x += blockDim.x) {
-        int acc = 0;
-        for (int y = 0; y < ty; ++y) {
-            acc += S[y * tx + x];
-            S[y * tx + x] = acc;
-        }
-    }
+// a (tile, triangle) pair into the tile's bin, or swept at once beyond its capacity
+__device__ __forceinline__ void cov_place(const CovBins& cb, const ViewImg& vi, int tile, int f, long long rec) {
+    const long long key = vi.tile + tile;
+    const int slot = cov_claim(cb, key);
+    if (slot < kCovCap) cb.bins[key * kCovCap + slot] = f;
+    else cov_sweep(cb, vi, tile, cb.rec[rec]);
 }
 
-// One thread per (view, triangle): its record, then its tiles.  Boxes of up
-// to kCovSmall tiles are binned by their own thread, one counter atomic per
-// entry; larger boxes are taken by the whole warp, a tile per lane, reading
-// the record back from global memory.
-// (all 32 lanes of the warp call it together: the big boxes are shared out
-// with warp votes; `sat` culls boxes without a needed tile)
-__device__ __forceinline__ void cov_bin_item(int view, int fi, bool live, int N, int F,
-                                             const int* __restrict__ faces, const float2* __restrict__ p2d,
-                                             const CovBins& cb, const ImgLayout& L, bool sat) {
+// The full binning, grid (triangle blocks, views), one thread per (view,
+// triangle): its record, then its tiles.  Boxes of up to kCovSmall tiles are
+// binned by their own thread, one counter atomic per entry; larger boxes are
+// taken by the whole warp, a tile per lane, reading the record back from
+// global memory.
+__global__ void __launch_bounds__(256, 4) k_cov_bin(int N, int F, const int3* __restrict__ faces,
+                                                    const float2* __restrict__ p2d, CovBins cb,
+                                                    const __grid_constant__ ImgLayout L) {
+    const int fi = blockIdx.x * blockDim.x + threadIdx.x, view = blockIdx.y;
     const unsigned lane = threadIdx.x & 31;
     const ViewImg vi = view_img(L, view);
     const long long i = (long long)view * F + fi;
-    int f = 0;
     CoverTri t;
     t.x0 = 0;
     t.x1 = -1;
     t.y0 = 0;
     t.y1 = -1;
     Footprint fp;
-    if (live) {
-        f = fi;
-        cover_tri(view, f, N, vi.W, vi.H, faces, p2d, t);
-    }
-    bool nonempty = live && t.x1 >= t.x0 && t.y1 >= t.y0;
+    if (fi < F) cover_tri(view, N, vi.W, vi.H, faces[fi], p2d, t);
+    const bool nonempty = fi < F && t.x1 >= t.x0 && t.y1 >= t.y0;
     const int tx0 = t.x0 / kCovTile, ty0 = t.y0 / kCovTile;
     const int ntx = nonempty ? t.x1 / kCovTile - tx0 + 1 : 0;
-    int nt = nonempty ? ntx * (t.y1 / kCovTile - ty0 + 1) : 0;
-    if (sat && nt > 0 &&  // a box without a needed tile needs nothing
-        need_in_box(cb.need_sum + vi.tile, vi.tiles_x, tx0, ty0, t.x1 / kCovTile, t.y1 / kCovTile) == 0) {
-        nonempty = false;
-        nt = 0;
-    }
+    const int nt = nonempty ? ntx * (t.y1 / kCovTile - ty0 + 1) : 0;
     if (nonempty) {
         fp = cover_footprint(t, vi.W, vi.H);
         cb.rec[i] = cover_record(t, fp);
@@ -496,23 +484,15 @@ __device__ __forceinline__ void cov_bin_item(int view, int fi, bool live, int N,
         if (nt > 1 && !footprint_overlaps(fp, max(tx * kCovTile, t.x0), min(tx * kCovTile + kCovTile - 1, t.x1),
                                           max(ty * kCovTile, t.y0), min(ty * kCovTile + kCovTile - 1, t.y1)))
             continue;
-        const int tile = ty * vi.tiles_x + tx;
-        if (cb.need && !cb.need[vi.tile + tile]) continue;
-        const long long key = vi.tile + tile;
-        const int slot = cov_claim(cb, key);
-        if (slot < kCovCap)
-            cb.bins[key * kCovCap + slot] = f;
-        else
-            cov_sweep(cb, vi, tile, cb.rec[i]);
+        cov_place(cb, vi, ty * vi.tiles_x + tx, fi, i);
     }
     __syncwarp();  // the records of big triangles are read back by the other lanes
     unsigned pending = __ballot_sync(0xffffffffu, big);
     while (pending) {
         const int src = __ffs(pending) - 1;
         pending &= pending - 1;
-        const int qv = __shfl_sync(0xffffffffu, view, src), qf = __shfl_sync(0xffffffffu, f, src);
-        const ViewImg qi = view_img(L, qv);
-        const CovTileTri q = cb.rec[(long long)qv * F + qf];
+        const int qf = __shfl_sync(0xffffffffu, fi, src);
+        const CovTileTri q = cb.rec[(long long)view * F + qf];
         const Footprint qfp = record_footprint(q);
         const int qx0 = q.bb.x & 0xffff, qx1 = q.bb.x >> 16, qy0 = q.bb.y & 0xffff, qy1 = q.bb.y >> 16;
         const int qtx0 = qx0 / kCovTile, qty0 = qy0 / kCovTile, qntx = qx1 / kCovTile - qtx0 + 1;
@@ -533,30 +513,21 @@ __device__ __forceinline__ void cov_bin_item(int view, int fi, bool live, int N,
             if (!footprint_overlaps(qfp, max(tx * kCovTile, qx0), min(tx * kCovTile + kCovTile - 1, qx1),
                                     max(ty * kCovTile, qy0), min(ty * kCovTile + kCovTile - 1, qy1)))
                 continue;
-            const int tile = ty * qi.tiles_x + tx;
-            const long long key = qi.tile + tile;
-            if (cb.need && !cb.need[key]) continue;
-            const int slot = cov_claim(cb, key);
-            if (slot < kCovCap)
-                cb.bins[key * kCovCap + slot] = qf;
-            else
-                cov_sweep(cb, qi, tile, q);
+            cov_place(cb, vi, ty * vi.tiles_x + tx, qf, (long long)view * F + qf);
         }
     }
 }
 
-// the unhinted binning: every (view, triangle), grid (triangle blocks, views)
-__global__ void __launch_bounds__(256, 4) k_cov_bin(int N, int F, const int* __restrict__ faces,
-                                                    const float2* __restrict__ p2d, CovBins cb,
-                                                    const __grid_constant__ ImgLayout L) {
-    const int fi = blockIdx.x * blockDim.x + threadIdx.x;
-    cov_bin_item(blockIdx.y, fi, fi < F, N, F, faces, p2d, cb, L, false);
-}
-
-// The hinted binning's first pass, light enough for full occupancy: the
-// (view, triangle) pairs whose tile box holds a needed tile (most hold none),
-// listed with one atomic per warp for k_cov_bin_list.
-__global__ void k_cov_cull(int N, int F, const int* __restrict__ faces, const float2* __restrict__ p2d,
+// The binning for marked tiles.  The marks are kept as one 64-bit word per 8x8
+// tiles, so the test of a box takes a load per word that it touches (one or
+// two for most) and the tiles to visit are the set bits.  Prefix sums of a
+// byte per tile took a kernel to form, and the boxes were then walked tile by
+// tile: 16 x 8 views of 81,920 triangles 1330 -> 555 us for the three.
+//
+// The first pass, light enough for full
+// occupancy: the (view, triangle) pairs whose tile box holds a needed tile
+// (most hold none), listed with one atomic per warp for k_cov_bin_list.
+__global__ void k_cov_cull(int N, int F, const int3* __restrict__ faces, const float2* __restrict__ p2d,
                            CovBins cb, const __grid_constant__ ImgLayout L) {
     const int fi = blockIdx.x * blockDim.x + threadIdx.x;
     const int view = blockIdx.y;
@@ -564,10 +535,9 @@ __global__ void k_cov_cull(int N, int F, const int* __restrict__ faces, const fl
     bool keep = false;
     if (fi < F) {  // no early exit: the whole warp takes part in the vote
         CoverTri t;
-        cover_tri(view, fi, N, vi.W, vi.H, faces, p2d, t);
+        cover_tri(view, N, vi.W, vi.H, faces[fi], p2d, t);
         keep = t.x1 >= t.x0 && t.y1 >= t.y0 &&
-               need_in_box(cb.need_sum + vi.tile, vi.tiles_x, t.x0 / kCovTile, t.y0 / kCovTile, t.x1 / kCovTile,
-                           t.y1 / kCovTile) > 0;
+               need_in_box(cb.need, vi, t.x0 / kCovTile, t.y0 / kCovTile, t.x1 / kCovTile, t.y1 / kCovTile);
     }
     const unsigned m = __ballot_sync(0xffffffffu, keep);
     if (!m) return;  // warp-uniform
@@ -578,19 +548,32 @@ __global__ void k_cov_cull(int N, int F, const int* __restrict__ faces, const fl
     if (keep) cb.items[base + __popc(m & ((1u << lane) - 1u))] = view * F + fi;
 }
 
-// the hinted binning proper over the listed pairs (persistent, whole warps)
-__global__ void __launch_bounds__(256, 4) k_cov_bin_list(int N, int F, const int* __restrict__ faces,
+// The second, over the listed pairs (persistent): a thread per pair writes its
+// record and walks the needed tiles of its box, the set bits of the box's words.
+__global__ void __launch_bounds__(256, 4) k_cov_bin_list(int N, int F, const int3* __restrict__ faces,
                                                          const float2* __restrict__ p2d, CovBins cb,
                                                          const __grid_constant__ ImgLayout L) {
     const int n = *cb.n_items;
-    const int lane = threadIdx.x & 31;
-    const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), nw = (int)((gridDim.x * blockDim.x) >> 5);
-    for (int base = 32 * gw; base < n; base += 32 * nw) {  // warp-uniform
-        const int i = base + lane;
-        const bool live = i < n;
-        const int item = live ? cb.items[i] : 0;
-        const int view = item / F;
-        cov_bin_item(view, item - view * F, live, N, F, faces, p2d, cb, L, false);
+    for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < n; it += gridDim.x * blockDim.x) {
+        const int item = cb.items[it], view = item / F, f = item - view * F;
+        const ViewImg vi = view_img(L, view);
+        CoverTri t;
+        cover_tri(view, N, vi.W, vi.H, faces[f], p2d, t);
+        const Footprint fp = cover_footprint(t, vi.W, vi.H);
+        cb.rec[item] = cover_record(t, fp);
+        const int tx0 = t.x0 / kCovTile, ty0 = t.y0 / kCovTile, tx1 = t.x1 / kCovTile, ty1 = t.y1 / kCovTile;
+        for (int wy = ty0 >> 3; wy <= ty1 >> 3; ++wy)
+            for (int wx = tx0 >> 3; wx <= tx1 >> 3; ++wx) {
+                unsigned long long bits =
+                    cb.need[vi.word + (long long)wy * vi.words_x + wx] & word_box(wx, wy, tx0, ty0, tx1, ty1);
+                for (; bits; bits &= bits - 1ull) {
+                    const int b = __ffsll((long long)bits) - 1, tx = 8 * wx + (b & 7), ty = 8 * wy + (b >> 3);
+                    if (!footprint_overlaps(fp, max(tx * kCovTile, t.x0), min(tx * kCovTile + kCovTile - 1, t.x1),
+                                            max(ty * kCovTile, t.y0), min(ty * kCovTile + kCovTile - 1, t.y1)))
+                        continue;
+                    cov_place(cb, vi, ty * vi.tiles_x + tx, f, item);
+                }
+            }
     }
 }
 
@@ -1160,7 +1143,7 @@ hc_status make_layout(int32_t batch, int32_t n_cameras, const int32_t* widths, c
                kMaxLayoutCams, n_cameras);
     memset(&L, 0, sizeof(L));
     L.n_cam = nc;
-    long long pix = 0, tile = 0, cell = 0;
+    long long pix = 0, tile = 0, cell = 0, word = 0;
     for (int c = 0; c < nc; ++c) {
         CamImg& k = L.cam[c];
         k.W = widths[c];
@@ -1168,9 +1151,12 @@ hc_status make_layout(int32_t batch, int32_t n_cameras, const int32_t* widths, c
         k.tiles_x = div_up(k.W, kCovTile);
         k.gx = div_up(k.W, 30) + 3;
         k.gy = div_up(k.H, 30) + 3;
+        k.words_x = div_up(k.tiles_x, 8);
         k.pix = pix;
         k.tile = tile;
         k.cell = cell;
+        k.word = word;
+        word += (long long)k.words_x * div_up(div_up(k.H, kCovTile), 8);
         HC_REQUIRE((long long)k.W * k.H < (1ll << 31), "too many pixels in one view");
         pix += (long long)k.W * k.H;
         tile += (long long)k.tiles_x * div_up(k.H, kCovTile);
@@ -1179,6 +1165,7 @@ hc_status make_layout(int32_t batch, int32_t n_cameras, const int32_t* widths, c
     L.P = pix;
     L.T = tile;
     L.G = cell;
+    L.Q = word;
     HC_REQUIRE(views / nc * L.T < (1ll << 31), "too many coverage tiles in one call");
     L.fd_T = FastDiv((unsigned)L.T);
     return HC_OK;
@@ -1208,8 +1195,15 @@ bool pixels_by_four(const ImgLayout& L) {
 
 struct hc_mesh_boundary_s {
     int F = 0, N = 0;
-    DevBuf faces, p2d, cover, count, bins, rec, need, need_sum, tile_list, items;
+    DevBuf faces, p2d, cover, count, bins, rec, need, tile_list, items;
 };
+
+static void release(hc_mesh_boundary h) {
+    DevBuf* bufs[] = {&h->faces, &h->p2d, &h->cover, &h->count, &h->bins,
+                      &h->rec, &h->need, &h->tile_list, &h->items};
+    for (DevBuf* b : bufs) b->release();
+    delete h;
+}
 
 extern "C" hc_status hc_mesh_boundary_create(hc_mesh_boundary* out, const int32_t* faces, int32_t n_faces,
                                              int32_t n_vertices) {
@@ -1222,7 +1216,7 @@ extern "C" hc_status hc_mesh_boundary_create(hc_mesh_boundary* out, const int32_
     h->N = n_vertices;
     hc_status st = upload(h->faces, faces, 3 * (size_t)n_faces);
     if (st != HC_OK) {
-        delete h;
+        release(h);
         return st;
     }
     *out = h;
@@ -1231,18 +1225,7 @@ extern "C" hc_status hc_mesh_boundary_create(hc_mesh_boundary* out, const int32_
 
 extern "C" hc_status hc_mesh_boundary_destroy(hc_mesh_boundary h) {
     clear_error();
-    if (!h) return HC_OK;
-    h->faces.release();
-    h->p2d.release();
-    h->cover.release();
-    h->count.release();
-    h->bins.release();
-    h->rec.release();
-    h->need.release();
-    h->need_sum.release();
-    h->tile_list.release();
-    h->items.release();
-    delete h;
+    if (h) release(h);
     return HC_OK;
 }
 
@@ -1253,8 +1236,7 @@ static hc_status mesh_boundary_reserve_layout(hc_mesh_boundary h, long long view
     HC_TRY(h->count.ensure(sizeof(int) * frames * (size_t)L.T));
     HC_TRY(h->bins.ensure(sizeof(int) * frames * (size_t)L.T * kCovCap));
     HC_TRY(h->rec.ensure(sizeof(CovTileTri) * (size_t)views * h->F));
-    HC_TRY(h->need.ensure(frames * (size_t)L.T));
-    HC_TRY(h->need_sum.ensure(sizeof(int) * frames * (size_t)L.T));
+    HC_TRY(h->need.ensure(sizeof(unsigned long long) * frames * (size_t)L.Q));
     HC_TRY(h->tile_list.ensure(sizeof(int) * (frames * (size_t)L.T + 1)));
     HC_REQUIRE(views * h->F < (1ll << 31), "too many (view, triangle) pairs in one call");
     HC_TRY(h->items.ensure(sizeof(int) * ((size_t)views * h->F + 1)));
@@ -1305,37 +1287,31 @@ static hc_status mesh_boundary_run(hc_mesh_boundary h, void* stream, int32_t bat
     cb.cover = h->cover.as<unsigned char>();
     cb.rec = h->rec.as<CovTileTri>();
     cb.need = nullptr;
-    cb.need_sum = nullptr;
     cb.n_tiles = h->tile_list.as<int>();
     cb.tiles = cb.n_tiles + 1;
     cb.n_items = h->items.as<int>();
     cb.items = cb.n_items + 1;
-    if (face_hint) {
-        // final flags of the vertices whose window the hint covers; open
-        // window pixels and their tiles for the binned passes
-        HC_CUDA(cudaMemsetAsync(h->need.ptr, 0, (size_t)n_keys, s));
-        k_bnd_hint<<<div_up(nv, 256), 256, 0, s>>>(nv, h->N, h->F, L, reinterpret_cast<const float2*>(p2d),
-                                                   h->faces.as<int>(), face_hint, h->cover.as<unsigned char>(),
-                                                   h->need.as<unsigned char>(), is_boundary);
-        HC_CHECK_LAUNCH();
-        k_need_sum<<<(unsigned)views, kNeedSumThreads, 0, s>>>(L, h->need.as<unsigned char>(), h->need_sum.as<int>());
-        HC_CHECK_LAUNCH();
-        cb.need = h->need.as<unsigned char>();
-        cb.need_sum = h->need_sum.as<int>();
-    } else {
-        HC_CUDA(cudaMemsetAsync(h->cover.ptr, 0, (size_t)(frames * L.P), s));
-    }
+    const float2* p2 = reinterpret_cast<const float2*>(p2d);
+    const int3* faces = h->faces.as<int3>();
+    unsigned long long* need = h->need.as<unsigned long long>();
     HC_CUDA(cudaMemsetAsync(cb.count, 0, sizeof(int) * (size_t)n_keys, s));
     HC_CUDA(cudaMemsetAsync(cb.n_tiles, 0, sizeof(int), s));
-    const float2* p2 = reinterpret_cast<const float2*>(p2d);
-    if (face_hint) {  // cull, then bin the listed pairs
+    if (face_hint) {
+        // final flags of the vertices whose windows the hint covers; open
+        // window pixels and their tiles for the binned passes
+        HC_CUDA(cudaMemsetAsync(need, 0, sizeof(unsigned long long) * (size_t)(frames * L.Q), s));
         HC_CUDA(cudaMemsetAsync(cb.n_items, 0, sizeof(int), s));
-        k_cov_cull<<<dim3(div_up(h->F, 256), (unsigned)views), 256, 0, s>>>(h->N, h->F, h->faces.as<int>(), p2, cb, L);
+        k_bnd_hint<<<div_up(nv, 256), 256, 0, s>>>(nv, h->N, h->F, L, p2, h->faces.as<int>(), face_hint, cb.cover, need,
+                                                   is_boundary);
         HC_CHECK_LAUNCH();
-        k_cov_bin_list<<<resident_grid(k_cov_bin_list, 256, views * h->F / 256 + 1), 256, 0, s>>>(
-            h->N, h->F, h->faces.as<int>(), p2, cb, L);
+        cb.need = need;  // cull, then bin the listed pairs
+        k_cov_cull<<<dim3(div_up(h->F, 256), (unsigned)views), 256, 0, s>>>(h->N, h->F, faces, p2, cb, L);
+        HC_CHECK_LAUNCH();
+        k_cov_bin_list<<<resident_grid(k_cov_bin_list, 256, views * h->F / 256 + 1), 256, 0, s>>>(h->N, h->F, faces, p2,
+                                                                                                  cb, L);
     } else {
-        k_cov_bin<<<dim3(div_up(h->F, 256), (unsigned)views), 256, 0, s>>>(h->N, h->F, h->faces.as<int>(), p2, cb, L);
+        HC_CUDA(cudaMemsetAsync(h->cover.ptr, 0, (size_t)(frames * L.P), s));
+        k_cov_bin<<<dim3(div_up(h->F, 256), (unsigned)views), 256, 0, s>>>(h->N, h->F, faces, p2, cb, L);
     }
     HC_CHECK_LAUNCH();
     k_cov_tile<<<resident_grid(k_cov_tile, kCovTile * kCovTile, n_keys), kCovTile * kCovTile, 0, s>>>(h->F, n_keys,
