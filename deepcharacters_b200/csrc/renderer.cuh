@@ -376,10 +376,9 @@ __device__ __forceinline__ unsigned pixel_mask(float a0, float b0, float c0, flo
 }
 
 // Bilinear texture lookup at texel coordinates (x, y), texel centres at
-// integer + 0.5, clamp-to-edge addressing: the four texel offsets (floats,
-// x3 channels) and weights.
+// integer + 0.5, clamp-to-edge addressing: the four texels and weights.
 struct BilinearTaps {
-    long long o00, o10, o01, o11;
+    long long i00, i10, i01, i11;
     float fx, fy;
 };
 
@@ -392,15 +391,15 @@ __device__ __forceinline__ BilinearTaps bilinear_taps(float x, float y, int tw, 
     const int x0 = (int)x0f, y0 = (int)y0f;
     const int xa = min(max(x0, 0), tw - 1), xb = min(max(x0 + 1, 0), tw - 1);
     const int ya = min(max(y0, 0), th - 1), yb = min(max(y0 + 1, 0), th - 1);
-    t.o00 = 3LL * ((long long)ya * tw + xa);
-    t.o10 = 3LL * ((long long)ya * tw + xb);
-    t.o01 = 3LL * ((long long)yb * tw + xa);
-    t.o11 = 3LL * ((long long)yb * tw + xb);
+    t.i00 = (long long)ya * tw + xa;
+    t.i10 = (long long)ya * tw + xb;
+    t.i01 = (long long)yb * tw + xa;
+    t.i11 = (long long)yb * tw + xb;
     return t;
 }
 
 __device__ __forceinline__ float3 bilinear_sample(const float* T, const BilinearTaps& t) {
-    const float3 c00 = ld3(T + t.o00), c10 = ld3(T + t.o10), c01 = ld3(T + t.o01), c11 = ld3(T + t.o11);
+    const float3 c00 = ld3(T + 3 * t.i00), c10 = ld3(T + 3 * t.i10), c01 = ld3(T + 3 * t.i01), c11 = ld3(T + 3 * t.i11);
     const float w00 = (1.f - t.fx) * (1.f - t.fy), w10 = t.fx * (1.f - t.fy), w01 = (1.f - t.fx) * t.fy,
                 w11 = t.fx * t.fy;
     return c00 * w00 + c10 * w10 + c01 * w01 + c11 * w11;

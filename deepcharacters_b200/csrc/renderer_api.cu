@@ -17,8 +17,9 @@ hc_status raster_reserve(RasterWorkspace& ws, int views, int F);
 hc_status raster_uv_maps(const Topology& topo, UvTable& tab, cudaStream_t s, int B, int C, long long P_frame, int mode,
                          const float* verts, int tex_h, int tex_w, float* bary, int* face, float* render,
                          float* vnormal, float* uv_map);
-hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vacc, cudaStream_t s, int B, int C,
-                          int albedo, int shading, int ifs, int tfs, const float* grad, const float* verts,
+hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vacc, DevBuf& tacc,
+                          DevBuf& tpad, cudaStream_t s,
+                          int B, int C, int albedo, int shading, int ifs, int tfs, const float* grad, const float* verts,
                           const float* colors, const float* texture, int tex_h, int tex_w, const float* sh,
                           const float* target, const float* vnormal, const float* bary, const int* face,
                           const float* extr, const float* intr, float* vpos_grad, float* vcol_grad, float* tex_grad,
@@ -106,6 +107,8 @@ struct hc_renderer_s {
     hc::Topology topo;
     hc::RasterWorkspace ws;
     hc::DevBuf vacc;      // backward: per-vertex gradient sums
+    hc::DevBuf tacc;      // backward: padded texel gradient sums
+    hc::DevBuf tpad;      // backward: the texture padded to 16 bytes per texel
     hc::UvTable uv;       // texel table of the UV-space maps
     int C = 0, W = 0, H = 0;
     int albedo = 0, shading = 0, normal_map = hc::kNmNone;
@@ -175,7 +178,7 @@ static void release_all(hc_renderer_s* r) {
     r->ws.clock.made = false;
     DevBuf* bufs[] = {&r->topo.faces, &r->topo.vf, &r->topo.vf_id, &r->topo.texcoords,
                       &r->ws.cams, &r->ws.tri_frame, &r->ws.tri_view, &r->ws.tile_state,
-                      &r->ws.bins, &r->ws.spill, &r->ws.spill_keys, &r->ws.stats, &r->vacc,
+                      &r->ws.bins, &r->ws.spill, &r->ws.spill_keys, &r->ws.stats, &r->vacc, &r->tacc, &r->tpad,
                       &r->uv.faces, &r->uv.table, &r->ws.layout, &r->ws.tile_cam, &r->ws.tile_cam_b, &r->ws.proj,
                       &r->ws.l1_part, &r->ws.claim, &r->ws.claim_b};
     for (DevBuf* b : bufs) b->release();
@@ -291,7 +294,7 @@ extern "C" hc_status hc_renderer_backward(hc_renderer h, void* stream, int32_t b
     if (h->albedo == kTextured || h->albedo == kTexturedBilinear)
         HC_REQUIRE(texture && texture_grad && texture_width > 0 && texture_height > 0, "textured mode needs a texture");
     if (h->shading == kShaded) HC_REQUIRE(sh_coeff && sh_coeff_grad, "shaded mode needs sh_coeff");
-    return raster_backward(h->topo, h->ws, h->vacc, (cudaStream_t)stream, batch, h->C, h->albedo,
+    return raster_backward(h->topo, h->ws, h->vacc, h->tacc, h->tpad, (cudaStream_t)stream, batch, h->C, h->albedo,
                            h->shading, h->image_filter, h->texture_filter, render_buffer_grad, vertex_pos,
                            vertex_color, texture, texture_height, texture_width, sh_coeff, target_image,
                            vertex_normal, barycentric_buffer, face_buffer, extrinsics, intrinsics, vertex_pos_grad,
@@ -355,7 +358,7 @@ extern "C" hc_status hc_renderer_backward_l1(hc_renderer h, void* stream, int32_
     l1.mask = foreground_mask;
     l1.state = const_cast<L1State*>(static_cast<const L1State*>(l1_state));
     l1.render = render_buffer;
-    return raster_backward(h->topo, h->ws, h->vacc, (cudaStream_t)stream, batch, h->C, h->albedo,
+    return raster_backward(h->topo, h->ws, h->vacc, h->tacc, h->tpad, (cudaStream_t)stream, batch, h->C, h->albedo,
                            h->shading, h->image_filter, h->texture_filter, nullptr, vertex_pos, vertex_color, texture,
                            texture_height, texture_width, sh_coeff, target_image, vertex_normal, barycentric_buffer,
                            face_buffer, extrinsics, intrinsics, vertex_pos_grad, vertex_color_grad, texture_grad,

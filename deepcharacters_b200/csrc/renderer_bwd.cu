@@ -12,8 +12,8 @@
 //  * per-vertex contributions (position, colour, pixel-normal gradients) are
 //    merged inside each warp (lanes matched by face id, a leader sums up to
 //    8 members) before 16-byte global reductions per vertex and leader;
-//  * SH gradients are reduced over the CTA (warp shuffles) before one atomic
-//    per coefficient;
+//  * SH gradients are summed per warp over the tiles of a view before one
+//    atomic per coefficient;
 //  * the shaded-mode normal chain is split in two: pixels accumulate the
 //    gradient w.r.t. each vertex's unnormalised normal, then a per-vertex
 //    gather over incident faces applies d(face normal)/d(vertex) once per
@@ -58,6 +58,8 @@ struct BwdArgs {
     const int* face;        // [V,H,W]
     float* vacc;            // [B,N,VertexSums::kStride] per-vertex sums (cleared before the launch)
     float* tex_grad;        // [B,TH,TW,3]
+    const float4* tex_pad;  // [B,TH,TW] the texture padded to 16 bytes per texel, or NULL
+    float4* tex_acc;        // [B,TH,TW] texel sums padded to 16 bytes (cleared before the launch), or NULL: tex_grad
     float* sh_grad;         // [V,27]
     // fused image L1: the image gradient is formed from the render and the
     // target instead of read from grad (NULL state: not fused)
@@ -126,15 +128,18 @@ __device__ __forceinline__ void bary_jacobian_apply(float3 o, float3 d, float3 v
 // Sobel-like image gradient of the reference (imageGradient, RendererUtil.h:566-620):
 // weights (x, y)/(x^2+y^2) over a (2k+1)^2 window, normalised by sum |x|/(x^2+y^2);
 // zero near the border.  `x`, `y` are the (possibly fractional) sample position.
-__device__ void image_gradient(const float* img, float x, float y, int w, int h, int fs, float3& du, float3& dv) {
-    du = dv = make_float3(0.f, 0.f, 0.f);
-    if (!(x >= (float)(fs + 1) && y >= (float)(fs + 1) && x < (float)(w - (fs + 1)) && y < (float)(h - (fs + 1))))
-        return;
+// FS: a filter size known at compile time, whose weights and normaliser fold
+// to constants (the run-time form divides twice per tap), or 0 for `size`;
+// the terms, their order and rounding are the same.
+template <int FS, class Tap>
+__device__ __forceinline__ void image_gradient_fs(Tap tap, float x, float y, int w, int size, float3& du, float3& dv) {
+    const int fs = FS ? FS : size;
     float norm = 0.f;
+#pragma unroll(FS ? 2 * FS + 1 : 1)
     for (int j = -fs; j <= fs; ++j)
+#pragma unroll(FS ? 2 * FS + 1 : 1)
         for (int i = -fs; i <= fs; ++i) {
-            const int idx = (int)((y + j) * w + (x + i));
-            const float3 I = ld3(img + 3LL * idx);
+            const float3 I = tap((int)((y + j) * w + (x + i)));
             const float den = (float)(i * i + j * j);
             float gu = 0.f, gv = 0.f;
             if (den != 0.f) {
@@ -147,6 +152,31 @@ __device__ void image_gradient(const float* img, float x, float y, int w, int h,
         }
     du = du / norm;
     dv = dv / norm;
+}
+
+template <class Tap>
+__device__ __forceinline__ void image_gradient(Tap tap, float x, float y, int w, int h, int fs, float3& du, float3& dv) {
+    du = dv = make_float3(0.f, 0.f, 0.f);
+    if (!(x >= (float)(fs + 1) && y >= (float)(fs + 1) && x < (float)(w - (fs + 1)) && y < (float)(h - (fs + 1))))
+        return;
+    switch (fs) {
+        case 1: image_gradient_fs<1>(tap, x, y, w, fs, du, dv); break;
+        case 2: image_gradient_fs<2>(tap, x, y, w, fs, du, dv); break;
+        default: image_gradient_fs<0>(tap, x, y, w, fs, du, dv);
+    }
+}
+
+// Sums of 32 values over the warp: lane k ends with the sum of value k (31
+// shuffles instead of five per value).
+__device__ __forceinline__ float warp_sum32(float v[32], int lane) {
+#pragma unroll
+    for (int h = 16; h > 0; h >>= 1)
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const float keep = (lane & h) ? v[i + h] : v[i], send = (lane & h) ? v[i] : v[i + h];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+        }
+    return v[0];
 }
 
 // Exact barycentric Jacobian of a ray hit.  With P = o + t d = l0 v0 + l1 v1 +
@@ -227,6 +257,18 @@ __device__ __forceinline__ void taps_fs(const float4* s_tgt, int s0, float3 G, f
         }
 }
 
+// adds g to a texel's gradient: one 16-byte reduction, or three floats
+__device__ __forceinline__ void add_texel(const BwdArgs& A, int b, long long texel, float3 g) {
+    const long long i = (long long)b * A.tex_h * A.tex_w + texel;
+    if (A.tex_acc) {  // launch-uniform
+        atomicAdd(A.tex_acc + i, make_float4(g.x, g.y, g.z, 0.f));
+    } else {
+        atomicAdd(A.tex_grad + 3 * i + 0, g.x);
+        atomicAdd(A.tex_grad + 3 * i + 1, g.y);
+        atomicAdd(A.tex_grad + 3 * i + 2, g.z);
+    }
+}
+
 // Albedo classes of the adjoint: vertex colours, texture, and the modes
 // whose albedo has no parameters (normal, lighting, mask, position, depth, uv).
 enum { kAlbVcol = 0, kAlbTex = 1, kAlbNone = 2, kAlbTexBilinear = 3 };
@@ -264,7 +306,7 @@ __global__ void __launch_bounds__(BNT, SHADED ? 2 : 4) k_render_grad(BwdArgs A, 
     constexpr int NVV = Sums::kVals;                  // values per vertex
     constexpr int NROW = (3 * NVV + 3) / 4 * 4;       // per-lane row, a multiple of 16 bytes
     __shared__ __align__(16) float s_red[BNT / 32][32][NROW];
-    __shared__ float s_sh[SHADED ? BNT / 32 : 1][27];
+    __shared__ float s_sh[SHADED ? BNT / 32 : 1][32];  // per warp: SH sums of the tiles of one view
     __shared__ __align__(128) float4 s_tgt2[2][TILE_S * TILE_S];  // target tile + halo, double-buffered
     __shared__ float2 s_tap[MAXTAPS];  // image-gradient tap weights (i, j) / (i^2 + j^2)
     __shared__ float s_norm;
@@ -371,6 +413,23 @@ __global__ void __launch_bounds__(BNT, SHADED ? 2 : 4) k_render_grad(BwdArgs A, 
         stage(g, 0);
     }
     asm volatile("cp.async.commit_group;\n" ::);
+    // the CTA's SH sums of a view: one atomic per coefficient when the view
+    // changes (a CTA walks many tiles of a view), instead of a reduction over
+    // the CTA and 27 atomics per tile
+    int sh_view = -1;
+    if constexpr (SHADED) s_sh[warp][lane] = 0.f;
+    auto flush_sh = [&](int v) {
+        __syncthreads();
+        if (v >= 0 && threadIdx.x < 27) {
+            float sum = 0.f;
+            for (int w = 0; w < BNT / 32; ++w) {
+                sum += s_sh[w][threadIdx.x];
+                s_sh[w][threadIdx.x] = 0.f;
+            }
+            if (sum != 0.f) atomicAdd(A.sh_grad + (long long)v * 27 + threadIdx.x, sum);
+        }
+        __syncthreads();
+    };
     for (int it = 0; g < n_tiles; ++it) {  // CTA-uniform
     const int buf = tma ? 0 : it & 1;
     const float4* s_tgt = s_tgt2[buf];
@@ -419,6 +478,12 @@ __global__ void __launch_bounds__(BNT, SHADED ? 2 : 4) k_render_grad(BwdArgs A, 
     const unsigned fb = A.fd_frame.div((unsigned)g);
     const int b = (int)fb;
     const int view = b * A.C + A.tile_cam_b[A.fd_frame.mod((unsigned)g, fb)];
+    if constexpr (SHADED) {
+        if (view != sh_view) {  // CTA-uniform: the sums of the view before
+            flush_sh(sh_view);
+            sh_view = view;
+        }
+    }
     const ViewCam& cam = cams[view];
     const int tile = (int)(g - cam.tile_base_b);
     const int W = cam.W, H = cam.H;
@@ -507,19 +572,15 @@ __global__ void __launch_bounds__(BNT, SHADED ? 2 : 4) k_render_grad(BwdArgs A, 
             const float2 uv = t0 * ba + t1 * bb + t2 * bc;
             const BilinearTaps tp = bilinear_taps(uv.x * A.tex_w, uv.y * A.tex_h, A.tex_w, A.tex_h);
             const float* T = A.texture + (long long)b * A.tex_h * A.tex_w * 3;
-            const float3 c00 = ld3(T + tp.o00), c10 = ld3(T + tp.o10), c01 = ld3(T + tp.o01), c11 = ld3(T + tp.o11);
+            const float3 c00 = ld3(T + 3 * tp.i00), c10 = ld3(T + 3 * tp.i10), c01 = ld3(T + 3 * tp.i01),
+                         c11 = ld3(T + 3 * tp.i11);
             const float w00 = (1.f - tp.fx) * (1.f - tp.fy), w10 = tp.fx * (1.f - tp.fy),
                         w01 = (1.f - tp.fx) * tp.fy, w11 = tp.fx * tp.fy;
             alb = c00 * w00 + c10 * w10 + c01 * w01 + c11 * w11;
-            float* tg = A.tex_grad + (long long)b * A.tex_h * A.tex_w * 3;
-            const long long off[4] = {tp.o00, tp.o10, tp.o01, tp.o11};
+            const long long texel[4] = {tp.i00, tp.i10, tp.i01, tp.i11};
             const float wt[4] = {w00, w10, w01, w11};
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                atomicAdd(tg + off[q] + 0, gA.x * wt[q]);
-                atomicAdd(tg + off[q] + 1, gA.y * wt[q]);
-                atomicAdd(tg + off[q] + 2, gA.z * wt[q]);
-            }
+            for (int q = 0; q < 4; ++q) add_texel(A, b, texel[q], gA * wt[q]);
             const float3 dx = (c10 - c00) * (1.f - tp.fy) + (c11 - c01) * tp.fy;
             const float3 dy = (c01 - c00) * (1.f - tp.fx) + (c11 - c10) * tp.fx;
             const float gu = dot(gA, dx) * A.tex_w, gv = dot(gA, dy) * A.tex_h;
@@ -544,14 +605,19 @@ __global__ void __launch_bounds__(BNT, SHADED ? 2 : 4) k_render_grad(BwdArgs A, 
             // (CUDABasedRasterizationGrad.cu:242-243), weight pairs as written there
             alb = (uv.y - LV) * (((uv.x - LU) * cLL) + ((HU - uv.x) * cHL)) +
                   (HV - uv.y) * (((uv.x - LU) * cLH) + ((HU - uv.x) * cHH));
-            if (!flipped) {
-                float* tg = A.tex_grad + (long long)b * A.tex_h * A.tex_w * 3 + 3LL * ((int)LV * A.tex_w + (int)LU);
-                atomicAdd(tg + 0, gA.x);
-                atomicAdd(tg + 1, gA.y);
-                atomicAdd(tg + 2, gA.z);
-            }
+            if (!flipped) add_texel(A, b, (int)LV * A.tex_w + (int)LU, gA);
             float3 du, dv;
-            image_gradient(T, uv.x, uv.y, A.tex_w, A.tex_h, A.tfs, du, dv);
+            if (A.tex_pad) {  // launch-uniform
+                const float4* T4 = A.tex_pad + (long long)b * A.tex_h * A.tex_w;
+                image_gradient(
+                    [&](int i) {
+                        const float4 q = T4[i];
+                        return make_float3(q.x, q.y, q.z);
+                    },
+                    uv.x, uv.y, A.tex_w, A.tex_h, A.tfs, du, dv);
+            } else {
+                image_gradient([&](int i) { return ld3(T + 3LL * i); }, uv.x, uv.y, A.tex_w, A.tex_h, A.tfs, du, dv);
+            }
             const float gu = dot(gA, du), gv = dot(gA, dv);
             gbc = make_float3(gu * (t0.x * A.tex_w) + gv * (t0.y * A.tex_h), gu * (t1.x * A.tex_w) + gv * (t1.y * A.tex_h),
                               gu * (t2.x * A.tex_w) + gv * (t2.y * A.tex_h));
@@ -721,26 +787,20 @@ __global__ void __launch_bounds__(BNT, SHADED ? 2 : 4) k_render_grad(BwdArgs A, 
                 add_vertex<NVV>(A.vacc + ((long long)b * A.N + vid[i]) * Sums::kStride, a + NVV * i);
         }
     }
-    // SH: reduce over the CTA, one atomic per coefficient
+    // SH: each warp adds its pixels to its own sums of the current view
     if constexpr (SHADED) {
+        if (__any_sync(0xffffffffu, f >= 0)) {
+            float v[32];
 #pragma unroll
-        for (int k = 0; k < 27; ++k) {
-            float v = shg[k];
-#pragma unroll
-            for (int o2 = 16; o2 > 0; o2 >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o2);
-            if (lane == 0) s_sh[warp][k] = v;
-        }
-        __syncthreads();
-        if (threadIdx.x < 27) {
-            float v = 0.f;
-            for (int w = 0; w < BNT / 32; ++w) v += s_sh[w][threadIdx.x];
-            if (v != 0.f) atomicAdd(A.sh_grad + (long long)view * 27 + threadIdx.x, v);
+            for (int k = 0; k < 32; ++k) v[k] = k < 27 ? shg[k < 27 ? k : 0] : 0.f;
+            s_sh[warp][lane] += warp_sum32(v, lane);
         }
     }
     __syncthreads();  // the next iteration's prefetch reuses this tile's buffer
     if constexpr (DYN) g = s_claimed[(it + 1) & 1];
     else g += gridDim.x;
     }
+    if constexpr (SHADED) flush_sh(sh_view);
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
@@ -786,6 +846,20 @@ __global__ void k_vertex_grad(int B, int N, const int3* __restrict__ faces, cons
     st3(vpos_grad + 3 * i, g0);
 }
 
+// the texture padded to 16 bytes per texel
+__global__ void k_texture_pad(long long n, const float* __restrict__ texture, float4* __restrict__ out) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i < n) out[i] = make_float4(texture[3 * i], texture[3 * i + 1], texture[3 * i + 2], 0.f);
+}
+
+// the texture gradient from the padded texel sums, a thread per float
+__global__ void k_texture_grad(long long n, const float* __restrict__ acc, float* __restrict__ out) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const long long t = i / 3;
+    out[i] = acc[4 * t + (i - 3 * t)];
+}
+
 }  // namespace
 
 hc_status raster_layout(RasterWorkspace& ws);
@@ -824,8 +898,9 @@ static bool target_tensor_map(const RasterWorkspace& ws, const float* target, in
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vacc, cudaStream_t s, int B, int C,
-                          int albedo, int shading, int ifs, int tfs, const float* grad,
+hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vacc, DevBuf& tacc,
+                          DevBuf& tpad, cudaStream_t s,
+                          int B, int C, int albedo, int shading, int ifs, int tfs, const float* grad,
                           const float* verts, const float* colors, const float* texture, int tex_h, int tex_w,
                           const float* sh, const float* target, const float* vnormal, const float* bary,
                           const int* face, const float* extr, const float* intr, float* vpos_grad,
@@ -841,8 +916,36 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vac
     const size_t vacc_bytes = sizeof(float) * (size_t)stride * (size_t)B * N;
     HC_TRY(vacc.ensure(vacc_bytes));
     HC_CUDA(cudaMemsetAsync(vacc.ptr, 0, vacc_bytes, s));
-    if (tex_grad && tex_h > 0 && tex_w > 0)
-        HC_CUDA(cudaMemsetAsync(tex_grad, 0, sizeof(float) * 3 * (size_t)B * tex_h * tex_w, s));
+    // Texels padded to 16 bytes where the padding's extra pass over the texture
+    // costs less than it saves.  Sums (a clear, a read and a write, 32 bytes per
+    // texel): two reductions per covered pixel (eight bilinear) become none;
+    // bilinear, 1024^2 texture: 4 x 2048^2 views 1144 -> 690 us, 4 x 1024^2 239 ->
+    // 206, one 1024^2 83 -> 84, one 512^2 51 -> 62; nearest: 4 x 512^2 views of a
+    // 32^2 texture 182 -> 92, of a 256^2 one and 4 x 1024^2 of 1024^2 no change.
+    // Taps of the nearest mode's texture gradient (28 bytes per texel): one load
+    // per tap instead of three; 1024^2 texture: 4 x 1024^2 views 400 -> 337 us,
+    // one 1024^2 131 -> 118, one 512^2 71 -> 67, one 256^2 56 -> 60.
+    // A capture does not allocate, and without memory for the padding the
+    // texture is used as it is.
+    const long long texels = tex_grad && tex_h > 0 && tex_w > 0 ? (long long)B * tex_h * tex_w : 0;
+    const long long pixels = (long long)B * ws.P_frame;
+    const size_t pad_bytes = sizeof(float4) * (size_t)texels;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    HC_CUDA(cudaStreamIsCapturing(s, &capture));
+    auto room = [&](DevBuf& buf) {
+        if (buf.bytes >= pad_bytes) return true;
+        if (capture == cudaStreamCaptureStatusNone && buf.ensure(pad_bytes) == HC_OK) return true;
+        cudaGetLastError();
+        clear_error();
+        return false;
+    };
+    const bool padded = texels > 0 &&
+                        ((albedo == kTexturedBilinear && pixels >= 2 * texels) ||
+                         (albedo == kTextured && pixels >= 16 * texels)) &&
+                        room(tacc);
+    const bool taps = albedo == kTextured && texels > 0 && 4 * pixels >= texels && room(tpad);
+    if (padded) HC_CUDA(cudaMemsetAsync(tacc.ptr, 0, pad_bytes, s));
+    else if (texels) HC_CUDA(cudaMemsetAsync(tex_grad, 0, sizeof(float) * 3 * (size_t)texels, s));
     if (sh_grad) HC_CUDA(cudaMemsetAsync(sh_grad, 0, sizeof(float) * 27 * (size_t)V, s));
     ViewCam* cams = ws.cams.as<ViewCam>();
     k_view_setup<<<div_up(V, 64), 64, 0, s>>>(V, C, extr, intr, ws.layout.as<CamLayout>(), ws.P_frame, ws.T_frame,
@@ -876,6 +979,12 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vac
     A.face = face;
     A.vacc = vacc.as<float>();
     A.tex_grad = tex_grad;
+    A.tex_acc = padded ? tacc.as<float4>() : nullptr;
+    A.tex_pad = taps ? tpad.as<float4>() : nullptr;
+    if (taps) {
+        k_texture_pad<<<div_up(texels, 256), 256, 0, s>>>(texels, texture, tpad.as<float4>());
+        HC_CHECK_LAUNCH();
+    }
     A.sh_grad = sh_grad;
     HC_TRY(ws.stats.ensure(sizeof(RasterStats)));
     A.err = &ws.stats.as<RasterStats>()->overflow;
@@ -944,6 +1053,10 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vac
     }
     HC_CHECK_LAUNCH();
     ws.clock.end(kKNormalChain, s);
+    if (padded) {
+        k_texture_grad<<<div_up(3 * texels, 256), 256, 0, s>>>(3 * texels, tacc.as<float>(), tex_grad);
+        HC_CHECK_LAUNCH();
+    }
     return HC_OK;
 }
 
