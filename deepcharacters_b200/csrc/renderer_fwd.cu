@@ -422,11 +422,11 @@ struct ShadeArgs {
     float* render;
     int* depth_q;
     int* tie_count;
-    // fused image L1 (NULL sums: not fused)
+    bool vec;  // rows of a multiple of four pixels, outputs 16-byte aligned
+    // fused image L1 (NULL state: not fused)
     const float* l1_target;
     const unsigned char* l1_mask;
-    float* l1_sum;     // [tiles * warps per tile]
-    unsigned* l1_cnt;  // [tiles * warps per tile]
+    L1State* l1_state;
 };
 
 // colour of a pixel hit by face f at barycentrics (a, bb)
@@ -553,6 +553,15 @@ __device__ __forceinline__ bool raster_hit_below(float3 ro_s, float3 dir, const 
     return (a / denom >= -0.001f) && (b / denom >= -0.001f) && (a / denom <= 1.001f) && (b / denom <= 1.001f);
 }
 
+__device__ __forceinline__ void store_bary(const ShadeArgs& A, long long pix, float a, float b) {
+    if (A.vec) {  // launch-uniform
+        reinterpret_cast<float2*>(A.bary)[pix] = make_float2(a, b);
+    } else {
+        A.bary[2 * pix + 0] = a;
+        A.bary[2 * pix + 1] = b;
+    }
+}
+
 // TIES: the call asked for the per-pixel count of hits at the winning depth
 // (diagnostics); without it the count is compiled out, which frees a register
 // of the scan and shortens its updates
@@ -585,7 +594,10 @@ __device__ __forceinline__ bool raster_hit_below(float3 ro_s, float3 dir, const 
 // the lockstep walk, the bound within the tile instead of the triangle's, and
 // claims sized to the call: 16 x 8 views of 1024^2, 8-px tiles 7.50 -> 6.73 ms;
 // 2 x 4 mixed-size views of a mesh of long thin triangles 751 -> 496 us;
-// 4 x 2048^2 at 16 px 1265 -> 968 us; one 512^2 view 84 -> 20 us.
+// 4 x 2048^2 at 16 px 1265 -> 968 us; one 512^2 view 84 -> 20 us.  Whole rows
+// of background, copies from a fixed piece per thread, and the image L1 kept
+// per thread over all tiles instead of reduced per warp and tile: 6.67 -> 6.05
+// ms, 486 -> 418 us, 960 -> 918 us.
 template <int TS, bool TIES>
 __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_resolve(ShadeArgs A, FastDiv fd_frame,
                                                    const int* __restrict__ tile_cam, int cap,
@@ -604,6 +616,7 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
     constexpr unsigned kNoKey = 0xffffffffu;
     constexpr int kRec = (sizeof(TriView) + sizeof(TriFrame)) / 16;  // 16-byte pieces of a record
     constexpr int kViewRec = sizeof(TriView) / 16;
+    static_assert(sizeof(TriView) == 48 && sizeof(TriFrame) == 48, "the copy's stride");
     __shared__ float4 s_rec[CHUNK * kRec];  // staged records (TriView, TriFrame), by slot
     __shared__ unsigned s_key[CHUNK];       // per warp: its keys, sorted
     __shared__ unsigned s_ord[CHUNK];       // the chunk's keys in order
@@ -612,10 +625,27 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
     // rewritten two claims later, after every thread has passed the next
     // claim's barrier
     __shared__ long long s_g[2];
+    // each thread's share of the image L1 (fused L1 only)
+    __shared__ double s_l1[NT];
+    __shared__ unsigned s_l1n[NT];
+    s_l1[threadIdx.x] = 0.0;
+    s_l1n[threadIdx.x] = 0u;
+    // the copy of the records: this thread's 16-byte piece and first record
+    const int piece = (int)threadIdx.x % kRec, rec0 = (int)threadIdx.x / kRec;
+    constexpr int kPerRound = NT / kRec;  // records per round
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned keep = 0;  // bit per stage of the bitonic network: this lane keeps the smaller key
+    {
+        int at = 0;
+#pragma unroll
+        for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+            for (int stride = size >> 1; stride > 0; stride >>= 1, ++at)
+                keep |= (unsigned)(((lane & stride) == 0) == ((lane & size) == 0)) << at;
+    }
     int left = 0, par = 1;  // tiles left of the current claim; its slot
     long long g = 0;
-    for (;; --left, ++g) {
+    for (;; --left, ++g) {  // (the background branch continues here too)
     if (left == 0) {
         par ^= 1;
         if (threadIdx.x == 0) s_g[par] = (long long)atomicAdd(claim, (unsigned long long)claim_n);
@@ -634,10 +664,39 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
     const int px = tx * TS + threadIdx.x % TS, py = ty * TS + threadIdx.x / TS;
     const float cx = px + 0.5f, cy = py + 0.5f;
     const bool valid = px < W && py < H;
-    const float3 ro_s = make_float3(cam.ro_s[0], cam.ro_s[1], cam.ro_s[2]);
-    const float3 dir = pixel_ray(cam, px, py);
     const int2 st = tile_state[g];
     const int n = min(st.x, cap);
+    if (n == 0) {  // background (a tile spills only beyond a full bin)
+        const long long pix = cam.pix_base + (long long)py * W + px;
+        if (A.vec && (tx + 1) * TS <= W && (ty + 1) * TS <= H) {
+            // whole rows: 16-byte stores, TS / 4 of the faces, twice that of the
+            // barycentrics, three times of the colours
+            constexpr int Q = TS / 4, kStores = TS * 6 * Q;
+            const long long first = cam.pix_base + (long long)ty * TS * W + tx * TS;
+#pragma unroll
+            for (int k = 0; k < (kStores + NT - 1) / NT; ++k) {
+                const int i = (int)threadIdx.x + k * NT, row = i / (6 * Q), q = i - row * (6 * Q);
+                if (kStores % NT != 0 && i >= kStores) break;
+                const long long p = first + (long long)row * W;
+                const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (q < 3 * Q) reinterpret_cast<float4*>(A.render + 3 * p)[q] = zero;
+                else if (q < 5 * Q) reinterpret_cast<float4*>(A.bary + 2 * p)[q - 3 * Q] = zero;
+                else reinterpret_cast<int4*>(A.face + p)[q - 5 * Q] = make_int4(-1, -1, -1, -1);
+            }
+        } else if (valid) {
+            A.face[pix] = -1;
+            A.bary[2 * pix + 0] = 0.f;
+            A.bary[2 * pix + 1] = 0.f;
+            A.render[3 * pix + 0] = 0.f;
+            A.render[3 * pix + 1] = 0.f;
+            A.render[3 * pix + 2] = 0.f;
+        }
+        if (valid && A.depth_q) A.depth_q[pix] = 0x7fffffff;
+        if (TIES && valid) A.tie_count[pix] = 0;
+        continue;
+    }
+    const float3 ro_s = make_float3(cam.ro_s[0], cam.ro_s[1], cam.ro_s[2]);
+    const float3 dir = pixel_ray(cam, px, py);
     const int* tb = bins + g * cap;
     unsigned best_d = 0xffffffffu;
     int best_f = 0x7fffffff;
@@ -646,16 +705,16 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
     for (int base = 0; base < n; base += CHUNK) {
         const int m = min(CHUNK, n - base);
         __syncthreads();  // the previous chunk's readers are done
-        for (int i = threadIdx.x; i < m * kRec; i += NT) {
-            const int r = i / kRec, c = i - r * kRec;
-            const int f = tb[base + r];
-            if (c == 0) s_face[r] = f;
-            const float4* src = c < kViewRec
-                                    ? reinterpret_cast<const float4*>(tri_view + (long long)view * A.F + f) + c
-                                    : reinterpret_cast<const float4*>(tri_frame + (long long)b * A.F + f) + (c - kViewRec);
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(
-                             (unsigned)__cvta_generic_to_shared(&s_rec[i])),
-                         "l"(src));
+        if (rec0 < kPerRound) {
+            // both records have kViewRec pieces of a 48-byte stride
+            const char* src = piece < kViewRec ? reinterpret_cast<const char*>(tri_view + (long long)view * A.F) + 16 * piece
+                                               : reinterpret_cast<const char*>(tri_frame + (long long)b * A.F) + 16 * (piece - kViewRec);
+            unsigned dst = (unsigned)__cvta_generic_to_shared(&s_rec[rec0 * kRec + piece]);
+            for (int r = rec0; r < m; r += kPerRound, dst += 16 * kRec * kPerRound) {
+                const int f = tb[base + r];
+                if (piece == 0) s_face[r] = f;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src + 48ll * f));
+            }
         }
         asm volatile("cp.async.wait_all;\n" ::: "memory");
         __syncthreads();
@@ -677,13 +736,13 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
             key = (front ? 0u : 0x80000000u) | (coarse << SB) | threadIdx.x;
         }
         if (threadIdx.x < CHUNK && (int)(threadIdx.x & ~31u) < m) {  // whole warps that hold keys
+            int at = 0;
 #pragma unroll
             for (int size = 2; size <= 32; size <<= 1) {
 #pragma unroll
-                for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                for (int stride = size >> 1; stride > 0; stride >>= 1, ++at) {
                     const unsigned o = __shfl_xor_sync(0xffffffffu, key, stride);
-                    const bool keep_min = ((lane & stride) == 0) == ((lane & size) == 0);
-                    key = keep_min ? min(key, o) : max(key, o);
+                    key = (keep >> at) & 1u ? min(key, o) : max(key, o);
                 }
             }
             s_key[threadIdx.x] = key;
@@ -756,8 +815,6 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
             }
         }
     }
-    float l1s = 0.f;  // this pixel's image L1 terms (fused L1 only)
-    unsigned l1c = 0;
     if (valid) {
         if (st.x > cap && st.y > 0 && st.y <= spill_tile_cap) {
             const unsigned long long key = spill_keys[(long long)(st.y - 1) * NT + threadIdx.x];
@@ -778,8 +835,7 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
         const long long pix = cam.pix_base + (long long)py * W + px;
         if (best_d == 0xffffffffu) {
             A.face[pix] = -1;
-            A.bary[2 * pix + 0] = 0.f;
-            A.bary[2 * pix + 1] = 0.f;
+            store_bary(A, pix, 0.f, 0.f);
             A.render[3 * pix + 0] = 0.f;
             A.render[3 * pix + 1] = 0.f;
             A.render[3 * pix + 2] = 0.f;
@@ -788,7 +844,7 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
         } else {
             // the fused L1's target, loaded before this pixel's stores (which
             // the compiler may not move it past)
-            const bool l1m = A.l1_sum && (!A.l1_mask || A.l1_mask[pix]);
+            const bool l1m = A.l1_state && (!A.l1_mask || A.l1_mask[pix]);
             const float3 tg = l1m ? ld3(A.l1_target + 3 * pix) : make_float3(0.f, 0.f, 0.f);
             // recompute the winner's barycentrics (same arithmetic as the hit test)
             // the winner's triangle and plane offset: from the staged chunk when
@@ -814,8 +870,7 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
             // every load of the shading before the first store of the pixel
             const float3 col = shade_pixel(A, cam, view, b, best_f, a, bb, dir);
             A.face[pix] = best_f;
-            A.bary[2 * pix + 0] = a;
-            A.bary[2 * pix + 1] = bb;
+            store_bary(A, pix, a, bb);
             A.render[3 * pix + 0] = col.x;
             A.render[3 * pix + 1] = col.y;
             A.render[3 * pix + 2] = col.z;
@@ -823,42 +878,24 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
             if (TIES) A.tie_count[pix] = ties;
             if (l1m) {
                 const float d0 = l1_diff(col.x, tg.x), d1 = l1_diff(col.y, tg.y), d2 = l1_diff(col.z, tg.z);
-                l1s = fabsf(d0) + fabsf(d1) + fabsf(d2);
-                l1c = (d0 != 0.f) + (d1 != 0.f) + (d2 != 0.f);
+                s_l1[threadIdx.x] += (double)(fabsf(d0) + fabsf(d1) + fabsf(d2));
+                s_l1n[threadIdx.x] += (d0 != 0.f) + (d1 != 0.f) + (d2 != 0.f);
             }
         }
     }
-    if (A.l1_sum) {  // launch-uniform: each warp's partial L1 sum and count
+    }
+    if (A.l1_state) {  // launch-uniform: the CTA's image L1, one atomic pair per warp
+        double l1s = s_l1[threadIdx.x];
+        unsigned long long l1c = s_l1n[threadIdx.x];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             l1s += __shfl_xor_sync(0xffffffffu, l1s, o);
             l1c += __shfl_xor_sync(0xffffffffu, l1c, o);
         }
-        if (lane == 0) {
-            A.l1_sum[g * (NT / 32) + warp] = l1s;
-            A.l1_cnt[g * (NT / 32) + warp] = l1c;
+        if (lane == 0 && l1c) {
+            atomicAdd(&A.l1_state->sum, l1s);
+            atomicAdd(&A.l1_state->count, l1c);
         }
-    }
-    }
-}
-
-// the fused L1's warp partials summed into the L1 state (zeroed before)
-__global__ void k_l1_tiles(long long n, const float* __restrict__ sums, const unsigned* __restrict__ cnts,
-                           L1State* __restrict__ state) {
-    double s = 0.0;
-    unsigned long long c = 0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        s += sums[i];
-        c += cnts[i];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        s += __shfl_xor_sync(0xffffffffu, s, o);
-        c += __shfl_xor_sync(0xffffffffu, c, o);
-    }
-    if ((threadIdx.x & 31) == 0 && (s != 0.0 || c != 0)) {
-        atomicAdd(&state->sum, s);
-        atomicAdd(&state->count, c);
     }
 }
 
@@ -1017,19 +1054,12 @@ hc_status raster_forward(const Topology& topo, RasterWorkspace& ws, cudaStream_t
     A.render = render;
     A.depth_q = depth_q;
     A.tie_count = tie_count;
-    A.l1_target = nullptr;
-    A.l1_mask = nullptr;
-    A.l1_sum = nullptr;
-    A.l1_cnt = nullptr;
-    const long long l1_n = tiles * (TS * TS / 32);  // warp partials of the fused L1
-    if (l1) {
-        HC_TRY(ws.l1_part.ensure(8 * (size_t)l1_n));
-        HC_CUDA(cudaMemsetAsync(l1->state, 0, sizeof(L1State), s));
-        A.l1_target = l1->target;
-        A.l1_mask = l1->mask;
-        A.l1_sum = ws.l1_part.as<float>();
-        A.l1_cnt = reinterpret_cast<unsigned*>(A.l1_sum + l1_n);
-    }
+    A.vec = (((uintptr_t)bary | (uintptr_t)face | (uintptr_t)render) & 15) == 0;
+    for (int w : ws.cam_w) A.vec = A.vec && w % 4 == 0;
+    A.l1_target = l1 ? l1->target : nullptr;
+    A.l1_mask = l1 ? l1->mask : nullptr;
+    A.l1_state = l1 ? l1->state : nullptr;
+    if (l1) HC_CUDA(cudaMemsetAsync(l1->state, 0, sizeof(L1State), s));
     const int* tcam = ws.tile_cam.as<int>();
     HC_REQUIRE(tiles < (1ll << 31), "too many tiles in one call (%lld)", tiles);
     HC_TRY(ws.claim.ensure(sizeof(unsigned long long)));
@@ -1058,8 +1088,6 @@ hc_status raster_forward(const Topology& topo, RasterWorkspace& ws, cudaStream_t
     HC_CHECK_LAUNCH();
     ws.clock.end(kKResolve, s);
     if (l1) {
-        k_l1_tiles<<<148 * 2, 256, 0, s>>>(l1_n, A.l1_sum, A.l1_cnt, l1->state);
-        HC_CHECK_LAUNCH();
         if (l1->loss) {
             k_l1_loss<<<1, 1, 0, s>>>(l1->state, l1->loss);
             HC_CHECK_LAUNCH();
