@@ -24,6 +24,7 @@
 #include "eg_rot.cuh"
 #include "hc_common.cuh"
 #include "hc_math.cuh"
+#include "renderer.cuh"  // FanFace
 
 namespace hc {
 namespace {
@@ -83,98 +84,101 @@ __global__ void k_eg_nodes(int B, int M, const float* __restrict__ base, const i
     }
 }
 
-// Deformed vertices (EmbeddedGraphGPUOp.cu:50-125), grid (vertex blocks,
-// frames).  The block's vertex -> node entries (a contiguous range of the
-// packed CSR) are staged in shared memory by coalesced loads; each (vertex,
-// node) pair then reads the node's rotation / translation rows as float4
-// loads of the 16-byte aligned table and the vertex as one float4.  Sums in
-// the reference's order: v_nr = sum_k w_k (R_dk (v - g_k) + g_k + t_dk) +
-// disp, then sum_k w_k (R_sk v_nr + t_sk).
+// The vertex pass, grid (vertex blocks, frames), a thread per vertex:
+//   kEgForward      the deformed vertex (EmbeddedGraphGPUOp.cu:50-125)
+//   kEgAdjoint      u_v = (sum_k w_k R_sk)^T g_v, the displacement gradient
+//   kEgAdjointFull  u_v, and (u, g, v_nr, base vertex) packed in three 16-byte
+//                   words per vertex for the node pass's gathers
+// Sums in the reference's order: v_nr = sum_k w_k (R_dk (v - g_k) + g_k + t_dk)
+// + disp, then sum_k w_k (R_sk v_nr + t_sk).
+// Bound by the wavefronts of its gathers (28 16-byte loads per vertex at four
+// nodes; copying a block's distinct nodes to shared memory first gained
+// nothing: a block's vertices lie all over the mesh and share few nodes).  16
+// frames x 40,962 vertices, 1000 nodes: 37 -> 33 us without the staging of the
+// entries; the adjoint 60 -> 36 us, the outer sum it does not need left out and
+// u_v formed in the same pass.
 constexpr int kEgBlock = 128;
-constexpr int kEgStage = 8 * kEgBlock;  // staged (node, weight) entries per block
+enum { kEgForward = 0, kEgAdjoint, kEgAdjointFull };
+constexpr int kEgRows = sizeof(NodeRT) / sizeof(float4);
 
-__global__ void __launch_bounds__(kEgBlock) k_eg_vertices(int B, int N, int M, const float4* __restrict__ base4,
+template <int MODE>
+__global__ void __launch_bounds__(kEgBlock) k_eg_vertices(int N, int M, const float4* __restrict__ base4,
                                                           const int* __restrict__ poff, const int* __restrict__ pidx,
-                                                          const float* __restrict__ pw, const NodeRT* __restrict__ tab,
-                                                          const float* __restrict__ disp, float* __restrict__ out,
-                                                          float* __restrict__ vnr_out) {
-    __shared__ int s_idx[kEgStage];
-    __shared__ float s_w[kEgStage];
+                                                          const float* __restrict__ pw,
+                                                          const NodeRT* __restrict__ tab,
+                                                          const float* __restrict__ disp,
+                                                          const float* __restrict__ gv, float* __restrict__ out,
+                                                          float4* __restrict__ packed) {
     const int b = blockIdx.y;
-    const int v0 = blockIdx.x * kEgBlock, v1 = min(v0 + kEgBlock, N);
-    const int e0 = poff[v0], e1 = poff[v1];
-    const bool staged = e1 - e0 <= kEgStage;  // block-uniform
-    if (staged)
-        for (int e = e0 + (int)threadIdx.x; e < e1; e += kEgBlock) {
-            s_idx[e - e0] = pidx[e];
-            s_w[e - e0] = pw[e];
-        }
-    __syncthreads();
-    const int v = v0 + (int)threadIdx.x;
+    const int v = blockIdx.x * kEgBlock + (int)threadIdx.x;
     if (v >= N) return;
+    const float4* T = reinterpret_cast<const float4*>(tab + (long long)b * M);
     const long long i = (long long)b * N + v;
     const int off = poff[v], cnt = poff[v + 1] - off;
-    const int* I = staged ? s_idx + (off - e0) : pidx + off;
-    const float* Wt = staged ? s_w + (off - e0) : pw + off;
+    auto weight = [&](int k) { return pw[off + k]; };
+    auto row = [&](int k, int r) { return T[(long long)pidx[off + k] * kEgRows + r]; };
+    auto rotation = [&](float4 a, float4 c, float4 d) {
+        R33 R;
+        R.m[0] = a.x;
+        R.m[1] = a.y;
+        R.m[2] = a.z;
+        R.m[3] = a.w;
+        R.m[4] = c.x;
+        R.m[5] = c.y;
+        R.m[6] = c.z;
+        R.m[7] = c.w;
+        R.m[8] = d.x;
+        return R;
+    };
     const float4 vb4 = base4[v];
-    const float3 vb = make_float3(vb4.x, vb4.y, vb4.z);
-    const float4* T = reinterpret_cast<const float4*>(tab + (long long)b * M);
-    constexpr int kRows = sizeof(NodeRT) / sizeof(float4);
     float3 vnr = make_float3(0.f, 0.f, 0.f);
-    for (int k = 0; k < cnt; ++k) {
-        const float4* q = T + (long long)I[k] * kRows;
-        const float w = Wt[k];
-        const float4 a = q[0], c = q[1], d = q[2], gg = q[6];
-        R33 R;
-        R.m[0] = a.x;
-        R.m[1] = a.y;
-        R.m[2] = a.z;
-        R.m[3] = a.w;
-        R.m[4] = c.x;
-        R.m[5] = c.y;
-        R.m[6] = c.z;
-        R.m[7] = c.w;
-        R.m[8] = d.x;
-        const float3 g = make_float3(gg.x, gg.y, gg.z);
-        vnr += w * (mv(R, vb - g) + g + make_float3(d.y, d.z, d.w));
+    if constexpr (MODE != kEgAdjoint) {
+        const float3 vb = make_float3(vb4.x, vb4.y, vb4.z);
+        for (int k = 0; k < cnt; ++k) {
+            const float w = weight(k);
+            const float4 d = row(k, 2), gg = row(k, 6);
+            const R33 R = rotation(row(k, 0), row(k, 1), d);
+            const float3 g = make_float3(gg.x, gg.y, gg.z);
+            vnr += w * (mv(R, vb - g) + g + make_float3(d.y, d.z, d.w));
+        }
+        vnr += ld3(disp + 3 * i);
     }
-    vnr += ld3(disp + 3 * i);
-    float3 dsum = make_float3(0.f, 0.f, 0.f);
-    for (int k = 0; k < cnt; ++k) {
-        const float4* q = T + (long long)I[k] * kRows;
-        const float w = Wt[k];
-        const float4 a = q[3], c = q[4], d = q[5];
-        R33 R;
-        R.m[0] = a.x;
-        R.m[1] = a.y;
-        R.m[2] = a.z;
-        R.m[3] = a.w;
-        R.m[4] = c.x;
-        R.m[5] = c.y;
-        R.m[6] = c.z;
-        R.m[7] = c.w;
-        R.m[8] = d.x;
-        dsum += w * (mv(R, vnr) + make_float3(d.y, d.z, d.w));
+    if constexpr (MODE == kEgForward) {
+        float3 dsum = make_float3(0.f, 0.f, 0.f);
+        for (int k = 0; k < cnt; ++k) {
+            const float w = weight(k);
+            const float4 d = row(k, 5);
+            const R33 R = rotation(row(k, 3), row(k, 4), d);
+            dsum += w * (mv(R, vnr) + make_float3(d.y, d.z, d.w));
+        }
+        st3(out + 3 * i, dsum);
+    } else {
+        float S[9];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) S[q] = 0.f;
+        for (int k = 0; k < cnt; ++k) {
+            const float w = weight(k);
+            const R33 R = rotation(row(k, 3), row(k, 4), row(k, 5));
+#pragma unroll
+            for (int q = 0; q < 9; ++q) S[q] = S[q] + R.m[q] * w;
+        }
+        const float3 g = ld3(gv + 3 * i), u = mtv(S, g);
+        st3(out + 3 * i, u);
+        if constexpr (MODE == kEgAdjointFull) {
+            packed[3 * i] = make_float4(u.x, u.y, u.z, vnr.x);
+            packed[3 * i + 1] = make_float4(g.x, g.y, g.z, vnr.y);
+            packed[3 * i + 2] = make_float4(vb4.x, vb4.y, vb4.z, vnr.z);
+        }
     }
-    st3(out + 3 * i, dsum);
-    if (vnr_out) st3(vnr_out + 3 * i, vnr);
 }
 
 // normalised area-weighted normal of the deformed mesh (EmbeddedGraphGPUOp.cu:180-225)
-__global__ void k_eg_normals(int B, int N, const int3* __restrict__ faces, const int* __restrict__ vf,
-                             const int2* __restrict__ vf_id, const float* __restrict__ dv, float* __restrict__ out) {
+__global__ void k_eg_normals(int B, int N, const int2* __restrict__ fan, const int2* __restrict__ vf_id,
+                             const float* __restrict__ dv, float* __restrict__ out) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= (long long)B * N) return;
     const int b = (int)(i / N), v = (int)(i % N);
-    const float* P = dv + (long long)b * N * 3;
-    const int2 r = vf_id[v];
-    float3 s = make_float3(0.f, 0.f, 0.f);
-    for (int k = r.x; k < r.x + r.y; ++k) {
-        const int3 f = faces[vf[k]];
-        const float3 v0 = ld3(P + 3 * f.x), v1 = ld3(P + 3 * f.y), v2 = ld3(P + 3 * f.z);
-        s += cross(v1 - v0, v2 - v0);
-    }
-    st3(out + 3 * i, normalize3(s));
+    st3(out + 3 * i, normalize3(fan_normal(dv + (long long)b * N * 3, fan, vf_id[v], v)));
 }
 
 // deformed markers (EmbeddedGraphGPUOp.cu:129-177)
@@ -201,105 +205,94 @@ __global__ void k_eg_markers(int B, int Mk, int M, const float* __restrict__ bas
 // adjoint
 // ---------------------------------------------------------------------------
 
-// per (frame, vertex): u_v = (sum_s w_s R_s)^T g_v (= the displacement gradient)
-__global__ void k_eg_grad_vertex(int B, int N, int M, const int* __restrict__ v2n_off, const int* __restrict__ v2n_size,
-                                 const int* __restrict__ v2n_idx, const float* __restrict__ v2n_w,
-                                 const NodeRT* __restrict__ tab, const float* __restrict__ gv,
-                                 float* __restrict__ u_out) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= (long long)B * N) return;
-    const int b = (int)(i / N), v = (int)(i % N);
-    const int off = v2n_off[v], cnt = v2n_size[v];
-    const NodeRT* T = tab + (long long)b * M;
-    float S[9];
-#pragma unroll
-    for (int q = 0; q < 9; ++q) S[q] = 0.f;
-    for (int k = 0; k < cnt; ++k) {
-        const int n = v2n_idx[off + k];
-        const float w = v2n_w[off + k];
-#pragma unroll
-        for (int q = 0; q < 9; ++q) S[q] = S[q] + T[n].rs[q] * w;
-    }
-    st3(u_out + 3 * i, mtv(S, ld3(gv + 3 * i)));
-}
-
-// per (frame, node): gather over the node's vertices (and its marker)
-__global__ void k_eg_grad_node(int B, int N, int M, int Mk, const float* __restrict__ base,
-                               const int* __restrict__ node_vertex, const int* __restrict__ n2v_off,
-                               const int* __restrict__ n2v_size, const int* __restrict__ n2v_idx,
-                               const float* __restrict__ n2v_w, const int* __restrict__ n2m,
-                               const float* __restrict__ markers, const float* __restrict__ dA,
-                               const float* __restrict__ sA, const float* __restrict__ gv,
-                               const float* __restrict__ gm, const float* __restrict__ u,
-                               const float* __restrict__ vnr, const NodeRT* __restrict__ tab, int full,
-                               float* __restrict__ gT, float* __restrict__ gA, float* __restrict__ gsT,
-                               float* __restrict__ gsA) {
-    // one warp per (frame, node): lanes split the node's vertex list, then a
-    // warp reduction; lane 0 adds the marker term and writes
+// Per (frame, node), a warp: gather over the node's vertices (and its marker).
+// The gradient of an Euler angle is sum_v w (dR (v - g)) . u_v = dR : W with W =
+// sum_v w u_v (v - g)^T, so the lanes sum the nine entries of W (12 operations
+// per vertex instead of 45 for the three angles) and the angle derivatives
+// enter once per node; FULL: the skinned gradients likewise from sum w g_v and
+// sum w g_v v_nr^T, read from the vertices' packed values.  The 24 sums take
+// one 31-shuffle reduction.  Bound by its gathers: 16 frames x 1000 nodes of
+// 164 vertices 49 -> 34 us.
+template <bool FULL>
+__global__ void __launch_bounds__(256) k_eg_grad_node(
+    int B, int N, int M, int Mk, const float4* __restrict__ base4, const int* __restrict__ node_vertex,
+    const int* __restrict__ n2v_off, const int* __restrict__ n2v_size, const int* __restrict__ n2v_idx,
+    const float* __restrict__ n2v_w, const int* __restrict__ n2m, const float* __restrict__ markers,
+    const float* __restrict__ dA, const float* __restrict__ sA, const float* __restrict__ gm,
+    const float* __restrict__ u, const float4* __restrict__ packed, const NodeRT* __restrict__ tab,
+    float* __restrict__ gT, float* __restrict__ gA, float* __restrict__ gsT, float* __restrict__ gsA) {
     const long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= (long long)B * M) return;  // warp-uniform
     const int b = (int)(i / M), n = (int)(i % M);
-    const float3 g = ld3(base + 3LL * node_vertex[n]);
-    R33 da, db, dc;
-    euler_rot_d(ld3(dA + 3 * i), da, db, dc);
-    R33 sda, sdb, sdc;
-    if (full) euler_rot_d(ld3(sA + 3 * i), sda, sdb, sdc);
-    float3 t = make_float3(0.f, 0.f, 0.f), a = make_float3(0.f, 0.f, 0.f);
-    float3 st = make_float3(0.f, 0.f, 0.f), sa = make_float3(0.f, 0.f, 0.f);
+    const float4 g4 = base4[node_vertex[n]];
+    const float3 g = make_float3(g4.x, g4.y, g4.z);
+    float a[32];  // t (3), W row-major (9); FULL: st (3), skinned W (9)
+#pragma unroll
+    for (int k = 0; k < 32; ++k) a[k] = 0.f;
+    auto moment = [&](int at, float3 x, float3 y) {  // x, and x y^T
+        a[at] += x.x;
+        a[at + 1] += x.y;
+        a[at + 2] += x.z;
+        a[at + 3] += x.x * y.x;
+        a[at + 4] += x.x * y.y;
+        a[at + 5] += x.x * y.z;
+        a[at + 6] += x.y * y.x;
+        a[at + 7] += x.y * y.y;
+        a[at + 8] += x.y * y.z;
+        a[at + 9] += x.z * y.x;
+        a[at + 10] += x.z * y.y;
+        a[at + 11] += x.z * y.z;
+    };
     const int off = n2v_off[n], cnt = n2v_size[n];
     for (int k = lane; k < cnt; k += 32) {
         const int v = n2v_idx[off + k];
         const float w = n2v_w[off + k];
         const long long vi = (long long)b * N + v;
-        const float3 uv = ld3(u + 3 * vi);
-        const float3 d = ld3(base + 3LL * v) - g;
-        t += w * uv;
-        a += w * make_float3(dot(mv(da, d), uv), dot(mv(db, d), uv), dot(mv(dc, d), uv));
-        if (full) {
-            const float3 gvv = ld3(gv + 3 * vi), p = ld3(vnr + 3 * vi);
-            st += w * gvv;
-            sa += w * make_float3(dot(mv(sda, p), gvv), dot(mv(sdb, p), gvv), dot(mv(sdc, p), gvv));
+        if constexpr (FULL) {
+            const float4 q0 = packed[3 * vi], q1 = packed[3 * vi + 1], q2 = packed[3 * vi + 2];
+            moment(0, w * make_float3(q0.x, q0.y, q0.z), make_float3(q2.x, q2.y, q2.z) - g);
+            moment(12, w * make_float3(q1.x, q1.y, q1.z), make_float3(q0.w, q1.w, q2.w));
+        } else {
+            const float4 v4 = base4[v];
+            moment(0, w * ld3(u + 3 * vi), make_float3(v4.x, v4.y, v4.z) - g);
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
-        t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
-        t.z += __shfl_xor_sync(0xffffffffu, t.z, o);
-        a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
-        a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
-        a.z += __shfl_xor_sync(0xffffffffu, a.z, o);
-        if (full) {
-            st.x += __shfl_xor_sync(0xffffffffu, st.x, o);
-            st.y += __shfl_xor_sync(0xffffffffu, st.y, o);
-            st.z += __shfl_xor_sync(0xffffffffu, st.z, o);
-            sa.x += __shfl_xor_sync(0xffffffffu, sa.x, o);
-            sa.y += __shfl_xor_sync(0xffffffffu, sa.y, o);
-            sa.z += __shfl_xor_sync(0xffffffffu, sa.z, o);
-        }
-    }
-    if (lane != 0) return;
     const int m = n2m ? n2m[n] : -1;
-    if (m >= 0 && gm) {
+    if (lane == 0 && m >= 0 && gm) {
         // marker residual (EmbeddedGraphGPUOpGrad.cu:90-123): weight 1, its own node
         const NodeRT& T = tab[i];
         const float3 gmm = ld3(gm + 3 * ((long long)b * Mk + m));
-        const float3 um = mtv(T.rs, gmm);
         const float3 d = ld3(markers + 3LL * m) - g;
-        t += um;
-        a += make_float3(dot(mv(da, d), um), dot(mv(db, d), um), dot(mv(dc, d), um));
-        if (full) {
+        moment(0, mtv(T.rs, gmm), d);
+        if constexpr (FULL) {
             R33 Rd;
 #pragma unroll
             for (int q = 0; q < 9; ++q) Rd.m[q] = T.rd[q];
-            const float3 p = mv(Rd, d) + g + make_float3(T.td[0], T.td[1], T.td[2]);
-            st += gmm;
-            sa += make_float3(dot(mv(sda, p), gmm), dot(mv(sdb, p), gmm), dot(mv(sdc, p), gmm));
+            moment(12, gmm, mv(Rd, d) + g + make_float3(T.td[0], T.td[1], T.td[2]));
         }
     }
-    st3(gT + 3 * i, t);
-    st3(gA + 3 * i, a);
+    const float sum = warp_sum32(a, lane);  // lane k: value k
+    float r[24];
+#pragma unroll
+    for (int k = 0; k < (FULL ? 24 : 12); ++k) r[k] = __shfl_sync(0xffffffffu, sum, k);
+    if (lane != 0) return;
+    auto angle = [&](const R33& D, int at) {  // D : W
+        float acc = 0.f;
+#pragma unroll
+        for (int q = 0; q < 9; ++q) acc += D.m[q] * r[at + q];
+        return acc;
+    };
+    R33 d0, d1, d2;
+    euler_rot_d(ld3(dA + 3 * i), d0, d1, d2);
+    st3(gT + 3 * i, make_float3(r[0], r[1], r[2]));
+    st3(gA + 3 * i, make_float3(angle(d0, 3), angle(d1, 3), angle(d2, 3)));
+    float3 st = make_float3(0.f, 0.f, 0.f), sa = st;
+    if constexpr (FULL) {
+        euler_rot_d(ld3(sA + 3 * i), d0, d1, d2);
+        st = make_float3(r[12], r[13], r[14]);
+        sa = make_float3(angle(d0, 15), angle(d1, 15), angle(d2, 15));
+    }
     st3(gsT + 3 * i, st);
     st3(gsA + 3 * i, sa);
 }
@@ -315,14 +308,14 @@ using namespace hc;
 struct hc_eg_s {
     int N = 0, M = 0, Mk = 0, F = 0;
     int full_skinned_grad = 0;
-    DevBuf base, node_vertex, v2n_off, v2n_size, v2n_idx, v2n_w, n2v_off, n2v_size, n2v_idx, n2v_w;
+    DevBuf base, node_vertex, n2v_off, n2v_size, n2v_idx, n2v_w;
     DevBuf base4, v2n_poff, v2n_pidx, v2n_pw;  // float4 base vertices; the vertex -> node CSR packed in vertex order
-    DevBuf markers, m2n, n2m, faces, vf, vf_id;
-    DevBuf tab, u, vnr;
+    DevBuf markers, m2n, n2m, fan, vf_id;
+    DevBuf tab, packed;
 };
 
 namespace hc {
-void build_vertex_faces(int N, const int32_t* faces, int F, std::vector<int>& vf, std::vector<int>& vf_id);
+void build_vertex_fans(int N, const int32_t* faces, int F, std::vector<int2>& fan, std::vector<int>& vf_id);
 }
 
 extern "C" hc_status hc_eg_create(hc_eg* out, int32_t n_vertices, const float* base_vertices, const int32_t* faces,
@@ -339,6 +332,7 @@ extern "C" hc_status hc_eg_create(hc_eg* out, int32_t n_vertices, const float* b
                    v2n_weights && n2v_offsets && n2v_sizes && n2v_indices && n2v_weights,
                "NULL graph array");
     HC_REQUIRE(n_markers == 0 || (base_markers && marker_to_node), "markers need positions and node ids");
+    HC_REQUIRE(n_vertices < (1 << 30), "too many vertices (%d)", n_vertices);
     long long nv2n = 0, nn2v = 0;
     for (int v = 0; v < n_vertices; ++v) {
         HC_REQUIRE(v2n_sizes[v] >= 0 && v2n_offsets[v] >= 0, "bad vertex->node range at %d", v);
@@ -368,24 +362,20 @@ extern "C" hc_status hc_eg_create(hc_eg* out, int32_t n_vertices, const float* b
     h->M = n_nodes;
     h->Mk = n_markers;
     h->F = n_faces;
-    std::vector<int> vf, vf_id;
-    build_vertex_faces(n_vertices, faces, n_faces, vf, vf_id);
+    std::vector<int2> fan;
+    std::vector<int> vf_id;
+    build_vertex_fans(n_vertices, faces, n_faces, fan, vf_id);
     hc_status st = HC_OK;
 #define UP(buf, ptr, n)                                   \
     if (st == HC_OK) st = upload(h->buf, ptr, (size_t)(n));
     UP(base, base_vertices, 3LL * n_vertices);
     UP(node_vertex, node_to_base_vertex, n_nodes);
-    UP(v2n_off, v2n_offsets, n_vertices);
-    UP(v2n_size, v2n_sizes, n_vertices);
-    UP(v2n_idx, v2n_indices, std::max<long long>(nv2n, 1));
-    UP(v2n_w, v2n_weights, std::max<long long>(nv2n, 1));
     UP(n2v_off, n2v_offsets, n_nodes);
     UP(n2v_size, n2v_sizes, n_nodes);
     UP(n2v_idx, n2v_indices, std::max<long long>(nn2v, 1));
     UP(n2v_w, n2v_weights, std::max<long long>(nn2v, 1));
     UP(n2m, n2m.data(), n_nodes);
-    UP(faces, faces, 3LL * n_faces);
-    UP(vf, vf.data(), vf.size());
+    UP(fan, fan.data(), fan.size());
     UP(vf_id, vf_id.data(), vf_id.size());
     if (n_markers > 0) {
         UP(markers, base_markers, 3LL * n_markers);
@@ -427,9 +417,9 @@ extern "C" hc_status hc_eg_create(hc_eg* out, int32_t n_vertices, const float* b
 extern "C" hc_status hc_eg_destroy(hc_eg h) {
     clear_error();
     if (!h) return HC_OK;
-    DevBuf* bufs[] = {&h->base, &h->node_vertex, &h->v2n_off, &h->v2n_size, &h->v2n_idx, &h->v2n_w, &h->n2v_off,
-                      &h->n2v_size, &h->n2v_idx, &h->n2v_w, &h->markers, &h->m2n, &h->n2m, &h->faces, &h->vf,
-                      &h->vf_id, &h->tab, &h->u, &h->vnr, &h->base4, &h->v2n_poff, &h->v2n_pidx, &h->v2n_pw};
+    DevBuf* bufs[] = {&h->base, &h->node_vertex, &h->n2v_off,
+                      &h->n2v_size, &h->n2v_idx, &h->n2v_w, &h->markers, &h->m2n, &h->n2m, &h->fan,
+                      &h->vf_id, &h->tab, &h->packed, &h->base4, &h->v2n_poff, &h->v2n_pidx, &h->v2n_pw};
     for (DevBuf* b : bufs) b->release();
     delete h;
     return HC_OK;
@@ -446,8 +436,17 @@ extern "C" hc_status hc_eg_reserve(hc_eg h, int32_t batch) {
     clear_error();
     HC_REQUIRE(h && batch > 0, "invalid handle or batch");
     HC_TRY(h->tab.ensure(sizeof(NodeRT) * (size_t)batch * h->M));
-    HC_TRY(h->u.ensure(sizeof(float) * 3 * (size_t)batch * h->N));
-    HC_TRY(h->vnr.ensure(sizeof(float) * 3 * (size_t)batch * h->N));
+    HC_TRY(h->packed.ensure(3 * sizeof(float4) * (size_t)batch * h->N));
+    return HC_OK;
+}
+
+template <int MODE>
+static hc_status launch_vertices(hc_eg h, cudaStream_t s, int B, const float* disp, const float* gv, float* out) {
+    HC_REQUIRE(B <= 65535, "too many frames in one call (%d)", B);
+    k_eg_vertices<MODE><<<dim3(div_up(h->N, kEgBlock), B), kEgBlock, 0, s>>>(
+        h->N, h->M, h->base4.as<float4>(), h->v2n_poff.as<int>(), h->v2n_pidx.as<int>(), h->v2n_pw.as<float>(),
+        h->tab.as<NodeRT>(), disp, gv, out, h->packed.as<float4>());
+    HC_CHECK_LAUNCH();
     return HC_OK;
 }
 
@@ -472,14 +471,10 @@ extern "C" hc_status hc_eg_forward(hc_eg h, void* stream, int32_t batch, const f
                                                nodes_skinned_translation, nodes_skinned_rotation, tab, deformed_graph,
                                                d_delta_rotation, d_skinned_rotation);
     HC_CHECK_LAUNCH();
-    HC_REQUIRE(batch <= 65535, "too many frames in one call (%d)", batch);
-    k_eg_vertices<<<dim3(div_up(h->N, kEgBlock), batch), kEgBlock, 0, s>>>(
-        batch, h->N, h->M, h->base4.as<float4>(), h->v2n_poff.as<int>(), h->v2n_pidx.as<int>(),
-        h->v2n_pw.as<float>(), tab, vertex_displacements, deformed_vertices, nullptr);
-    HC_CHECK_LAUNCH();
+    HC_TRY(launch_vertices<kEgForward>(h, s, batch, vertex_displacements, nullptr, deformed_vertices));
     if (deformed_normals) {
-        k_eg_normals<<<div_up(BN, 128), 128, 0, s>>>(batch, h->N, h->faces.as<int3>(), h->vf.as<int>(),
-                                                     h->vf_id.as<int2>(), deformed_vertices, deformed_normals);
+        k_eg_normals<<<div_up(BN, 128), 128, 0, s>>>(batch, h->N, h->fan.as<int2>(), h->vf_id.as<int2>(),
+                                                     deformed_vertices, deformed_normals);
         HC_CHECK_LAUNCH();
     }
     if (h->Mk > 0) {
@@ -519,26 +514,18 @@ extern "C" hc_status hc_eg_backward(hc_eg h, void* stream, int32_t batch, const 
                                                nullptr, nullptr);
     HC_CHECK_LAUNCH();
     if (full) {
-        HC_TRY(h->vnr.ensure(sizeof(float) * 3 * (size_t)BN));
-        HC_TRY(h->u.ensure(sizeof(float) * 3 * (size_t)BN));
-        // v_nr of every vertex (the outer sum's argument); the deformed output
-        // goes to the scratch u buffer and is overwritten below
-        HC_REQUIRE(batch <= 65535, "too many frames in one call (%d)", batch);
-        k_eg_vertices<<<dim3(div_up(h->N, kEgBlock), batch), kEgBlock, 0, s>>>(
-            batch, h->N, h->M, h->base4.as<float4>(), h->v2n_poff.as<int>(), h->v2n_pidx.as<int>(),
-            h->v2n_pw.as<float>(), tab, vertex_displacements, h->u.as<float>(), h->vnr.as<float>());
-        HC_CHECK_LAUNCH();
+        HC_TRY(h->packed.ensure(3 * sizeof(float4) * (size_t)BN));
+        HC_TRY(launch_vertices<kEgAdjointFull>(h, s, batch, vertex_displacements, deformed_vertices_grad,
+                                               vertex_displacements_grad));
+    } else {
+        HC_TRY(launch_vertices<kEgAdjoint>(h, s, batch, nullptr, deformed_vertices_grad, vertex_displacements_grad));
     }
-    k_eg_grad_vertex<<<div_up(BN, 128), 128, 0, s>>>(batch, h->N, h->M, h->v2n_off.as<int>(), h->v2n_size.as<int>(),
-                                                     h->v2n_idx.as<int>(), h->v2n_w.as<float>(), tab,
-                                                     deformed_vertices_grad, vertex_displacements_grad);
-    HC_CHECK_LAUNCH();
-    k_eg_grad_node<<<div_up(BM * 32, 256), 256, 0, s>>>(
-        batch, h->N, h->M, h->Mk, h->base.as<float>(), h->node_vertex.as<int>(), h->n2v_off.as<int>(),
+    auto kernel = full ? k_eg_grad_node<true> : k_eg_grad_node<false>;
+    kernel<<<div_up(BM * 32, 256), 256, 0, s>>>(
+        batch, h->N, h->M, h->Mk, h->base4.as<float4>(), h->node_vertex.as<int>(), h->n2v_off.as<int>(),
         h->n2v_size.as<int>(), h->n2v_idx.as<int>(), h->n2v_w.as<float>(), h->n2m.as<int>(), h->markers.as<float>(),
-        d_delta_a, d_skinned_a, deformed_vertices_grad, deformed_markers_grad, vertex_displacements_grad,
-        full ? h->vnr.as<float>() : nullptr, tab, full ? 1 : 0, nodes_t_grad, nodes_r_grad, nodes_skinned_t_grad,
-        nodes_skinned_r_grad);
+        d_delta_a, d_skinned_a, deformed_markers_grad, vertex_displacements_grad, h->packed.as<float4>(), tab,
+        nodes_t_grad, nodes_r_grad, nodes_skinned_t_grad, nodes_skinned_r_grad);
     HC_CHECK_LAUNCH();
     return HC_OK;
 }

@@ -134,6 +134,21 @@ HC_HD M44 inverse44(const M44& m) {
     return r;
 }
 
+#ifdef __CUDACC__
+// Sums of 32 values over the warp: lane k ends with the sum of value k (31
+// shuffles instead of five per value).
+__device__ __forceinline__ float warp_sum32(float v[32], int lane) {
+#pragma unroll
+    for (int h = 16; h > 0; h >>= 1)
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const float keep = (lane & h) ? v[i + h] : v[i], send = (lane & h) ? v[i] : v[i + h];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+        }
+    return v[0];
+}
+#endif
+
 // Masked image L1 of the training step (Projects/HoloportedCharacters/
 // HPCMeshDL.py:642-688).  One channel's difference: render and target scaled
 // by 255 and then subtracted, each product rounded on its own as the separate

@@ -405,6 +405,45 @@ __device__ __forceinline__ float3 bilinear_sample(const float* T, const Bilinear
     return c00 * w00 + c10 * w10 + c01 * w01 + c11 * w11;
 }
 
+// One incident face of a vertex: the ids of its other two vertices in the
+// face's order, and the vertex's own place in the face (0 to 2) in the top two
+// bits of the second.  A fan walk reads one 8-byte entry and two vertices per
+// face, where face ids would cost the id, three vertex ids and three vertices.
+struct FanFace {
+    int p, q, place;
+    __device__ __forceinline__ explicit FanFace(int2 e) : p(e.x), q(e.y & 0x3fffffff), place((unsigned)e.y >> 30) {}
+    // the face's three values in its order, from the own one and the others'
+    template <class T>
+    __device__ __forceinline__ void order(const T& own, const T& a, const T& b, T& v0, T& v1, T& v2) const {
+        v0 = place == 0 ? own : a;
+        v1 = place == 0 ? a : place == 1 ? own : b;
+        v2 = place == 2 ? own : b;
+    }
+};
+
+// Sum of a vertex's incident face normals in increasing face order.
+__device__ __forceinline__ float3 fan_normal(const float* __restrict__ P, const int2* __restrict__ fan, int2 range,
+                                             int v) {
+    const float3 own = ld3(P + 3 * v);
+    float3 s = make_float3(0.f, 0.f, 0.f);
+#pragma unroll 3
+    for (int k = 0; k < range.y; ++k) {
+        const FanFace f(fan[range.x + k]);
+        const float3 a = ld3(P + 3 * f.p), b = ld3(P + 3 * f.q);
+        float3 v0, v1, v2;
+        f.order(own, a, b, v0, v1, v2);
+        const float3 fn = cross(v1 - v0, v2 - v0);
+        if (k == 0) {
+            s = fn;
+        } else {
+            s.x = s.x + fn.x;
+            s.y = s.y + fn.y;
+            s.z = s.z + fn.z;
+        }
+    }
+    return s;
+}
+
 // Second-order SH shading of an albedo (reference getShading,
 // CudaRenderer/cpp/src/Utils/RendererUtil.h:135-173), one band set per channel.
 __device__ __forceinline__ float sh_channel(const float* s, float3 d, float3 d2) {
@@ -428,7 +467,7 @@ __device__ __forceinline__ float3 sh_illum(const float* sh, float3 n) {
 struct Topology {
     int N = 0, F = 0;
     DevBuf faces;        // int3[F]
-    DevBuf vf;           // int[3F]  vertex -> faces, increasing face id
+    DevBuf fan;          // int2[3F]  vertex -> incident faces, increasing face id (FanFace)
     DevBuf vf_id;        // int2[N]  (start, count)
     DevBuf texcoords;    // float[6F]
     bool has_texcoords = false;

@@ -51,10 +51,11 @@ static int parse_normal_map(const char* m) {
 
 // Vertex -> incident faces in increasing face order, by counting sort
 // (the reference builds the same lists with an O(N*F) scan,
-// CudaRenderer/cpp/src/Renderer/CUDABasedRasterization.cpp:154-183).  A face
-// that names a vertex twice is listed once for it.  Vertices without faces get
-// an empty range (the reference drops them from the offset table).
-void build_vertex_faces(int N, const int32_t* faces, int F, std::vector<int>& vf, std::vector<int>& vf_id) {
+// CudaRenderer/cpp/src/Renderer/CUDABasedRasterization.cpp:154-183), each face
+// as the other two vertices and the vertex's own place in it (see FanFace).  A
+// face that names a vertex twice is listed once for it.  Vertices without faces
+// get an empty range (the reference drops them from the offset table).
+void build_vertex_fans(int N, const int32_t* faces, int F, std::vector<int2>& fan, std::vector<int>& vf_id) {
     std::vector<int> cnt(N + 1, 0);
     for (int f = 0; f < F; ++f) {
         const int a = faces[3 * f], b = faces[3 * f + 1], c = faces[3 * f + 2];
@@ -69,25 +70,28 @@ void build_vertex_faces(int N, const int32_t* faces, int F, std::vector<int>& vf
         vf_id[2 * v] = start[v];
         vf_id[2 * v + 1] = cnt[v];
     }
-    vf.assign(start[N], 0);
+    fan.assign(start[N], make_int2(0, 0));
     std::vector<int> fill(start.begin(), start.end() - 1);
+    auto entry = [](int p, int q, unsigned place) { return make_int2(p, (int)((unsigned)q | place << 30)); };
     for (int f = 0; f < F; ++f) {
         const int a = faces[3 * f], b = faces[3 * f + 1], c = faces[3 * f + 2];
-        vf[fill[a]++] = f;
-        if (b != a) vf[fill[b]++] = f;
-        if (c != a && c != b) vf[fill[c]++] = f;
+        fan[fill[a]++] = entry(b, c, 0);
+        if (b != a) fan[fill[b]++] = entry(a, c, 1);
+        if (c != a && c != b) fan[fill[c]++] = entry(a, b, 2);
     }
 }
 
 hc_status topology_upload(Topology& t, int N, const int32_t* faces, int F, const float* texcoords, int n_tc) {
     for (int i = 0; i < 3 * F; ++i)
         HC_REQUIRE(faces[i] >= 0 && faces[i] < N, "face %d references vertex %d outside [0,%d)", i / 3, faces[i], N);
-    std::vector<int> vf, vf_id;
-    build_vertex_faces(N, faces, F, vf, vf_id);
+    HC_REQUIRE(N < (1 << 30), "too many vertices (%d)", N);
+    std::vector<int2> fan;
+    std::vector<int> vf_id;
+    build_vertex_fans(N, faces, F, fan, vf_id);
     t.N = N;
     t.F = F;
     HC_TRY(upload(t.faces, faces, (size_t)3 * F));
-    HC_TRY(upload(t.vf, vf.data(), vf.size()));
+    HC_TRY(upload(t.fan, fan.data(), fan.size()));
     HC_TRY(upload(t.vf_id, vf_id.data(), vf_id.size()));
     if (texcoords && n_tc == 6 * F) {
         HC_TRY(upload(t.texcoords, texcoords, (size_t)6 * F));
@@ -176,7 +180,7 @@ static void release_all(hc_renderer_s* r) {
     if (r->ws.clock.made)
         for (cudaEvent_t& e : r->ws.clock.ev) cudaEventDestroy(e);
     r->ws.clock.made = false;
-    DevBuf* bufs[] = {&r->topo.faces, &r->topo.vf, &r->topo.vf_id, &r->topo.texcoords,
+    DevBuf* bufs[] = {&r->topo.faces, &r->topo.fan, &r->topo.vf_id, &r->topo.texcoords,
                       &r->ws.cams, &r->ws.tri_frame, &r->ws.tri_view, &r->ws.tile_state,
                       &r->ws.bins, &r->ws.spill, &r->ws.spill_keys, &r->ws.stats, &r->vacc, &r->tacc, &r->tpad,
                       &r->uv.faces, &r->uv.table, &r->ws.layout, &r->ws.tile_cam, &r->ws.tile_cam_b, &r->ws.proj,

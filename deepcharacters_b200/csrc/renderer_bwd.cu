@@ -166,19 +166,6 @@ __device__ __forceinline__ void image_gradient(Tap tap, float x, float y, int w,
     }
 }
 
-// Sums of 32 values over the warp: lane k ends with the sum of value k (31
-// shuffles instead of five per value).
-__device__ __forceinline__ float warp_sum32(float v[32], int lane) {
-#pragma unroll
-    for (int h = 16; h > 0; h >>= 1)
-#pragma unroll
-        for (int i = 0; i < h; ++i) {
-            const float keep = (lane & h) ? v[i + h] : v[i], send = (lane & h) ? v[i] : v[i + h];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
-        }
-    return v[0];
-}
-
 // Exact barycentric Jacobian of a ray hit.  With P = o + t d = l0 v0 + l1 v1 +
 // l2 v2 (l2 = 1 - l0 - l1), perturbing vertex i moves (t, l0, l1) by
 // l_i M^-1 dv_i with M = [d, -(v0 - v2), -(v1 - v2)], so
@@ -813,8 +800,8 @@ __global__ void __launch_bounds__(BNT, SHADED ? 2 : 4) k_render_grad(BwdArgs A, 
 //   x: g x (z - y),  y: (z - x) x g,  z: g x (y - x).
 // Bound by its gathers; the sums are at most 48 bytes per vertex.
 template <bool SHADED, int ALB>
-__global__ void k_vertex_grad(int B, int N, const int3* __restrict__ faces, const int* __restrict__ vf,
-                              const int2* __restrict__ vf_id, const float* __restrict__ verts,
+__global__ void k_vertex_grad(int B, int N, const int2* __restrict__ fan, const int2* __restrict__ vf_id,
+                              const float* __restrict__ verts,
                               const float* __restrict__ vacc, float* __restrict__ vpos_grad,
                               float* __restrict__ vcol_grad) {
     using Sums = VertexSums<SHADED, ALB>;
@@ -829,14 +816,17 @@ __global__ void k_vertex_grad(int B, int N, const int3* __restrict__ faces, cons
         const float* P = verts + (long long)b * N * 3;
         const float* Gn = vacc + (long long)b * N * Sums::kStride + Sums::kNormal;
         const int2 r = vf_id[v];
+        const float3 own = ld3(P + 3 * v), own_g = ld3(Gn + (long long)Sums::kStride * v);
         float3 acc = make_float3(0.f, 0.f, 0.f);
         for (int k = r.x; k < r.x + r.y; ++k) {
-            const int3 f = faces[vf[k]];
-            const float3 g = ld3(Gn + (long long)Sums::kStride * f.x) + ld3(Gn + (long long)Sums::kStride * f.y) +
-                             ld3(Gn + (long long)Sums::kStride * f.z);
-            const float3 x = ld3(P + 3 * f.x), y = ld3(P + 3 * f.y), z = ld3(P + 3 * f.z);
-            if (v == f.x) acc += cross(g, z - y);
-            else if (v == f.y) acc += cross(z - x, g);
+            const FanFace f(fan[k]);
+            const float3 p = ld3(P + 3 * f.p), q = ld3(P + 3 * f.q);
+            float3 x, y, z, gx, gy, gz;
+            f.order(own, p, q, x, y, z);
+            f.order(own_g, ld3(Gn + (long long)Sums::kStride * f.p), ld3(Gn + (long long)Sums::kStride * f.q), gx, gy, gz);
+            const float3 g = gx + gy + gz;
+            if (f.place == 0) acc += cross(g, z - y);
+            else if (f.place == 1) acc += cross(z - x, g);
             else acc += cross(g, y - x);
         }
         g0.x += acc.x;
@@ -1038,7 +1028,7 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vac
 #define HC_VERTEX_CASE(SH, AL)                                                                                \
     case (SH ? 4 : 0) + AL:                                                                                   \
         k_vertex_grad<SH, AL><<<div_up((long long)B * N, 256), 256, 0, s>>>(                                  \
-            B, N, topo.faces.as<int3>(), topo.vf.as<int>(), topo.vf_id.as<int2>(), verts, vacc.as<float>(),   \
+            B, N, topo.fan.as<int2>(), topo.vf_id.as<int2>(), verts, vacc.as<float>(),                        \
             vpos_grad, vcol_grad);                                                                            \
         break;
         HC_VERTEX_CASE(false, kAlbVcol)

@@ -99,28 +99,15 @@ __global__ void k_view_setup(int V, int C, const float* __restrict__ extr, const
 // CUDABasedRasterization.cu:122-174, computed once per frame and written for
 // every camera of the [B,C,N,3] output)
 // ---------------------------------------------------------------------------
-__global__ void k_vertex_normals(int B, int C, int N, const int3* __restrict__ faces,
-                                 const int* __restrict__ vf, const int2* __restrict__ vf_id,
+// Bound by its gathers (FanFace): 16 frames x 40,962 vertices, 8 cameras, 43 ->
+// 25 us.
+__global__ void k_vertex_normals(int B, int C, int N, const int2* __restrict__ fan, const int2* __restrict__ vf_id,
                                  const float* __restrict__ verts, float* __restrict__ out) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= (long long)B * N) return;
     const int b = (int)(i / N);
     const int v = (int)(i % N);
-    const float* P = verts + (long long)b * N * 3;
-    const int2 r = vf_id[v];
-    float3 s = make_float3(0.f, 0.f, 0.f);
-    for (int k = r.x; k < r.x + r.y; ++k) {
-        const int3 f = faces[vf[k]];
-        const float3 v0 = ld3(P + 3 * f.x), v1 = ld3(P + 3 * f.y), v2 = ld3(P + 3 * f.z);
-        const float3 fn = cross(v1 - v0, v2 - v0);
-        if (k == r.x) {
-            s = fn;
-        } else {
-            s.x = s.x + fn.x;
-            s.y = s.y + fn.y;
-            s.z = s.z + fn.z;
-        }
-    }
+    const float3 s = fan_normal(verts + (long long)b * N * 3, fan, vf_id[v], v);
     for (int c = 0; c < C; ++c) st3(out + (((long long)b * C + c) * N + v) * 3, s);
 }
 
@@ -1005,7 +992,7 @@ hc_status raster_forward(const Topology& topo, RasterWorkspace& ws, cudaStream_t
     ws.clock.end(kKViewSetup, s);
     ws.clock.begin(kKVertexNormals, s);
     k_vertex_normals<<<div_up((long long)B * N, 256), 256, 0, s>>>(
-        B, C, N, topo.faces.as<int3>(), topo.vf.as<int>(), topo.vf_id.as<int2>(), verts, vnormal);
+        B, C, N, topo.fan.as<int2>(), topo.vf_id.as<int2>(), verts, vnormal);
     HC_CHECK_LAUNCH();
     ws.clock.end(kKVertexNormals, s);
     ws.clock.begin(kKTriFrame, s);

@@ -133,9 +133,8 @@ __global__ void k_uv_map(int B, int C, int N, int n_texels, int mode, const int3
 
 }  // namespace
 
-__global__ void k_vertex_normals(int B, int C, int N, const int3* __restrict__ faces, const int* __restrict__ vf,
-                                 const int2* __restrict__ vf_id, const float* __restrict__ verts,
-                                 float* __restrict__ out);
+__global__ void k_vertex_normals(int B, int C, int N, const int2* __restrict__ fan, const int2* __restrict__ vf_id,
+                                 const float* __restrict__ verts, float* __restrict__ out);
 
 hc_status raster_uv_maps(const Topology& topo, UvTable& tab, cudaStream_t s, int B, int C, long long P_frame, int mode,
                          const float* verts, int tex_h, int tex_w, float* bary, int* face, float* render,
@@ -148,7 +147,7 @@ hc_status raster_uv_maps(const Topology& topo, UvTable& tab, cudaStream_t s, int
     HC_CUDA(cudaMemsetAsync(bary, 0, sizeof(float) * 2 * px, s));
     HC_CUDA(cudaMemsetAsync(render, 0, sizeof(float) * 3 * px, s));
     const int N = topo.N, F = topo.F;
-    k_vertex_normals<<<div_up((long long)B * N, 256), 256, 0, s>>>(B, C, N, topo.faces.as<int3>(), topo.vf.as<int>(),
+    k_vertex_normals<<<div_up((long long)B * N, 256), 256, 0, s>>>(B, C, N, topo.fan.as<int2>(),
                                                                     topo.vf_id.as<int2>(), verts, vnormal);
     HC_CHECK_LAUNCH();
     const int nt = tex_h * tex_w;
