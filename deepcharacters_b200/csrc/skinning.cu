@@ -19,6 +19,7 @@
 // A_s = sum_v w (v x g_v) and G_s = sum_v w g_v, so a single parallel
 // reduction over vertices replaces the serial loops.
 #include <math.h>
+#include <string.h>
 
 #include <algorithm>
 #include <vector>
@@ -118,7 +119,7 @@ struct Skel {
     // the adjoint's vertex blocks: each block's (vertex, slot) pairs by skinning joint
     int grad_block;          // vertices per block
     const int* bone_off;     // [blocks, S+1]
-    const int2* bone_slot;   // [N,K]: (vertex * K + slot, vertex) within the block
+    const unsigned* bone_slot;  // [N,K]: (vertex * K + slot) << 8 | vertex, within the block
     const int* skin_idx;   // [N,K] skinning joint per vertex slot
     const float* base_v;   // [N,3]
     const float* base_n;   // [N,3]
@@ -601,10 +602,10 @@ __global__ void __launch_bounds__(256) k_skin_grad(Skel sk, int B, const float* 
         if (e0 == e1) continue;
         float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         for (int e = e0 + lane; e < e1; e += 32) {
-            const int2 q = sk.bone_slot[e];
-            const float wk = s_w[q.x];
+            const unsigned q = sk.bone_slot[e];
+            const float wk = s_w[q >> 8];
 #pragma unroll
-            for (int c = 0; c < 6; ++c) a[c] += wk * s_m[c * G + q.y];
+            for (int c = 0; c < 6; ++c) a[c] += wk * s_m[c * G + (q & 255u)];
         }
         const float t = warp_sum8(a, lane);
         if (lane < 6 && t != 0.f) atomicAdd(mom + ((long long)b * sk.S + s) * 6 + lane, t);
@@ -883,7 +884,8 @@ struct hc_skin_s {
     int parity = 1;
     DevBuf parent, type, offset, axis, jscale, dof_off, dof_joint, dof_w, skin_joint, skin_scale, t0inv, in_chain,
         skin_idx, base_v, base_n, base_v4, base_n4;
-    DevBuf joint_off, joint_dof, joint_w, level_off, level_joint, bone_off, bone_slot;
+    DevBuf tree;   // joint_off, joint_dof, joint_w, level_off, level_joint of Skel
+    DevBuf bones;  // bone_off, bone_slot of Skel
     DevBuf mom, gpos, gaxis, dq_ws, gdq;
     int levels = 0, grad_block = 0;
     Skel skel() const {
@@ -911,14 +913,14 @@ struct hc_skin_s {
         s.base_v4 = base_v4.as<float4>();
         s.base_n4 = base_n4.as<float4>();
         s.levels = levels;
-        s.joint_off = joint_off.as<int>();
-        s.joint_dof = joint_dof.as<int>();
-        s.joint_w = joint_w.as<float>();
-        s.level_off = level_off.as<int>();
-        s.level_joint = level_joint.as<int>();
+        s.joint_off = tree.as<int>();
+        s.joint_dof = s.joint_off + J + 1;
+        s.joint_w = reinterpret_cast<const float*>(s.joint_dof + E);
+        s.level_off = s.joint_dof + 2 * E;
+        s.level_joint = s.level_off + levels + 1;
         s.grad_block = grad_block;
-        s.bone_off = bone_off.as<int>();
-        s.bone_slot = bone_slot.as<int2>();
+        s.bone_off = bones.as<int>();
+        s.bone_slot = bones.as<unsigned>() + (size_t)((N + grad_block - 1) / grad_block) * (S + 1);
         return s;
     }
 };
@@ -1032,54 +1034,54 @@ extern "C" hc_status hc_skin_create(hc_skin* out, int32_t n_joints, const int32_
         UP(base_n4, bn4.data(), bn4.size());
     }
     {
-        // the dof entries by joint (in dof order), and the joints by depth
-        std::vector<int> joff(n_joints + 1, 0), jdof(std::max(E, 1), 0), depth(n_joints, 0);
-        std::vector<float> jw(std::max(E, 1), 0.f);
+        // the dof entries by joint (in dof order), and the joints by depth, in
+        // one buffer: joint offsets, dofs, weights (as bits), level offsets, joints
+        std::vector<int> depth(n_joints, 0), joff(n_joints + 1, 0);
         for (int e = 0; e < E; ++e) joff[dof_joint[e] + 1]++;
         for (int j = 0; j < n_joints; ++j) joff[j + 1] += joff[j];
-        std::vector<int> at(joff.begin(), joff.end() - 1);
-        for (int d = 0; d < n_dofs; ++d)
-            for (int e = dof_offsets[d]; e < dof_offsets[d + 1]; ++e) {
-                jdof[at[dof_joint[e]]] = d;
-                jw[at[dof_joint[e]]++] = dof_weight[e];
-            }
         for (int j = 0; j < n_joints; ++j) {
             depth[j] = parent[j] < 0 ? 0 : depth[parent[j]] + 1;
             h->levels = std::max(h->levels, depth[j] + 1);
         }
-        std::vector<int> loff(h->levels + 1, 0), lj;
-        for (int l = 0; l < h->levels; ++l) {
-            for (int j = 0; j < n_joints; ++j)
-                if (depth[j] == l) lj.push_back((int)((unsigned)j << 16 | (unsigned)(parent[j] + 1)));
-            loff[l + 1] = (int)lj.size();
-        }
-        UP(joint_off, joff.data(), joff.size());
-        UP(joint_dof, jdof.data(), jdof.size());
-        UP(joint_w, jw.data(), jw.size());
-        UP(level_off, loff.data(), loff.size());
-        UP(level_joint, lj.data(), lj.size());
+        std::vector<int> tree(joff);
+        tree.resize((size_t)n_joints + 1 + 2 * (size_t)E + h->levels + 1);
+        int* jdof = tree.data() + n_joints + 1;
+        int* level_off = jdof + 2 * (size_t)E;
+        std::vector<int> at(joff.begin(), joff.end() - 1);
+        for (int d = 0; d < n_dofs; ++d)
+            for (int e = dof_offsets[d]; e < dof_offsets[d + 1]; ++e) {
+                const int k = at[dof_joint[e]]++;
+                jdof[k] = d;
+                memcpy(jdof + E + k, dof_weight + e, sizeof(float));
+            }
+        for (int j = 0; j < n_joints; ++j) level_off[depth[j] + 1]++;
+        for (int l = 0; l < h->levels; ++l) level_off[l + 1] += level_off[l];
+        std::vector<int> order(n_joints), next(level_off, level_off + h->levels);
+        for (int j = 0; j < n_joints; ++j)
+            order[next[depth[j]]++] = (int)((unsigned)j << 16 | (unsigned)(parent[j] + 1));
+        tree.insert(tree.end(), order.begin(), order.end());
+        UP(tree, tree.data(), tree.size());
     }
     {
-        // each adjoint block's (vertex, slot) pairs by skinning joint, vertices ascending
+        // each adjoint block's (vertex, slot) pairs by skinning joint, vertices
+        // ascending: the blocks' offsets, then the pairs
         const int G = h->grad_block = skin_grad_smem(n_skin, 12, k, 256) <= (96u << 10) ? 256 : 128;
-        const int blocks = div_up(n_vertices, G);
-        std::vector<int> off;
-        std::vector<int2> slot((size_t)n_vertices * k);
-        off.reserve((size_t)blocks * (n_skin + 1));
-        std::vector<int> cnt(n_skin + 1);
-        for (int q = 0; q < blocks; ++q) {
-            const int v0 = q * G, v1 = std::min(v0 + G, n_vertices);
-            std::fill(cnt.begin(), cnt.end(), 0);
+        const size_t blocks = (size_t)div_up(n_vertices, G);
+        std::vector<unsigned> bones(blocks * (n_skin + 1) + (size_t)n_vertices * k);
+        unsigned* slot = bones.data() + blocks * (n_skin + 1);
+        std::vector<unsigned> cnt(n_skin + 1);
+        for (size_t q = 0; q < blocks; ++q) {
+            const int v0 = (int)q * G, v1 = std::min(v0 + G, n_vertices);
+            std::fill(cnt.begin(), cnt.end(), 0u);
             for (long long i = (long long)v0 * k; i < (long long)v1 * k; ++i) cnt[skin_index[i] + 1]++;
-            cnt[0] = v0 * k;
+            cnt[0] = (unsigned)(v0 * k);
             for (int s = 0; s < n_skin; ++s) cnt[s + 1] += cnt[s];
-            off.insert(off.end(), cnt.begin(), cnt.end());
+            std::copy(cnt.begin(), cnt.end(), bones.begin() + q * (n_skin + 1));
             for (int v = v0; v < v1; ++v)
                 for (int c = 0; c < k; ++c)
-                    slot[cnt[skin_index[(long long)v * k + c]]++] = make_int2((v - v0) * k + c, v - v0);
+                    slot[cnt[skin_index[(long long)v * k + c]]++] = (unsigned)((v - v0) * k + c) << 8 | (unsigned)(v - v0);
         }
-        UP(bone_off, off.data(), off.size());
-        UP(bone_slot, slot.data(), slot.size());
+        UP(bones, bones.data(), bones.size());
     }
 #undef UP
     if (st != HC_OK) {
@@ -1095,8 +1097,7 @@ extern "C" hc_status hc_skin_destroy(hc_skin h) {
     if (!h) return HC_OK;
     DevBuf* bufs[] = {&h->parent, &h->type, &h->offset, &h->axis, &h->jscale, &h->dof_off, &h->dof_joint, &h->dof_w,
                       &h->skin_joint, &h->skin_scale, &h->t0inv, &h->in_chain, &h->skin_idx, &h->base_v,
-                      &h->base_n, &h->joint_off, &h->joint_dof, &h->joint_w, &h->level_off, &h->level_joint,
-                      &h->bone_off, &h->bone_slot, &h->mom, &h->gpos, &h->gaxis,
+                      &h->base_n, &h->tree, &h->bones, &h->mom, &h->gpos, &h->gaxis,
                       &h->dq_ws, &h->gdq};
     for (DevBuf* b : bufs) b->release();
     delete h;
