@@ -587,16 +587,23 @@ __global__ void __launch_bounds__(256, 4) k_cov_bin_list(int N, int F, const int
 // record that one of its open pixels still needed).  A warp stops when all its
 // pixels are covered, the tile at the chunk after which all are.
 // Bound by instruction issue.  16 views of 81,920 triangles at 1024^2: 552 ->
-// 382 us.
+// 374 us.
 __global__ void __launch_bounds__(kCovTile* kCovTile) k_cov_tile(int F, long long n_keys, CovBins cb,
                                                                   const __grid_constant__ ImgLayout L) {
     constexpr int NT = kCovTile * kCovTile, RW = 32 / kCovTile, kRec = sizeof(CovTileTri) / 16;
     static_assert(sizeof(CovTileTri) == 16 * kRec, "records are copied in 16-byte pieces");
     __shared__ __align__(16) CovTileTri s_t[NT];
     const int listed = *cb.n_tiles, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // the next tile's index and count are loaded while this one is processed
+    long long next = blockIdx.x < listed ? cb.tiles[blockIdx.x] : 0;
+    int next_n = blockIdx.x < listed ? cb.count[next] : 0;
     for (int it = blockIdx.x; it < listed; it += gridDim.x) {
-        const long long key = cb.tiles[it];
-        const int n = min(cb.count[key], kCovCap);
+        const long long key = next;
+        const int n = min(next_n, kCovCap);
+        if (it + (int)gridDim.x < listed) {
+            next = cb.tiles[it + gridDim.x];
+            next_n = cb.count[next];
+        }
         int tile;
         const int view = view_of_tile(L, key, tile);
         const ViewImg vi = view_img(L, view);
@@ -927,88 +934,81 @@ __device__ __forceinline__ void sil_pixel_warp(long long view, const ViewImg& vi
     }
 }
 
-// Four consecutive pixels per thread, grid (pixel blocks of one view, views):
-// one 4-byte DT load and 16-byte stores when the buffers allow (vec), and
-// 32-bit index arithmetic.  Most pixels are not on the boundary and only
-// write their zero outputs; in the vec path each boundary pixel is searched
-// by a whole warp (sil_pixel_warp), the block's boundary pixels dealt to its
-// warps in turn, instead of leaving one lane to search while the others wait.
-// Launched with 256 threads (the shared lists hold the block's 1024 pixels).
-__global__ void __launch_bounds__(256, 5) k_sil_pixels(int N, const __grid_constant__ ImgLayout L, SilGrid g,
+// Data -> model term of a block of consecutive pixels of one view, grid (pixel
+// blocks, views).  Most pixels are not on the boundary and only get their zero
+// outputs, so a block stores those first, in consecutive 16-byte words that
+// wait for nothing, while its distance pixels are loaded, 16 per thread.  The
+// boundary pixels (value 127) are listed in shared memory and dealt to the
+// block's warps in turn (a contour running along a row can put dozens in one
+// warp's pixels); a warp searches one at a time (sil_pixel_warp) and overwrites
+// its outputs after the barrier.
+// vec: views of a multiple of four pixels and aligned buffers; otherwise four
+// pixels per thread, each searched by its thread.
+// Bound by HBM: 13 bytes per pixel.  16 views of 1024^2: 67 -> 46 us.
+constexpr int kSilBlock = 256;
+constexpr int kSilPixels = 16 * kSilBlock;  // pixels of a block (vec)
+
+__global__ void __launch_bounds__(kSilBlock) k_sil_pixels(int N, const __grid_constant__ ImgLayout L, SilGrid g,
                              const float* __restrict__ p2d, const unsigned char* __restrict__ dt,
                              const float* __restrict__ crops, float* __restrict__ residual1,
                              float* __restrict__ closest, int vec, double* __restrict__ sumsq1) {
     const long long view = blockIdx.y;
     const ViewImg vi = view_img(L, (int)view);
     const int P = vi.W * vi.H;
-    const int p0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
-    if (4 * (int)(blockIdx.x * blockDim.x) >= P) return;  // blocks past a smaller view's pixels (CTA-uniform)
     const unsigned char* D = dt + vi.pix;
-    const long long i0 = vi.pix + p0;
-    if (vec) {  // P % 4 == 0 and aligned buffers: all four pixels of an active thread exist
-        // The block's boundary pixels are listed in shared memory and dealt to
-        // its warps in turn (a contour running along a row can put dozens in
-        // one warp's 128 pixels); their results come back through shared
-        // memory to the threads that own the pixels and store them.
+    if (vec) {
         __shared__ int s_n;
-        __shared__ unsigned short s_list[4 * 256];
-        __shared__ float2 s_r[4 * 256];
-        __shared__ float s_c[4 * 256];
-        const bool active = p0 < P;  // no early exit: every thread takes part in the barriers
-        int dv[4] = {0, 0, 0, 0};
-        if (active) {
-            const uchar4 d4 = *reinterpret_cast<const uchar4*>(D + p0);
-            dv[0] = d4.x;
-            dv[1] = d4.y;
-            dv[2] = d4.z;
-            dv[3] = d4.w;
-        }
+        __shared__ unsigned short s_list[kSilPixels];
+        const int pb = kSilPixels * blockIdx.x, m = min(kSilPixels, P - pb);
+        if (m <= 0) return;  // blocks past a smaller view's pixels (CTA-uniform)
+        const long long i0 = vi.pix + pb;
         if (threadIdx.x == 0) s_n = 0;
+        uchar4 d[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int q = (int)threadIdx.x + k * kSilBlock;  // word of four pixels
+            d[k] = 4 * q < m ? reinterpret_cast<const uchar4*>(D + pb)[q] : make_uchar4(0, 0, 0, 0);
+        }
+        float4* r4 = reinterpret_cast<float4*>(residual1 + 2 * i0);
+        float4* c4 = reinterpret_cast<float4*>(closest + i0);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int q = (int)threadIdx.x + k * kSilBlock;
+            if (2 * q < m) r4[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int q = (int)threadIdx.x + k * kSilBlock;
+            if (4 * q < m) c4[q] = make_float4(-1.f, -1.f, -1.f, -1.f);
+        }
         __syncthreads();
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (dv[k] == 127) s_list[atomicAdd(&s_n, 1)] = (unsigned short)(4 * threadIdx.x + k);
+        for (int k = 0; k < 4; ++k) {
+            const int p = 4 * ((int)threadIdx.x + k * kSilBlock);
+            if (d[k].x == 127) s_list[atomicAdd(&s_n, 1)] = (unsigned short)p;
+            if (d[k].y == 127) s_list[atomicAdd(&s_n, 1)] = (unsigned short)(p + 1);
+            if (d[k].z == 127) s_list[atomicAdd(&s_n, 1)] = (unsigned short)(p + 2);
+            if (d[k].w == 127) s_list[atomicAdd(&s_n, 1)] = (unsigned short)(p + 3);
+        }
         __syncthreads();
         const int n = s_n, lane = threadIdx.x & 31;
-        const int pb = 4 * (int)(blockIdx.x * blockDim.x);  // the block's first pixel
-        for (int e = threadIdx.x >> 5; e < n; e += blockDim.x >> 5) {  // warp-uniform
+        float q = 0.f;
+        for (int e = threadIdx.x >> 5; e < n; e += kSilBlock >> 5) {  // warp-uniform
             const int lp = s_list[e];
             float a0, a1, cl;
             sil_pixel_warp(view, vi, pb + lp, N, g, p2d, D, crops, lane, a0, a1, cl);
-            if (lane == 0) {
-                s_r[lp] = make_float2(a0, a1);
-                s_c[lp] = cl;
+            if (lane == 0 && cl >= 0.f) {
+                reinterpret_cast<float2*>(residual1)[i0 + lp] = make_float2(a0, a1);
+                closest[i0 + lp] = cl;
+                q += a0 * a0 + a1 * a1;
             }
         }
-        __syncthreads();
-        float r[8], c[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            r[2 * k] = r[2 * k + 1] = 0.f;
-            c[k] = -1.f;
-            if (dv[k] == 127) {
-                const float2 q = s_r[4 * threadIdx.x + k];
-                r[2 * k] = q.x;
-                r[2 * k + 1] = q.y;
-                c[k] = s_c[4 * threadIdx.x + k];
-            }
-        }
-        if (active) {
-            reinterpret_cast<float4*>(residual1 + 2 * i0)[0] = make_float4(r[0], r[1], r[2], r[3]);
-            reinterpret_cast<float4*>(residual1 + 2 * i0)[1] = make_float4(r[4], r[5], r[6], r[7]);
-            *reinterpret_cast<float4*>(closest + i0) = make_float4(c[0], c[1], c[2], c[3]);
-        }
-        if (sumsq1) {  // launch-uniform: the squared residuals, one reduction per warp that has any
-            float q = 0.f;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) q += r[k] * r[k];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-            if (lane == 0 && q != 0.f) atomicAdd(sumsq1, (double)q);
-        }
+        if (sumsq1 && lane == 0 && q != 0.f) atomicAdd(sumsq1, (double)q);
         return;
     }
+    const int p0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (p0 >= P) return;
+    const long long i0 = vi.pix + p0;
     float q = 0.f;
     for (int k = 0; k < 4 && p0 + k < P; ++k) {
         float r0, r1, cl;
@@ -1034,36 +1034,48 @@ __global__ void k_sil_grad_points(long long n, const float* __restrict__ dtgrad,
     out[2 * i + 1] = dtgrad[2 * i + 1] * g[i];
 }
 
-// four pixels per thread on a (pixel block, view) grid: one 16-byte load of
-// closest_vertex_id when the buffer allows (vec); the rare boundary pixels
-// scatter their residual gradient to the closest vertex
-__global__ void k_sil_grad_pixels(int N, const __grid_constant__ ImgLayout L, const float* __restrict__ g1,
-                                  float s1, const float* __restrict__ closest, const float* __restrict__ crops,
-                                  float* __restrict__ out, int vec) {
+// sixteen pixels per thread on a (pixel block, view) grid: four consecutive
+// 16-byte loads of closest_vertex_id per warp when the buffer allows (vec),
+// all in flight at once; the rare boundary pixels scatter their residual
+// gradient to the closest vertex
+__global__ void __launch_bounds__(kSilBlock) k_sil_grad_pixels(int N, const __grid_constant__ ImgLayout L,
+                                                               const float* __restrict__ g1, float s1,
+                                                               const float* __restrict__ closest,
+                                                               const float* __restrict__ crops,
+                                                               float* __restrict__ out, int vec) {
     const long long view = blockIdx.y;
     const ViewImg vi = view_img(L, (int)view);
-    const int P = vi.W * vi.H;
-    const int p0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
-    if (p0 >= P) return;
-    const long long i0 = vi.pix + p0;
-    float cl[4];
-    if (vec) {
-        const float4 c4 = *reinterpret_cast<const float4*>(closest + i0);
-        cl[0] = c4.x;
-        cl[1] = c4.y;
-        cl[2] = c4.z;
-        cl[3] = c4.w;
-    } else {
-        for (int k = 0; k < 4; ++k) cl[k] = p0 + k < P ? closest[i0 + k] : -1.f;
+    const int P = vi.W * vi.H, pb = kSilPixels * blockIdx.x;
+    const long long i0 = vi.pix + pb;
+    float4 c[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int p = 4 * ((int)threadIdx.x + k * kSilBlock);
+        c[k] = make_float4(-1.f, -1.f, -1.f, -1.f);
+        if (pb + p >= P) continue;
+        if (vec) {
+            c[k] = *reinterpret_cast<const float4*>(closest + i0 + p);
+        } else {
+            c[k].x = closest[i0 + p];
+            if (pb + p + 1 < P) c[k].y = closest[i0 + p + 1];
+            if (pb + p + 2 < P) c[k].z = closest[i0 + p + 2];
+            if (pb + p + 3 < P) c[k].w = closest[i0 + p + 3];
+        }
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const int cv = (int)cl[k];
-        if (cv < 0) continue;
-        const float scale = crops[view * 7 + 2];
-        float* o = out + (view * N + cv) * 2;
-        atomicAdd(o, s1 * g1[2 * (i0 + k)] / (30.f * scale));  // (s1 x g) exact for s1 = 1
-        atomicAdd(o + 1, s1 * g1[2 * (i0 + k) + 1] / (30.f * scale));
+        const float cl[4] = {c[k].x, c[k].y, c[k].z, c[k].w};
+        if (fmaxf(fmaxf(cl[0], cl[1]), fmaxf(cl[2], cl[3])) < 0.f) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int cv = (int)cl[j];
+            if (cv < 0) continue;
+            const long long i = i0 + 4 * ((int)threadIdx.x + k * kSilBlock) + j;
+            const float scale = crops[view * 7 + 2];
+            float* o = out + (view * N + cv) * 2;
+            atomicAdd(o, s1 * g1[2 * i] / (30.f * scale));  // (s1 x g) exact for s1 = 1
+            atomicAdd(o + 1, s1 * g1[2 * i + 1] / (30.f * scale));
+        }
     }
 }
 
@@ -1453,7 +1465,8 @@ hc_status sil_forward_run(cudaStream_t s, int* base, const ImgLayout& L, int32_t
     {
         const int vec = pixels_by_four(L) && ((uintptr_t)distance_transform_image & 3) == 0 &&
                         ((uintptr_t)mv_dt_residual_1 & 15) == 0 && ((uintptr_t)closest_vertex_id & 15) == 0;
-        k_sil_pixels<<<dim3(div_up(max_view_pixels(L), 4 * 256), (unsigned)views), 256, 0, s>>>(
+        k_sil_pixels<<<dim3(div_up(max_view_pixels(L), vec ? kSilPixels : 4 * kSilBlock), (unsigned)views), kSilBlock, 0,
+                       s>>>(
             N, L, g, points_image_space, distance_transform_image, multi_view_crops, mv_dt_residual_1,
             closest_vertex_id, vec, sumsq_1);
     }
@@ -1480,7 +1493,7 @@ hc_status sil_backward_run(cudaStream_t s, int32_t batch, int32_t n_cameras, int
     k_sil_grad_points<<<div_up(np, 256), 256, 0, s>>>(np, dt_image_grad, mv_dt_grad, points_image_space_grad);
     HC_CHECK_LAUNCH();
     const int vec = pixels_by_four(L) && ((uintptr_t)closest_vertex_id & 15) == 0;
-    k_sil_grad_pixels<<<dim3(div_up(max_view_pixels(L), 4 * 256), (unsigned)views), 256, 0, s>>>(
+    k_sil_grad_pixels<<<dim3(div_up(max_view_pixels(L), kSilPixels), (unsigned)views), kSilBlock, 0, s>>>(
         n_points, L, mv_dt_grad_1, scale_1, closest_vertex_id, multi_view_crops, points_image_space_grad, vec);
     HC_CHECK_LAUNCH();
     return HC_OK;
