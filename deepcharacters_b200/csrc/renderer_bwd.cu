@@ -285,8 +285,15 @@ __device__ __forceinline__ void add_vertex(float* slot, const float* a) {
     if constexpr (rest == 1) atomicAdd(slot + at, a[at]);
 }
 
+// Resident CTAs per SM the adjoint is compiled for (registers per thread): it
+// waits on gathers, so more CTAs help until their spills cost more.  4 (64) for
+// the closed form, 3 (80) with the parity formula (1784 -> 1766 us at 4 x 8 x
+// 1024^2) or shading (9 x 643 x 477: 160 -> 144 us), 2 (128) with both (207 us
+// at 3, 187 at 2).
+constexpr int adjoint_ctas(bool shaded, bool parity) { return 4 - (shaded ? 1 : 0) - (parity ? 1 : 0); }
+
 template <bool SHADED, int ALB, bool PARITY, bool DYN>
-__global__ void __launch_bounds__(BNT, SHADED ? 2 : 4) k_render_grad(BwdArgs A, const ViewCam* __restrict__ cams, long long n_tiles,
+__global__ void __launch_bounds__(BNT, adjoint_ctas(SHADED, PARITY)) k_render_grad(BwdArgs A, const ViewCam* __restrict__ cams, long long n_tiles,
                                                                      const __grid_constant__ CUtensorMap tmap,
                                                                      int use_tma) {
     using Sums = VertexSums<SHADED, ALB>;
