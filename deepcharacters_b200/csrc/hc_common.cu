@@ -41,6 +41,16 @@ int resident_ctas(const void* kernel, int threads) {
     return sms * per_sm;
 }
 
+__global__ void k_fill(FillRuns runs) {
+    fill_runs(runs, blockIdx.x * (long long)blockDim.x + threadIdx.x, gridDim.x * (long long)blockDim.x);
+}
+
+hc_status fill(const FillRuns& runs, cudaStream_t s) {
+    k_fill<<<runs.blocks(256), 256, 0, s>>>(runs);
+    HC_CHECK_LAUNCH();
+    return HC_OK;
+}
+
 }  // namespace hc
 
 extern "C" const char* hc_last_error(void) { return hc::g_last_error.c_str(); }

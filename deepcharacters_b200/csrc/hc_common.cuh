@@ -97,4 +97,46 @@ unsigned resident_grid(K kernel, int threads, long long items) {
 
 inline int div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
 
+// Device ranges to fill with a byte each, by one launch or by spare blocks of a
+// kernel that is launched anyway: a memset of its own costs a launch (0.8 to 1.4
+// us of device time and its gap) for a few bytes.
+struct FillRuns {
+    static constexpr int kMost = 6;
+    char* p[kMost];
+    long long n[kMost];
+    unsigned word[kMost];  // the byte, four times
+    int count = 0;
+    void add(void* ptr, size_t bytes, unsigned char value = 0) {
+        p[count] = static_cast<char*>(ptr);
+        n[count] = (long long)bytes;
+        word[count++] = 0x01010101u * value;
+    }
+    // blocks of `threads` that fill with four 16-byte stores a thread, at most a
+    // few waves (the loop strides over the rest)
+    unsigned blocks(int threads) const {
+        long long b = 0;
+        for (int i = 0; i < count; ++i) b += n[i];
+        b = (b / 64 + threads - 1) / threads;
+        return (unsigned)(b < 1 ? 1 : b < 148 * 16 ? b : 148 * 16);
+    }
+};
+
+// thread t of nt fills its share of the ranges (any alignment, any size)
+__device__ __forceinline__ void fill_runs(const FillRuns& r, long long t, long long nt) {
+#pragma unroll
+    for (int i = 0; i < FillRuns::kMost; ++i) {
+        if (i >= r.count) break;
+        char* p = r.p[i];
+        const long long off = (long long)(-(uintptr_t)p & 15), head = off < r.n[i] ? off : r.n[i];
+        const long long body = (r.n[i] - head) >> 4, tail = head + (body << 4);
+        uint4* q = reinterpret_cast<uint4*>(p + head);
+        const uint4 w = make_uint4(r.word[i], r.word[i], r.word[i], r.word[i]);
+        for (long long k = t; k < body; k += nt) q[k] = w;
+        for (long long k = t; k < head; k += nt) p[k] = (char)r.word[i];
+        for (long long k = tail + t; k < r.n[i]; k += nt) p[k] = (char)r.word[i];
+    }
+}
+
+hc_status fill(const FillRuns& runs, cudaStream_t s);
+
 }  // namespace hc

@@ -477,7 +477,42 @@ struct Topology {
 struct UvTable {
     int th = 0, tw = 0;
     DevBuf faces, table;
+    DevBuf unit;  // normalised vertex normals of a call, 16 bytes each
 };
+
+// v / |v| (zero stays zero).  The contraction of |v|^2 is written out, so that
+// every kernel gives the same values: a vertex normal's and a texel's differ in
+// which of x^2 and y^2 is rounded first.
+template <bool TEXEL>
+__device__ __forceinline__ float3 unit_or_zero(float3 v) {
+    const float l = sqrtf(TEXEL ? __fmaf_rn(v.z, v.z, __fmaf_rn(v.y, v.y, v.x * v.x))
+                                : __fmaf_rn(v.z, v.z, __fmaf_rn(v.x, v.x, v.y * v.y)));
+    return l != 0.f ? v / l : v;
+}
+
+// Work on a frame's mesh before any tile: vertex normals, triangle constants
+// and projected vertices, one thread each.  They do not depend on one another,
+// so one launch covers them, and ranges to fill, by its blocks in this order;
+// a part without blocks is left out.
+struct FrameSetup {
+    int B, C, N, F;
+    const int3* faces;
+    const int2 *fan, *vf_id;
+    const float* verts;
+    float* vnormal;   // [B,C,N,3]
+    float4* unit;     // with the normals: normalised, [B,N], or NULL
+    TriFrame* tri;    // [B,F]
+    const ViewCam* cams;
+    float4* proj;     // [B*C,N]
+    unsigned normal_blocks = 0, tri_blocks = 0, project_blocks = 0;
+    FillRuns fills;
+};
+constexpr int kSetupThreads = 256, kViewThreads = 128;
+__global__ void k_frame_setup(FrameSetup S);
+// camera set-up, and ranges to fill by the blocks after the first view_blocks
+__global__ void k_view_setup(int V, int C, const float* __restrict__ extr, const float* __restrict__ intr,
+                             const CamLayout* __restrict__ layout, long long P_frame, long long T_frame,
+                             long long Tb_frame, ViewCam* __restrict__ cams, int view_blocks, FillRuns fills);
 
 // Optional per-kernel timing of the renderer (CUDA events around each
 // launch on the launching stream), for benchmarks; off by default.

@@ -183,7 +183,7 @@ static void release_all(hc_renderer_s* r) {
     DevBuf* bufs[] = {&r->topo.faces, &r->topo.fan, &r->topo.vf_id, &r->topo.texcoords,
                       &r->ws.cams, &r->ws.tri_frame, &r->ws.tri_view, &r->ws.tile_state,
                       &r->ws.bins, &r->ws.spill, &r->ws.spill_keys, &r->ws.stats, &r->vacc, &r->tacc, &r->tpad,
-                      &r->uv.faces, &r->uv.table, &r->ws.layout, &r->ws.tile_cam, &r->ws.tile_cam_b, &r->ws.proj,
+                      &r->uv.faces, &r->uv.table, &r->uv.unit, &r->ws.layout, &r->ws.tile_cam, &r->ws.tile_cam_b, &r->ws.proj,
                       &r->ws.claim, &r->ws.claim_b};
     for (DevBuf* b : bufs) b->release();
 }
@@ -203,6 +203,7 @@ extern "C" hc_status hc_renderer_reserve(hc_renderer h, int32_t batch) {
     HC_TRY(h->ws.tri_frame.ensure(sizeof(TriFrame) * (size_t)batch * h->topo.F));
     HC_TRY(h->ws.proj.ensure(sizeof(float4) * (size_t)batch * h->C * h->topo.N));
     HC_TRY(h->vacc.ensure(sizeof(float) * 12 * (size_t)batch * h->topo.N));  // the widest VertexSums
+    if (h->normal_map == kNmOriginal) HC_TRY(h->uv.unit.ensure(sizeof(float4) * (size_t)batch * h->topo.N));
     return HC_OK;
 }
 

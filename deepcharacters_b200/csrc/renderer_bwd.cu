@@ -25,11 +25,6 @@
 #include "renderer.cuh"
 
 namespace hc {
-
-__global__ void k_view_setup(int V, int C, const float* __restrict__ extr, const float* __restrict__ intr,
-                             const CamLayout* __restrict__ layout, long long P_frame, long long T_frame,
-                             long long Tb_frame, ViewCam* __restrict__ cams);
-
 namespace {
 
 constexpr int BT = 16;           // backward tile edge
@@ -912,7 +907,6 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vac
     const int stride = (3 + (alb == kAlbVcol ? 3 : 0) + (shaded ? 3 : 0) + 3) / 4 * 4;  // VertexSums::kStride
     const size_t vacc_bytes = sizeof(float) * (size_t)stride * (size_t)B * N;
     HC_TRY(vacc.ensure(vacc_bytes));
-    HC_CUDA(cudaMemsetAsync(vacc.ptr, 0, vacc_bytes, s));
     // Texels padded to 16 bytes where the padding's extra pass over the texture
     // costs less than it saves.  Sums (a clear, a read and a write, 32 bytes per
     // texel): two reductions per covered pixel (eight bilinear) become none;
@@ -941,12 +935,17 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vac
                          (albedo == kTextured && pixels >= 16 * texels)) &&
                         room(tacc);
     const bool taps = albedo == kTextured && texels > 0 && 4 * pixels >= texels && room(tpad);
-    if (padded) HC_CUDA(cudaMemsetAsync(tacc.ptr, 0, pad_bytes, s));
-    else if (texels) HC_CUDA(cudaMemsetAsync(tex_grad, 0, sizeof(float) * 3 * (size_t)texels, s));
-    if (sh_grad) HC_CUDA(cudaMemsetAsync(sh_grad, 0, sizeof(float) * 27 * (size_t)V, s));
+    HC_TRY(ws.claim_b.ensure(sizeof(unsigned)));
+    FillRuns zeros;
+    zeros.add(vacc.ptr, vacc_bytes);
+    if (padded) zeros.add(tacc.ptr, pad_bytes);
+    else if (texels) zeros.add(tex_grad, sizeof(float) * 3 * (size_t)texels);
+    if (sh_grad) zeros.add(sh_grad, sizeof(float) * 27 * (size_t)V);
+    zeros.add(ws.claim_b.ptr, sizeof(unsigned));
     ViewCam* cams = ws.cams.as<ViewCam>();
-    k_view_setup<<<div_up(V, 64), 64, 0, s>>>(V, C, extr, intr, ws.layout.as<CamLayout>(), ws.P_frame, ws.T_frame,
-                                              ws.Tb_frame, cams);
+    const int view_blocks = div_up(V, kViewThreads);
+    k_view_setup<<<view_blocks + zeros.blocks(kViewThreads), kViewThreads, 0, s>>>(
+        V, C, extr, intr, ws.layout.as<CamLayout>(), ws.P_frame, ws.T_frame, ws.Tb_frame, cams, view_blocks, zeros);
     HC_CHECK_LAUNCH();
     BwdArgs A;
     A.B = B;
@@ -990,10 +989,8 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vac
     A.l1_mask = l1 ? l1->mask : nullptr;
     const long long tiles = (long long)B * ws.Tb_frame;
     HC_REQUIRE(tiles < (1ll << 31), "too many adjoint tiles in one call (%lld)", tiles);
-    HC_TRY(ws.claim_b.ensure(sizeof(unsigned)));
     A.claim = ws.claim_b.as<unsigned>();
     const bool dyn = ws.adjoint_dynamic != 0;
-    if (dyn) HC_CUDA(cudaMemsetAsync(A.claim, 0, sizeof(unsigned), s));
     // the target's tensor map for the TMA staging, where its layout allows it
     CUtensorMap tmap;
     memset(&tmap, 0, sizeof(tmap));

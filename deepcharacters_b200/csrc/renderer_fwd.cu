@@ -24,7 +24,12 @@ namespace hc {
 // ---------------------------------------------------------------------------
 __global__ void k_view_setup(int V, int C, const float* __restrict__ extr, const float* __restrict__ intr,
                              const CamLayout* __restrict__ layout, long long P_frame, long long T_frame,
-                             long long Tb_frame, ViewCam* __restrict__ cams) {
+                             long long Tb_frame, ViewCam* __restrict__ cams, int view_blocks, FillRuns fills) {
+    if ((int)blockIdx.x >= view_blocks) {
+        fill_runs(fills, (blockIdx.x - view_blocks) * (long long)blockDim.x + threadIdx.x,
+                  (gridDim.x - view_blocks) * (long long)blockDim.x);
+        return;
+    }
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= V) return;
     {
@@ -94,58 +99,66 @@ __global__ void k_view_setup(int V, int C, const float* __restrict__ extr, const
 }
 
 // ---------------------------------------------------------------------------
-// vertex normals: unnormalised sum of incident face normals, in increasing
-// face order (reference renderFaceNormalDevice / renderVertexNormalDevice,
-// CUDABasedRasterization.cu:122-174, computed once per frame and written for
-// every camera of the [B,C,N,3] output)
+// a frame's mesh:
+// - vertex normals: unnormalised sum of incident face normals, in increasing
+//   face order (reference renderFaceNormalDevice / renderVertexNormalDevice,
+//   CUDABasedRasterization.cu:122-174, computed once per frame and written for
+//   every camera of the [B,C,N,3] output).  Bound by their gathers (FanFace).
+// - per-frame triangle constants
+// - per-view vertex projection (reference projectVerticesDevice,
+//   CUDABasedRasterization.cu:98-115): once per (view, vertex) instead of three
+//   times per (view, triangle); the same function, so the same values
+// One launch for the three (FrameSetup): with the camera set-up and the fills,
+// 8 launches and 13.8 us became 2 launches and 6.1 us (one 512^2 view of 20,480
+// triangles).
 // ---------------------------------------------------------------------------
-// Bound by its gathers (FanFace): 16 frames x 40,962 vertices, 8 cameras, 43 ->
-// 25 us.
-__global__ void k_vertex_normals(int B, int C, int N, const int2* __restrict__ fan, const int2* __restrict__ vf_id,
-                                 const float* __restrict__ verts, float* __restrict__ out) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= (long long)B * N) return;
-    const int b = (int)(i / N);
-    const int v = (int)(i % N);
-    const float3 s = fan_normal(verts + (long long)b * N * 3, fan, vf_id[v], v);
-    for (int c = 0; c < C; ++c) st3(out + (((long long)b * C + c) * N + v) * 3, s);
-}
-
-// ---------------------------------------------------------------------------
-// per-frame triangle constants
-// ---------------------------------------------------------------------------
-__global__ void k_tri_frame(int B, int F, int N, const int3* __restrict__ faces,
-                            const float* __restrict__ verts, TriFrame* __restrict__ out) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= (long long)B * F) return;
-    const int b = (int)(i / F);
-    const int f = (int)(i % F);
-    const float* P = verts + (long long)b * N * 3;
-    const int3 id = faces[f];
-    const float3 s0 = ld3(P + 3 * id.x) / 1000.f;
-    const float3 s1 = ld3(P + 3 * id.y) / 1000.f;
-    const float3 s2 = ld3(P + 3 * id.z) / 1000.f;
-    const float3 n = cross(s1 - s0, s2 - s0);
-    TriFrame t;
-    t.a = make_float4(s0.x, s0.y, s0.z, n.x);
-    t.b = make_float4(s1.x, s1.y, s1.z, n.y);
-    t.c = make_float4(s2.x, s2.y, s2.z, n.z);
-    out[i] = t;
-}
-
-// ---------------------------------------------------------------------------
-// per-view vertex projection (reference projectVerticesDevice,
-// CUDABasedRasterization.cu:98-115): once per (view, vertex) instead of three
-// times per (view, triangle); the same function, so the same values
-// ---------------------------------------------------------------------------
-__global__ void k_project_vertices(int V, int C, int N, const float* __restrict__ verts,
-                                   const ViewCam* __restrict__ cams, float4* __restrict__ proj) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= (long long)V * N) return;
-    const int view = (int)(i / N), v = (int)(i % N);
-    const ViewCam& cam = cams[view];
-    const float3 p = project_point(cam.ext, cam.intr, ld3(verts + ((long long)(view / C) * N + v) * 3));
-    proj[i] = make_float4(p.x, p.y, p.z, 0.f);
+__global__ void __launch_bounds__(kSetupThreads) k_frame_setup(FrameSetup S) {
+    unsigned blk = blockIdx.x;
+    if (blk < S.normal_blocks) {
+        const long long i = blk * (long long)blockDim.x + threadIdx.x;
+        if (i >= (long long)S.B * S.N) return;
+        const int b = (int)(i / S.N);
+        const int v = (int)(i % S.N);
+        const float3 s = fan_normal(S.verts + (long long)b * S.N * 3, S.fan, S.vf_id[v], v);
+        for (int c = 0; c < S.C; ++c) st3(S.vnormal + (((long long)b * S.C + c) * S.N + v) * 3, s);
+        if (S.unit) {
+            const float3 u = unit_or_zero<false>(s);
+            S.unit[i] = make_float4(u.x, u.y, u.z, 0.f);
+        }
+        return;
+    }
+    blk -= S.normal_blocks;
+    if (blk < S.tri_blocks) {
+        const long long i = blk * (long long)blockDim.x + threadIdx.x;
+        if (i >= (long long)S.B * S.F) return;
+        const int b = (int)(i / S.F);
+        const int f = (int)(i % S.F);
+        const float* P = S.verts + (long long)b * S.N * 3;
+        const int3 id = S.faces[f];
+        const float3 s0 = ld3(P + 3 * id.x) / 1000.f;
+        const float3 s1 = ld3(P + 3 * id.y) / 1000.f;
+        const float3 s2 = ld3(P + 3 * id.z) / 1000.f;
+        const float3 n = cross(s1 - s0, s2 - s0);
+        TriFrame t;
+        t.a = make_float4(s0.x, s0.y, s0.z, n.x);
+        t.b = make_float4(s1.x, s1.y, s1.z, n.y);
+        t.c = make_float4(s2.x, s2.y, s2.z, n.z);
+        S.tri[i] = t;
+        return;
+    }
+    blk -= S.tri_blocks;
+    if (blk < S.project_blocks) {
+        const long long i = blk * (long long)blockDim.x + threadIdx.x;
+        if (i >= (long long)S.B * S.C * S.N) return;
+        const int view = (int)(i / S.N), v = (int)(i % S.N);
+        const ViewCam& cam = S.cams[view];
+        const float3 p = project_point(cam.ext, cam.intr, ld3(S.verts + ((long long)(view / S.C) * S.N + v) * 3));
+        S.proj[i] = make_float4(p.x, p.y, p.z, 0.f);
+        return;
+    }
+    blk -= S.project_blocks;
+    const unsigned first = S.normal_blocks + S.tri_blocks + S.project_blocks;
+    fill_runs(S.fills, blk * (long long)blockDim.x + threadIdx.x, (gridDim.x - first) * (long long)blockDim.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -983,25 +996,57 @@ hc_status raster_forward(const Topology& topo, RasterWorkspace& ws, cudaStream_t
     int2* tstate = ws.tile_state.as<int2>();
     RasterStats* stats = ws.stats.as<RasterStats>();
 
-    HC_CUDA(cudaMemsetAsync(tstate, 0, sizeof(int2) * (size_t)tiles, s));
-    HC_CUDA(cudaMemsetAsync(stats, 0, sizeof(RasterStats), s));
+    HC_TRY(ws.claim.ensure(sizeof(unsigned long long)));
+    unsigned long long* claim = ws.claim.as<unsigned long long>();
+
+    FillRuns zeros;
+    zeros.add(tstate, sizeof(int2) * (size_t)tiles);
+    zeros.add(stats, sizeof(RasterStats));
+    zeros.add(claim, sizeof(unsigned long long));
+    if (l1) zeros.add(l1->state, sizeof(L1State));
+    const int view_blocks = div_up(V, kViewThreads);
     ws.clock.begin(kKViewSetup, s);
-    k_view_setup<<<div_up(V, 64), 64, 0, s>>>(V, C, extr, intr, ws.layout.as<CamLayout>(), ws.P_frame, ws.T_frame,
-                                              ws.Tb_frame, cams);
+    k_view_setup<<<view_blocks + zeros.blocks(kViewThreads), kViewThreads, 0, s>>>(
+        V, C, extr, intr, ws.layout.as<CamLayout>(), ws.P_frame, ws.T_frame, ws.Tb_frame, cams, view_blocks, zeros);
     HC_CHECK_LAUNCH();
     ws.clock.end(kKViewSetup, s);
-    ws.clock.begin(kKVertexNormals, s);
-    k_vertex_normals<<<div_up((long long)B * N, 256), 256, 0, s>>>(
-        B, C, N, topo.fan.as<int2>(), topo.vf_id.as<int2>(), verts, vnormal);
-    HC_CHECK_LAUNCH();
-    ws.clock.end(kKVertexNormals, s);
-    ws.clock.begin(kKTriFrame, s);
-    k_tri_frame<<<div_up((long long)B * F, 256), 256, 0, s>>>(B, F, N, topo.faces.as<int3>(), verts, tf);
-    HC_CHECK_LAUNCH();
-    ws.clock.end(kKTriFrame, s);
-    ws.clock.begin(kKBin, s);
-    k_project_vertices<<<div_up((long long)V * N, 256), 256, 0, s>>>(V, C, N, verts, cams, ws.proj.as<float4>());
-    HC_CHECK_LAUNCH();
+    FrameSetup S;
+    S.B = B;
+    S.C = C;
+    S.N = N;
+    S.F = F;
+    S.faces = topo.faces.as<int3>();
+    S.fan = topo.fan.as<int2>();
+    S.vf_id = topo.vf_id.as<int2>();
+    S.verts = verts;
+    S.vnormal = vnormal;
+    S.unit = nullptr;
+    S.tri = tf;
+    S.cams = cams;
+    S.proj = ws.proj.as<float4>();
+    // kernel timing names the parts: a launch each then
+    const unsigned nb = div_up((long long)B * N, kSetupThreads), fb = div_up((long long)B * F, kSetupThreads),
+                   pb = div_up((long long)V * N, kSetupThreads);
+    auto setup = [&](unsigned normals, unsigned tris, unsigned projected) -> hc_status {
+        S.normal_blocks = normals;
+        S.tri_blocks = tris;
+        S.project_blocks = projected;
+        k_frame_setup<<<normals + tris + projected, kSetupThreads, 0, s>>>(S);
+        HC_CHECK_LAUNCH();
+        return HC_OK;
+    };
+    if (ws.clock.on) {
+        ws.clock.begin(kKVertexNormals, s);
+        HC_TRY(setup(nb, 0, 0));
+        ws.clock.end(kKVertexNormals, s);
+        ws.clock.begin(kKTriFrame, s);
+        HC_TRY(setup(0, fb, 0));
+        ws.clock.end(kKTriFrame, s);
+        ws.clock.begin(kKBin, s);
+        HC_TRY(setup(0, 0, pb));
+    } else {
+        HC_TRY(setup(nb, fb, pb));
+    }
     HC_REQUIRE(V <= 65535, "too many views in one call (%d)", V);
     HC_REQUIRE(tiles < (1ll << 31), "too many tiles in one call (%lld)", tiles);
     const int ts_shift = TS == 8 ? 3 : (TS == 16 ? 4 : 5);
@@ -1046,12 +1091,8 @@ hc_status raster_forward(const Topology& topo, RasterWorkspace& ws, cudaStream_t
     A.l1_target = l1 ? l1->target : nullptr;
     A.l1_mask = l1 ? l1->mask : nullptr;
     A.l1_state = l1 ? l1->state : nullptr;
-    if (l1) HC_CUDA(cudaMemsetAsync(l1->state, 0, sizeof(L1State), s));
     const int* tcam = ws.tile_cam.as<int>();
     HC_REQUIRE(tiles < (1ll << 31), "too many tiles in one call (%lld)", tiles);
-    HC_TRY(ws.claim.ensure(sizeof(unsigned long long)));
-    unsigned long long* claim = ws.claim.as<unsigned long long>();
-    HC_CUDA(cudaMemsetAsync(claim, 0, sizeof(unsigned long long), s));
     const int* kbins = ws.bins.as<int>();
     const unsigned long long* kspill = ws.spill_keys.as<unsigned long long>();
     ws.clock.begin(kKResolve, s);

@@ -1306,13 +1306,19 @@ static hc_status mesh_boundary_run(hc_mesh_boundary h, void* stream, int32_t bat
     const float2* p2 = reinterpret_cast<const float2*>(p2d);
     const int3* faces = h->faces.as<int3>();
     unsigned long long* need = h->need.as<unsigned long long>();
-    HC_CUDA(cudaMemsetAsync(cb.count, 0, sizeof(int) * (size_t)n_keys, s));
-    HC_CUDA(cudaMemsetAsync(cb.n_tiles, 0, sizeof(int), s));
+    FillRuns zeros;
+    zeros.add(cb.count, sizeof(int) * (size_t)n_keys);
+    zeros.add(cb.n_tiles, sizeof(int));
+    if (face_hint) {
+        zeros.add(need, sizeof(unsigned long long) * (size_t)(frames * L.Q));
+        zeros.add(cb.n_items, sizeof(int));
+    } else {
+        zeros.add(cb.cover, (size_t)(frames * L.P));
+    }
+    HC_TRY(fill(zeros, s));
     if (face_hint) {
         // final flags of the vertices whose windows the hint covers; open
         // window pixels and their tiles for the binned passes
-        HC_CUDA(cudaMemsetAsync(need, 0, sizeof(unsigned long long) * (size_t)(frames * L.Q), s));
-        HC_CUDA(cudaMemsetAsync(cb.n_items, 0, sizeof(int), s));
         k_bnd_hint<<<div_up(nv, 256), 256, 0, s>>>(nv, h->N, h->F, L, p2, h->faces.as<int>(), face_hint, cb.cover, need,
                                                    is_boundary);
         HC_CHECK_LAUNCH();
@@ -1322,7 +1328,6 @@ static hc_status mesh_boundary_run(hc_mesh_boundary h, void* stream, int32_t bat
         k_cov_bin_list<<<resident_grid(k_cov_bin_list, 256, views * h->F / 256 + 1), 256, 0, s>>>(h->N, h->F, faces, p2,
                                                                                                   cb, L);
     } else {
-        HC_CUDA(cudaMemsetAsync(h->cover.ptr, 0, (size_t)(frames * L.P), s));
         k_cov_bin<<<dim3(div_up(h->F, 256), (unsigned)views), 256, 0, s>>>(h->N, h->F, faces, p2, cb, L);
     }
     HC_CHECK_LAUNCH();
@@ -1447,7 +1452,10 @@ hc_status sil_forward_run(cudaStream_t s, int* base, const ImgLayout& L, int32_t
     g.start = base + cells;
     g.cursor = base + 2 * cells + 1;
     g.items = base + 3 * cells + 1;
-    HC_CUDA(cudaMemsetAsync(g.count, 0, sizeof(int) * (size_t)cells, s));
+    FillRuns zeros;
+    zeros.add(g.count, sizeof(int) * (size_t)cells);
+    if (sumsq_1) zeros.add(sumsq_1, sizeof(double));
+    HC_TRY(fill(zeros, s));
     const long long np = views * N;
     k_sil_points<<<div_up(np, 256), 256, 0, s>>>(batch, n_cameras, N, L, points_image_space, normals_image_space,
                                                  is_boundary, distance_transform_image, multi_view_crops,
@@ -1461,7 +1469,6 @@ hc_status sil_forward_run(cudaStream_t s, int* base, const ImgLayout& L, int32_t
     k_grid_fill<<<div_up(np, 256), 256, 0, s>>>(batch, n_cameras, N, L, g, points_image_space, is_boundary,
                                                 multi_view_crops);
     HC_CHECK_LAUNCH();
-    if (sumsq_1) HC_CUDA(cudaMemsetAsync(sumsq_1, 0, sizeof(double), s));
     {
         const int vec = pixels_by_four(L) && ((uintptr_t)distance_transform_image & 3) == 0 &&
                         ((uintptr_t)mv_dt_residual_1 & 15) == 0 && ((uintptr_t)closest_vertex_id & 15) == 0;

@@ -164,7 +164,9 @@ class RendererEngine:
             img + (3,), device=dev, dtype=torch.float32)
         vnormal = o.get("vnormal") if o.get("vnormal") is not None else torch.empty(
             (B, self.C, self.N, 3), device=dev, dtype=torch.float32)
-        normal_map = torch.zeros((B, max(TH, 1), max(TW, 1), 3), device=dev, dtype=torch.float32)
+        # the UV maps write every texel
+        normal_map = (torch.zeros if self.compute_normal_map == "none" or not TH * TW else torch.empty)(
+            (B, max(TH, 1), max(TW, 1), 3), device=dev, dtype=torch.float32)
         depth_q = tie = None
         if diagnostics:
             depth_q = torch.empty(img, device=dev, dtype=torch.int32)
