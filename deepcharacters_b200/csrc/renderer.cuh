@@ -308,6 +308,100 @@ __device__ __forceinline__ bool footprint_overlaps(const Footprint& fp, int x0, 
     return true;
 }
 
+// The same for the rows of a box, an interval of columns per row: edge k leaves
+// or enters a row [y0, y1] at x = s y + c for the better of its ends.  A pixel
+// column outside the interval fails one edge in every pixel of the row.  Against
+// a test of each tile of the box it costs one row's share of the edges, and no
+// tile that is missed is visited.  (Each value differs from the sum above by
+// rounding only, at most 0.05 px of the edge's distance against its margin of
+// kEdgeMargin; edges with a nearly 0 bound no column.)
+struct TileRows {
+    float s[3], c[3];
+    int low;  // bit k: edge k bounds the columns from below; bit 3 + k: b > 0
+    __device__ __forceinline__ TileRows() {}
+    __device__ __forceinline__ explicit TileRows(const Footprint& fp) : low(0) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const bool bounds = fabsf(fp.a[k]) > 1e-6f;
+            const float inv = __fdividef(-1.f, fp.a[k]);
+            s[k] = bounds ? fp.b[k] * inv : 0.f;
+            c[k] = bounds ? fp.c[k] * inv - 0.5f : -1e30f;
+            low |= (!bounds || fp.a[k] > 0.f ? 1 << k : 0) | (fp.b[k] > 0.f ? 8 << k : 0);
+        }
+    }
+    // pixel columns of the row inside [x0, x1]; none if hi < lo
+    __device__ __forceinline__ void span(int x0, int x1, int y0, int y1, int& lo, int& hi) const {
+        const float ya = y0 + 0.5f, yb = y1 + 0.5f;
+        float l = (float)x0, h = (float)x1;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float x = s[k] * (low & (8 << k) ? yb : ya) + c[k];
+            if (low & (1 << k)) l = fmaxf(l, x);
+            else h = fminf(h, x);
+        }
+        lo = __float2int_ru(fminf(l, x1 + 1.f));
+        hi = __float2int_rd(fmaxf(h, x0 - 1.f));
+    }
+    // the tiles (edge 1 << sh) of a box of at most 32 that the footprint
+    // reaches: bit ntx * row + column
+    __device__ __forceinline__ unsigned tiles(int sh, int x0, int x1, int y0, int y1) const {
+        const int tx0 = x0 >> sh, ty0 = y0 >> sh, ty1 = y1 >> sh, ntx = (x1 >> sh) - tx0 + 1;
+        unsigned reached = 0u;
+        int at = 0;
+        for (int ty = ty0; ty <= ty1; ++ty, at += ntx) {
+            int lo, hi;
+            span(x0, x1, max(ty << sh, y0), min((ty << sh) + (1 << sh) - 1, y1), lo, hi);
+            if (hi >= lo) reached |= ((2u << ((hi >> sh) - tx0)) - (1u << ((lo >> sh) - tx0))) << at;
+        }
+        return reached;
+    }
+    __device__ __forceinline__ TileRows from_lane(int src) const {
+        TileRows q;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            q.s[k] = __shfl_sync(0xffffffffu, s[k], src);
+            q.c[k] = __shfl_sync(0xffffffffu, c[k], src);
+        }
+        q.low = __shfl_sync(0xffffffffu, low, src);
+        return q;
+    }
+};
+
+// A warp visits the tiles of one box that a footprint reaches: a row per lane
+// for the intervals, then the tiles of up to 32 rows dealt out evenly.  All
+// lanes call it with the same box; visit(tx, ty) runs in the lanes that have one.
+template <class Visit>
+__device__ __forceinline__ void warp_tiles(const TileRows& rows, int sh, int x0, int x1, int y0, int y1, int lane,
+                                           Visit visit) {
+    const int ty0 = y0 >> sh, ty1 = y1 >> sh;
+    for (int r = ty0; r <= ty1; r += 32) {
+        const int ty = r + lane;
+        int lo = 0, count = 0;
+        if (ty <= ty1) {
+            int hi;
+            rows.span(x0, x1, max(ty << sh, y0), min((ty << sh) + (1 << sh) - 1, y1), lo, hi);
+            count = hi >= lo ? (hi >> sh) - (lo >> sh) + 1 : 0;
+            lo >>= sh;
+        }
+        int upto = count;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        const int total = __shfl_sync(0xffffffffu, upto, 31), first = lo - (upto - count);
+        for (int k0 = 0; k0 < total; k0 += 32) {
+            const int k = k0 + lane;
+            int row = 0;  // the first row whose tiles reach beyond k
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                if (__shfl_sync(0xffffffffu, upto, row + o - 1) <= k) row += o;
+            const int tx = __shfl_sync(0xffffffffu, first, row & 31) + k;
+            if (k < total) visit(tx, r + row);
+        }
+    }
+}
+
 // bit n alone; 0 for n = 32 (the hardware shift saturates)
 __device__ __forceinline__ unsigned bit_at(unsigned n) {
     unsigned r;
