@@ -75,6 +75,26 @@ struct DevBuf {
     T* as() const { return reinterpret_cast<T*>(ptr); }
 };
 
+// Scratch that a call is faster with and can do without: there is no room where
+// memory is short, where a capture would have to allocate it, and where growing it
+// would free what a captured graph addresses.
+struct SpareBuf : DevBuf {
+    bool captured = false;  // a graph holds its address: it keeps its size
+    bool room(size_t need, cudaStreamCaptureStatus capture) {
+        const bool recording = capture != cudaStreamCaptureStatusNone;
+        if (bytes < need) {
+            if (captured || recording) return false;
+            if (ensure(need) != HC_OK) {
+                cudaGetLastError();
+                clear_error();
+                return false;
+            }
+        }
+        captured = captured || recording;
+        return true;
+    }
+};
+
 template <class T>
 hc_status upload(DevBuf& b, const T* host, size_t count) {
     HC_TRY(b.ensure(count * sizeof(T)));

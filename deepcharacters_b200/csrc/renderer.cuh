@@ -571,7 +571,7 @@ struct Topology {
 struct UvTable {
     int th = 0, tw = 0;
     DevBuf faces, table;
-    DevBuf unit;  // normalised vertex normals of a call, 16 bytes each
+    SpareBuf unit;  // normalised vertex normals of a call, 16 bytes each
 };
 
 // v / |v| (zero stays zero).  The contraction of |v|^2 is written out, so that

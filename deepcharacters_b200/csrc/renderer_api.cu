@@ -17,8 +17,8 @@ hc_status raster_reserve(RasterWorkspace& ws, int views, int F);
 hc_status raster_uv_maps(const Topology& topo, UvTable& tab, cudaStream_t s, int B, int C, long long P_frame, int mode,
                          const float* verts, int tex_h, int tex_w, float* bary, int* face, float* render,
                          float* vnormal, float* uv_map);
-hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vacc, DevBuf& tacc,
-                          DevBuf& tpad, cudaStream_t s,
+hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vacc, SpareBuf& tacc,
+                          SpareBuf& tpad, cudaStream_t s,
                           int B, int C, int albedo, int shading, int ifs, int tfs, const float* grad, const float* verts,
                           const float* colors, const float* texture, int tex_h, int tex_w, const float* sh,
                           const float* target, const float* vnormal, const float* bary, const int* face,
@@ -111,8 +111,8 @@ struct hc_renderer_s {
     hc::Topology topo;
     hc::RasterWorkspace ws;
     hc::DevBuf vacc;      // backward: per-vertex gradient sums
-    hc::DevBuf tacc;      // backward: padded texel gradient sums
-    hc::DevBuf tpad;      // backward: the texture padded to 16 bytes per texel
+    hc::SpareBuf tacc;      // backward: padded texel gradient sums
+    hc::SpareBuf tpad;      // backward: the texture padded to 16 bytes per texel
     hc::UvTable uv;       // texel table of the UV-space maps
     int C = 0, W = 0, H = 0;
     int albedo = 0, shading = 0, normal_map = hc::kNmNone;
@@ -203,7 +203,7 @@ extern "C" hc_status hc_renderer_reserve(hc_renderer h, int32_t batch) {
     HC_TRY(h->ws.tri_frame.ensure(sizeof(TriFrame) * (size_t)batch * h->topo.F));
     HC_TRY(h->ws.proj.ensure(sizeof(float4) * (size_t)batch * h->C * h->topo.N));
     HC_TRY(h->vacc.ensure(sizeof(float) * 12 * (size_t)batch * h->topo.N));  // the widest VertexSums
-    if (h->normal_map == kNmOriginal) HC_TRY(h->uv.unit.ensure(sizeof(float4) * (size_t)batch * h->topo.N));
+    if (h->normal_map == kNmOriginal) h->uv.unit.room(sizeof(float4) * (size_t)batch * h->topo.N, cudaStreamCaptureStatusNone);
     return HC_OK;
 }
 

@@ -890,8 +890,8 @@ static bool target_tensor_map(const RasterWorkspace& ws, const float* target, in
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vacc, DevBuf& tacc,
-                          DevBuf& tpad, cudaStream_t s,
+hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vacc, SpareBuf& tacc,
+                          SpareBuf& tpad, cudaStream_t s,
                           int B, int C, int albedo, int shading, int ifs, int tfs, const float* grad,
                           const float* verts, const float* colors, const float* texture, int tex_h, int tex_w,
                           const float* sh, const float* target, const float* vnormal, const float* bary,
@@ -906,7 +906,8 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vac
                     : albedo == kTexturedBilinear ? kAlbTexBilinear : kAlbNone;
     const int stride = (3 + (alb == kAlbVcol ? 3 : 0) + (shaded ? 3 : 0) + 3) / 4 * 4;  // VertexSums::kStride
     const size_t vacc_bytes = sizeof(float) * (size_t)stride * (size_t)B * N;
-    HC_TRY(vacc.ensure(vacc_bytes));
+    // sized with the cameras, so that it grows only where those do
+    HC_TRY(vacc.ensure(vacc_bytes / B * std::max(B, ws.cap_views / C)));
     // Texels padded to 16 bytes where the padding's extra pass over the texture
     // costs less than it saves.  Sums (a clear, a read and a write, 32 bytes per
     // texel): two reductions per covered pixel (eight bilinear) become none;
@@ -916,25 +917,17 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vac
     // Taps of the nearest mode's texture gradient (28 bytes per texel): one load
     // per tap instead of three; 1024^2 texture: 4 x 1024^2 views 400 -> 337 us,
     // one 1024^2 131 -> 118, one 512^2 71 -> 67, one 256^2 56 -> 60.
-    // A capture does not allocate, and without memory for the padding the
-    // texture is used as it is.
+    // Without room for the padding (SpareBuf) the texture is used as it is.
     const long long texels = tex_grad && tex_h > 0 && tex_w > 0 ? (long long)B * tex_h * tex_w : 0;
     const long long pixels = (long long)B * ws.P_frame;
     const size_t pad_bytes = sizeof(float4) * (size_t)texels;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     HC_CUDA(cudaStreamIsCapturing(s, &capture));
-    auto room = [&](DevBuf& buf) {
-        if (buf.bytes >= pad_bytes) return true;
-        if (capture == cudaStreamCaptureStatusNone && buf.ensure(pad_bytes) == HC_OK) return true;
-        cudaGetLastError();
-        clear_error();
-        return false;
-    };
     const bool padded = texels > 0 &&
                         ((albedo == kTexturedBilinear && pixels >= 2 * texels) ||
                          (albedo == kTextured && pixels >= 16 * texels)) &&
-                        room(tacc);
-    const bool taps = albedo == kTextured && texels > 0 && 4 * pixels >= texels && room(tpad);
+                        tacc.room(pad_bytes, capture);
+    const bool taps = albedo == kTextured && texels > 0 && 4 * pixels >= texels && tpad.room(pad_bytes, capture);
     HC_TRY(ws.claim_b.ensure(sizeof(unsigned)));
     FillRuns zeros;
     zeros.add(vacc.ptr, vacc_bytes);

@@ -183,19 +183,10 @@ hc_status raster_uv_maps(const Topology& topo, UvTable& tab, cudaStream_t s, int
     S.vf_id = topo.vf_id.as<int2>();
     S.verts = verts;
     S.vnormal = vnormal;
-    // a capture does not allocate, and without memory for them the normals are
-    // normalised where they are used
-    const size_t unit_bytes = sizeof(float4) * (size_t)B * N;
+    // without room for them the normals are normalised where they are used
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     HC_CUDA(cudaStreamIsCapturing(s, &capture));
-    if (mode == kNmOriginal &&
-        (tab.unit.bytes >= unit_bytes ||
-         (capture == cudaStreamCaptureStatusNone && tab.unit.ensure(unit_bytes) == HC_OK))) {
-        S.unit = tab.unit.as<float4>();
-    } else {
-        cudaGetLastError();
-        clear_error();
-    }
+    if (mode == kNmOriginal && tab.unit.room(sizeof(float4) * (size_t)B * N, capture)) S.unit = tab.unit.as<float4>();
     S.fills.add(face, sizeof(int) * (size_t)px, 0xff);
     S.fills.add(bary, sizeof(float) * 2 * (size_t)px);
     S.fills.add(render, sizeof(float) * 3 * (size_t)px);
