@@ -570,7 +570,7 @@ struct Topology {
 // texel -> (face, barycentrics) table of the UV-space maps, per texture size
 struct UvTable {
     int th = 0, tw = 0;
-    DevBuf faces, table;
+    DevBuf table;   // float4 per texel, then the int face per texel it is made from
     SpareBuf unit;  // normalised vertex normals of a call, 16 bytes each
 };
 

@@ -195,12 +195,12 @@ hc_status raster_uv_maps(const Topology& topo, UvTable& tab, cudaStream_t s, int
     HC_CHECK_LAUNCH();
     const int nt = tex_h * tex_w;
     if (tab.th != tex_h || tab.tw != tex_w) {
-        HC_TRY(tab.faces.ensure(sizeof(int) * (size_t)nt));
-        HC_TRY(tab.table.ensure(sizeof(float4) * (size_t)nt));
-        HC_CUDA(cudaMemsetAsync(tab.faces.ptr, 0xff, sizeof(int) * (size_t)nt, s));
-        k_texel_faces<<<div_up(F, 128), 128, 0, s>>>(F, tex_w, tex_h, topo.texcoords.as<float>(), tab.faces.as<int>());
+        HC_TRY(tab.table.ensure((sizeof(float4) + sizeof(int)) * (size_t)nt));  // one allocation for both
+        int* texel_face = reinterpret_cast<int*>(tab.table.as<float4>() + nt);
+        HC_CUDA(cudaMemsetAsync(texel_face, 0xff, sizeof(int) * (size_t)nt, s));
+        k_texel_faces<<<div_up(F, 128), 128, 0, s>>>(F, tex_w, tex_h, topo.texcoords.as<float>(), texel_face);
         HC_CHECK_LAUNCH();
-        k_texel_table<<<div_up(nt, 256), 256, 0, s>>>(tex_w, tex_h, topo.texcoords.as<float>(), tab.faces.as<int>(),
+        k_texel_table<<<div_up(nt, 256), 256, 0, s>>>(tex_w, tex_h, topo.texcoords.as<float>(), texel_face,
                                                       tab.table.as<float4>());
         HC_CHECK_LAUNCH();
         tab.th = tex_h;
