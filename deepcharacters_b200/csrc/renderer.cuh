@@ -567,11 +567,51 @@ struct Topology {
     bool has_texcoords = false;
 };
 
-// texel -> (face, barycentrics) table of the UV-space maps, per texture size
+// texel -> (face, barycentrics) table of the UV-space maps for one texture size
 struct UvTable {
     int th = 0, tw = 0;
-    DevBuf table;   // float4 per texel, then the int face per texel it is made from
+    bool valid = false;     // built by a call that ran (one recorded into a graph builds it at each replay)
+    bool captured = false;  // a graph holds its address: it keeps its size and its texture size
+    DevBuf buf;             // float4 per texel, then the int face per texel it is made from
+};
+
+struct UvTables {
+    std::vector<UvTable> tables;  // one for each size that a graph holds, and at most one besides
     SpareBuf unit;  // normalised vertex normals of a call, 16 bytes each
+    // the table of a texture size; the call has to build it unless it is valid
+    hc_status get(int th, int tw, cudaStreamCaptureStatus capture, UvTable** out) {
+        const bool recording = capture != cudaStreamCaptureStatusNone;
+        const size_t need = (sizeof(float4) + sizeof(int)) * (size_t)th * tw;
+        UvTable* t = nullptr;
+        bool held = false;  // a table that a graph holds would have the room
+        for (UvTable& k : tables) {
+            if (k.th == th && k.tw == tw) {
+                k.captured = k.captured || recording;
+                *out = &k;
+                return HC_OK;
+            }
+            if (!k.captured) t = &k;
+            else held = held || k.buf.bytes >= need;
+        }
+        // under capture nothing is allocated, but for what another graph's table keeps from use
+        const bool extra = recording && held && (!t || t->buf.bytes < need);
+        if (!t || extra) {
+            tables.emplace_back();
+            t = &tables.back();
+        }
+        t->th = t->tw = 0;
+        t->valid = false;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        if (extra) HC_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        const hc_status st = t->buf.ensure(need);
+        if (extra) HC_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        HC_TRY(st);
+        t->th = th;
+        t->tw = tw;
+        t->captured = recording;
+        *out = t;
+        return HC_OK;
+    }
 };
 
 // v / |v| (zero stays zero).  The contraction of |v|^2 is written out, so that

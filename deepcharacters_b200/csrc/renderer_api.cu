@@ -14,7 +14,7 @@ hc_status raster_forward(const Topology& topo, RasterWorkspace& ws, cudaStream_t
                          float* render, float* vnormal, int* depth_q, int* tie_count,
                          const L1Fuse* l1 = nullptr);
 hc_status raster_reserve(RasterWorkspace& ws, int views, int F);
-hc_status raster_uv_maps(const Topology& topo, UvTable& tab, cudaStream_t s, int B, int C, long long P_frame, int mode,
+hc_status raster_uv_maps(const Topology& topo, UvTables& tab, cudaStream_t s, int B, int C, long long P_frame, int mode,
                          const float* verts, int tex_h, int tex_w, float* bary, int* face, float* render,
                          float* vnormal, float* uv_map);
 hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vacc, SpareBuf& tacc,
@@ -113,7 +113,7 @@ struct hc_renderer_s {
     hc::DevBuf vacc;      // backward: per-vertex gradient sums
     hc::SpareBuf tacc;      // backward: padded texel gradient sums
     hc::SpareBuf tpad;      // backward: the texture padded to 16 bytes per texel
-    hc::UvTable uv;       // texel table of the UV-space maps
+    hc::UvTables uv;        // texel tables of the UV-space maps
     int C = 0, W = 0, H = 0;
     int albedo = 0, shading = 0, normal_map = hc::kNmNone;
     int image_filter = 2, texture_filter = 2;
@@ -183,9 +183,10 @@ static void release_all(hc_renderer_s* r) {
     DevBuf* bufs[] = {&r->topo.faces, &r->topo.fan, &r->topo.vf_id, &r->topo.texcoords,
                       &r->ws.cams, &r->ws.tri_frame, &r->ws.tri_view, &r->ws.tile_state,
                       &r->ws.bins, &r->ws.spill, &r->ws.spill_keys, &r->ws.stats, &r->vacc, &r->tacc, &r->tpad,
-                      &r->uv.table, &r->uv.unit, &r->ws.layout, &r->ws.tile_cam, &r->ws.tile_cam_b, &r->ws.proj,
+                      &r->uv.unit, &r->ws.layout, &r->ws.tile_cam, &r->ws.tile_cam_b, &r->ws.proj,
                       &r->ws.claim, &r->ws.claim_b};
     for (DevBuf* b : bufs) b->release();
+    for (UvTable& t : r->uv.tables) t.buf.release();
 }
 
 extern "C" hc_status hc_renderer_destroy(hc_renderer h) {

@@ -166,7 +166,7 @@ __global__ void k_uv_map(int B, int C, int N, int n_texels, int mode, const int3
 
 }  // namespace
 
-hc_status raster_uv_maps(const Topology& topo, UvTable& tab, cudaStream_t s, int B, int C, long long P_frame, int mode,
+hc_status raster_uv_maps(const Topology& topo, UvTables& tab, cudaStream_t s, int B, int C, long long P_frame, int mode,
                          const float* verts, int tex_h, int tex_w, float* bary, int* face, float* render,
                          float* vnormal, float* uv_map) {
     HC_REQUIRE(topo.has_texcoords, "compute_normal_map needs texture_coordinates");
@@ -194,20 +194,20 @@ hc_status raster_uv_maps(const Topology& topo, UvTable& tab, cudaStream_t s, int
     k_frame_setup<<<S.normal_blocks + S.fills.blocks(kSetupThreads), kSetupThreads, 0, s>>>(S);
     HC_CHECK_LAUNCH();
     const int nt = tex_h * tex_w;
-    if (tab.th != tex_h || tab.tw != tex_w) {
-        HC_TRY(tab.table.ensure((sizeof(float4) + sizeof(int)) * (size_t)nt));  // one allocation for both
-        int* texel_face = reinterpret_cast<int*>(tab.table.as<float4>() + nt);
+    UvTable* table = nullptr;
+    HC_TRY(tab.get(tex_h, tex_w, capture, &table));
+    float4* texels = table->buf.as<float4>();
+    if (!table->valid) {
+        int* texel_face = reinterpret_cast<int*>(texels + nt);  // one allocation for both
         HC_CUDA(cudaMemsetAsync(texel_face, 0xff, sizeof(int) * (size_t)nt, s));
         k_texel_faces<<<div_up(F, 128), 128, 0, s>>>(F, tex_w, tex_h, topo.texcoords.as<float>(), texel_face);
         HC_CHECK_LAUNCH();
-        k_texel_table<<<div_up(nt, 256), 256, 0, s>>>(tex_w, tex_h, topo.texcoords.as<float>(), texel_face,
-                                                      tab.table.as<float4>());
+        k_texel_table<<<div_up(nt, 256), 256, 0, s>>>(tex_w, tex_h, topo.texcoords.as<float>(), texel_face, texels);
         HC_CHECK_LAUNCH();
-        tab.th = tex_h;
-        tab.tw = tex_w;
+        table->valid = capture == cudaStreamCaptureStatusNone;
     }
     k_uv_map<<<dim3(div_up(nt, 256), std::min(div_up(B, kUvFrames), 65535)), 256, 0, s>>>(
-        B, C, N, nt, mode, topo.faces.as<int3>(), tab.table.as<float4>(), verts, vnormal, S.unit, uv_map);
+        B, C, N, nt, mode, topo.faces.as<int3>(), texels, verts, vnormal, S.unit, uv_map);
     HC_CHECK_LAUNCH();
     return HC_OK;
 }

@@ -1,0 +1,138 @@
+// Host checks of the library's buffers, against a fake of the CUDA runtime calls
+// that they make: run with the name of a check, exit code 0 when it holds.
+#include <cstdlib>
+#include <cstring>
+#include <map>
+
+#include "../deepcharacters_b200/csrc/renderer.cuh"
+
+namespace fake {
+size_t room = ~(size_t)0;  // the largest allocation that succeeds
+int mallocs = 0, frees = 0;
+std::map<void*, size_t> live;
+cudaError_t last = cudaSuccess;
+cudaStreamCaptureMode mode = cudaStreamCaptureModeGlobal;
+bool recording = false;  // allocations and frees are refused unless the mode is relaxed
+bool refused() { return recording && mode != cudaStreamCaptureModeRelaxed; }
+cudaError_t fail(cudaError_t e) { return last = e; }
+}  // namespace fake
+
+#ifndef __CUDA_ARCH__
+extern "C" {
+cudaError_t cudaMalloc(void** p, size_t n) {
+    ++fake::mallocs;
+    if (fake::refused()) return fake::fail(cudaErrorStreamCaptureUnsupported);
+    if (n > fake::room) return fake::fail(cudaErrorMemoryAllocation);
+    fake::live[*p = std::malloc(16)] = n;  // never freed: each has an address of its own
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void* p) {
+    ++fake::frees;
+    if (fake::refused()) return fake::fail(cudaErrorStreamCaptureUnsupported);
+    return fake::live.erase(p) ? cudaSuccess : fake::fail(cudaErrorInvalidValue);
+}
+cudaError_t cudaGetLastError() {
+    const cudaError_t e = fake::last;
+    fake::last = cudaSuccess;
+    return e;
+}
+const char* cudaGetErrorString(cudaError_t) { return "fake"; }
+cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode* m) {
+    std::swap(*m, fake::mode);
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpy(void*, const void*, size_t, cudaMemcpyKind) { return cudaSuccess; }
+void** __cudaRegisterFatBinary(void*) { return nullptr; }
+void __cudaRegisterFatBinaryEnd(void**) {}
+void __cudaUnregisterFatBinary(void**) {}
+char __cudaInitModule(void**) { return 0; }
+}
+#endif
+
+namespace hc {
+void set_error(const char*, ...) {}
+void clear_error() {}
+}  // namespace hc
+
+using namespace hc;
+
+#define CHECK(c)                                                  \
+    do {                                                          \
+        if (!(c)) {                                               \
+            fprintf(stderr, "line %d: %s\n", __LINE__, #c);       \
+            return 1;                                             \
+        }                                                         \
+    } while (0)
+
+const cudaStreamCaptureStatus kEager = cudaStreamCaptureStatusNone, kRecord = cudaStreamCaptureStatusActive;
+
+// A call at a size, as the UV maps make it; the table it used, NULL where it failed.
+static UvTable* uv_call(UvTables& t, int size, cudaStreamCaptureStatus capture, bool* built = nullptr) {
+    fake::recording = capture != kEager;
+    UvTable* k = nullptr;
+    const hc_status st = t.get(size, size, capture, &k);
+    fake::recording = false;
+    if (st != HC_OK) return nullptr;
+    if (built) *built = !k->valid;
+    if (!k->valid) k->valid = capture == kEager;
+    return k;
+}
+
+// a table that a graph holds is neither replaced nor built again for another size
+static int uv_held() {
+    UvTables t;
+    bool built = false;
+    CHECK(uv_call(t, 37, kEager, &built) && built);
+    void* at = uv_call(t, 37, kRecord, &built)->buf.ptr;
+    CHECK(!built && fake::mallocs == 1);
+    const UvTable* big = uv_call(t, 64, kEager, &built);
+    CHECK(big && built && big->buf.ptr != at && fake::frees == 0);
+    const UvTable* small = uv_call(t, 16, kEager, &built);  // in the place of the 64^2 table
+    CHECK(small && built && small->buf.ptr != at && t.tables.size() == 2);
+    const UvTable* again = uv_call(t, 37, kEager, &built);
+    CHECK(again->buf.ptr == at && !built && again->th == 37 && fake::live.count(at));
+    return 0;
+}
+
+// a table whose build was only recorded does not count as built
+static int uv_recorded() {
+    UvTables t;
+    bool built = false;
+    CHECK(uv_call(t, 64, kEager));
+    void* at = uv_call(t, 37, kRecord, &built)->buf.ptr;  // fits, and is built at each replay
+    CHECK(built && fake::mallocs == 1);
+    CHECK(uv_call(t, 64, kEager, &built)->buf.ptr != at && built);
+    CHECK(uv_call(t, 37, kEager, &built)->buf.ptr == at && built);
+    CHECK(uv_call(t, 37, kEager, &built)->buf.ptr == at && !built);
+    // a second graph of the size shares the table; one of another size that only a held
+    // table has room for gets its own
+    CHECK(uv_call(t, 37, kRecord)->buf.ptr == at);
+    CHECK(uv_call(t, 64, kRecord, &built)->buf.ptr != at && !built);
+    const size_t n = t.tables.size();
+    const UvTable* k = uv_call(t, 20, kRecord, &built);
+    CHECK(k && built && k->buf.ptr != at && t.tables.size() == n + 1 && fake::mode == cudaStreamCaptureModeGlobal);
+    CHECK(!uv_call(t, 1024, kRecord));  // no table of that size was ever made: refused
+    return 0;
+}
+
+// after a failed allocation no size is taken for built
+static int uv_no_memory() {
+    UvTables t;
+    bool built = false;
+    CHECK(uv_call(t, 37, kEager));
+    fake::room = 1 << 16;
+    CHECK(!uv_call(t, 64, kEager));
+    const UvTable* k = uv_call(t, 37, kEager, &built);
+    CHECK(k && built && k->buf.ptr && k->buf.bytes >= 20u * 37 * 37);
+    return 0;
+}
+
+int main(int argc, char** argv) {
+    const std::map<std::string, int (*)()> checks = {
+        {"uv_held", uv_held},
+        {"uv_recorded", uv_recorded},
+        {"uv_no_memory", uv_no_memory},
+    };
+    const auto it = checks.find(argc > 1 ? argv[1] : "");
+    return it == checks.end() ? 2 : it->second();
+}
