@@ -44,6 +44,15 @@ struct ViewCam {
 
 constexpr int kAdjointTile = 16;  // tile edge of the renderer adjoint
 
+// Values that the adjoint sums per vertex (position; colour with vertex colours;
+// normal if shaded), and the floats they take: a multiple of 16 bytes.
+__host__ __device__ constexpr int vertex_sum_values(bool vertex_colors, bool shaded) {
+    return 3 + (vertex_colors ? 3 : 0) + (shaded ? 3 : 0);
+}
+__host__ __device__ constexpr int vertex_sum_floats(bool vertex_colors, bool shaded) {
+    return (vertex_sum_values(vertex_colors, shaded) + 3) / 4 * 4;
+}
+
 // One camera's image inside a frame: the frame's cameras are concatenated,
 // so views of different resolutions share one launch.
 struct CamLayout {
@@ -696,6 +705,14 @@ struct RasterWorkspace {
     DevBuf proj;  // float4 [V,N]: projected vertices of the current call
     DevBuf claim;    // the tile resolve's tile counter
     DevBuf claim_b;  // the adjoint's tile counter
+    // the adjoint's per-vertex gradient sums: once a call has needed them (floats
+    // per frame, 0 before), sized with the cameras, so that they are replaced
+    // only where those are
+    DevBuf vacc;
+    size_t vacc_floats = 0;
+    hc_status size_vacc() {
+        return vacc.ensure(sizeof(float) * vacc_floats * (cams.bytes / sizeof(ViewCam) / cam_w.size()));
+    }
     int adjoint_dynamic = 1;  // the adjoint's tile schedule (hc_renderer_set_adjoint_schedule)
     KernelClock clock;
 };

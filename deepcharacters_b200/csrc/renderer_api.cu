@@ -17,8 +17,7 @@ hc_status raster_reserve(RasterWorkspace& ws, int views, int F);
 hc_status raster_uv_maps(const Topology& topo, UvTables& tab, cudaStream_t s, int B, int C, long long P_frame, int mode,
                          const float* verts, int tex_h, int tex_w, float* bary, int* face, float* render,
                          float* vnormal, float* uv_map);
-hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vacc, SpareBuf& tacc,
-                          SpareBuf& tpad, cudaStream_t s,
+hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, SpareBuf& tacc, SpareBuf& tpad, cudaStream_t s,
                           int B, int C, int albedo, int shading, int ifs, int tfs, const float* grad, const float* verts,
                           const float* colors, const float* texture, int tex_h, int tex_w, const float* sh,
                           const float* target, const float* vnormal, const float* bary, const int* face,
@@ -110,7 +109,6 @@ hc_status topology_upload(Topology& t, int N, const int32_t* faces, int F, const
 struct hc_renderer_s {
     hc::Topology topo;
     hc::RasterWorkspace ws;
-    hc::DevBuf vacc;      // backward: per-vertex gradient sums
     hc::SpareBuf tacc;      // backward: padded texel gradient sums
     hc::SpareBuf tpad;      // backward: the texture padded to 16 bytes per texel
     hc::UvTables uv;        // texel tables of the UV-space maps
@@ -121,6 +119,11 @@ struct hc_renderer_s {
 };
 
 using namespace hc;
+
+// the albedo modes that the adjoint is defined for
+static bool has_gradients(const hc_renderer_s* h) {
+    return h->albedo == kVertexColor || h->albedo == kTextured || h->albedo == kTexturedBilinear;
+}
 
 static long long frame_pixels(const hc_renderer_s* h) {
     long long p = 0;
@@ -182,7 +185,7 @@ static void release_all(hc_renderer_s* r) {
     r->ws.clock.made = false;
     DevBuf* bufs[] = {&r->topo.faces, &r->topo.fan, &r->topo.vf_id, &r->topo.texcoords,
                       &r->ws.cams, &r->ws.tri_frame, &r->ws.tri_view, &r->ws.tile_state,
-                      &r->ws.bins, &r->ws.spill, &r->ws.spill_keys, &r->ws.stats, &r->vacc, &r->tacc, &r->tpad,
+                      &r->ws.bins, &r->ws.spill, &r->ws.spill_keys, &r->ws.stats, &r->ws.vacc, &r->tacc, &r->tpad,
                       &r->uv.unit, &r->ws.layout, &r->ws.tile_cam, &r->ws.tile_cam_b, &r->ws.proj,
                       &r->ws.claim, &r->ws.claim_b};
     for (DevBuf* b : bufs) b->release();
@@ -203,7 +206,10 @@ extern "C" hc_status hc_renderer_reserve(hc_renderer h, int32_t batch) {
     HC_TRY(raster_reserve(h->ws, batch * h->C, h->topo.F));
     HC_TRY(h->ws.tri_frame.ensure(sizeof(TriFrame) * (size_t)batch * h->topo.F));
     HC_TRY(h->ws.proj.ensure(sizeof(float4) * (size_t)batch * h->C * h->topo.N));
-    HC_TRY(h->vacc.ensure(sizeof(float) * 12 * (size_t)batch * h->topo.N));  // the widest VertexSums
+    if (has_gradients(h)) {
+        h->ws.vacc_floats = (size_t)vertex_sum_floats(h->albedo == kVertexColor, h->shading == kShaded) * h->topo.N;
+        HC_TRY(h->ws.size_vacc());
+    }
     if (h->normal_map == kNmOriginal) h->uv.unit.room(sizeof(float4) * (size_t)batch * h->topo.N, cudaStreamCaptureStatusNone);
     return HC_OK;
 }
@@ -291,8 +297,7 @@ extern "C" hc_status hc_renderer_backward(hc_renderer h, void* stream, int32_t b
     clear_error();
     HC_REQUIRE(h, "invalid handle");
     HC_REQUIRE(batch > 0, "batch must be positive (%d)", batch);
-    HC_REQUIRE(h->albedo == kVertexColor || h->albedo == kTextured || h->albedo == kTexturedBilinear,
-               "renderer gradients exist only for vertexColor and textured albedo");
+    HC_REQUIRE(has_gradients(h), "renderer gradients exist only for vertexColor and textured albedo");
     HC_REQUIRE(render_buffer_grad && vertex_pos && target_image && vertex_normal && barycentric_buffer &&
                    face_buffer && extrinsics && intrinsics && vertex_pos_grad,
                "NULL input/output pointer");
@@ -300,7 +305,7 @@ extern "C" hc_status hc_renderer_backward(hc_renderer h, void* stream, int32_t b
     if (h->albedo == kTextured || h->albedo == kTexturedBilinear)
         HC_REQUIRE(texture && texture_grad && texture_width > 0 && texture_height > 0, "textured mode needs a texture");
     if (h->shading == kShaded) HC_REQUIRE(sh_coeff && sh_coeff_grad, "shaded mode needs sh_coeff");
-    return raster_backward(h->topo, h->ws, h->vacc, h->tacc, h->tpad, (cudaStream_t)stream, batch, h->C, h->albedo,
+    return raster_backward(h->topo, h->ws, h->tacc, h->tpad, (cudaStream_t)stream, batch, h->C, h->albedo,
                            h->shading, h->image_filter, h->texture_filter, render_buffer_grad, vertex_pos,
                            vertex_color, texture, texture_height, texture_width, sh_coeff, target_image,
                            vertex_normal, barycentric_buffer, face_buffer, extrinsics, intrinsics, vertex_pos_grad,
@@ -350,8 +355,7 @@ extern "C" hc_status hc_renderer_backward_l1(hc_renderer h, void* stream, int32_
     clear_error();
     HC_REQUIRE(h, "invalid handle");
     HC_REQUIRE(batch > 0, "batch must be positive (%d)", batch);
-    HC_REQUIRE(h->albedo == kVertexColor || h->albedo == kTextured || h->albedo == kTexturedBilinear,
-               "renderer gradients exist only for vertexColor and textured albedo");
+    HC_REQUIRE(has_gradients(h), "renderer gradients exist only for vertexColor and textured albedo");
     HC_REQUIRE(l1_state && render_buffer && vertex_pos && target_image && vertex_normal && barycentric_buffer &&
                    face_buffer && extrinsics && intrinsics && vertex_pos_grad,
                "NULL input/output pointer");
@@ -364,7 +368,7 @@ extern "C" hc_status hc_renderer_backward_l1(hc_renderer h, void* stream, int32_
     l1.mask = foreground_mask;
     l1.state = const_cast<L1State*>(static_cast<const L1State*>(l1_state));
     l1.render = render_buffer;
-    return raster_backward(h->topo, h->ws, h->vacc, h->tacc, h->tpad, (cudaStream_t)stream, batch, h->C, h->albedo,
+    return raster_backward(h->topo, h->ws, h->tacc, h->tpad, (cudaStream_t)stream, batch, h->C, h->albedo,
                            h->shading, h->image_filter, h->texture_filter, nullptr, vertex_pos, vertex_color, texture,
                            texture_height, texture_width, sh_coeff, target_image, vertex_normal, barycentric_buffer,
                            face_buffer, extrinsics, intrinsics, vertex_pos_grad, vertex_color_grad, texture_grad,

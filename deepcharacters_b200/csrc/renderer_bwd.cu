@@ -263,8 +263,8 @@ enum { kAlbVcol = 0, kAlbTex = 1, kAlbNone = 2, kAlbTexBilinear = 3 };
 // colours); k_vertex_grad writes the op's outputs from it.
 template <bool SHADED, int ALB>
 struct VertexSums {
-    static constexpr int kVals = 3 + (ALB == kAlbVcol ? 3 : 0) + (SHADED ? 3 : 0);
-    static constexpr int kStride = (kVals + 3) / 4 * 4;
+    static constexpr int kVals = vertex_sum_values(ALB == kAlbVcol, SHADED);
+    static constexpr int kStride = vertex_sum_floats(ALB == kAlbVcol, SHADED);
     static constexpr int kNormal = ALB == kAlbVcol ? 6 : 3;  // first normal value
 };
 
@@ -890,8 +890,7 @@ static bool target_tensor_map(const RasterWorkspace& ws, const float* target, in
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vacc, SpareBuf& tacc,
-                          SpareBuf& tpad, cudaStream_t s,
+hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, SpareBuf& tacc, SpareBuf& tpad, cudaStream_t s,
                           int B, int C, int albedo, int shading, int ifs, int tfs, const float* grad,
                           const float* verts, const float* colors, const float* texture, int tex_h, int tex_w,
                           const float* sh, const float* target, const float* vnormal, const float* bary,
@@ -904,10 +903,13 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vac
     const int alb = albedo == kVertexColor ? kAlbVcol
                     : albedo == kTextured ? kAlbTex
                     : albedo == kTexturedBilinear ? kAlbTexBilinear : kAlbNone;
-    const int stride = (3 + (alb == kAlbVcol ? 3 : 0) + (shaded ? 3 : 0) + 3) / 4 * 4;  // VertexSums::kStride
-    const size_t vacc_bytes = sizeof(float) * (size_t)stride * (size_t)B * N;
-    // sized with the cameras, so that it grows only where those do
-    HC_TRY(vacc.ensure(vacc_bytes / B * std::max(B, ws.cap_views / C)));
+    ws.vacc_floats = (size_t)vertex_sum_floats(alb == kAlbVcol, shaded) * N;
+    const size_t vacc_bytes = sizeof(float) * ws.vacc_floats * B;
+    if (ws.size_vacc() != HC_OK) {  // no room for as many frames as there are cameras for: this call's
+        cudaGetLastError();
+        clear_error();
+        HC_TRY(ws.vacc.ensure(vacc_bytes));
+    }
     // Texels padded to 16 bytes where the padding's extra pass over the texture
     // costs less than it saves.  Sums (a clear, a read and a write, 32 bytes per
     // texel): two reductions per covered pixel (eight bilinear) become none;
@@ -930,7 +932,7 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vac
     const bool taps = albedo == kTextured && texels > 0 && 4 * pixels >= texels && tpad.room(pad_bytes, capture);
     HC_TRY(ws.claim_b.ensure(sizeof(unsigned)));
     FillRuns zeros;
-    zeros.add(vacc.ptr, vacc_bytes);
+    zeros.add(ws.vacc.ptr, vacc_bytes);
     if (padded) zeros.add(tacc.ptr, pad_bytes);
     else if (texels) zeros.add(tex_grad, sizeof(float) * 3 * (size_t)texels);
     if (sh_grad) zeros.add(sh_grad, sizeof(float) * 27 * (size_t)V);
@@ -966,7 +968,7 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vac
     A.vnormal = vnormal;
     A.bary = bary;
     A.face = face;
-    A.vacc = vacc.as<float>();
+    A.vacc = ws.vacc.as<float>();
     A.tex_grad = tex_grad;
     A.tex_acc = padded ? tacc.as<float4>() : nullptr;
     A.tex_pad = taps ? tpad.as<float4>() : nullptr;
@@ -1025,7 +1027,7 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, DevBuf& vac
 #define HC_VERTEX_CASE(SH, AL)                                                                                \
     case (SH ? 4 : 0) + AL:                                                                                   \
         k_vertex_grad<SH, AL><<<div_up((long long)B * N, 256), 256, 0, s>>>(                                  \
-            B, N, topo.fan.as<int2>(), topo.vf_id.as<int2>(), verts, vacc.as<float>(),                        \
+            B, N, topo.fan.as<int2>(), topo.vf_id.as<int2>(), verts, ws.vacc.as<float>(),                      \
             vpos_grad, vcol_grad);                                                                            \
         break;
         HC_VERTEX_CASE(false, kAlbVcol)
