@@ -321,13 +321,14 @@ __device__ __forceinline__ unsigned long long word_box(int wx, int wy, int tx0, 
     return row * 0x0101010101010101ull & (~0ull >> (56 - 8 * y1)) & (~0ull << (8 * y0));
 }
 
-// a needed tile of a view lies in the box
+// a needed tile of a view lies in the box (a row of words at a time: its loads do not wait for one another)
 __device__ __forceinline__ bool need_in_box(const unsigned long long* need, const ViewImg& vi, int tx0, int ty0, int tx1,
                                             int ty1) {
-    for (int wy = ty0 >> 3; wy <= ty1 >> 3; ++wy)
+    unsigned long long any = 0ull;
+    for (int wy = ty0 >> 3; wy <= ty1 >> 3 && !any; ++wy)
         for (int wx = tx0 >> 3; wx <= tx1 >> 3; ++wx)
-            if (need[vi.word + (long long)wy * vi.words_x + wx] & word_box(wx, wy, tx0, ty0, tx1, ty1)) return true;
-    return false;
+            any |= need[vi.word + (long long)wy * vi.words_x + wx] & word_box(wx, wy, tx0, ty0, tx1, ty1);
+    return any != 0ull;
 }
 
 // the pixels of one tile that a triangle covers, written at once (a pair
@@ -513,32 +514,71 @@ __global__ void k_cov_cull(int N, int F, const int3* __restrict__ faces, const f
     if (keep) cb.items[base + __popc(m & ((1u << lane) - 1u))] = view * F + fi;
 }
 
-// The second, over the listed pairs (persistent): a thread per pair writes its
-// record and walks the needed tiles of its box, the set bits of the box's words.
+// The second, over the listed pairs (persistent, whole warps): a thread per pair
+// writes its record and walks the needed tiles of its box, the set bits of the
+// box's words; a box with more than kCovNeeded of them is taken by the warp, as
+// in the full binning.  A poor hint leaves large triangles thousands of needed
+// tiles: 1024^2, an empty hint, 81,920 small triangles and two that span the view
+// 269 us (a thread per box throughout 1599), 10,000 triangles of 200 px 198 (484).
+// kCovNeeded of 32: 270 and 147 us, but 195 instead of 132 with the first mesh's
+// own face buffer as the hint; of 512: 272, 349 and 132.
+constexpr int kCovNeeded = 128;
+
 __global__ void __launch_bounds__(256, 4) k_cov_bin_list(int N, int F, const int3* __restrict__ faces,
                                                          const float2* __restrict__ p2d, CovBins cb,
                                                          const __grid_constant__ ImgLayout L) {
-    const int n = *cb.n_items;
-    for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < n; it += gridDim.x * blockDim.x) {
-        const int item = cb.items[it], view = item / F, f = item - view * F;
-        const ViewImg vi = view_img(L, view);
+    const int n = *cb.n_items, lane = threadIdx.x & 31;
+    for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += gridDim.x * blockDim.x) {
+        const int it = base + lane;
+        int item = 0;
         CoverTri t;
-        cover_tri(view, N, vi.W, vi.H, faces[f], p2d, t);
-        const Footprint fp = cover_footprint(t, vi.W, vi.H);
-        cb.rec[item] = cover_record(t, fp);
-        const int tx0 = t.x0 / kCovTile, ty0 = t.y0 / kCovTile, tx1 = t.x1 / kCovTile, ty1 = t.y1 / kCovTile;
-        for (int wy = ty0 >> 3; wy <= ty1 >> 3; ++wy)
-            for (int wx = tx0 >> 3; wx <= tx1 >> 3; ++wx) {
-                unsigned long long bits =
-                    cb.need[vi.word + (long long)wy * vi.words_x + wx] & word_box(wx, wy, tx0, ty0, tx1, ty1);
-                for (; bits; bits &= bits - 1ull) {
-                    const int b = __ffsll((long long)bits) - 1, tx = 8 * wx + (b & 7), ty = 8 * wy + (b >> 3);
-                    if (!footprint_overlaps(fp, max(tx * kCovTile, t.x0), min(tx * kCovTile + kCovTile - 1, t.x1),
-                                            max(ty * kCovTile, t.y0), min(ty * kCovTile + kCovTile - 1, t.y1)))
-                        continue;
-                    cov_place(cb, vi, ty * vi.tiles_x + tx, f, item);
-                }
+        t.x0 = t.x1 = t.y0 = t.y1 = 0;
+        TileRows rows;
+        bool many = false;
+        if (it < n) {
+            item = cb.items[it];
+            const int view = item / F, f = item - view * F;
+            const ViewImg vi = view_img(L, view);
+            cover_tri(view, N, vi.W, vi.H, faces[f], p2d, t);
+            const Footprint fp = cover_footprint(t, vi.W, vi.H);
+            cb.rec[item] = cover_record(t, fp);
+            const int tx0 = t.x0 / kCovTile, ty0 = t.y0 / kCovTile, tx1 = t.x1 / kCovTile, ty1 = t.y1 / kCovTile;
+            auto needed = [&](int wx, int wy) {
+                return cb.need[vi.word + (long long)wy * vi.words_x + wx] & word_box(wx, wy, tx0, ty0, tx1, ty1);
+            };
+            if ((tx1 - tx0 + 1) * (ty1 - ty0 + 1) > kCovNeeded) {
+                int count = 0;
+                for (int wy = ty0 >> 3; wy <= ty1 >> 3 && count <= kCovNeeded; ++wy)
+                    for (int wx = tx0 >> 3; wx <= tx1 >> 3; ++wx) count += __popcll(needed(wx, wy));
+                many = count > kCovNeeded;
             }
+            if (many) {
+                rows = TileRows(fp);
+            } else {
+                for (int wy = ty0 >> 3; wy <= ty1 >> 3; ++wy)
+                    for (int wx = tx0 >> 3; wx <= tx1 >> 3; ++wx)
+                        for (unsigned long long bits = needed(wx, wy); bits; bits &= bits - 1ull) {
+                            const int b = __ffsll((long long)bits) - 1, tx = 8 * wx + (b & 7), ty = 8 * wy + (b >> 3);
+                            if (footprint_overlaps(fp, max(tx * kCovTile, t.x0), min(tx * kCovTile + kCovTile - 1, t.x1),
+                                                   max(ty * kCovTile, t.y0), min(ty * kCovTile + kCovTile - 1, t.y1)))
+                                cov_place(cb, vi, ty * vi.tiles_x + tx, f, item);
+                        }
+            }
+        }
+        __syncwarp();  // the records of large triangles are read by the other lanes where a bin overflows
+        unsigned pending = __ballot_sync(0xffffffffu, many);
+        while (pending) {
+            const int src = __ffs(pending) - 1;
+            pending &= pending - 1;
+            const int q = __shfl_sync(0xffffffffu, item, src), view = q / F, f = q - view * F;
+            const ViewImg vi = view_img(L, view);
+            const int qx0 = __shfl_sync(0xffffffffu, t.x0, src), qx1 = __shfl_sync(0xffffffffu, t.x1, src);
+            const int qy0 = __shfl_sync(0xffffffffu, t.y0, src), qy1 = __shfl_sync(0xffffffffu, t.y1, src);
+            warp_tiles(rows.from_lane(src), kCovShift, qx0, qx1, qy0, qy1, lane, [&](int tx, int ty) {
+                if (cb.need[vi.word + (long long)(ty >> 3) * vi.words_x + (tx >> 3)] >> (8 * (ty & 7) + (tx & 7)) & 1ull)
+                    cov_place(cb, vi, ty * vi.tiles_x + tx, f, q);
+            });
+        }
     }
 }
 
