@@ -513,7 +513,8 @@ __device__ __forceinline__ float3 shade_pixel(const ShadeArgs& A, const ViewCam&
 // Accepted hits and their depth are those of raster_hit.  The barycentric
 // window (a, b <= 1.001 |N|^2 after the sign tests) is decided without the two
 // divisions unless a value is near its end or not a number, or |N|^2 is near
-// underflow or overflow (there the quotients are NaN and the hit is refused).
+// overflow (there the quotients are NaN and the hit is refused); it is never near
+// underflow, since |N| is at least the |dir . N| of 1e-7 tested first.
 __device__ __forceinline__ bool raster_hit_below(float3 ro_s, float3 dir, const TriS& T, float num,
                                                  unsigned best_d, bool inside, int& depth_q) {
     const float ndr = dot(dir, T.n);
@@ -533,7 +534,7 @@ __device__ __forceinline__ bool raster_hit_below(float3 ro_s, float3 dir, const 
     const float b = dot(T.n, C);
     if (b < 0.f) return false;
     const float denom = dot(T.n, T.n);
-    if (denom > 1e-30f && denom < 1e30f && a <= 1.0005f * denom && b <= 1.0005f * denom) return true;
+    if (denom < 1e30f && a <= 1.0005f * denom && b <= 1.0005f * denom) return true;
     return (a / denom >= -0.001f) && (b / denom >= -0.001f) && (a / denom <= 1.001f) && (b / denom <= 1.001f);
 }
 
