@@ -925,12 +925,18 @@ struct hc_skin_s {
     }
 };
 
-// Opt a kernel in to more than 48 KB of dynamic shared memory (hc_skin_create
-// bounds what a handle needs).
+// The dynamic shared memory that a handle's blocks may need: hc_skin_create
+// bounds the staged block, the adjoint adds six values per vertex.
+constexpr size_t kSkinStaged = 200u << 10, kSkinSmem = kSkinStaged + sizeof(float) * 6 * kSkinBlock;
+static_assert(kSkinSmem <= 227u << 10, "shared memory of a block");
+
+// Opt a kernel in to more than 48 KB of dynamic shared memory.  The limit is the
+// kernel's, not the handle's: always the same one, so that a handle cannot lower it
+// between another one's call and its launch.
 template <typename K>
 static hc_status skin_allow_smem(K kernel, size_t bytes) {
     if (bytes <= (48u << 10)) return HC_OK;
-    HC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    HC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSkinSmem));
     return HC_OK;
 }
 
@@ -950,7 +956,7 @@ extern "C" hc_status hc_skin_create(hc_skin* out, int32_t n_joints, const int32_
     *out = nullptr;
     HC_REQUIRE(n_joints > 0 && n_dofs > 0 && n_skin > 0 && n_vertices > 0 && k > 0, "empty skeleton or mesh");
     HC_REQUIRE(n_skin <= 1024, "at most 1024 skinning joints (got %d)", n_skin);
-    HC_REQUIRE(skin_block_smem(n_skin, 12, k, kSkinBlock) <= (200u << 10),
+    HC_REQUIRE(skin_block_smem(n_skin, 12, k, kSkinBlock) <= kSkinStaged,
                "%d skinning joints with %d per vertex exceed the staged skinning block", n_skin, k);
     HC_REQUIRE(parent && joint_type && offset && axis && dof_offsets && dof_joint && dof_weight && skin_joint &&
                    base_vertices && base_normals && skin_index,
