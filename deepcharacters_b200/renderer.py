@@ -81,6 +81,13 @@ class RendererEngine:
                       self.N, self.C, self.W, self.H, albedo_mode.encode(), shading_mode.encode(),
                       self.image_filter_size, self.texture_filter_size, compute_normal_map.encode())
         self._h = h
+        self.device = torch.cuda.current_device()  # owns the handle's allocations
+
+    def _elsewhere(self, device: torch.device):
+        """For a call outside the engine's device: its tensors have to be there, then it is made current."""
+        if device.index != self.device:
+            raise ValueError(f"vertex_pos is on {device}, the engine on cuda:{self.device}")
+        return torch.cuda.device(self.device)
 
     def image_shape(self, B: int) -> tuple:
         """Leading shape of the per-pixel buffers: [B, C, H, W] or, with
@@ -121,7 +128,8 @@ class RendererEngine:
         return self._h
 
     def reserve(self, batch: int):
-        _lib.call("hc_renderer_reserve", self._h, int(batch))
+        with torch.cuda.device(self.device):
+            _lib.call("hc_renderer_reserve", self._h, int(batch))
 
     def set_tuning(self, tile: int, bin_capacity: int):
         _lib.call("hc_renderer_set_tuning", self._h, int(tile), int(bin_capacity))
@@ -139,7 +147,8 @@ class RendererEngine:
     def stats(self) -> tuple[int, int]:
         b = C.c_int64()
         s = C.c_int64()
-        _lib.call("hc_renderer_stats", self._h, _stream(), C.byref(b), C.byref(s))
+        with torch.cuda.device(self.device):
+            _lib.call("hc_renderer_stats", self._h, _stream(), C.byref(b), C.byref(s))
         return b.value, s.value
 
     def forward(self, vertex_pos, vertex_color, texture, sh_coeff, extrinsics, intrinsics, batch: int | None = None,
@@ -148,6 +157,11 @@ class RendererEngine:
         vp = _f32(vertex_pos, "vertex_pos")
         B = int(batch if batch is not None else vp.shape[0])
         dev = vp.device
+        stream = torch.cuda.current_stream()
+        if dev.index != self.device or stream.device_index != self.device:
+            with self._elsewhere(dev):
+                return self.forward(vertex_pos, vertex_color, texture, sh_coeff, extrinsics, intrinsics, batch,
+                                    diagnostics, out)
         vc = _f32(vertex_color, "vertex_color")
         tex = _f32(texture, "texture")
         sh = _f32(sh_coeff, "sh_coeff")
@@ -172,8 +186,8 @@ class RendererEngine:
             depth_q = torch.empty(img, device=dev, dtype=torch.int32)
             tie = torch.empty(img, device=dev, dtype=torch.int32)
         P = _lib.ptr
-        _lib.call("hc_renderer_forward_ex", self._h, _stream(), B, P(vp), P(vc), P(tex), TH, TW, P(sh), P(ex), P(it),
-                  P(bary), P(face), P(render), P(vnormal),
+        _lib.call("hc_renderer_forward_ex", self._h, stream.cuda_stream, B, P(vp), P(vc), P(tex), TH, TW, P(sh), P(ex),
+                  P(it), P(bary), P(face), P(render), P(vnormal),
                   P(normal_map) if self.compute_normal_map != "none" else None, P(depth_q), P(tie))
         res = (bary, face, render, vnormal, normal_map)
         if diagnostics:
@@ -181,12 +195,12 @@ class RendererEngine:
         return res
 
 
-# Engines by attribute set, the most recently used last.  An engine is found by
+# Engines by attribute set and device, the most recently used last.  An engine is found by
 # comparing its topology's contents with the call's: a comparison of the two
 # arrays costs a fraction of copying and hashing them into a key (12 MB at
 # 327,680 faces with texture coordinates took 3 ms of every call).
-_ENGINES: list = []  # (attributes, faces, texture coordinates or None, engine)
-_ENGINES_MOST = 16
+_ENGINES: list = []  # (attributes and device, faces, texture coordinates or None, engine)
+_ENGINES_MOST = 16  # on each device
 _ENGINES_LOCK = threading.Lock()
 _memcmp = C.CDLL(None).memcmp
 _memcmp.argtypes, _memcmp.restype = [C.c_void_p, C.c_void_p, C.c_size_t], C.c_int
@@ -199,23 +213,27 @@ def _same_bytes(a, b) -> bool:
 
 
 def get_engine(faces, tex_coords, n_vertices, n_cameras, width, height, albedo_mode, shading_mode,
-               image_filter_size, texture_filter_size, compute_normal_map) -> RendererEngine:
-    """Engine per attribute set, like one TF op instance per graph node."""
+               image_filter_size, texture_filter_size, compute_normal_map, device: int | None = None) -> RendererEngine:
+    """Engine per attribute set and device (default: the current one), like one TF op instance per graph node."""
+    device = torch.cuda.current_device() if device is None else int(device)
     f = np.ascontiguousarray(np.asarray(faces, dtype=np.int32).reshape(-1))
     tc = None if tex_coords is None or len(tex_coords) == 0 else np.ascontiguousarray(
         np.asarray(tex_coords, dtype=np.float32).reshape(-1))
     attrs = (int(n_vertices), int(n_cameras), int(width), int(height), albedo_mode, shading_mode,
              int(image_filter_size), int(texture_filter_size), compute_normal_map)
+    key = attrs + (device,)
     with _ENGINES_LOCK:
         for i in range(len(_ENGINES) - 1, -1, -1):
             e = _ENGINES[i]
-            if e[0] == attrs and _same_bytes(e[1], f) and _same_bytes(e[2], tc):
+            if e[0] == key and _same_bytes(e[1], f) and _same_bytes(e[2], tc):
                 _ENGINES.append(_ENGINES.pop(i))
                 return e[3]
         f, tc = f.copy(), None if tc is None else tc.copy()  # the caller's arrays may change later
-        engine = RendererEngine(f, tc, *attrs)
-        _ENGINES.append((attrs, f, tc, engine))
-        del _ENGINES[:-_ENGINES_MOST]
+        with torch.cuda.device(device):
+            engine = RendererEngine(f, tc, *attrs)
+        _ENGINES.append((key, f, tc, engine))
+        for i in [i for i, e in enumerate(_ENGINES) if e[0][-1] == device][-_ENGINES_MOST - 1::-1]:
+            del _ENGINES[i]  # from the end: the indices before stay
         return engine
 
 
@@ -259,6 +277,12 @@ def renderer_backward(engine: RendererEngine, render_buffer_grad, vertex_pos, ve
     vp = _f32(vertex_pos, "vertex_pos")
     B = int(batch if batch is not None else vp.shape[0])
     dev = vp.device
+    stream = torch.cuda.current_stream()
+    if dev.index != engine.device or stream.device_index != engine.device:
+        with engine._elsewhere(dev):
+            return renderer_backward(engine, render_buffer_grad, vertex_pos, vertex_color, texture, sh_coeff,
+                                     target_image, vertex_normal, barycentric_buffer, face_buffer, extrinsics,
+                                     intrinsics, batch)
     g = _f32(render_buffer_grad, "render_buffer_grad")
     vc = _f32(vertex_color, "vertex_color")
     tex = _f32(texture, "texture")
@@ -278,8 +302,8 @@ def renderer_backward(engine: RendererEngine, render_buffer_grad, vertex_pos, ve
                                                                dtype=torch.float32)
     gsh = torch.empty((B, engine.C, 27), device=dev, dtype=torch.float32)
     P = _lib.ptr
-    _lib.call("hc_renderer_backward", engine.handle, _stream(), B, P(g), P(vp), P(vc), P(tex), TH, TW, P(sh), P(tgt),
-              P(vn), P(bary), P(face), P(ex), P(it), P(gpos), P(gcol), P(gtex) if TH > 0 else None, P(gsh))
+    _lib.call("hc_renderer_backward", engine.handle, stream.cuda_stream, B, P(g), P(vp), P(vc), P(tex), TH, TW, P(sh),
+              P(tgt), P(vn), P(bary), P(face), P(ex), P(it), P(gpos), P(gcol), P(gtex) if TH > 0 else None, P(gsh))
     return gpos, gcol, gtex, gsh
 
 
@@ -313,7 +337,8 @@ class CudaRendererGpu:
         self.nodeName = nodeName
         self.engine = get_engine(faces_attr, texCoords_attr, numberOfVertices_attr, numberOfCameras_attr,
                                  renderResolutionU_attr, renderResolutionV_attr, albedoMode_attr, shadingMode_attr,
-                                 image_filter_size_attr, texture_filter_size_attr, compute_normal_map_attr)
+                                 image_filter_size_attr, texture_filter_size_attr, compute_normal_map_attr,
+                                 vertexPos_input.device.index if getattr(vertexPos_input, "is_cuda", False) else None)
         self.cudaRendererOperator = _RenderFn.apply(self.engine, vertexPos_input, vertexColor_input, texture_input,
                                                     shCoeff_input, targetImage_input, extrinsics_input,
                                                     intrinsics_input)
