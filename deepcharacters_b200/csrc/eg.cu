@@ -315,7 +315,7 @@ struct hc_eg_s {
 };
 
 namespace hc {
-void build_vertex_fans(int N, const int32_t* faces, int F, std::vector<int2>& fan, std::vector<int>& vf_id);
+void build_vertex_faces(int N, const int32_t* faces, int F, std::vector<int>& vf, std::vector<int>& vf_id);
 }
 
 extern "C" hc_status hc_eg_create(hc_eg* out, int32_t n_vertices, const float* base_vertices, const int32_t* faces,
@@ -362,9 +362,12 @@ extern "C" hc_status hc_eg_create(hc_eg* out, int32_t n_vertices, const float* b
     h->M = n_nodes;
     h->Mk = n_markers;
     h->F = n_faces;
-    std::vector<int2> fan;
-    std::vector<int> vf_id;
-    build_vertex_fans(n_vertices, faces, n_faces, fan, vf_id);
+    std::vector<int> vf, vf_id;
+    build_vertex_faces(n_vertices, faces, n_faces, vf, vf_id);
+    std::vector<int2> fan(vf.size());
+    for (int v = 0; v < n_vertices; ++v)
+        for (int k = vf_id[2 * v]; k < vf_id[2 * v] + vf_id[2 * v + 1]; ++k)
+            fan[k] = fan_entry(v, faces[3 * vf[k]], faces[3 * vf[k] + 1], faces[3 * vf[k] + 2]);
     hc_status st = HC_OK;
 #define UP(buf, ptr, n)                                   \
     if (st == HC_OK) st = upload(h->buf, ptr, (size_t)(n));

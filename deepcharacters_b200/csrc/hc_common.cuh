@@ -75,6 +75,13 @@ struct DevBuf {
     T* as() const { return reinterpret_cast<T*>(ptr); }
 };
 
+// One of several arrays in an allocation.
+struct DevPart {
+    void* ptr = nullptr;
+    template <class T>
+    T* as() const { return reinterpret_cast<T*>(ptr); }
+};
+
 // Scratch that a call is faster with and can do without: there is no room where
 // memory is short, where a capture would have to allocate it, and where growing it
 // would free what a captured graph addresses.

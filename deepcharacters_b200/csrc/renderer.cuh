@@ -524,6 +524,12 @@ struct FanFace {
     }
 };
 
+// the entry of vertex v for its face (a, b, c)
+__host__ __device__ __forceinline__ int2 fan_entry(int v, int a, int b, int c) {
+    const unsigned place = v == a ? 0u : v == b ? 1u : 2u;
+    return make_int2(place == 0u ? b : a, (int)((unsigned)(place == 2u ? b : c) | place << 30));
+}
+
 // Sum of a vertex's incident face normals in increasing face order.
 __device__ __forceinline__ float3 fan_normal(const float* __restrict__ P, const int2* __restrict__ fan, int2 range,
                                              int v) {
@@ -569,12 +575,19 @@ __device__ __forceinline__ float3 sh_illum(const float* sh, float3 n) {
 
 struct Topology {
     int N = 0, F = 0;
-    DevBuf faces;        // int3[F]
-    DevBuf fan;          // int2[3F]  vertex -> incident faces, increasing face id (FanFace)
-    DevBuf vf_id;        // int2[N]  (start, count)
-    DevBuf texcoords;    // float[6F]
+    DevBuf mem;          // the arrays below, in one allocation
+    DevPart faces;       // int3[F]
+    DevPart fan;         // int2[3F]  vertex -> incident faces, increasing face id (FanFace)
+    DevPart vf_id;       // int2[N]  (start, count)
+    DevPart texcoords;   // float[6F]
+    DevPart unit;        // float4[unit_frames * N]  normalised vertex normals of a UV map call
+    int unit_frames = 0;
     bool has_texcoords = false;
 };
+// Frames whose normalised vertex normals have a place beside the topology: an
+// allocation of their own makes an engine's first UV maps take 1.27 instead of
+// 0.90 ms (40,962 vertices).
+constexpr int kUnitFrames = 4;
 
 // texel -> (face, barycentrics) table of the UV-space maps for one texture size
 struct UvTable {
@@ -586,7 +599,7 @@ struct UvTable {
 
 struct UvTables {
     std::vector<UvTable> tables;  // one for each size that a graph holds, and at most one besides
-    SpareBuf unit;  // normalised vertex normals of a call, 16 bytes each
+    SpareBuf unit;  // normalised vertex normals of a call of more than Topology::unit_frames frames, 16 bytes each
     // the table of a texture size; the call has to build it unless it is valid
     hc_status get(int th, int tw, cudaStreamCaptureStatus capture, UvTable** out) {
         const bool recording = capture != cudaStreamCaptureStatusNone;

@@ -186,7 +186,10 @@ hc_status raster_uv_maps(const Topology& topo, UvTables& tab, cudaStream_t s, in
     // without room for them the normals are normalised where they are used
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     HC_CUDA(cudaStreamIsCapturing(s, &capture));
-    if (mode == kNmOriginal && tab.unit.room(sizeof(float4) * (size_t)B * N, capture)) S.unit = tab.unit.as<float4>();
+    if (mode == kNmOriginal) {
+        if (B <= topo.unit_frames) S.unit = topo.unit.as<float4>();
+        else if (tab.unit.room(sizeof(float4) * (size_t)B * N, capture)) S.unit = tab.unit.as<float4>();
+    }
     S.fills.add(face, sizeof(int) * (size_t)px, 0xff);
     S.fills.add(bary, sizeof(float) * 2 * (size_t)px);
     S.fills.add(render, sizeof(float) * 3 * (size_t)px);

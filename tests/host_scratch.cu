@@ -127,11 +127,26 @@ static int uv_no_memory() {
     return 0;
 }
 
+// a vertex's entry names its place in the face and the others in the face's order
+static int fan_entries() {
+    const int face[5][3] = {{4, 7, 9}, {7, 4, 9}, {9, 7, 4}, {4, 4, 9}, {9, 4, 4}};  // the last two degenerate
+    for (const auto& f : face)
+        for (int v : {4, 7, 9}) {
+            const int place = v == f[0] ? 0 : v == f[1] ? 1 : v == f[2] ? 2 : -1;
+            if (place < 0) continue;
+            const int2 e = fan_entry(v, f[0], f[1], f[2]);
+            CHECK((unsigned)e.y >> 30 == (unsigned)place && e.x == f[place == 0 ? 1 : 0] &&
+                  (e.y & 0x3fffffff) == f[place == 2 ? 1 : 2]);
+        }
+    return 0;
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, int (*)()> checks = {
         {"uv_held", uv_held},
         {"uv_recorded", uv_recorded},
         {"uv_no_memory", uv_no_memory},
+        {"fan_entries", fan_entries},
     };
     const auto it = checks.find(argc > 1 ? argv[1] : "");
     return it == checks.end() ? 2 : it->second();

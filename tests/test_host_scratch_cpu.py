@@ -22,7 +22,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("check", ["uv_held", "uv_recorded", "uv_no_memory"])
+@pytest.mark.parametrize("check", ["uv_held", "uv_recorded", "uv_no_memory", "fan_entries"])
 def test_host_buffers(program, check):
     r = subprocess.run([program, check], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
