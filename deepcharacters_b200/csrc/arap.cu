@@ -137,6 +137,12 @@ struct hc_arap_s {
     }
 };
 
+static void release(hc_arap h) {
+    DevBuf* bufs[] = {&h->base, &h->node_vertex, &h->off, &h->size, &h->idx, &h->rev, &h->rigid};
+    for (DevBuf* b : bufs) b->release();
+    delete h;
+}
+
 extern "C" hc_status hc_arap_create(hc_arap* out, int32_t n_vertices, const float* base_vertices, int32_t n_nodes,
                                     const int32_t* node_to_base_vertex, const int32_t* n2n_offsets,
                                     const int32_t* n2n_sizes, const int32_t* n2n_indices,
@@ -186,7 +192,7 @@ extern "C" hc_status hc_arap_create(hc_arap* out, int32_t n_vertices, const floa
     UP(rigid, rigidity_weights, n_nodes);
 #undef UP
     if (st != HC_OK) {
-        delete h;
+        release(h);
         return st;
     }
     *out = h;
@@ -195,10 +201,7 @@ extern "C" hc_status hc_arap_create(hc_arap* out, int32_t n_vertices, const floa
 
 extern "C" hc_status hc_arap_destroy(hc_arap h) {
     clear_error();
-    if (!h) return HC_OK;
-    DevBuf* bufs[] = {&h->base, &h->node_vertex, &h->off, &h->size, &h->idx, &h->rev, &h->rigid};
-    for (DevBuf* b : bufs) b->release();
-    delete h;
+    if (h) release(h);
     return HC_OK;
 }
 

@@ -314,6 +314,14 @@ struct hc_eg_s {
     DevBuf tab, packed;
 };
 
+static void release(hc_eg h) {
+    DevBuf* bufs[] = {&h->base, &h->node_vertex, &h->n2v_off, &h->n2v_size, &h->n2v_idx, &h->n2v_w, &h->markers,
+                      &h->m2n, &h->n2m, &h->fan, &h->vf_id, &h->tab, &h->packed, &h->base4, &h->v2n_poff,
+                      &h->v2n_pidx, &h->v2n_pw};
+    for (DevBuf* b : bufs) b->release();
+    delete h;
+}
+
 namespace hc {
 void build_vertex_faces(int N, const int32_t* faces, int F, std::vector<int>& vf, std::vector<int>& vf_id);
 }
@@ -410,7 +418,7 @@ extern "C" hc_status hc_eg_create(hc_eg* out, int32_t n_vertices, const float* b
     }
 #undef UP
     if (st != HC_OK) {
-        delete h;
+        release(h);
         return st;
     }
     *out = h;
@@ -419,12 +427,7 @@ extern "C" hc_status hc_eg_create(hc_eg* out, int32_t n_vertices, const float* b
 
 extern "C" hc_status hc_eg_destroy(hc_eg h) {
     clear_error();
-    if (!h) return HC_OK;
-    DevBuf* bufs[] = {&h->base, &h->node_vertex, &h->n2v_off,
-                      &h->n2v_size, &h->n2v_idx, &h->n2v_w, &h->markers, &h->m2n, &h->n2m, &h->fan,
-                      &h->vf_id, &h->tab, &h->packed, &h->base4, &h->v2n_poff, &h->v2n_pidx, &h->v2n_pw};
-    for (DevBuf* b : bufs) b->release();
-    delete h;
+    if (h) release(h);
     return HC_OK;
 }
 

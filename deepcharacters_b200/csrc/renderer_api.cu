@@ -151,6 +151,20 @@ static long long frame_pixels(const hc_renderer_s* h) {
     return p;
 }
 
+static void release_all(hc_renderer_s* r) {
+    if (r->ws.clock.made)
+        for (cudaEvent_t& e : r->ws.clock.ev) cudaEventDestroy(e);
+    r->ws.clock.made = false;
+    DevBuf* bufs[] = {&r->topo.mem,
+                      &r->ws.cams, &r->ws.tri_frame, &r->ws.tri_view, &r->ws.tile_state,
+                      &r->ws.bins, &r->ws.spill, &r->ws.spill_keys, &r->ws.stats, &r->ws.vacc, &r->tacc, &r->tpad,
+                      &r->uv.unit, &r->ws.layout, &r->ws.tile_cam, &r->ws.tile_cam_b, &r->ws.proj,
+                      &r->ws.claim, &r->ws.claim_b};
+    for (DevBuf* b : bufs) b->release();
+    for (UvTable& t : r->uv.tables) t.buf.release();
+    delete r;
+}
+
 extern "C" hc_status hc_renderer_create(hc_renderer* out, const int32_t* faces, int32_t n_faces,
                                         const float* texture_coordinates, int32_t n_texcoords,
                                         int32_t number_of_vertices, int32_t number_of_cameras,
@@ -183,7 +197,7 @@ extern "C" hc_status hc_renderer_create(hc_renderer* out, const int32_t* faces, 
     hc_status st = topology_upload(r->topo, number_of_vertices, faces, n_faces, texture_coordinates, n_texcoords,
                                    nm == kNmOriginal ? kUnitFrames : 0);
     if (st != HC_OK) {
-        delete r;
+        release_all(r);
         return st;
     }
     r->C = number_of_cameras;
@@ -200,24 +214,9 @@ extern "C" hc_status hc_renderer_create(hc_renderer* out, const int32_t* faces, 
     return HC_OK;
 }
 
-static void release_all(hc_renderer_s* r) {
-    if (r->ws.clock.made)
-        for (cudaEvent_t& e : r->ws.clock.ev) cudaEventDestroy(e);
-    r->ws.clock.made = false;
-    DevBuf* bufs[] = {&r->topo.mem,
-                      &r->ws.cams, &r->ws.tri_frame, &r->ws.tri_view, &r->ws.tile_state,
-                      &r->ws.bins, &r->ws.spill, &r->ws.spill_keys, &r->ws.stats, &r->ws.vacc, &r->tacc, &r->tpad,
-                      &r->uv.unit, &r->ws.layout, &r->ws.tile_cam, &r->ws.tile_cam_b, &r->ws.proj,
-                      &r->ws.claim, &r->ws.claim_b};
-    for (DevBuf* b : bufs) b->release();
-    for (UvTable& t : r->uv.tables) t.buf.release();
-}
-
 extern "C" hc_status hc_renderer_destroy(hc_renderer h) {
     clear_error();
-    if (!h) return HC_OK;
-    release_all(h);
-    delete h;
+    if (h) release_all(h);
     return HC_OK;
 }
 

@@ -97,7 +97,6 @@ __device__ __forceinline__ void mat_to_quat(const float* R, float* q) {
 
 struct Skel {
     int J, D, S, K, N;
-    const int* parent;
     const int* type;
     const float* offset;   // [J,3]
     const float* axis;     // [J,3] local
@@ -117,14 +116,11 @@ struct Skel {
     const int* level_off;    // [levels+1]
     const int* level_joint;  // [J]: joint << 16 | parent + 1
     // the adjoint's vertex blocks: each block's (vertex, slot) pairs by skinning joint
-    int grad_block;          // vertices per block
     const int* bone_off;     // [blocks, S+1]
     const unsigned* bone_slot;  // [N,K]: (vertex * K + slot) << 8 | vertex, within the block
     const int* skin_idx;   // [N,K] skinning joint per vertex slot
-    const float* base_v;   // [N,3]
-    const float* base_n;   // [N,3]
-    const float4* base_v4;  // [N] the same, padded to float4 (one 16-byte load per vertex)
-    const float4* base_n4;  // [N]
+    const float4* base_v4;  // [N] base vertices, padded to float4 (one 16-byte load per vertex)
+    const float4* base_n4;  // [N] base normals
 };
 
 // Forward kinematics, one CTA per frame.  Every joint sums its dof entries (in
@@ -882,8 +878,8 @@ using namespace hc;
 struct hc_skin_s {
     int J = 0, D = 0, S = 0, K = 0, N = 0, E = 0;
     int parity = 1;
-    DevBuf parent, type, offset, axis, jscale, dof_off, dof_joint, dof_w, skin_joint, skin_scale, t0inv, in_chain,
-        skin_idx, base_v, base_n, base_v4, base_n4;
+    DevBuf type, offset, axis, jscale, dof_off, dof_joint, dof_w, skin_joint, skin_scale, t0inv, in_chain, skin_idx,
+        base_v4, base_n4;
     DevBuf tree;   // joint_off, joint_dof, joint_w, level_off, level_joint of Skel
     DevBuf bones;  // bone_off, bone_slot of Skel
     DevBuf mom, gpos, gaxis, dq_ws, gdq;
@@ -895,7 +891,6 @@ struct hc_skin_s {
         s.S = S;
         s.K = K;
         s.N = N;
-        s.parent = parent.as<int>();
         s.type = type.as<int>();
         s.offset = offset.as<float>();
         s.axis = axis.as<float>();
@@ -908,8 +903,6 @@ struct hc_skin_s {
         s.t0inv = t0inv.as<float>();
         s.in_chain = in_chain.as<unsigned char>();
         s.skin_idx = skin_idx.as<int>();
-        s.base_v = base_v.as<float>();
-        s.base_n = base_n.as<float>();
         s.base_v4 = base_v4.as<float4>();
         s.base_n4 = base_n4.as<float4>();
         s.levels = levels;
@@ -918,12 +911,19 @@ struct hc_skin_s {
         s.joint_w = reinterpret_cast<const float*>(s.joint_dof + E);
         s.level_off = s.joint_dof + 2 * E;
         s.level_joint = s.level_off + levels + 1;
-        s.grad_block = grad_block;
         s.bone_off = bones.as<int>();
         s.bone_slot = bones.as<unsigned>() + (size_t)((N + grad_block - 1) / grad_block) * (S + 1);
         return s;
     }
 };
+
+static void release(hc_skin h) {
+    DevBuf* bufs[] = {&h->type, &h->offset, &h->axis, &h->jscale, &h->dof_off, &h->dof_joint, &h->dof_w,
+                      &h->skin_joint, &h->skin_scale, &h->t0inv, &h->in_chain, &h->skin_idx, &h->base_v4,
+                      &h->base_n4, &h->tree, &h->bones, &h->mom, &h->gpos, &h->gaxis, &h->dq_ws, &h->gdq};
+    for (DevBuf* b : bufs) b->release();
+    delete h;
+}
 
 // The dynamic shared memory that a handle's blocks may need: hc_skin_create
 // bounds the staged block, the adjoint adds six values per vertex.
@@ -1015,7 +1015,6 @@ extern "C" hc_status hc_skin_create(hc_skin* out, int32_t n_joints, const int32_
     hc_status st = HC_OK;
 #define UP(buf, ptr, n) \
     if (st == HC_OK) st = upload(h->buf, ptr, (size_t)(n));
-    UP(parent, parent, n_joints);
     UP(type, joint_type, n_joints);
     UP(offset, offset, 3LL * n_joints);
     UP(axis, axis, 3LL * n_joints);
@@ -1028,8 +1027,6 @@ extern "C" hc_status hc_skin_create(hc_skin* out, int32_t n_joints, const int32_
     UP(t0inv, t0.data(), t0.size());
     UP(in_chain, chain.data(), chain.size());
     UP(skin_idx, skin_index, (long long)n_vertices * k);
-    UP(base_v, base_vertices, 3LL * n_vertices);
-    UP(base_n, base_normals, 3LL * n_vertices);
     {
         std::vector<float4> bv4((size_t)n_vertices), bn4((size_t)n_vertices);
         for (int v = 0; v < n_vertices; ++v) {
@@ -1091,7 +1088,7 @@ extern "C" hc_status hc_skin_create(hc_skin* out, int32_t n_joints, const int32_
     }
 #undef UP
     if (st != HC_OK) {
-        delete h;
+        release(h);
         return st;
     }
     *out = h;
@@ -1100,13 +1097,7 @@ extern "C" hc_status hc_skin_create(hc_skin* out, int32_t n_joints, const int32_
 
 extern "C" hc_status hc_skin_destroy(hc_skin h) {
     clear_error();
-    if (!h) return HC_OK;
-    DevBuf* bufs[] = {&h->parent, &h->type, &h->offset, &h->axis, &h->jscale, &h->dof_off, &h->dof_joint, &h->dof_w,
-                      &h->skin_joint, &h->skin_scale, &h->t0inv, &h->in_chain, &h->skin_idx, &h->base_v,
-                      &h->base_n, &h->tree, &h->bones, &h->mom, &h->gpos, &h->gaxis,
-                      &h->dq_ws, &h->gdq};
-    for (DevBuf* b : bufs) b->release();
-    delete h;
+    if (h) release(h);
     return HC_OK;
 }
 
