@@ -116,7 +116,7 @@ struct Skel {
     const int* level_off;    // [levels+1]
     const int* level_joint;  // [J]: joint << 16 | parent + 1
     // the adjoint's vertex blocks: each block's (vertex, slot) pairs by skinning joint
-    const int* bone_off;     // [blocks, S+1]
+    const int* bone_off;     // [blocks, S+1], within the block
     const unsigned* bone_slot;  // [N,K]: (vertex * K + slot) << 8 | vertex, within the block
     const int* skin_idx;   // [N,K] skinning joint per vertex slot
     const float4* base_v4;  // [N] base vertices, padded to float4 (one 16-byte load per vertex)
@@ -539,11 +539,41 @@ __device__ __forceinline__ float3 lbs_grads(const Skel& sk, int B, int b, int v,
                        M[6] * g.x + M[7] * g.y + M[8] * g.z);
 }
 
+// The adjoint's pair lists of a vertex block of G, a CTA each, when a handle is
+// made: where each bone's (vertex, slot) pairs begin, and the pairs, a warp per
+// bone, in vertex order.
+constexpr int kListBlock = 256;
+__global__ void __launch_bounds__(kListBlock) k_bone_lists(int N, int K, int S, int G, const int* __restrict__ skin_idx,
+                                                           int* __restrict__ off, unsigned* __restrict__ slot) {
+    extern __shared__ int s_at[];  // [S+1]
+    const int v0 = blockIdx.x * G, n = min(G, N - v0) * K, lane = threadIdx.x & 31;
+    const int* I = skin_idx + (long long)v0 * K;
+    for (int s = threadIdx.x; s <= S; s += kListBlock) s_at[s] = 0;
+    __syncthreads();
+    for (int e = threadIdx.x; e < n; e += kListBlock) atomicAdd(s_at + I[e] + 1, 1);
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int s = 0; s < S; ++s) s_at[s + 1] += s_at[s];
+    __syncthreads();
+    for (int s = threadIdx.x; s <= S; s += kListBlock) off[(long long)blockIdx.x * (S + 1) + s] = s_at[s];
+    unsigned* out = slot + (long long)v0 * K;
+    for (int s = threadIdx.x >> 5; s < S; s += kListBlock >> 5) {  // warp-uniform
+        const int end = s_at[s + 1];
+        for (int at = s_at[s], e0 = 0; at < end; e0 += 32) {
+            const int e = e0 + lane;
+            const bool mine = e < n && I[e] == s;
+            const unsigned m = __ballot_sync(0xffffffffu, mine);
+            if (mine) out[at + __popc(m & ((1u << lane) - 1u))] = (unsigned)e << 8 | (unsigned)(e / K);
+            at += __popc(m);
+        }
+    }
+}
+
 // The skinning adjoint of a block of vertices of one frame (grid (vertex
 // blocks, frames)): a thread per vertex forms the gradients of its weights
 // (and, LBS, its displacement) from the staged joint table, and the block adds
 // its part of the bone moments A_s = sum w (v x g), G_s = sum w g.  The block's
-// (vertex, slot) pairs are listed by bone when the handle is made, so a warp
+// (vertex, slot) pairs are listed by bone when the handle is made (k_bone_lists), so a warp
 // sums a bone's pairs in registers and adds six values per bone.
 // Reads and writes 100 bytes per vertex at K = 4; bound by instruction issue.
 // 16 frames x 40,962 vertices, 24 joints: 41 us, where six shared-memory
@@ -593,12 +623,13 @@ __global__ void __launch_bounds__(256) k_skin_grad(Skel sk, int B, const float* 
     }
     const int lane = threadIdx.x & 31;
     const int* off = sk.bone_off + (long long)blockIdx.x * (sk.S + 1);
+    const unsigned* slots = sk.bone_slot + (long long)v0 * K;
     for (int s = threadIdx.x >> 5; s < sk.S; s += G >> 5) {  // warp-uniform
         const int e0 = off[s], e1 = off[s + 1];
         if (e0 == e1) continue;
         float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         for (int e = e0 + lane; e < e1; e += 32) {
-            const unsigned q = sk.bone_slot[e];
+            const unsigned q = slots[e];
             const float wk = s_w[q >> 8];
 #pragma unroll
             for (int c = 0; c < 6; ++c) a[c] += wk * s_m[c * G + (q & 255u)];
@@ -1027,6 +1058,20 @@ extern "C" hc_status hc_skin_create(hc_skin* out, int32_t n_joints, const int32_
     UP(t0inv, t0.data(), t0.size());
     UP(in_chain, chain.data(), chain.size());
     UP(skin_idx, skin_index, (long long)n_vertices * k);
+    // each adjoint block's (vertex, slot) pairs by skinning joint; the copies below wait for the kernel
+    const int G = h->grad_block = skin_grad_smem(n_skin, 12, k, 256) <= (96u << 10) ? 256 : 128;
+    const long long blocks = div_up(n_vertices, G);
+    if (st == HC_OK) st = h->bones.ensure(sizeof(int) * (size_t)(blocks * (n_skin + 1) + (long long)n_vertices * k));
+    if (st == HC_OK) {
+        const Skel sk = h->skel();
+        k_bone_lists<<<(unsigned)blocks, kListBlock, sizeof(int) * (n_skin + 1)>>>(
+            n_vertices, k, n_skin, G, sk.skin_idx, const_cast<int*>(sk.bone_off), const_cast<unsigned*>(sk.bone_slot));
+        count_launch();
+        if (cudaGetLastError() != cudaSuccess) {
+            set_error("the adjoint's lists could not be made");
+            st = HC_ERR_CUDA;
+        }
+    }
     {
         std::vector<float4> bv4((size_t)n_vertices), bn4((size_t)n_vertices);
         for (int v = 0; v < n_vertices; ++v) {
@@ -1064,27 +1109,6 @@ extern "C" hc_status hc_skin_create(hc_skin* out, int32_t n_joints, const int32_
             order[next[depth[j]]++] = (int)((unsigned)j << 16 | (unsigned)(parent[j] + 1));
         tree.insert(tree.end(), order.begin(), order.end());
         UP(tree, tree.data(), tree.size());
-    }
-    {
-        // each adjoint block's (vertex, slot) pairs by skinning joint, vertices
-        // ascending: the blocks' offsets, then the pairs
-        const int G = h->grad_block = skin_grad_smem(n_skin, 12, k, 256) <= (96u << 10) ? 256 : 128;
-        const size_t blocks = (size_t)div_up(n_vertices, G);
-        std::vector<unsigned> bones(blocks * (n_skin + 1) + (size_t)n_vertices * k);
-        unsigned* slot = bones.data() + blocks * (n_skin + 1);
-        std::vector<unsigned> cnt(n_skin + 1);
-        for (size_t q = 0; q < blocks; ++q) {
-            const int v0 = (int)q * G, v1 = std::min(v0 + G, n_vertices);
-            std::fill(cnt.begin(), cnt.end(), 0u);
-            for (long long i = (long long)v0 * k; i < (long long)v1 * k; ++i) cnt[skin_index[i] + 1]++;
-            cnt[0] = (unsigned)(v0 * k);
-            for (int s = 0; s < n_skin; ++s) cnt[s + 1] += cnt[s];
-            std::copy(cnt.begin(), cnt.end(), bones.begin() + q * (n_skin + 1));
-            for (int v = v0; v < v1; ++v)
-                for (int c = 0; c < k; ++c)
-                    slot[cnt[skin_index[(long long)v * k + c]]++] = (unsigned)((v - v0) * k + c) << 8 | (unsigned)(v - v0);
-        }
-        UP(bones, bones.data(), bones.size());
     }
 #undef UP
     if (st != HC_OK) {
