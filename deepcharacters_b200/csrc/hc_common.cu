@@ -5,7 +5,7 @@
 
 #include <map>
 #include <mutex>
-#include <utility>
+#include <tuple>
 
 namespace hc {
 
@@ -27,18 +27,19 @@ void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
 int resident_ctas(const void* kernel, int threads) {
     static std::mutex mu;
-    static std::map<std::pair<const void*, int>, int> known;  // a few kernels per device
-    int dev = 0;
-    cudaGetDevice(&dev);
+    static std::map<std::tuple<const void*, int, int>, int> known;  // a few kernels per device
+    int dev = 0, sms = 0, per_sm = 0;
     std::lock_guard<std::mutex> lock(mu);
-    auto it = known.find({kernel, dev});
+    bool ok = cudaGetDevice(&dev) == cudaSuccess;
+    const auto it = ok ? known.find({kernel, threads, dev}) : known.end();
     if (it != known.end()) return it->second;
-    int sms = 0, per_sm = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess || per_sm <= 0)
-        per_sm = 1;
-    known[{kernel, dev}] = sms * per_sm;
-    return sms * per_sm;
+    ok = ok && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0 &&
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) == cudaSuccess && per_sm > 0;
+    if (!ok) {  // a guess for this call alone; the error is not the launch's
+        cudaGetLastError();
+        return 148;
+    }
+    return known[{kernel, threads, dev}] = sms * per_sm;
 }
 
 __global__ void k_fill(FillRuns runs) {

@@ -110,7 +110,8 @@ hc_status upload(DevBuf& b, const T* host, size_t count) {
 }
 
 // CTAs of a kernel that are resident on the current device at once (SMs x CTAs
-// per SM without dynamic shared memory); looked up once per kernel and device
+// per SM without dynamic shared memory); looked up once per kernel, block size
+// and device
 int resident_ctas(const void* kernel, int threads);
 
 // grid of a persistent kernel: as many CTAs as are resident at once (a second

@@ -15,6 +15,8 @@ cudaStreamCaptureMode mode = cudaStreamCaptureModeGlobal;
 bool recording = false;  // allocations and frees are refused unless the mode is relaxed
 bool refused() { return recording && mode != cudaStreamCaptureModeRelaxed; }
 cudaError_t fail(cudaError_t e) { return last = e; }
+int device = 0, queries = 0;
+bool occupancy_fails = false;
 }  // namespace fake
 
 #ifndef __CUDA_ARCH__
@@ -41,6 +43,24 @@ cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode* m) {
     std::swap(*m, fake::mode);
     return cudaSuccess;
 }
+cudaError_t cudaGetDevice(int* d) {
+    *d = fake::device;
+    return cudaSuccess;
+}
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) {
+    *v = 10;
+    return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void*, int threads, size_t) {
+    ++fake::queries;
+    if (fake::occupancy_fails) return fake::fail(cudaErrorInvalidValue);
+    *n = 1024 / threads + fake::device;
+    return cudaSuccess;
+}
+cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t) { return cudaSuccess; }
+unsigned __cudaPushCallConfiguration(dim3, dim3, size_t, struct CUstream_st*) { return 0; }
+cudaError_t __cudaPopCallConfiguration(dim3*, dim3*, size_t*, void*) { return cudaSuccess; }
+void __cudaRegisterFunction(void**, const char*, char*, const char*, int, uint3*, uint3*, dim3*, dim3*, int*) {}
 cudaError_t cudaMemcpy(void*, const void*, size_t, cudaMemcpyKind) { return cudaSuccess; }
 void** __cudaRegisterFatBinary(void*) { return nullptr; }
 void __cudaRegisterFatBinaryEnd(void**) {}
@@ -48,11 +68,6 @@ void __cudaUnregisterFatBinary(void**) {}
 char __cudaInitModule(void**) { return 0; }
 }
 #endif
-
-namespace hc {
-void set_error(const char*, ...) {}
-void clear_error() {}
-}  // namespace hc
 
 using namespace hc;
 
@@ -141,12 +156,28 @@ static int fan_entries() {
     return 0;
 }
 
+// the resident CTAs are those of the kernel, the block size and the device; a failed
+// query is neither kept nor left for the next launch to report
+static int resident() {
+    const void *a = &fake::room, *b = &fake::last;
+    CHECK(resident_ctas(a, 256) == 40 && resident_ctas(a, 64) == 160 && resident_ctas(a, 256) == 40);
+    CHECK(fake::queries == 2);
+    fake::device = 1;
+    CHECK(resident_ctas(a, 256) == 50 && resident_ctas(a, 64) == 170);
+    fake::occupancy_fails = true;
+    CHECK(resident_ctas(b, 256) > 0 && fake::last == cudaSuccess);
+    fake::occupancy_fails = false;
+    CHECK(resident_ctas(b, 256) == 50);
+    return 0;
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, int (*)()> checks = {
         {"uv_held", uv_held},
         {"uv_recorded", uv_recorded},
         {"uv_no_memory", uv_no_memory},
         {"fan_entries", fan_entries},
+        {"resident", resident},
     };
     const auto it = checks.find(argc > 1 ? argv[1] : "");
     return it == checks.end() ? 2 : it->second();

@@ -17,12 +17,13 @@ def program(tmp_path_factory):
         pytest.skip("nvcc not found")
     exe = str(tmp_path_factory.mktemp("host") / "host_scratch")
     subprocess.run([NVCC, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "--expt-relaxed-constexpr",
-                    "-diag-suppress", "177", "-cudart", "none", os.path.join(HERE, "host_scratch.cu"), "-o", exe],
+                    "-diag-suppress", "177", "-cudart", "none", os.path.join(HERE, "host_scratch.cu"),
+                    os.path.join(HERE, "..", "deepcharacters_b200", "csrc", "hc_common.cu"), "-o", exe],
                    check=True)
     return exe
 
 
-@pytest.mark.parametrize("check", ["uv_held", "uv_recorded", "uv_no_memory", "fan_entries"])
+@pytest.mark.parametrize("check", ["uv_held", "uv_recorded", "uv_no_memory", "fan_entries", "resident"])
 def test_host_buffers(program, check):
     r = subprocess.run([program, check], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
