@@ -61,6 +61,7 @@ struct DevBuf {
         cudaError_t e = cudaMalloc(&ptr, need);
         if (e != cudaSuccess) {
             ptr = nullptr;
+            cudaGetLastError();  // reported here, not by the next launch's check
             HC_FAIL(HC_ERR_ALLOC, "cudaMalloc(%zu) failed: %s", need, cudaGetErrorString(e));
         }
         bytes = need;
@@ -92,7 +93,6 @@ struct SpareBuf : DevBuf {
         if (bytes < need) {
             if (captured || recording) return false;
             if (ensure(need) != HC_OK) {
-                cudaGetLastError();
                 clear_error();
                 return false;
             }

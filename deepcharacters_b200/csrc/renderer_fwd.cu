@@ -947,7 +947,6 @@ hc_status raster_reserve(RasterWorkspace& ws, int views, int F) {
     if (views > ws.cap_views || ws.bins.bytes < (size_t)tiles * ws.bin_cap * sizeof(int)) {
         HC_TRY(ws.cams.ensure(sizeof(ViewCam) * views));
         if (ws.vacc_floats && ws.size_vacc() != HC_OK) {  // an adjoint that needs it will say so
-            cudaGetLastError();
             clear_error();
         }
         HC_TRY(ws.tri_view.ensure(sizeof(TriView) * (size_t)views * F));

@@ -156,6 +156,16 @@ static int fan_entries() {
     return 0;
 }
 
+// a failed allocation is reported once, by the call that needed it
+static int failed_allocation() {
+    DevBuf b;
+    CHECK(b.ensure(100) == HC_OK);
+    fake::room = 1000;
+    CHECK(b.ensure(2000) == HC_ERR_ALLOC && fake::last == cudaSuccess && !b.ptr && b.bytes == 0);
+    CHECK(b.ensure(500) == HC_OK && b.bytes == 500);
+    return 0;
+}
+
 // the resident CTAs are those of the kernel, the block size and the device; a failed
 // query is neither kept nor left for the next launch to report
 static int resident() {
@@ -178,6 +188,7 @@ int main(int argc, char** argv) {
         {"uv_no_memory", uv_no_memory},
         {"fan_entries", fan_entries},
         {"resident", resident},
+        {"failed_allocation", failed_allocation},
     };
     const auto it = checks.find(argc > 1 ? argv[1] : "");
     return it == checks.end() ? 2 : it->second();
