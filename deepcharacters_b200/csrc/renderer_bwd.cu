@@ -905,7 +905,8 @@ hc_status raster_backward(const Topology& topo, RasterWorkspace& ws, SpareBuf& t
                     : albedo == kTexturedBilinear ? kAlbTexBilinear : kAlbNone;
     ws.vacc_floats = (size_t)vertex_sum_floats(alb == kAlbVcol, shaded) * N;
     const size_t vacc_bytes = sizeof(float) * ws.vacc_floats * B;
-    if (ws.size_vacc() != HC_OK) {  // no room for as many frames as there are cameras for: this call's
+    // where there is no room for as many frames as there are cameras for: for this call's
+    if (ws.vacc.bytes < vacc_bytes && ws.size_vacc() != HC_OK) {
         clear_error();
         HC_TRY(ws.vacc.ensure(vacc_bytes));
     }
