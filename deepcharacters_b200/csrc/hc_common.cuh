@@ -88,14 +88,19 @@ struct DevPart {
 // would free what a captured graph addresses.
 struct SpareBuf : DevBuf {
     bool captured = false;  // a graph holds its address: it keeps its size
+    size_t refused = ~(size_t)0;  // there was no memory for this size
+    int patience = 0;             // calls until it is asked for again (a failed attempt costs more than the scratch gains)
     bool room(size_t need, cudaStreamCaptureStatus capture) {
         const bool recording = capture != cudaStreamCaptureStatusNone;
         if (bytes < need) {
-            if (captured || recording) return false;
+            if (captured || recording || (need >= refused && patience-- > 0)) return false;
             if (ensure(need) != HC_OK) {
                 clear_error();
+                refused = need;
+                patience = 1000;
                 return false;
             }
+            refused = ~(size_t)0;
         }
         captured = captured || recording;
         return true;

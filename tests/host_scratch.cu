@@ -156,6 +156,33 @@ static int fan_entries() {
     return 0;
 }
 
+// spare scratch that a graph holds is neither replaced nor grown
+static int spare_held() {
+    SpareBuf b;
+    CHECK(!b.room(100, kRecord) && !b.captured && b.room(100, kEager) && b.room(300, kEager));
+    void* at = b.ptr;
+    CHECK(b.room(200, kRecord) && b.captured);
+    const int mallocs = fake::mallocs, frees = fake::frees;
+    CHECK(!b.room(400, kEager) && !b.room(400, kRecord) && b.room(300, kEager));
+    CHECK(b.ptr == at && b.bytes == 300 && fake::mallocs == mallocs && fake::frees == frees && fake::live.count(at));
+    return 0;
+}
+
+// where memory is short the allocation is not tried again in every call
+static int spare_no_memory() {
+    SpareBuf b;
+    CHECK(b.room(100, kEager));
+    fake::room = 1000;
+    for (int k = 0; k < 500; ++k) CHECK(!b.room(5000, kEager));
+    CHECK(fake::mallocs == 2 && fake::last == cudaSuccess);
+    CHECK(b.room(900, kEager) && b.bytes == 900);
+    fake::room = 10000;
+    bool found = false;
+    for (int k = 0; k < 1000; ++k) found = found || b.room(5000, kEager);
+    CHECK(found && b.bytes == 5000 && fake::mallocs == 4);
+    return 0;
+}
+
 // a failed allocation is reported once, by the call that needed it
 static int failed_allocation() {
     DevBuf b;
@@ -188,6 +215,8 @@ int main(int argc, char** argv) {
         {"uv_no_memory", uv_no_memory},
         {"fan_entries", fan_entries},
         {"resident", resident},
+        {"spare_held", spare_held},
+        {"spare_no_memory", spare_no_memory},
         {"failed_allocation", failed_allocation},
     };
     const auto it = checks.find(argc > 1 ? argv[1] : "");

@@ -24,7 +24,7 @@ def program(tmp_path_factory):
 
 
 @pytest.mark.parametrize("check", ["uv_held", "uv_recorded", "uv_no_memory", "fan_entries", "resident",
-                                   "failed_allocation"])
+                                   "spare_held", "spare_no_memory", "failed_allocation"])
 def test_host_buffers(program, check):
     r = subprocess.run([program, check], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
