@@ -312,6 +312,11 @@ struct hc_eg_s {
     DevBuf base4, v2n_poff, v2n_pidx, v2n_pw;  // float4 base vertices; the vertex -> node CSR packed in vertex order
     DevBuf markers, m2n, n2m, fan, vf_id;
     DevBuf tab, packed;
+    int reserved = 0;  // frames asked for with hc_eg_reserve
+    // the packed vertices, which only the full skinned gradient reads
+    hc_status reserve_packed(long long frames) {
+        return full_skinned_grad ? packed.ensure(3 * sizeof(float4) * (size_t)frames * N) : HC_OK;
+    }
 };
 
 static void release(hc_eg h) {
@@ -435,15 +440,15 @@ extern "C" hc_status hc_eg_set_full_skinned_gradient(hc_eg h, int32_t enable) {
     clear_error();
     HC_REQUIRE(h, "invalid handle");
     h->full_skinned_grad = enable ? 1 : 0;
-    return HC_OK;
+    return h->reserve_packed(h->reserved);
 }
 
 extern "C" hc_status hc_eg_reserve(hc_eg h, int32_t batch) {
     clear_error();
     HC_REQUIRE(h && batch > 0, "invalid handle or batch");
     HC_TRY(h->tab.ensure(sizeof(NodeRT) * (size_t)batch * h->M));
-    HC_TRY(h->packed.ensure(3 * sizeof(float4) * (size_t)batch * h->N));
-    return HC_OK;
+    h->reserved = std::max(h->reserved, batch);
+    return h->reserve_packed(h->reserved);
 }
 
 template <int MODE>
@@ -509,7 +514,7 @@ extern "C" hc_status hc_eg_backward(hc_eg h, void* stream, int32_t batch, const 
                "the full skinned gradient needs nodes_delta_translation and vertex_displacements");
     cudaStream_t s = (cudaStream_t)stream;
     HC_TRY(h->tab.ensure(sizeof(NodeRT) * (size_t)batch * h->M));
-    const long long BM = (long long)batch * h->M, BN = (long long)batch * h->N;
+    const long long BM = (long long)batch * h->M;
     NodeRT* tab = h->tab.as<NodeRT>();
     // node table from the saved angles; the backward reads the rotations, and
     // (full mode) the delta translations -- the skinned-translation slot of
@@ -520,7 +525,7 @@ extern "C" hc_status hc_eg_backward(hc_eg h, void* stream, int32_t batch, const 
                                                nullptr, nullptr);
     HC_CHECK_LAUNCH();
     if (full) {
-        HC_TRY(h->packed.ensure(3 * sizeof(float4) * (size_t)BN));
+        HC_TRY(h->reserve_packed(batch));
         HC_TRY(launch_vertices<kEgAdjointFull>(h, s, batch, vertex_displacements, deformed_vertices_grad,
                                                vertex_displacements_grad));
     } else {
