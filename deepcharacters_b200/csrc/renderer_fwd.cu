@@ -962,6 +962,8 @@ hc_status raster_reserve(RasterWorkspace& ws, int views, int F) {
         ws.spill_tile_cap = (int)(tiles * per_tile <= (4ll << 30) ? tiles : std::max<long long>(256, tiles / 4));
         HC_TRY(ws.spill_keys.ensure(sizeof(unsigned long long) * (size_t)ws.spill_tile_cap * TS * TS));
         HC_TRY(ws.stats.ensure(sizeof(RasterStats)));
+        HC_TRY(ws.claim.ensure(sizeof(unsigned long long)));
+        HC_TRY(ws.claim_b.ensure(sizeof(unsigned)));
         ws.cap_views = views;
     }
     return HC_OK;
@@ -984,7 +986,6 @@ hc_status raster_forward(const Topology& topo, RasterWorkspace& ws, cudaStream_t
     int2* tstate = ws.tile_state.as<int2>();
     RasterStats* stats = ws.stats.as<RasterStats>();
 
-    HC_TRY(ws.claim.ensure(sizeof(unsigned long long)));
     unsigned long long* claim = ws.claim.as<unsigned long long>();
 
     FillRuns zeros;

@@ -68,3 +68,14 @@ def test_captured_backward_after_a_larger_one(shading):
     g.replay()
     torch.cuda.synchronize()
     _same(got, want)
+
+
+def test_capture_after_reserve_alone():
+    make, forward, backward = _setup("shaded")
+    want = backward(make(), *forward(make(), 4))  # loads the kernels too
+    eng = make()
+    eng.reserve(4)
+    g, got = _graph(lambda: backward(eng, *forward(eng, 4)))
+    g.replay()
+    torch.cuda.synchronize()
+    _same(got, want)
