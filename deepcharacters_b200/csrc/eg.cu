@@ -398,9 +398,8 @@ extern "C" hc_status hc_eg_create(hc_eg* out, int32_t n_vertices, const float* b
         UP(m2n, marker_to_node, n_markers);
     }
     {
-        // the vertex -> node lists packed contiguously in vertex order (the
-        // vertex kernel stages a block's range in one coalesced sweep), and
-        // the base vertices padded to float4
+        // the vertex -> node lists packed contiguously in vertex order (a warp's
+        // lists lie side by side), and the base vertices padded to float4
         std::vector<int> poff((size_t)n_vertices + 1, 0), pidx;
         std::vector<float> pw;
         std::vector<float4> b4((size_t)n_vertices);

@@ -300,7 +300,6 @@ __global__ void __launch_bounds__(BNT, adjoint_ctas(SHADED, PARITY)) k_render_gr
     __shared__ float2 s_tap[MAXTAPS];  // image-gradient tap weights (i, j) / (i^2 + j^2)
     __shared__ float s_norm;
     __shared__ __align__(8) unsigned long long s_mbar;
-    constexpr bool shaded = SHADED;
     constexpr bool vcol = ALB == kAlbVcol;
     constexpr bool textured = ALB == kAlbTex;
     constexpr bool bilinear = ALB == kAlbTexBilinear;

@@ -190,7 +190,7 @@ struct BinSink {
     int spill_tile_cap;
     RasterStats* stats;
 
-    __device__ __forceinline__ int place(int slot, long long key, int view, int local_tile, int f) const {
+    __device__ __forceinline__ int place(int slot, long long key, int f) const {
         if (slot < cap) {
             bins[key * cap + slot] = f;
             return 1;
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(256, 6) k_bin(int V, int C, int F, int N, int 
         }
 #pragma unroll
         for (int j = 0; j < 2; ++j)
-            if (slot[j] >= 0) nbinned += sink.place(slot[j], tile_base + tile[j], view, tile[j], f);
+            if (slot[j] >= 0) nbinned += sink.place(slot[j], tile_base + tile[j], f);
     }
     // larger boxes: the warp takes them one at a time
     unsigned pending = __ballot_sync(0xffffffffu, big);
@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(256, 6) k_bin(int V, int C, int F, int N, int 
         const int qy0 = __shfl_sync(0xffffffffu, y0, src), qy1 = __shfl_sync(0xffffffffu, y1, src);
         warp_tiles(rows.from_lane(src), ts_shift, qx0, qx1, qy0, qy1, (int)lane, [&](int tx, int ty) {
             const int tile = ty * tiles_x + tx;
-            nbinned += sink.place(atomicAdd(&tile_state[tile_base + tile].x, 1), tile_base + tile, view, tile, qf);
+            nbinned += sink.place(atomicAdd(&tile_state[tile_base + tile].x, 1), tile_base + tile, qf);
         });
     }
     // one counter update per warp
@@ -390,7 +390,6 @@ __global__ void k_spill(int C, int F, int TS, long long T_frame, const int* __re
 // ---------------------------------------------------------------------------
 struct ShadeArgs {
     int B, C, N, F;
-    const float4* proj;  // [V,N] projected vertices
     int albedo, shading;
     const int3* faces;
     const float* texcoords;
@@ -1058,7 +1057,6 @@ hc_status raster_forward(const Topology& topo, RasterWorkspace& ws, cudaStream_t
     A.C = C;
     A.N = N;
     A.F = F;
-    A.proj = ws.proj.as<float4>();
     A.albedo = albedo;
     A.shading = shading;
     A.faces = topo.faces.as<int3>();

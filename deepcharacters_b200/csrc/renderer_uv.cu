@@ -119,8 +119,9 @@ __device__ __forceinline__ float3 blend(float3 a, float3 b, float3 c, float4 t) 
 // A thread takes one texel of kUvFrames frames: the table entry and the face's
 // ids are read once for them.  unit: the vertex normals already normalised, one
 // 16-byte load each (k_frame_setup; 40,962 normalisations instead of three per
-// texel); NULL: from vnormal.  4 frames of 512^2 texels, 81,920 triangles:
-// 17.0 -> 10.1 us.
+// texel); NULL: from vnormal.  512^2 texels, 81,920 triangles, 4 frames: 17.0 us
+// without either, 13.5 with the unit normals, 9.8 with four frames per thread
+// too (1, 2, 3 and 16 frames: 4.9, 7.8, 10.7 and 46.6 us -> 5.0, 6.6, 8.2 and 28.3).
 constexpr int kUvFrames = 4;
 __global__ void k_uv_map(int B, int C, int N, int n_texels, int mode, const int3* __restrict__ faces,
                          const float4* __restrict__ table, const float* __restrict__ verts,

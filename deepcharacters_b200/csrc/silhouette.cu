@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(256, 4) k_cov_bin_list(int N, int F, const int
 // pixels are covered, the tile at the chunk after which all are.
 // Bound by instruction issue.  16 views of 81,920 triangles at 1024^2: 552 ->
 // 374 us.
-__global__ void __launch_bounds__(kCovTile* kCovTile) k_cov_tile(int F, long long n_keys, CovBins cb,
+__global__ void __launch_bounds__(kCovTile* kCovTile) k_cov_tile(int F, CovBins cb,
                                                                   const __grid_constant__ ImgLayout L) {
     constexpr int NT = kCovTile * kCovTile, RW = 32 / kCovTile, kRec = sizeof(CovTileTri) / 16;
     static_assert(sizeof(CovTileTri) == 16 * kRec, "records are copied in 16-byte pieces");
@@ -1336,8 +1336,7 @@ static hc_status mesh_boundary_run(hc_mesh_boundary h, void* stream, int32_t bat
         k_cov_bin<<<dim3(div_up(h->F, 256), (unsigned)views), 256, 0, s>>>(h->N, h->F, faces, p2, cb, L);
     }
     HC_CHECK_LAUNCH();
-    k_cov_tile<<<resident_grid(k_cov_tile, kCovTile * kCovTile, n_keys), kCovTile * kCovTile, 0, s>>>(h->F, n_keys,
-                                                                                                      cb, L);
+    k_cov_tile<<<resident_grid(k_cov_tile, kCovTile * kCovTile, n_keys), kCovTile * kCovTile, 0, s>>>(h->F, cb, L);
     HC_CHECK_LAUNCH();
     k_boundary_cover<<<div_up(nv, 256), 256, 0, s>>>(batch, n_cameras, h->N, L, p2d, h->cover.as<unsigned char>(),
                                                      face_hint != nullptr, is_boundary);

@@ -9,8 +9,8 @@
 // The reference copies the dofs to the host on every call, runs the Eigen
 // kinematic chain there, and copies dual quaternions / joint frames back
 // (DQSkinningGPUOp.cpp:351-389) -- a serialising round trip that cannot be
-// captured in a CUDA graph.  Here one thread per frame walks the joint list
-// (parents precede children) entirely on the device.
+// captured in a CUDA graph.  Here a CTA per frame composes the chain level by
+// level of the tree, entirely on the device.
 //
 // The dof gradient of the reference is a per-dof serial loop over an
 // influence list of (vertex, bone, weight, joint) entries (DQSkinningGPUOpGrad.cu:
@@ -1134,7 +1134,9 @@ extern "C" hc_status hc_skin_set_parity(hc_skin h, int32_t parity) {
 
 static hc_status fk(hc_skin h, cudaStream_t s, int B, const float* dofs, float* gpos, float* gaxis, float* dq,
                     float* xf) {
-    // two transforms and up to two words per joint, two per dof entry
+    // The sizes that this entry point takes: 48 KB for two transforms and two words
+    // per joint and two words per dof entry.  The kernel itself holds two transforms
+    // and a word per joint, whose ids fit level_joint's 16 bits far below that.
     const size_t most = sizeof(float) * (2 * (size_t)((h->J + 3) & ~3) + 2 * (size_t)((h->E + 3) & ~3)) +
                         2 * sizeof(Xf) * (size_t)h->J;
     HC_REQUIRE(most <= 48 * 1024, "skeleton too large for the kinematics kernel (%d joints)", h->J);
