@@ -302,8 +302,10 @@ struct CovBins {
     const unsigned long long* need;  // tiles with a pixel still open: a word per 8x8 tiles of a view, bit 8 row + column
     int* tiles;                 // [tiles of the call]: the tiles that received an entry, in no order
     int* n_tiles;               // their number (cleared before the binning pass)
-    int* items;                 // [V*F]: hinted binning, the (view * F + triangle) pairs left by the cull
-    int* n_items;               // their number (cleared before the cull)
+    // hinted binning: the (view * F + triangle) pairs left by the cull, those of boxes
+    // of more than kCovLarge tiles from the end
+    int* items;                 // [V*F]
+    int* n_items;               // the numbers of both (cleared before the cull)
 };
 
 // a bin slot of tile `key`; the tile's first slot also lists the tile for the
@@ -321,14 +323,13 @@ __device__ __forceinline__ unsigned long long word_box(int wx, int wy, int tx0, 
     return row * 0x0101010101010101ull & (~0ull >> (56 - 8 * y1)) & (~0ull << (8 * y0));
 }
 
-// a needed tile of a view lies in the box (a row of words at a time: its loads do not wait for one another)
+// a needed tile of a view lies in the box
 __device__ __forceinline__ bool need_in_box(const unsigned long long* need, const ViewImg& vi, int tx0, int ty0, int tx1,
                                             int ty1) {
-    unsigned long long any = 0ull;
-    for (int wy = ty0 >> 3; wy <= ty1 >> 3 && !any; ++wy)
+    for (int wy = ty0 >> 3; wy <= ty1 >> 3; ++wy)
         for (int wx = tx0 >> 3; wx <= tx1 >> 3; ++wx)
-            any |= need[vi.word + (long long)wy * vi.words_x + wx] & word_box(wx, wy, tx0, ty0, tx1, ty1);
-    return any != 0ull;
+            if (need[vi.word + (long long)wy * vi.words_x + wx] & word_box(wx, wy, tx0, ty0, tx1, ty1)) return true;
+    return false;
 }
 
 // the pixels of one tile that a triangle covers, written at once (a pair
@@ -490,20 +491,28 @@ __global__ void __launch_bounds__(256, 4) k_cov_bin(int N, int F, const int3* __
 // byte per tile took a kernel to form, and the boxes were then walked tile by
 // tile: 16 x 8 views of 81,920 triangles 1330 -> 555 us for the three.
 //
-// The first pass, light enough for full
-// occupancy: the (view, triangle) pairs whose tile box holds a needed tile
-// (most hold none), listed with one atomic per warp for k_cov_bin_list.
+// The first pass, light enough for full occupancy (32 registers): the (view,
+// triangle) pairs whose tile box holds a needed tile (most hold none), listed for
+// k_cov_bin_list with one atomic per warp, boxes of more than kCovLarge tiles from
+// the list's end.
+constexpr int kCovLarge = 128;
+
 __global__ void k_cov_cull(int N, int F, const int3* __restrict__ faces, const float2* __restrict__ p2d,
                            CovBins cb, const __grid_constant__ ImgLayout L) {
     const int fi = blockIdx.x * blockDim.x + threadIdx.x;
     const int view = blockIdx.y;
     const ViewImg vi = view_img(L, view);
-    bool keep = false;
+    bool keep = false, large = false;
     if (fi < F) {  // no early exit: the whole warp takes part in the vote
         CoverTri t;
         cover_tri(view, N, vi.W, vi.H, faces[fi], p2d, t);
-        keep = t.x1 >= t.x0 && t.y1 >= t.y0 &&
-               need_in_box(cb.need, vi, t.x0 / kCovTile, t.y0 / kCovTile, t.x1 / kCovTile, t.y1 / kCovTile);
+        const int tx0 = t.x0 / kCovTile, ty0 = t.y0 / kCovTile, tx1 = t.x1 / kCovTile, ty1 = t.y1 / kCovTile;
+        keep = t.x1 >= t.x0 && t.y1 >= t.y0 && need_in_box(cb.need, vi, tx0, ty0, tx1, ty1);
+        large = keep && (tx1 - tx0 + 1) * (ty1 - ty0 + 1) > kCovLarge;
+    }
+    if (large) {  // rare
+        cb.items[(long long)gridDim.y * F - 1 - atomicAdd(cb.n_items + 1, 1)] = view * F + fi;
+        keep = false;
     }
     const unsigned m = __ballot_sync(0xffffffffu, keep);
     if (!m) return;  // warp-uniform
@@ -514,70 +523,72 @@ __global__ void k_cov_cull(int N, int F, const int3* __restrict__ faces, const f
     if (keep) cb.items[base + __popc(m & ((1u << lane) - 1u))] = view * F + fi;
 }
 
-// The second, over the listed pairs (persistent, whole warps): a thread per pair
-// writes its record and walks the needed tiles of its box, the set bits of the
-// box's words; a box with more than kCovNeeded of them is taken by the warp, as
-// in the full binning.  A poor hint leaves large triangles thousands of needed
-// tiles: 1024^2, an empty hint, 81,920 small triangles and two that span the view
-// 269 us (a thread per box throughout 1599), 10,000 triangles of 200 px 198 (484).
-// kCovNeeded of 32: 270 and 147 us, but 195 instead of 132 with the first mesh's
-// own face buffer as the hint; of 512: 272, 349 and 132.
+// The second, over the listed pairs (persistent): a thread per pair writes its
+// record and walks the needed tiles of its box, the set bits of the box's words.
+// The large boxes follow, a warp each: a poor hint leaves them thousands of needed
+// tiles, which are dealt out as in the full binning; up to kCovNeeded are walked
+// by words, a lane each.  1024^2, an empty hint: 81,920 small triangles and two that
+// span the view 185 us (a thread per box throughout 1599; prefix sums and a warp per
+// box of nine tiles 383), 10,000 triangles of 200 px 235 (484; 208), 1000 that span
+// the view 343 (2072; 2494).
 constexpr int kCovNeeded = 128;
 
-__global__ void __launch_bounds__(256, 4) k_cov_bin_list(int N, int F, const int3* __restrict__ faces,
+__global__ void __launch_bounds__(256, 4) k_cov_bin_list(int N, int F, int V, const int3* __restrict__ faces,
                                                          const float2* __restrict__ p2d, CovBins cb,
                                                          const __grid_constant__ ImgLayout L) {
-    const int n = *cb.n_items, lane = threadIdx.x & 31;
-    for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += gridDim.x * blockDim.x) {
-        const int it = base + lane;
-        int item = 0;
+    const int n = cb.n_items[0], large = cb.n_items[1];
+    for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < n; it += gridDim.x * blockDim.x) {
+        const int item = cb.items[it], view = item / F, f = item - view * F;
+        const ViewImg vi = view_img(L, view);
         CoverTri t;
-        t.x0 = t.x1 = t.y0 = t.y1 = 0;
-        TileRows rows;
-        bool many = false;
-        if (it < n) {
-            item = cb.items[it];
-            const int view = item / F, f = item - view * F;
-            const ViewImg vi = view_img(L, view);
-            cover_tri(view, N, vi.W, vi.H, faces[f], p2d, t);
-            const Footprint fp = cover_footprint(t, vi.W, vi.H);
-            cb.rec[item] = cover_record(t, fp);
-            const int tx0 = t.x0 / kCovTile, ty0 = t.y0 / kCovTile, tx1 = t.x1 / kCovTile, ty1 = t.y1 / kCovTile;
-            auto needed = [&](int wx, int wy) {
-                return cb.need[vi.word + (long long)wy * vi.words_x + wx] & word_box(wx, wy, tx0, ty0, tx1, ty1);
-            };
-            if ((tx1 - tx0 + 1) * (ty1 - ty0 + 1) > kCovNeeded) {
-                int count = 0;
-                for (int wy = ty0 >> 3; wy <= ty1 >> 3 && count <= kCovNeeded; ++wy)
-                    for (int wx = tx0 >> 3; wx <= tx1 >> 3; ++wx) count += __popcll(needed(wx, wy));
-                many = count > kCovNeeded;
+        cover_tri(view, N, vi.W, vi.H, faces[f], p2d, t);
+        const Footprint fp = cover_footprint(t, vi.W, vi.H);
+        cb.rec[item] = cover_record(t, fp);
+        const int tx0 = t.x0 / kCovTile, ty0 = t.y0 / kCovTile, tx1 = t.x1 / kCovTile, ty1 = t.y1 / kCovTile;
+        for (int wy = ty0 >> 3; wy <= ty1 >> 3; ++wy)
+            for (int wx = tx0 >> 3; wx <= tx1 >> 3; ++wx) {
+                unsigned long long bits =
+                    cb.need[vi.word + (long long)wy * vi.words_x + wx] & word_box(wx, wy, tx0, ty0, tx1, ty1);
+                for (; bits; bits &= bits - 1ull) {
+                    const int b = __ffsll((long long)bits) - 1, tx = 8 * wx + (b & 7), ty = 8 * wy + (b >> 3);
+                    if (!footprint_overlaps(fp, max(tx * kCovTile, t.x0), min(tx * kCovTile + kCovTile - 1, t.x1),
+                                            max(ty * kCovTile, t.y0), min(ty * kCovTile + kCovTile - 1, t.y1)))
+                        continue;
+                    cov_place(cb, vi, ty * vi.tiles_x + tx, f, item);
+                }
             }
-            if (many) {
-                rows = TileRows(fp);
-            } else {
-                for (int wy = ty0 >> 3; wy <= ty1 >> 3; ++wy)
-                    for (int wx = tx0 >> 3; wx <= tx1 >> 3; ++wx)
-                        for (unsigned long long bits = needed(wx, wy); bits; bits &= bits - 1ull) {
-                            const int b = __ffsll((long long)bits) - 1, tx = 8 * wx + (b & 7), ty = 8 * wy + (b >> 3);
-                            if (footprint_overlaps(fp, max(tx * kCovTile, t.x0), min(tx * kCovTile + kCovTile - 1, t.x1),
-                                                   max(ty * kCovTile, t.y0), min(ty * kCovTile + kCovTile - 1, t.y1)))
-                                cov_place(cb, vi, ty * vi.tiles_x + tx, f, item);
-                        }
-            }
-        }
-        __syncwarp();  // the records of large triangles are read by the other lanes where a bin overflows
-        unsigned pending = __ballot_sync(0xffffffffu, many);
-        while (pending) {
-            const int src = __ffs(pending) - 1;
-            pending &= pending - 1;
-            const int q = __shfl_sync(0xffffffffu, item, src), view = q / F, f = q - view * F;
-            const ViewImg vi = view_img(L, view);
-            const int qx0 = __shfl_sync(0xffffffffu, t.x0, src), qx1 = __shfl_sync(0xffffffffu, t.x1, src);
-            const int qy0 = __shfl_sync(0xffffffffu, t.y0, src), qy1 = __shfl_sync(0xffffffffu, t.y1, src);
-            warp_tiles(rows.from_lane(src), kCovShift, qx0, qx1, qy0, qy1, lane, [&](int tx, int ty) {
-                if (cb.need[vi.word + (long long)(ty >> 3) * vi.words_x + (tx >> 3)] >> (8 * (ty & 7) + (tx & 7)) & 1ull)
-                    cov_place(cb, vi, ty * vi.tiles_x + tx, f, q);
+    }
+    const int lane = threadIdx.x & 31, warps = (int)((gridDim.x * blockDim.x) >> 5);
+    for (int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); w < large; w += warps) {  // warp-uniform
+        const int item = cb.items[(long long)V * F - 1 - w], view = item / F, f = item - view * F;
+        const ViewImg vi = view_img(L, view);
+        CoverTri t;
+        cover_tri(view, N, vi.W, vi.H, faces[f], p2d, t);
+        const Footprint fp = cover_footprint(t, vi.W, vi.H);
+        if (lane == 0) cb.rec[item] = cover_record(t, fp);
+        __syncwarp();  // read by the other lanes where a bin overflows
+        const int tx0 = t.x0 / kCovTile, ty0 = t.y0 / kCovTile, tx1 = t.x1 / kCovTile, ty1 = t.y1 / kCovTile;
+        const int wx0 = tx0 >> 3, wy0 = ty0 >> 3, nwx = (tx1 >> 3) - wx0 + 1, words = nwx * ((ty1 >> 3) - wy0 + 1);
+        auto needed = [&](int wx, int wy) {
+            return cb.need[vi.word + (long long)wy * vi.words_x + wx] & word_box(wx, wy, tx0, ty0, tx1, ty1);
+        };
+        int count = 0;
+        for (int q = lane; q < words; q += 32) count += __popcll(needed(wx0 + q % nwx, wy0 + q / nwx));
+        if (__reduce_add_sync(0xffffffffu, count) > kCovNeeded) {
+            warp_tiles(TileRows(fp), kCovShift, t.x0, t.x1, t.y0, t.y1, lane, [&](int tx, int ty) {
+                if (needed(tx >> 3, ty >> 3) >> (8 * (ty & 7) + (tx & 7)) & 1ull)
+                    cov_place(cb, vi, ty * vi.tiles_x + tx, f, item);
             });
+        } else {
+            for (int q = lane; q < words; q += 32) {
+                const int wx = wx0 + q % nwx, wy = wy0 + q / nwx;
+                for (unsigned long long bits = needed(wx, wy); bits; bits &= bits - 1ull) {
+                    const int b = __ffsll((long long)bits) - 1, tx = 8 * wx + (b & 7), ty = 8 * wy + (b >> 3);
+                    if (footprint_overlaps(fp, max(tx * kCovTile, t.x0), min(tx * kCovTile + kCovTile - 1, t.x1),
+                                           max(ty * kCovTile, t.y0), min(ty * kCovTile + kCovTile - 1, t.y1)))
+                        cov_place(cb, vi, ty * vi.tiles_x + tx, f, item);
+                }
+            }
         }
     }
 }
@@ -1256,7 +1267,7 @@ static hc_status mesh_boundary_reserve_layout(hc_mesh_boundary h, long long view
     HC_TRY(h->need.ensure(sizeof(unsigned long long) * frames * (size_t)L.Q));
     HC_TRY(h->tile_list.ensure(sizeof(int) * (frames * (size_t)L.T + 1)));
     HC_REQUIRE(views * h->F < (1ll << 31), "too many (view, triangle) pairs in one call");
-    HC_TRY(h->items.ensure(sizeof(int) * ((size_t)views * h->F + 1)));
+    HC_TRY(h->items.ensure(sizeof(int) * ((size_t)views * h->F + 2)));
     return HC_OK;
 }
 
@@ -1307,7 +1318,7 @@ static hc_status mesh_boundary_run(hc_mesh_boundary h, void* stream, int32_t bat
     cb.n_tiles = h->tile_list.as<int>();
     cb.tiles = cb.n_tiles + 1;
     cb.n_items = h->items.as<int>();
-    cb.items = cb.n_items + 1;
+    cb.items = cb.n_items + 2;
     const float2* p2 = reinterpret_cast<const float2*>(p2d);
     const int3* faces = h->faces.as<int3>();
     unsigned long long* need = h->need.as<unsigned long long>();
@@ -1316,7 +1327,7 @@ static hc_status mesh_boundary_run(hc_mesh_boundary h, void* stream, int32_t bat
     zeros.add(cb.n_tiles, sizeof(int));
     if (face_hint) {
         zeros.add(need, sizeof(unsigned long long) * (size_t)(frames * L.Q));
-        zeros.add(cb.n_items, sizeof(int));
+        zeros.add(cb.n_items, 2 * sizeof(int));
     } else {
         zeros.add(cb.cover, (size_t)(frames * L.P));
     }
@@ -1330,8 +1341,10 @@ static hc_status mesh_boundary_run(hc_mesh_boundary h, void* stream, int32_t bat
         cb.need = need;  // cull, then bin the listed pairs
         k_cov_cull<<<dim3(div_up(h->F, 256), (unsigned)views), 256, 0, s>>>(h->N, h->F, faces, p2, cb, L);
         HC_CHECK_LAUNCH();
-        k_cov_bin_list<<<resident_grid(k_cov_bin_list, 256, views * h->F / 256 + 1), 256, 0, s>>>(h->N, h->F, faces, p2,
-                                                                                                  cb, L);
+        // a thread per pair, but a CTA per SM for the large boxes of meshes of a thousand triangles or more
+        const long long pairs = views * h->F, ctas = std::max(pairs / 256, std::min(148ll, pairs / 8)) + 1;
+        k_cov_bin_list<<<resident_grid(k_cov_bin_list, 256, ctas), 256, 0, s>>>(
+            h->N, h->F, (int)views, faces, p2, cb, L);
     } else {
         k_cov_bin<<<dim3(div_up(h->F, 256), (unsigned)views), 256, 0, s>>>(h->N, h->F, faces, p2, cb, L);
     }
