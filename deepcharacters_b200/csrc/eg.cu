@@ -450,13 +450,17 @@ extern "C" hc_status hc_eg_reserve(hc_eg h, int32_t batch) {
     return h->reserve_packed(h->reserved);
 }
 
+// the vertex pass over B frames, at most 65535 (the grid's limit) at a time
 template <int MODE>
 static hc_status launch_vertices(hc_eg h, cudaStream_t s, int B, const float* disp, const float* gv, float* out) {
-    HC_REQUIRE(B <= 65535, "too many frames in one call (%d)", B);
-    k_eg_vertices<MODE><<<dim3(div_up(h->N, kEgBlock), B), kEgBlock, 0, s>>>(
-        h->N, h->M, h->base4.as<float4>(), h->v2n_poff.as<int>(), h->v2n_pidx.as<int>(), h->v2n_pw.as<float>(),
-        h->tab.as<NodeRT>(), disp, gv, out, h->packed.as<float4>());
-    HC_CHECK_LAUNCH();
+    for (int b = 0; b < B; b += 65535) {
+        const size_t at = 3 * (size_t)b * h->N;
+        k_eg_vertices<MODE><<<dim3(div_up(h->N, kEgBlock), std::min(B - b, 65535)), kEgBlock, 0, s>>>(
+            h->N, h->M, h->base4.as<float4>(), h->v2n_poff.as<int>(), h->v2n_pidx.as<int>(), h->v2n_pw.as<float>(),
+            h->tab.as<NodeRT>() + (size_t)b * h->M, disp ? disp + at : nullptr, gv ? gv + at : nullptr, out + at,
+            h->packed.as<float4>() + at);
+        HC_CHECK_LAUNCH();
+    }
     return HC_OK;
 }
 
@@ -481,6 +485,7 @@ extern "C" hc_status hc_eg_forward(hc_eg h, void* stream, int32_t batch, const f
                                                nodes_skinned_translation, nodes_skinned_rotation, tab, deformed_graph,
                                                d_delta_rotation, d_skinned_rotation);
     HC_CHECK_LAUNCH();
+    HC_REQUIRE(batch <= 65535, "too many frames in one call (%d)", batch);
     HC_TRY(launch_vertices<kEgForward>(h, s, batch, vertex_displacements, nullptr, deformed_vertices));
     if (deformed_normals) {
         k_eg_normals<<<div_up(BN, 128), 128, 0, s>>>(batch, h->N, h->fan.as<int2>(), h->vf_id.as<int2>(),
@@ -524,6 +529,7 @@ extern "C" hc_status hc_eg_backward(hc_eg h, void* stream, int32_t batch, const 
                                                nullptr, nullptr);
     HC_CHECK_LAUNCH();
     if (full) {
+        HC_REQUIRE(batch <= 65535, "too many frames in one call (%d)", batch);
         HC_TRY(h->reserve_packed(batch));
         HC_TRY(launch_vertices<kEgAdjointFull>(h, s, batch, vertex_displacements, deformed_vertices_grad,
                                                vertex_displacements_grad));
