@@ -645,9 +645,10 @@ __global__ void __launch_bounds__(256) k_skin_grad(Skel sk, int B, const float* 
 // joint
 __global__ void k_dof_grad(Skel sk, int B, const float* __restrict__ mom, const float* __restrict__ gpos,
                            const float* __restrict__ gaxis, float* __restrict__ gdof) {
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (i >= B * sk.D) return;  // warp-uniform
-    const int b = i / sk.D, d = i % sk.D;
+    const long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= (long long)B * sk.D) return;  // warp-uniform
+    const int b = (int)(i / sk.D), d = (int)(i % sk.D);
     float acc = 0.f;
     for (int e = sk.dof_off[d]; e < sk.dof_off[d + 1]; ++e) {
         const int j = sk.dof_joint[e];
@@ -863,9 +864,10 @@ __global__ void k_pose2eg_grad_nodes(Skel sk, int M, const int* __restrict__ nod
 __global__ void k_pose2eg_grad_dofs(Skel sk, int B, const float* __restrict__ dq, const float* __restrict__ gdq,
                                     const float* __restrict__ gpos, const float* __restrict__ gaxis,
                                     float* __restrict__ gdof) {
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (i >= B * sk.D) return;  // warp-uniform
-    const int b = i / sk.D, d = i % sk.D;
+    const long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= (long long)B * sk.D) return;  // warp-uniform
+    const int b = (int)(i / sk.D), d = (int)(i % sk.D);
     float acc = 0.f;
     for (int e = sk.dof_off[d]; e < sk.dof_off[d + 1]; ++e) {
         const int j = sk.dof_joint[e];
