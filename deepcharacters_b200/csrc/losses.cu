@@ -280,9 +280,12 @@ struct SmoothTaps {
 template <int S>
 constexpr int smooth_columns() { return S <= 3 ? 4 : S <= 7 ? 2 : 1; }
 
-// CN: channels, or 0 to take them from Cn
+// CN: channels, or 0 to take them from Cn.  The n columns from `in` and `out` on
+// are written; columns lo to hi (exclusive) belong to the image, whose rows have
+// WC.
 template <int S, int CN>
-__global__ void __launch_bounds__(kSmoothBlock) k_smooth(int H, int WC, int Cn, int rows_per_strip, SmoothTaps taps,
+__global__ void __launch_bounds__(kSmoothBlock) k_smooth(int H, long long WC, int lo, int hi, int n, int Cn,
+                                                         int rows_per_strip, SmoothTaps taps,
                                                          const float* __restrict__ in, float* __restrict__ out) {
     constexpr int T = kSmoothBlock, NC = smooth_columns<S>(), K = 2 * S + 1;
     static_assert(2 * kSmoothMax * 4 <= T, "one extra load per thread covers the halo");
@@ -296,11 +299,11 @@ __global__ void __launch_bounds__(kSmoothBlock) k_smooth(int H, int WC, int Cn, 
     auto fetch = [&](int r) {
         const int y = y0 - S + r;
         const bool ok = y >= 0 && y < H;
-        const float* row = I + (long long)y * WC;
+        const float* row = I + y * WC;
 #pragma unroll
         for (int c = 0; c <= NC; ++c) {
             const int x = x0 - halo + t + c * T;
-            next[c] = ok && x >= 0 && x < WC && (c < NC || t < 2 * halo) ? row[x] : 0.f;
+            next[c] = ok && x >= lo && x < hi && (c < NC || t < 2 * halo) ? row[x] : 0.f;
         }
     };
     fetch(0);
@@ -325,13 +328,13 @@ __global__ void __launch_bounds__(kSmoothBlock) k_smooth(int H, int WC, int Cn, 
                     ring[c][u] = acc;
                 }
                 if (r >= 2 * S) {
-                    float* row = O + (long long)(y0 + r - 2 * S) * WC + x0;
+                    float* row = O + (y0 + r - 2 * S) * WC + x0;
 #pragma unroll
                     for (int c = 0; c < NC; ++c) {
                         float acc = 0.f;
 #pragma unroll
                         for (int k = 0; k < K; ++k) acc += taps.w[k] * ring[c][(u + 1 + k) % K];  // oldest row first
-                        if (x0 + t + c * T < WC) row[t + c * T] = acc;
+                        if (x0 + t + c * T < n) row[t + c * T] = acc;
                     }
                 }
             }
@@ -339,16 +342,26 @@ __global__ void __launch_bounds__(kSmoothBlock) k_smooth(int H, int WC, int Cn, 
     }
 }
 
+// Columns of a launch: a row of an image may have more floats than 32 bits count.
+constexpr long long kSmoothColumns = 1ll << 30;
+
 template <int S>
-void launch_smooth(cudaStream_t s, int n, int H, int W, int Cn, const SmoothTaps& taps, const float* in, float* out) {
-    const int WC = W * Cn, gx = div_up(WC, kSmoothBlock * smooth_columns<S>());
-    // 64-row strips; shorter ones while they leave SMs idle (their halos cost less than that)
-    int rows = 64;
-    while (rows > 8 && (long long)gx * div_up(H, rows) * n < 4 * 148) rows /= 2;
-    while (div_up(H, rows) > 65535) rows *= 2;  // grid limit
-    const dim3 grid(gx, div_up(H, rows), n);
-    if (Cn == 3) k_smooth<S, 3><<<grid, kSmoothBlock, 0, s>>>(H, WC, Cn, rows, taps, in, out);
-    else k_smooth<S, 0><<<grid, kSmoothBlock, 0, s>>>(H, WC, Cn, rows, taps, in, out);
+hc_status launch_smooth(cudaStream_t s, int images, int H, int W, int Cn, const SmoothTaps& taps, const float* in,
+                        float* out) {
+    const long long WC = (long long)W * Cn;
+    for (long long x = 0; x < WC; x += kSmoothColumns) {
+        const int n = (int)std::min(kSmoothColumns, WC - x), gx = div_up(n, kSmoothBlock * smooth_columns<S>());
+        const int lo = x > 0 ? -S * Cn : 0, hi = (int)std::min(WC - x, (long long)n + S * Cn);
+        // 64-row strips; shorter ones while they leave SMs idle (their halos cost less than that)
+        int rows = 64;
+        while (rows > 8 && (long long)gx * div_up(H, rows) * images < 4 * 148) rows /= 2;
+        while (div_up(H, rows) > 65535) rows *= 2;  // grid limit
+        const dim3 grid(gx, div_up(H, rows), images);
+        if (Cn == 3) k_smooth<S, 3><<<grid, kSmoothBlock, 0, s>>>(H, WC, lo, hi, n, Cn, rows, taps, in + x, out + x);
+        else k_smooth<S, 0><<<grid, kSmoothBlock, 0, s>>>(H, WC, lo, hi, n, Cn, rows, taps, in + x, out + x);
+        HC_CHECK_LAUNCH();
+    }
+    return HC_OK;
 }
 
 }  // namespace
@@ -380,16 +393,14 @@ extern "C" hc_status hc_gaussian_smooth(void* stream, int32_t n_images, int32_t 
         sum += v[k];
     }
     for (int k = 0; k <= 2 * size; ++k) t.w[k] = (float)(v[k] / sum);
-    HC_REQUIRE((long long)width * channels < (1ll << 31), "image rows too long");
     switch (size) {
 #define HC_SMOOTH_CASE(S) \
-    case S: launch_smooth<S>(s, n_images, height, width, channels, t, image, out); break;
+    case S: return launch_smooth<S>(s, n_images, height, width, channels, t, image, out);
         HC_SMOOTH_CASE(1) HC_SMOOTH_CASE(2) HC_SMOOTH_CASE(3) HC_SMOOTH_CASE(4) HC_SMOOTH_CASE(5)
         HC_SMOOTH_CASE(6) HC_SMOOTH_CASE(7) HC_SMOOTH_CASE(8) HC_SMOOTH_CASE(9) HC_SMOOTH_CASE(10)
         HC_SMOOTH_CASE(11) HC_SMOOTH_CASE(12) HC_SMOOTH_CASE(13) HC_SMOOTH_CASE(14) HC_SMOOTH_CASE(15)
 #undef HC_SMOOTH_CASE
     }
-    HC_CHECK_LAUNCH();
     return HC_OK;
 }
 
