@@ -1022,11 +1022,12 @@ __global__ void __launch_bounds__(kSilBlock) k_sil_pixels(int N, const __grid_co
         if (sumsq1 && lane == 0 && q != 0.f) atomicAdd(sumsq1, (double)q);
         return;
     }
-    const int p0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
-    if (p0 >= P) return;
+    const unsigned p = 4u * (blockIdx.x * blockDim.x + threadIdx.x);  // may pass 2^31
+    if (p >= (unsigned)P) return;
+    const int p0 = (int)p;
     const long long i0 = vi.pix + p0;
     float q = 0.f;
-    for (int k = 0; k < 4 && p0 + k < P; ++k) {
+    for (int k = 0; k < 4 && k < P - p0; ++k) {
         float r0, r1, cl;
         sil_pixel(view, vi, p0 + k, D[p0 + k], N, g, p2d, D, crops, r0, r1, cl);
         residual1[2 * (i0 + k)] = r0;
@@ -1068,14 +1069,14 @@ __global__ void __launch_bounds__(kSilBlock) k_sil_grad_pixels(int N, const __gr
     for (int k = 0; k < 4; ++k) {
         const int p = 4 * ((int)threadIdx.x + k * kSilBlock);
         c[k] = make_float4(-1.f, -1.f, -1.f, -1.f);
-        if (pb + p >= P) continue;
+        if (p >= P - pb) continue;
         if (vec) {
             c[k] = *reinterpret_cast<const float4*>(closest + i0 + p);
         } else {
             c[k].x = closest[i0 + p];
-            if (pb + p + 1 < P) c[k].y = closest[i0 + p + 1];
-            if (pb + p + 2 < P) c[k].z = closest[i0 + p + 2];
-            if (pb + p + 3 < P) c[k].w = closest[i0 + p + 3];
+            if (p + 1 < P - pb) c[k].y = closest[i0 + p + 1];
+            if (p + 2 < P - pb) c[k].z = closest[i0 + p + 2];
+            if (p + 3 < P - pb) c[k].w = closest[i0 + p + 3];
         }
     }
 #pragma unroll
