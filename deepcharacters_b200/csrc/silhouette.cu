@@ -964,7 +964,7 @@ __device__ __forceinline__ void sil_pixel_warp(long long view, const ViewImg& vi
 constexpr int kSilBlock = 256;
 constexpr int kSilPixels = 16 * kSilBlock;  // pixels of a block (vec)
 
-__global__ void __launch_bounds__(kSilBlock) k_sil_pixels(int N, const __grid_constant__ ImgLayout L, SilGrid g,
+__global__ void __launch_bounds__(kSilBlock, 5) k_sil_pixels(int N, const __grid_constant__ ImgLayout L, SilGrid g,
                              const float* __restrict__ p2d, const unsigned char* __restrict__ dt,
                              const float* __restrict__ crops, float* __restrict__ residual1,
                              float* __restrict__ closest, int vec, double* __restrict__ sumsq1) {
@@ -1008,7 +1008,7 @@ __global__ void __launch_bounds__(kSilBlock) k_sil_pixels(int N, const __grid_co
         }
         __syncthreads();
         const int n = s_n, lane = threadIdx.x & 31;
-        float q = 0.f;
+        double q = 0.0;  // hundreds of a block's terms in turn: a tree's accuracy or better
         for (int e = threadIdx.x >> 5; e < n; e += kSilBlock >> 5) {  // warp-uniform
             const int lp = s_list[e];
             float a0, a1, cl;
@@ -1016,10 +1016,10 @@ __global__ void __launch_bounds__(kSilBlock) k_sil_pixels(int N, const __grid_co
             if (lane == 0 && cl >= 0.f) {
                 reinterpret_cast<float2*>(residual1)[i0 + lp] = make_float2(a0, a1);
                 closest[i0 + lp] = cl;
-                q += a0 * a0 + a1 * a1;
+                q += (double)(a0 * a0 + a1 * a1);
             }
         }
-        if (sumsq1 && lane == 0 && q != 0.f) atomicAdd(sumsq1, (double)q);
+        if (sumsq1 && lane == 0 && q != 0.0) atomicAdd(sumsq1, q);
         return;
     }
     const unsigned p = 4u * (blockIdx.x * blockDim.x + threadIdx.x);  // may pass 2^31
