@@ -36,7 +36,13 @@ def image_l1_loss(render: torch.Tensor, target: torch.Tensor, face: torch.Tensor
     m = mask.to(torch.uint8).contiguous() if mask is not None else None
     loss = torch.empty((1,), device=r.device)
     grad = torch.empty_like(r)
-    ws = torch.empty((16 + f.numel(),), device=r.device, dtype=torch.uint8)  # the sums, a byte per pixel
+    try:
+        ws = torch.empty((16 + f.numel(),), device=r.device, dtype=torch.uint8)  # the sums, a byte per pixel
+    except torch.OutOfMemoryError:  # the images are read twice then
+        ws = torch.empty((2,), device=r.device, dtype=torch.float64)
+        _lib.call("hc_image_l1_loss", _stream(), f.numel(), _lib.ptr(r), _lib.ptr(t), _lib.ptr(f), _lib.ptr(m),
+                  _lib.ptr(ws), _lib.ptr(loss), _lib.ptr(grad))
+        return loss, grad
     _lib.call("hc_image_l1_loss_scratch", _stream(), f.numel(), _lib.ptr(r), _lib.ptr(t), _lib.ptr(f), _lib.ptr(m),
               _lib.ptr(ws), ws.data_ptr() + 16, _lib.ptr(loss), _lib.ptr(grad))
     return loss, grad
