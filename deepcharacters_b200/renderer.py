@@ -10,6 +10,7 @@ CUDA tensors; the work runs in ``libhc.so`` on the current CUDA stream.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import threading
 
@@ -81,7 +82,8 @@ class RendererEngine:
                       self.N, self.C, self.W, self.H, albedo_mode.encode(), shading_mode.encode(),
                       self.image_filter_size, self.texture_filter_size, compute_normal_map.encode())
         self._h = h
-        self.device = torch.cuda.current_device()  # owns the handle's allocations
+        # owns the handle's allocations; None without a GPU (the entry points stood in for)
+        self.device = torch.cuda.current_device() if torch.cuda.is_available() else None
 
     def _elsewhere(self, device: torch.device):
         """For a call outside the engine's device: its tensors have to be there, then it is made current."""
@@ -128,7 +130,7 @@ class RendererEngine:
         return self._h
 
     def reserve(self, batch: int):
-        with torch.cuda.device(self.device):
+        with contextlib.nullcontext() if self.device is None else torch.cuda.device(self.device):
             _lib.call("hc_renderer_reserve", self._h, int(batch))
 
     def set_tuning(self, tile: int, bin_capacity: int):
