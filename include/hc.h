@@ -90,7 +90,10 @@ hc_status hc_renderer_create_multires(hc_renderer* out, const int32_t* faces, in
 hc_status hc_renderer_frame_pixels(hc_renderer h, int64_t* pixels);
 hc_status hc_renderer_destroy(hc_renderer h);
 
-/* Pre-size the workspace for up to `batch` frames (no allocation afterwards). */
+/* Pre-size the workspace for up to `batch` frames.  What is still allocated
+ * afterwards: scratch that a call can do without (the textured adjoint's padded
+ * texels, never under capture), and the texel table of a UV map size that the
+ * handle meets for the first time. */
 hc_status hc_renderer_reserve(hc_renderer h, int32_t batch);
 
 /* Raster tuning: screen tile edge in pixels (8, 16 or 32) and per-tile bin
@@ -246,7 +249,8 @@ hc_status hc_eg_create(hc_eg* out, int32_t n_vertices, const float* base_vertice
 hc_status hc_eg_destroy(hc_eg h);
 hc_status hc_eg_reserve(hc_eg h, int32_t batch);
 /* 0 (default): skinned-rotation/translation gradients are zero, as in the
- * reference (EmbeddedGraphGPUOpGrad.cu:136-142); 1: return them. */
+ * reference (EmbeddedGraphGPUOpGrad.cu:136-142); 1: return them.  After
+ * hc_eg_reserve the workspace that they need is taken here. */
 hc_status hc_eg_set_full_skinned_gradient(hc_eg h, int32_t enable);
 
 /*
