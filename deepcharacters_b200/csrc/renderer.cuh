@@ -575,7 +575,7 @@ __device__ __forceinline__ float3 sh_illum(const float* sh, float3 n) {
 
 struct Topology {
     int N = 0, F = 0;
-    DevBuf mem;          // the arrays below, in one allocation
+    DevBuf mem[5];       // the arrays below, all in the first or each in its own
     DevPart faces;       // int3[F]
     DevPart fan;         // int2[3F]  vertex -> incident faces, increasing face id (FanFace)
     DevPart vf_id;       // int2[N]  (start, count)
