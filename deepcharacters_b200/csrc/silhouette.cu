@@ -112,6 +112,13 @@ __global__ void k_project_grad(int B, int C, int N, const float* __restrict__ gi
     st3(out + i * 3, g);
 }
 
+// The 3x3 window around pixel (u, v) lies in the image.  u and v may be any: the
+// projection of a vertex behind the camera is converted to the largest int, to which
+// nothing may be added.
+__device__ __forceinline__ bool window_inside(int u, int v, int W, int H) {
+    return u >= 1 && u < W - 1 && v >= 1 && v < H - 1;
+}
+
 // Boundary vertices of the projected mesh: a vertex is on the boundary of a
 // view if a pixel of the 3x3 window around its (truncated) projection is not
 // covered (Skeletool/Mesh/CUDABasedRasterization.cu:168-200).  Coverage is the
@@ -123,7 +130,7 @@ __global__ void k_boundary(int B, int C, int N, int W, int H, const float* __res
     const long long view = i / N;
     const int u = (int)p2d[2 * i], v = (int)p2d[2 * i + 1];
     unsigned char r = 0;
-    if (u - 1 >= 0 && u + 1 < W && v - 1 >= 0 && v + 1 < H) {
+    if (window_inside(u, v, W, H)) {
         const int* F = face + view * H * W;
         for (int c = u - 1; c <= u + 1; ++c)
             for (int rr = v - 1; rr <= v + 1; ++rr)
@@ -401,7 +408,7 @@ __global__ void __launch_bounds__(256, 6) k_bnd_hint(long long n, int N, int F, 
     const float2 q = p2d[i];
     const int u = (int)q.x, v = (int)q.y;
     unsigned char r = 0;
-    if (u - 1 >= 0 && u + 1 < W && v - 1 >= 0 && v + 1 < H) {
+    if (window_inside(u, v, W, H)) {
         int last = -1;
         CoverTri t;
         unsigned open = 0;  // bit 3 j + k: window pixel (row j, column k) is open
@@ -677,7 +684,7 @@ __global__ void k_boundary_cover(int B, int C, int N, const __grid_constant__ Im
     const int W = vi.W, H = vi.H;
     const int u = (int)p2d[2 * i], v = (int)p2d[2 * i + 1];
     unsigned char r = 0;
-    if (u - 1 >= 0 && u + 1 < W && v - 1 >= 0 && v + 1 < H) {
+    if (window_inside(u, v, W, H)) {
         const unsigned char* img = cover + vi.pix;
         for (int c = u - 1; c <= u + 1; ++c)
             for (int rr = v - 1; rr <= v + 1; ++rr)
