@@ -164,6 +164,21 @@ __device__ __forceinline__ bool cover_test(const CoverTri& t, float pu, float pv
     return e0 >= -0.001f && e1 >= -0.001f && e2 >= -0.001f && e0 <= 1.001f && e1 <= 1.001f && e2 <= 1.001f;
 }
 
+// The same for a record, its contraction written out so that every kernel decides
+// alike the pixels whose barycentric is the tolerance to the last bits.  apart: the
+// triangle's own products rounded by themselves, as they have always been where a
+// large box is swept.
+__device__ __forceinline__ bool cover_test_record(float2 a, float2 b, float2 c, float d1, float d2, float pu, float pv,
+                                                  bool apart) {
+    auto numerator = [&](float2 q) {  // of the edge a -> q
+        const float s = __fmaf_rn(q.x - a.x, pv, __fmul_rn(a.y - q.y, pu));
+        return apart ? __fsub_rn(__fadd_rn(s, __fmul_rn(a.x, q.y)), __fmul_rn(q.x, a.y))
+                     : __fmaf_rn(-q.x, a.y, __fmaf_rn(a.x, q.y, s));
+    };
+    const float e2 = numerator(b) / d2, e1 = numerator(c) / d1, e0 = 1.f - e2 - e1;
+    return e0 >= -0.001f && e1 >= -0.001f && e2 >= -0.001f && e0 <= 1.001f && e1 <= 1.001f && e2 <= 1.001f;
+}
+
 __device__ __forceinline__ Footprint cover_footprint(const CoverTri& t, int W, int H) {
     const float M = fmaxf(fmaxf(fmaxf(fabsf(t.a.x), fabsf(t.a.y)), fmaxf(fabsf(t.b.x), fabsf(t.b.y))),
                           fmaxf(fmaxf(fabsf(t.c.x), fabsf(t.c.y)), (float)max(W, H)));
@@ -285,20 +300,14 @@ __device__ __forceinline__ CovTileTri cover_record(const CoverTri& t, const Foot
 // the reference's test of one pixel centre (only pixels of the triangle's
 // clamped box are tested: a centre just outside the box can pass the widened
 // barycentric test), with the footprint cull and the interior shortcut first
-__device__ __forceinline__ bool cover_record_test(const CovTileTri& e, int px, int py) {
+__device__ __forceinline__ bool cover_record_test(const CovTileTri& e, int px, int py, bool apart) {
     if (px < (e.bb.x & 0xffff) || px > (e.bb.x >> 16) || py < (e.bb.y & 0xffff) || py > (e.bb.y >> 16)) return false;
     const float pu = px + 0.5f, pv = py + 0.5f;
     const float f0 = e.e0.x * pu + e.e0.y * pv + e.e0.z, f1 = e.e0.w * pu + e.e1.x * pv + e.e1.y,
                 f2 = e.e1.z * pu + e.e1.w * pv + e.e2.x;
     if (f0 < 0.f || f1 < 0.f || f2 < 0.f) return false;
     if (f0 >= e.e2.w && f1 >= e.e2.w && f2 >= e.e2.w) return true;  // clearly inside
-    CoverTri t;
-    t.a = make_float2(e.ab.x, e.ab.y);
-    t.b = make_float2(e.ab.z, e.ab.w);
-    t.c = e.c;
-    t.d1 = e.e2.y;
-    t.d2 = e.e2.z;
-    return cover_test(t, pu, pv);
+    return cover_test_record(make_float2(e.ab.x, e.ab.y), make_float2(e.ab.z, e.ab.w), e.c, e.e2.y, e.e2.z, pu, pv, apart);
 }
 
 struct CovBins {
@@ -339,14 +348,15 @@ __device__ __forceinline__ bool need_in_box(const unsigned long long* need, cons
     return false;
 }
 
-// the pixels of one tile that a triangle covers, written at once (a pair
+// the pixels of tile (tx, ty) that a triangle covers, written at once (a pair
 // beyond the tile's bin capacity)
-__device__ void cov_sweep(const CovBins& cb, const ViewImg& vi, int tile, const CovTileTri& e) {
-    const int ty = tile / vi.tiles_x, tx = tile - ty * vi.tiles_x;
-    unsigned char* img = cb.cover + vi.pix;
-    for (int v = ty * kCovTile; v < min(ty * kCovTile + kCovTile, vi.H); ++v)
-        for (int u = tx * kCovTile; u < min(tx * kCovTile + kCovTile, vi.W); ++u)
-            if (cover_record_test(e, u, v)) img[(long long)v * vi.W + u] = 1;
+__device__ __forceinline__ void cov_sweep(unsigned char* img, int W, int H, int tx, int ty, const CovTileTri& e) {
+    const int nx = ((e.bb.x >> 16) >> kCovShift) - ((e.bb.x & 0xffff) >> kCovShift) + 1,
+              ny = ((e.bb.y >> 16) >> kCovShift) - ((e.bb.y & 0xffff) >> kCovShift) + 1;
+    const bool large = nx * ny > 9;
+    for (int v = ty * kCovTile; v < min(ty * kCovTile + kCovTile, H); ++v)
+        for (int u = tx * kCovTile; u < min(tx * kCovTile + kCovTile, W); ++u)
+            if (cover_record_test(e, u, v, large)) img[(long long)v * W + u] = 1;
 }
 
 // Boundary flags from a per-pixel face hint (a renderer face buffer of the
@@ -434,11 +444,11 @@ __global__ void __launch_bounds__(256, 6) k_bnd_hint(long long n, int N, int F, 
 }
 
 // a (tile, triangle) pair into the tile's bin, or swept at once beyond its capacity
-__device__ __forceinline__ void cov_place(const CovBins& cb, const ViewImg& vi, int tile, int f, long long rec) {
-    const long long key = vi.tile + tile;
+__device__ __forceinline__ void cov_place(const CovBins& cb, const ViewImg& vi, int tx, int ty, int f, long long rec) {
+    const long long key = vi.tile + ty * vi.tiles_x + tx;
     const int slot = cov_claim(cb, key);
     if (slot < kCovCap) cb.bins[key * kCovCap + slot] = f;
-    else cov_sweep(cb, vi, tile, cb.rec[rec]);
+    else cov_sweep(cb.cover + vi.pix, vi.W, vi.H, tx, ty, cb.rec[rec]);
 }
 
 // The full binning, grid (triangle blocks, views), one thread per (view,
@@ -476,7 +486,7 @@ __global__ void __launch_bounds__(256, 4) k_cov_bin(int N, int F, const int3* __
     const float rn = __fdividef(1.f, (float)ntx);
     for (; reached; reached &= reached - 1u) {
         const int k = __ffs(reached) - 1, r = (int)((k + 0.5f) * rn);
-        cov_place(cb, vi, (ty0 + r) * vi.tiles_x + tx0 + (k - r * ntx), fi, i);
+        cov_place(cb, vi, tx0 + (k - r * ntx), ty0 + r, fi, i);
     }
     __syncwarp();  // the records of big triangles are read by the other lanes where a bin overflows
     unsigned pending = __ballot_sync(0xffffffffu, big);
@@ -487,7 +497,7 @@ __global__ void __launch_bounds__(256, 4) k_cov_bin(int N, int F, const int3* __
         const int qx0 = __shfl_sync(0xffffffffu, t.x0, src), qx1 = __shfl_sync(0xffffffffu, t.x1, src);
         const int qy0 = __shfl_sync(0xffffffffu, t.y0, src), qy1 = __shfl_sync(0xffffffffu, t.y1, src);
         warp_tiles(rows.from_lane(src), kCovShift, qx0, qx1, qy0, qy1, (int)lane, [&](int tx, int ty) {
-            cov_place(cb, vi, ty * vi.tiles_x + tx, qf, (long long)view * F + qf);
+            cov_place(cb, vi, tx, ty, qf, (long long)view * F + qf);
         });
     }
 }
@@ -561,7 +571,7 @@ __global__ void __launch_bounds__(256, 4) k_cov_bin_list(int N, int F, int V, co
                     if (!footprint_overlaps(fp, max(tx * kCovTile, t.x0), min(tx * kCovTile + kCovTile - 1, t.x1),
                                             max(ty * kCovTile, t.y0), min(ty * kCovTile + kCovTile - 1, t.y1)))
                         continue;
-                    cov_place(cb, vi, ty * vi.tiles_x + tx, f, item);
+                    cov_place(cb, vi, tx, ty, f, item);
                 }
             }
     }
@@ -584,7 +594,7 @@ __global__ void __launch_bounds__(256, 4) k_cov_bin_list(int N, int F, int V, co
         if (__reduce_add_sync(0xffffffffu, count) > kCovNeeded) {
             warp_tiles(TileRows(fp), kCovShift, t.x0, t.x1, t.y0, t.y1, lane, [&](int tx, int ty) {
                 if (needed(tx >> 3, ty >> 3) >> (8 * (ty & 7) + (tx & 7)) & 1ull)
-                    cov_place(cb, vi, ty * vi.tiles_x + tx, f, item);
+                    cov_place(cb, vi, tx, ty, f, item);
             });
         } else {
             for (int q = lane; q < words; q += 32) {
@@ -593,7 +603,7 @@ __global__ void __launch_bounds__(256, 4) k_cov_bin_list(int N, int F, int V, co
                     const int b = __ffsll((long long)bits) - 1, tx = 8 * wx + (b & 7), ty = 8 * wy + (b >> 3);
                     if (footprint_overlaps(fp, max(tx * kCovTile, t.x0), min(tx * kCovTile + kCovTile - 1, t.x1),
                                            max(ty * kCovTile, t.y0), min(ty * kCovTile + kCovTile - 1, t.y1)))
-                        cov_place(cb, vi, ty * vi.tiles_x + tx, f, item);
+                        cov_place(cb, vi, tx, ty, f, item);
                 }
             }
         }
@@ -663,7 +673,7 @@ __global__ void __launch_bounds__(kCovTile* kCovTile) k_cov_tile(int F, CovBins 
                 }
                 w = transpose_bits(w, lane);
                 while (w && !covered) {
-                    covered = cover_record_test(s_t[s0 + __ffs(w) - 1], px, py);
+                    covered = cover_record_test(s_t[s0 + __ffs(w) - 1], px, py, false);
                     w &= w - 1u;
                 }
             }
