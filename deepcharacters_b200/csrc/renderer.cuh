@@ -89,16 +89,24 @@ struct RasterStats {
 // Pixel-centre camera ray (reference getRayCuda2 / backprojectPixelCuda,
 // CudaRenderer/cpp/src/Utils/CameraUtil.h:223-258): the pixel centre is lifted
 // to depth 1000 through inv(K*E) and the direction from the camera centre is
-// normalised with rsqrtf.
+// normalised with rsqrtf.  The roundings are written out: left to the compiler,
+// the order in which it contracts a row's products changes with the code
+// around it, and with it the last bits of a ray and the side of an edge that it
+// falls on.  In the tile resolve (RESOLVE) the x row rounds its first product
+// before the second is added, elsewhere its second, as the other rows do.
+template <bool FIRST>
+__device__ __forceinline__ float lifted(const float* m, float u, float v) {
+    const float s = FIRST ? __fmaf_rn(m[1], v, __fmul_rn(m[0], u)) : __fmaf_rn(m[0], u, __fmul_rn(m[1], v));
+    return __fadd_rn(__fmaf_rn(m[2], 1000.f, s), m[3]);
+}
+
+template <bool RESOLVE>
 __device__ __forceinline__ float3 pixel_ray(const ViewCam& c, int px, int py) {
-    const float u = px + 0.5f;
-    const float v = py + 0.5f;
-    const float4 tp = make_float4(u * 1000.f, v * 1000.f, 1000.f, 1.f);
-    const float4 r0 = make_float4(c.invP[0], c.invP[1], c.invP[2], c.invP[3]);
-    const float4 r1 = make_float4(c.invP[4], c.invP[5], c.invP[6], c.invP[7]);
-    const float4 r2 = make_float4(c.invP[8], c.invP[9], c.invP[10], c.invP[11]);
-    const float3 q = make_float3(dot(r0, tp), dot(r1, tp), dot(r2, tp));
-    return normalize3(q - make_float3(c.ro[0], c.ro[1], c.ro[2]));
+    const float u = __fmul_rn(px + 0.5f, 1000.f), v = __fmul_rn(py + 0.5f, 1000.f);
+    const float3 q = make_float3(lifted<RESOLVE>(c.invP, u, v), lifted<false>(c.invP + 4, u, v),
+                                 lifted<false>(c.invP + 8, u, v));
+    const float3 d = q - make_float3(c.ro[0], c.ro[1], c.ro[2]);
+    return d * rsqrtf(__fmaf_rn(d.z, d.z, __fmaf_rn(d.x, d.x, __fmul_rn(d.y, d.y))));
 }
 
 struct TriS {

@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(BNT, adjoint_ctas(SHADED, PARITY)) k_render_gr
     float3 d = make_float3(0.f, 0.f, 1.f), v0 = d, v1 = d, v2 = d, G = d, frag = d;
     float3 gbc = make_float3(0.f, 0.f, 0.f);  // d loss / d (a, b, c)
     if (f >= 0) {
-        d = pixel_ray(cam, px, py);
+        d = pixel_ray<false>(cam, px, py);
         const float ba = A.bary[2 * pix], bb = A.bary[2 * pix + 1];
         const float bc = 1.f - ba - bb;
         const int3 id = A.faces[f];

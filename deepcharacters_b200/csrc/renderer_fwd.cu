@@ -368,7 +368,7 @@ __global__ void k_spill(int C, int F, int TS, long long T_frame, const int* __re
         for (int q = lane; q < bw * bh; q += 32) {
             {
                 const int px = px0 + q % bw, py = py0 + q / bw;
-                const float3 dir = pixel_ray(cam, px, py);
+                const float3 dir = pixel_ray<false>(cam, px, py);
                 int dq;
                 float a, b;
                 if (!raster_hit(ro_s, dir, Tr, tv.num, dq, a, b)) continue;
@@ -680,7 +680,7 @@ __global__ void __launch_bounds__(TS* TS, TS == 8 ? 20 : (TS == 16 ? 5 : 1)) k_r
         continue;
     }
     const float3 ro_s = make_float3(cam.ro_s[0], cam.ro_s[1], cam.ro_s[2]);
-    const float3 dir = pixel_ray(cam, px, py);
+    const float3 dir = pixel_ray<true>(cam, px, py);
     const int* tb = bins + g * cap;
     unsigned best_d = 0xffffffffu;
     int best_f = 0x7fffffff;
