@@ -125,8 +125,11 @@ __device__ __forceinline__ void bary_jacobian_apply(float3 o, float3 d, float3 v
 // zero near the border.  `x`, `y` are the (possibly fractional) sample position.
 // FS: a filter size known at compile time, whose weights and normaliser fold
 // to constants (the run-time form divides twice per tap), or 0 for `size`;
-// the terms, their order and rounding are the same.
-template <int FS, class Tap>
+// the terms, their order and rounding are the same.  A tap's texel is the whole
+// part of (y + j) w + (x + i), which near a whole number depends on the rounding:
+// written out, since the compiler's choice follows the loop's form.  APART (with
+// shading): the product is rounded before the sum; otherwise the sum alone is.
+template <int FS, bool APART, class Tap>
 __device__ __forceinline__ void image_gradient_fs(Tap tap, float x, float y, int w, int size, float3& du, float3& dv) {
     const int fs = FS ? FS : size;
     float norm = 0.f;
@@ -134,7 +137,8 @@ __device__ __forceinline__ void image_gradient_fs(Tap tap, float x, float y, int
     for (int j = -fs; j <= fs; ++j)
 #pragma unroll(FS ? 2 * FS + 1 : 1)
         for (int i = -fs; i <= fs; ++i) {
-            const float3 I = tap((int)((y + j) * w + (x + i)));
+            const float3 I = tap((int)(APART ? __fadd_rn(__fmul_rn(y + j, (float)w), x + i)
+                                             : __fmaf_rn(y + j, (float)w, x + i)));
             const float den = (float)(i * i + j * j);
             float gu = 0.f, gv = 0.f;
             if (den != 0.f) {
@@ -149,15 +153,15 @@ __device__ __forceinline__ void image_gradient_fs(Tap tap, float x, float y, int
     dv = dv / norm;
 }
 
-template <class Tap>
+template <bool APART, class Tap>
 __device__ __forceinline__ void image_gradient(Tap tap, float x, float y, int w, int h, int fs, float3& du, float3& dv) {
     du = dv = make_float3(0.f, 0.f, 0.f);
     if (!(x >= (float)(fs + 1) && y >= (float)(fs + 1) && x < (float)(w - (fs + 1)) && y < (float)(h - (fs + 1))))
         return;
     switch (fs) {
-        case 1: image_gradient_fs<1>(tap, x, y, w, fs, du, dv); break;
-        case 2: image_gradient_fs<2>(tap, x, y, w, fs, du, dv); break;
-        default: image_gradient_fs<0>(tap, x, y, w, fs, du, dv);
+        case 1: image_gradient_fs<1, APART>(tap, x, y, w, fs, du, dv); break;
+        case 2: image_gradient_fs<2, APART>(tap, x, y, w, fs, du, dv); break;
+        default: image_gradient_fs<0, APART>(tap, x, y, w, fs, du, dv);
     }
 }
 
@@ -597,14 +601,14 @@ __global__ void __launch_bounds__(BNT, adjoint_ctas(SHADED, PARITY)) k_render_gr
             float3 du, dv;
             if (A.tex_pad) {  // launch-uniform
                 const float4* T4 = A.tex_pad + (long long)b * A.tex_h * A.tex_w;
-                image_gradient(
+                image_gradient<SHADED>(
                     [&](int i) {
                         const float4 q = T4[i];
                         return make_float3(q.x, q.y, q.z);
                     },
                     uv.x, uv.y, A.tex_w, A.tex_h, A.tfs, du, dv);
             } else {
-                image_gradient([&](int i) { return ld3(T + 3LL * i); }, uv.x, uv.y, A.tex_w, A.tex_h, A.tfs, du, dv);
+                image_gradient<SHADED>([&](int i) { return ld3(T + 3LL * i); }, uv.x, uv.y, A.tex_w, A.tex_h, A.tfs, du, dv);
             }
             const float gu = dot(gA, du), gv = dot(gA, dv);
             gbc = make_float3(gu * (t0.x * A.tex_w) + gv * (t0.y * A.tex_h), gu * (t1.x * A.tex_w) + gv * (t1.y * A.tex_h),
